@@ -133,6 +133,23 @@ def test_gemm_f32_is_true_fp32_and_cut_invariant(M, N, K):
     assert np.array_equal(one[0], c[M - 1])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 4), (1, 1024, 3072), (2, 4096, 1024), (3, 33, 132), (4, 4735, 128), (5, 4736, 260), (13, 18943, 124),
+                                   (16, 18944, 512), (17, 31, 36), (32, 33, 68), (33, 1000, 1024), (65, 4100, 96), (129, 129, 32), (300, 3000, 640)])
+def test_gemm_f32_kernels_walk_the_same_chain(M, N, K):
+    """Aligned rows take the tiled and the few-rows kernel, rows at an odd pitch the general one: the same bits."""
+    k = _k()
+    g = torch.Generator().manual_seed(M + N + K)
+    wide = torch.randn((M, K + 1), generator=g).to(DEV)
+    w = torch.randn((N, K), generator=g).to(DEV)
+    if M > 1:
+        general = k.linear(wide[:, :K], w)                                           # a row pitch of K + 1 elements
+    else:
+        padded = torch.empty((K + 1,), device=DEV)[1:]                               # one row, four bytes off alignment
+        padded.copy_(wide[0, :K])
+        general = k.linear(padded[None, :], w)
+    assert torch.equal(k.linear(wide[:, :K].contiguous(), w), general)
+
+
 def _paged(kv: np.ndarray, page_ids, n_pages, dt, poison=None):
     """Scatter [T, KV, HD] into pages [n_pages, KV, 64, HD]."""
     T, KV, HD = kv.shape
