@@ -29,6 +29,7 @@ from ..cache.pages import PAGE_TOKENS, CacheError
 from ..cache.storage import Cache
 from ..config.spec import ModelSpec
 from ..ops import kernels
+from ..ops.decode_layers import DecodeLayers
 from ..ops.lib import KernelError
 from ..parts.base import Residual
 from ..registry import read_config_folder
@@ -252,6 +253,8 @@ class Engine:
         self._layer_weights = [[t for p in self.model.layers[e.layer].parts() for t in p.streamed_tensors()]
                                for e in self.model.schedule]
         self._feeds_embedding = any(e.add_embedding for e in self.model.schedule)
+        # decode steps of a few rows run all layers in one launch, where the model's layers are of the kind it takes
+        self.decode_layers = DecodeLayers.plan(self.model, self.cache, self.runtime)
         self.launches = 0                          # kernels of this package launched (see count_launches)
         self.vocab_size = spec.vocab_size
 
@@ -348,6 +351,9 @@ class Engine:
         receives copies of the residual stream on the way (see `step`)."""
         x = self._embed(ctx)
         stream = Residual(x)
+        if taps is None and self.decode_layers is not None and self.decode_layers.takes(ctx):
+            self.decode_layers.forward(x, ctx, self.runtime)
+            return self.model.head.forward(self.model.final_norm.apply(stream, rows=want_rows, lazy=want_rows is None))
         if taps is not None:
             taps["embed"] = x.clone()
         x0 = x.clone() if self._feeds_embedding else None      # the stream itself is added to in place
@@ -709,6 +715,8 @@ class Engine:
             word.zero_()
             if st & 16:
                 from ..ops.lib import call, stream_ptr
+                if self.decode_layers is not None:
+                    self.decode_layers.sync[1].zero_()               # a count that a step which gave up may have left
                 call("mynah_gemm_tcgen05_reset", stream_ptr())       # flags that a product which gave up may have left raised
             what = [name for bit, name in ((kernels.ST_PAGE_RANGE, "a position without a page"),
                                            (kernels.ST_POS_RANGE, "a position outside the rotation table"),

@@ -1,0 +1,126 @@
+"""All layers of a decode step of a few rows in one launch (csrc/decode_layers.cu).
+
+`DecodeLayers.plan(...)` looks a model over: it is taken when every run of the schedule is the dense design's layer (RMSNorm,
+grouped-query attention with a rotation of whole heads or none, RMSNorm, SwiGLU) of one set of sizes, in bfloat16, each
+with a cache of its own. Any other model has no plan, and its layers run one by one. The plan holds the layers' descriptors
+(addresses of weights, gains and caches, which live as long as the engine) on the device, and the words that the launch's
+CTAs exchange, kept with their tags from step to step: a plan's steps follow one another on one stream, as an engine's do.
+"""
+from __future__ import annotations
+
+import ctypes
+from typing import Optional
+
+import torch
+
+from ..cache.pages import PAGE_TOKENS
+from . import lib
+from .lib import KernelError, call, code, ptr, stream_ptr
+
+KERNEL_ROWS = 8         # rows that the kernel takes at most
+# Rows up to which a step takes the one launch. 0: never.
+MAX_ROWS = 8
+# And rows times the widest product's columns: every CTA reads all of a product's rows, twice their size with the tags. One launch
+# against the layers one by one, ms a step: 0.6B shape (3,072 columns) 1 row 0.59 / 0.87, 3 rows 0.80 / 1.01, 8 rows 0.89 / 1.01;
+# 4B shape's first 8 layers (9,728 columns) 1 row 0.60 / 0.80, 4 rows 0.68 / 0.69, 8 rows 0.83 / 0.75.
+MAX_ROW_COLUMNS = 40000
+
+
+class DecodeLayers:
+    def __init__(self, rows, sizes: dict, groups: list, device):
+        self.host_table = torch.tensor(rows, dtype=torch.int64)                 # [layers, 12]
+        self.table = self.host_table.to(device)
+        self.sizes = sizes
+        self.groups = groups                       # (K cache, V cache, window) of every storage group
+        z = sizes
+        self.words = torch.zeros((KERNEL_ROWS * (z["D"] // 2 + z["D"] // 8 + ((z["H"] + z["KV"]) * z["HD"] * 2 + z["F"]) // 2),),
+                                 dtype=torch.int64, device=device)
+        self.sync = torch.zeros((2,), dtype=torch.int32, device=device)
+        self.part: Optional[torch.Tensor] = None
+        self._retired: list[torch.Tensor] = []     # outgrown buffers stay alive: a captured graph may still hold their address
+
+    @classmethod
+    def plan(cls, model, cache, runtime) -> Optional["DecodeLayers"]:
+        from ..parts.attention import GQAttention
+        from ..parts.block import PreNormResidual
+        from ..parts.feedforward import SwiGLUDense
+        from ..parts.norms import OffsetRMSNorm, RMSNorm
+        from ..parts.position import NoPosition, RopeNeox
+        if runtime.act_dtype != torch.bfloat16 or not model.schedule:
+            return None
+        rows, sizes, windows = [], None, {}
+        for i, e in enumerate(model.schedule):
+            block, view = model.layers[e.layer], cache.views[i]
+            if type(block) is not PreNormResidual or block.mult != 1.0 or e.add_embedding or e.add_vector is not None or not view.writes:
+                return None
+            mix, ffn = block.mixer, block.ffn
+            n1, n2 = block.norms.get("mixer"), block.norms.get("ffn")
+            if type(mix) is not GQAttention or type(ffn) is not SwiGLUDense or ffn.out_dtype is not None:
+                return None
+            if type(n1) not in (RMSNorm, OffsetRMSNorm) or type(n2) not in (RMSNorm, OffsetRMSNorm) or n1.eps != n2.eps:
+                return None
+            if type(mix.position) not in (RopeNeox, NoPosition):
+                return None
+            cos, sin, rot = mix.position.fused_tables()
+            if cos is not None and rot != mix.HD:
+                return None
+            qg, kg = mix.q_gain, mix.k_gain
+            if (qg is None) != (kg is None) or (qg is not None and (qg.dtype != kg.dtype or qg.numel() != mix.HD or kg.numel() != mix.HD)):
+                return None
+            if n1.gain.dtype != n2.gain.dtype or n1.gain.numel() != mix.D or n2.gain.numel() != mix.D or ffn.D != mix.D:
+                return None
+            own = dict(D=mix.D, H=mix.H, KV=mix.KV, HD=mix.HD, F=ffn.F, eps=n1.eps, qk_eps=mix.qk_eps, gain_dtype=code(n1.gain.dtype),
+                       qk_dtype=code(qg.dtype) if qg is not None else 0, cos=cos, sin=sin)
+            if sizes is None:
+                sizes = own
+            elif any(own[k] is not sizes[k] if k in ("cos", "sin") else own[k] != sizes[k] for k in own):
+                return None
+            weights = [mix.w_qkv, mix.w_o, ffn.w_gate_up, ffn.w_down]
+            shapes = [((mix.H + 2 * mix.KV) * mix.HD, mix.D), (mix.D, mix.H * mix.HD), (2 * ffn.F, mix.D), (mix.D, ffn.F)]
+            if any(w.dtype != torch.bfloat16 or not w.is_contiguous() or tuple(w.shape) != s for w, s in zip(weights, shapes)):
+                return None
+            if windows.setdefault(view.group, mix.window or 0) != (mix.window or 0):
+                return None
+            k, v = view.k, view.v
+            if v is None or k.dtype != torch.bfloat16 or v.dtype != k.dtype or k.shape != v.shape or tuple(k.shape[1:]) != (mix.KV, PAGE_TOKENS, mix.HD):
+                return None
+            row0, rest = divmod(k.data_ptr() - cache.keys[view.group].data_ptr(), mix.HD * 2)
+            if rest or v.data_ptr() - cache.values[view.group].data_ptr() != row0 * mix.HD * 2:
+                return None
+            words = [t.data_ptr() if t is not None else 0 for t in [*weights, n1.gain, n2.gain, qg, kg, k, v]]
+            if any(w % 16 for w in words):
+                return None                        # (the copies and vector loads want 16-byte boundaries)
+            rows.append(words + [row0, view.group])
+        groups = [(cache.keys[g], cache.values[g], windows.get(g, 0)) for g in range(len(cache.keys))]
+        if any(v is None or k.numel() // sizes["HD"] > 0x7fffffff for k, v, _ in groups):
+            return None
+        if not lib.load().mynah_decode_layers_supported(1, sizes["D"], sizes["H"], sizes["KV"], sizes["HD"], sizes["F"], len(rows), len(groups)):
+            return None
+        return cls(rows, sizes, groups, runtime.device)
+
+    def takes(self, ctx) -> bool:
+        z = self.sizes
+        return ctx.is_decode and ctx.T <= min(MAX_ROWS, KERNEL_ROWS) and ctx.T * max(z["D"], z["H"] * z["HD"], z["F"]) <= MAX_ROW_COLUMNS
+
+    def _partials(self, splits: int) -> torch.Tensor:
+        need = KERNEL_ROWS * self.sizes["H"] * splits * (self.sizes["HD"] + 2)
+        if self.part is None or self.part.numel() < need:
+            if torch.cuda.is_current_stream_capturing():
+                raise KernelError("decode_layers: the pages' partial results would have to grow during graph capture")
+            if self.part is not None:
+                self._retired.append(self.part)
+            self.part = torch.zeros((need,), dtype=torch.int64, device=self.words.device)
+        return self.part
+
+    def forward(self, x: torch.Tensor, ctx, runtime) -> torch.Tensor:
+        """The residual stream x [T, D] (fp32, updated in place) behind all layers."""
+        z, M, S = self.sizes, ctx.T, ctx.decode_splits
+        words = []
+        for (k, v, window), p in zip(self.groups, ctx.pages):
+            words += [k.data_ptr(), v.data_ptr(), k.numel() // z["HD"], window, p.indptr.data_ptr(), p.ids.data_ptr(), p.base.data_ptr(), p.n_pages]
+        cos, sin = z["cos"], z["sin"]
+        call("mynah_decode_layers", ptr(self.table), ptr(self.host_table), self.table.shape[0], M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S,
+             ptr(x), ptr(self.words), ptr(self._partials(S)), ptr(self.sync),
+             z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,
+             ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, stream_ptr())
+        return x

@@ -1,0 +1,73 @@
+"""Decode steps whose layers run in one launch (ops/decode_layers.py), against the plain implementation and against the
+layers run one by one."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import BF16_REL, assert_close, make_folder
+from plain.model import PlainQwen3
+
+pytestmark = pytest.mark.gpu
+
+
+def _cfg(layers, hidden, heads, kv, dim, ffn, window=None):
+    return dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", num_hidden_layers=layers, hidden_size=hidden,
+                num_attention_heads=heads, num_key_value_heads=kv, head_dim=dim, intermediate_size=ffn, vocab_size=515,
+                rope_theta=10000.0, rms_norm_eps=1e-6, tie_word_embeddings=True, max_position_embeddings=4096, hidden_act="silu",
+                attention_bias=False, rope_scaling=None, use_sliding_window=window is not None, sliding_window=window,
+                max_window_layers=1, eos_token_id=1)
+
+
+# one sequence of a single page and several rows that are not a power of two; pages that end where the step begins or ends
+# (63 -> 64 -> 65); more units a CTA than are summed at a time (feed-forwards of 8,192); columns that are no multiple of a
+# slot's 1,024 or of a warp's 128; groups of 1, 2, 3, 4 and 16 query heads; windows shorter than a page and longer; more page
+# jobs a CTA than its table holds is beyond a test's memory: 17 kv heads of 64 with 700 positions come to 1.4 a CTA
+CASES = [
+    (_cfg(2, 64, 1, 1, 64, 64), [5]),
+    (_cfg(2, 192, 6, 2, 64, 320), [63, 1, 130]),
+    (_cfg(3, 1088, 16, 1, 64, 1216), [64, 3, 700, 65, 128, 62, 191]),
+    (_cfg(2, 1024, 16, 8, 128, 3072), [62, 126, 500, 1, 1000, 333, 64, 129]),
+    (_cfg(2, 2560, 8, 2, 128, 8192), [200, 31]),
+    (_cfg(3, 256, 4, 4, 128, 8192, window=20), [300, 19, 70]),
+    (_cfg(3, 512, 34, 17, 64, 704, window=100), [700, 99, 101, 230]),
+]
+
+
+@pytest.mark.parametrize("i", range(len(CASES)))
+def test_one_launch_a_step(tmp_path, i):
+    from mynah_slm_b200.engine.engine import Engine, StepEntry
+    cfg, lens = CASES[i]
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=i)
+    plain = PlainQwen3.from_folder(folder)
+    rng = np.random.default_rng(i)
+    steps = 4
+    seqs = [rng.integers(0, cfg["vocab_size"], size=n + steps).tolist() for n in lens]
+    refs = [plain.forward(q) for q in seqs]
+    room = sum(-(-(n + steps) // 64) * 64 for n in lens)
+    rows = {}
+    for one in (True, False):
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=room + 64, max_seqs=len(lens) + 1)
+        assert eng.decode_layers is not None
+        took = []
+        takes = eng.decode_layers.takes
+        eng.decode_layers.takes = lambda ctx: took.append(takes(ctx) and one) or took[-1]
+        # what a page holds beyond its sequence's end must not matter
+        for t in eng.cache.keys + eng.cache.values:
+            t.fill_(float("nan"))
+        slots = [eng.open_sequence() for _ in lens]
+        eng.step([StepEntry(s, q[:n], ()) for s, q, n in zip(slots, seqs, lens)])
+        rows[one] = [eng.step([StepEntry(s, [q[n + t]], (0,)) for s, q, n in zip(slots, seqs, lens)]).cpu().numpy() for t in range(steps)]
+        eng.check_status()
+        assert any(took) == one
+        if one:
+            # a step again, with the rows in another order: a sequence's bits do not depend on its row or its company
+            for s in slots:
+                eng.close_sequence(s)
+            slots = [eng.open_sequence() for _ in lens]
+            eng.step([StepEntry(s, q[:n], ()) for s, q, n in zip(slots, seqs, lens)])
+            back = eng.step([StepEntry(s, [q[n]], (0,)) for s, q, n in list(zip(slots, seqs, lens))[::-1]]).cpu().numpy()
+            assert np.array_equal(back[::-1], rows[True][0])
+    for t in range(steps):
+        for b, n in enumerate(lens):
+            assert_close(refs[b][n + t][None], rows[True][t][b][None], BF16_REL, f"one launch, sequence {b}, step {t}")
+            assert_close(refs[b][n + t][None], rows[False][t][b][None], BF16_REL, f"layer by layer, sequence {b}, step {t}")
