@@ -20,9 +20,9 @@
 // added in a fixed order. A row's bits do not depend on the other rows. Who owns a column of the residual stream publishes it
 // times the norm's gain, and its share of the row's squares; 1/rms is a factor on the finished sums.
 //
-// Attention takes the sequences' pages as jobs of four warps (attn_page.cuh, the arithmetic of the per-page kernels). The
-// group of warps that has a (sequence, kv head)'s newest page merges all of its pages when its own jobs are done, in an order
-// that depends on their number only.
+// Attention's jobs are runs of up to four pages of a (sequence, kv head), cut by the sequence alone, four warps a job: each warp
+// keeps its own 16 keys of every page, with a running maximum, and meets the others once a run. The warps that have a
+// sequence's newest run merge all of its runs when their own jobs are done, in an order that depends on their number only.
 //
 // All CTAs must be resident at once: the launch is cooperative, and every wait is bounded (status bit 16). Registers: twelve
 // warps leave 168 a thread. (Sixteen multiplying warps at 96 spilled, and beside this much shared memory L1 holds no spills:
@@ -40,13 +40,15 @@ constexpr int PAGE_GROUPS = CWARPS / 4;                  // page jobs that a CTA
 constexpr int KC = 1024, KW = KC / CWARPS, PIECES = KW / 32;         // a slot's columns, a warp's share of them, in pieces of 32
 constexpr int UR = 8;                                    // output rows of a unit
 constexpr int SLOT_BYTES = UR * KC * 2;                  // eight rows in blocks of 64 columns [block][row][64], or a K or V tile
-constexpr int SLOTS = 11;                                // as many as the rest leaves room for
+constexpr int SLOTS = 10;                                // as many as the rest leaves room for
 constexpr int TG = 6;                                    // units whose sums a warp holds at a time
 constexpr int MAX_LAYERS = 48, MAX_GROUPS = 4, MAX_ROWS = 8;
 constexpr uint32_t WAIT_LOOKS = 1u << 22;                // trips to L2 after which a wait is given up (a second and more)
-constexpr int TABLE = 64;                                // page jobs of a CTA that are looked up once for all layers
+constexpr int RUN = 4;                                   // pages of a job at most
+constexpr int TABLE = 32;                                // jobs of a CTA that are looked up once for all layers
 constexpr int BAR_ALL = 5, BAR_NORM = 6;                 // named barriers of the eight warps, and with the helpers (1, 2: a page's four warps)
 static_assert(KEYS * 128 * 2 <= SLOT_BYTES && KW % 64 == 0, "a slot holds either kind of tile; a warp takes whole blocks of columns");
+static_assert(SLOTS > 2 * RUN, "a warp that passes over the other group's job has seen a filling of every slot since the one before");
 
 struct LayerDesc {                                       // as the host lays them out: 12 words of 64 bits
     const bf16 *w_qkv, *w_o, *w_gu, *w_down;
@@ -59,6 +61,8 @@ static_assert(sizeof(LayerDesc) == 96, "the host's layout");
 
 struct StepArgs {
     int M, D, H, KV, F, L, S;
+    int run;                                             // pages of a job
+    int lg_rows;                                         // M, rounded up to a power of two: its logarithm
     int gain_dtype, qk_dtype, n_pos;
     float eps, qk_eps, scale;
     int window[MAX_GROUPS];
@@ -77,22 +81,26 @@ struct StepMaps {
     CUtensorMap w[MAX_LAYERS][4];                        // q/k/v, o, gate/up, down as [block of 64 columns][row][64]
 };
 
-// a page job's place to work
+// a job's place to work
+constexpr int CHUNK = 2;                                 // heads whose outputs the four warps add at a time
 template <int HD> struct alignas(16) AttnWork {
     bf16 q[MAX_G * (HD + 8)];                            // the group's queries
-    bf16 p[MAX_G * KEYS];                                // the probabilities, then the merge's sums
-    float red_m[4][MAX_G], red_l[4][MAX_G];
+    float o[4][CHUNK][HD];                               // the warps' outputs, and the merge's sums
+    float m[4][MAX_G], l[4][MAX_G];
 };
+constexpr int STAGE_PITCH = KW * 2 + 16;                 // bytes of a staged row: eight rows' pieces of 16 bytes in different banks
 
 template <int HD>
 struct Smem {
     unsigned char slots[SLOTS][SLOT_BYTES];
     AttnWork<HD> a[PAGE_GROUPS];
+    unsigned char stage[CWARPS][MAX_ROWS * STAGE_PITCH]; // a warp's share of the rows at hand
     float sums[2][CWARPS][TG][UR * MAX_ROWS];            // two, used in turn: one barrier a turn is enough
     LayerDesc layers[MAX_LAYERS];
-    int2 table[MAX_GROUPS][TABLE];                       // a job's sequence, kv head and page number; the page's place
+    int table[MAX_GROUPS][TABLE];                        // a job's sequence, kv head and run
+    int pages[MAX_GROUPS][TABLE][RUN];                   // the places of its pages, -1: none
     unsigned long long full[SLOTS], empty[SLOTS];
-    int pg0[MAX_GROUPS][MAX_ROWS], cnt[MAX_GROUPS][MAX_ROWS], cum[MAX_GROUPS][MAX_ROWS + 1];   // pages seen by a sequence; jobs before it
+    int pg0[MAX_GROUPS][MAX_ROWS], cnt[MAX_GROUPS][MAX_ROWS], cum[MAX_GROUPS][MAX_ROWS + 1];   // pages seen by a sequence, jobs before it
     float inv_rms[MAX_ROWS];
     int hi[MAX_ROWS];
     int abort;
@@ -113,23 +121,29 @@ __device__ __forceinline__ int my_units(int n_units) {
     return (int)blockIdx.x < n_units ? (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 }
 
-// Page jobs are numbered sequence by sequence, kv head by kv head, page by page; a CTA takes a run of them.
-struct Job { int b, g, s; };
+// Jobs are numbered sequence by sequence, kv head by kv head, run by run; a CTA takes consecutive ones.
+struct Job {
+    int b, g, r, n;                                      // run r of n pages
+};
+__device__ __forceinline__ int runs_of(int pages, int run) { return (pages + run - 1) / run; }
 template <class SM>
-__device__ __noinline__ Job find_job(const SM& sm, const PageTable& pt, int grp, int j, int M, int& page) {
+__device__ __noinline__ int find_job(const SM& sm, int grp, int j, int M, int run) {
     int b = 0;
     while (b + 1 < M && j >= sm.cum[grp][b + 1]) b++;
-    const int r = j - sm.cum[grp][b], n = sm.cnt[grp][b];
-    const Job job{b, r / n, r % n};
-    page = page_of(pt, job.b, (sm.pg0[grp][job.b] + job.s) * PAGE_TOKENS);       // the physical page, -1: none
-    return job;
+    const int r = j - sm.cum[grp][b], n = runs_of(sm.cnt[grp][b], run);
+    return (int)((unsigned)b << 28) | (r / n) << 20 | r % n;
 }
 template <class SM>
-__device__ __forceinline__ Job look_up(const SM& sm, const PageTable& pt, int grp, int j, int j0, int M, int& page) {
-    if (j - j0 >= TABLE) return find_job(sm, pt, grp, j, M, page);
-    const int2 e = sm.table[grp][j - j0];
-    page = e.y;
-    return {(int)((unsigned)e.x >> 28), (e.x >> 20) & 255, e.x & 0xfffff};
+__device__ __forceinline__ Job look_up(const SM& sm, int grp, int j, int j0, int M, int run) {
+    const int e = j - j0 < TABLE ? sm.table[grp][j - j0] : find_job(sm, grp, j, M, run);
+    Job job{(int)((unsigned)e >> 28), (e >> 20) & 255, e & 0xfffff, 0};
+    job.n = min(run, sm.cnt[grp][job.b] - job.r * run);
+    return job;
+}
+// The physical page of a run's page i, -1: none.
+template <class SM>
+__device__ __forceinline__ int page_at(const SM& sm, const PageTable& pt, int grp, const Job& job, int j, int j0, int run, int i) {
+    return j - j0 < TABLE ? sm.pages[grp][j - j0][i] : page_of(pt, job.b, (sm.pg0[grp][job.b] + job.r * run + i) * PAGE_TOKENS);
 }
 __device__ __forceinline__ int first_job(int jobs, int cta) { return (int)((long long)jobs * cta / gridDim.x); }
 
@@ -195,21 +209,17 @@ struct Producer {
     __device__ __forceinline__ void pages(const StepArgs& a, const StepMaps& maps, const LayerDesc& d) {
         const int grp = (int)d.group, J = sm.cum[grp][a.M];
         const int j0 = first_job(J, blockIdx.x), j1 = first_job(J, blockIdx.x + 1);
-        for (int jb = j0; jb < j1; jb += 32) {
-            int row = -1;                                // every lane finds one job's tile
-            if (jb + lane < j1) {
-                int page;
-                const Job job = look_up(sm, a.pt[grp], grp, jb + lane, j0, a.M, page);
-                if (page >= 0) row = (int)d.map_row0 + (page * a.KV + job.g) * PAGE_TOKENS;
-            }
-            for (int i = 0; i < 32 && jb + i < j1; i++) {
-                const int r = __shfl_sync(0xffffffffu, row, i);
+        for (int j = j0; j < j1; j++) {
+            const Job job = look_up(sm, grp, j, j0, a.M, a.run);
+            for (int i = 0; i < job.n; i++) {
+                const int page = page_at(sm, a.pt[grp], grp, job, j, j0, a.run, i);
+                const int r = (int)d.map_row0 + (page * a.KV + job.g) * PAGE_TOKENS;
 #pragma unroll
                 for (int kv = 0; kv < 2; kv++, it++) {
                     if (!wait_empty(it)) return;
                     if (lane == 0) {
                         const uint32_t bar = tc5::smem_u32(&sm.full[it % SLOTS]), dst = tc5::smem_u32(sm.slots[it % SLOTS]);
-                        if (r >= 0) {
+                        if (page >= 0) {
                             const CUtensorMap* m = kv ? &maps.v[grp] : &maps.k[grp];
                             tc5::mbar_expect_tx(bar, KEYS * HD * 2);
 #pragma unroll
@@ -244,6 +254,7 @@ struct Worker {
     const StepArgs& a;
     uint32_t it = 0;                                     // slots taken so far
     int turn = 0;                                        // which of the two buffers of sums is next
+    uint32_t live = 0;                                   // the rows in use, a bit each
     int tid, warp, lane;
 
     // After `n` fruitless looks (of `limit`): whether to stop waiting, because the limit ran out here or somewhere in this CTA
@@ -265,17 +276,23 @@ struct Worker {
             : "=r"(done) : "r"(tc5::smem_u32(&sm.full[i % SLOTS])), "r"((i / SLOTS) & 1) : "memory");
         return done != 0;
     }
-    __device__ __forceinline__ void wait_full(uint32_t i) {
-        unsigned long long t0 = 0;                       // (a look may take a hardware wait of its own: a clock, not a count)
-        while (!is_full(i)) {
-            if (*(volatile int*)&sm.abort != 0) break;
+    // Until the n slots from number i on are full; a lane looks after a slot (a look may take a hardware wait of its own, so this
+    // limit is a clock, not a count).
+    __device__ __forceinline__ void wait_full(uint32_t i, int n) {
+        unsigned long long t0 = 0;
+        while (!__all_sync(0xffffffffu, lane >= n || is_full(i + lane))) {
             const unsigned long long now = tc5::now_ns();
             if (t0 == 0) t0 = now;
             else if (now - t0 > tc5::WAIT_LIMIT_NS) tired(~0u, 0);
+            if (__any_sync(0xffffffffu, *(volatile int*)&sm.abort != 0)) break;
         }
-        __syncwarp();
     }
-    __device__ __forceinline__ bool row_in_use(int m) const { return m < a.M && sm.hi[m] > 0; }
+    // This warp is through with the n slots from number i on.
+    __device__ __forceinline__ void release(uint32_t i, int n, int arrivals) {
+        __syncwarp();
+        if (lane < n * arrivals) tc5::mbar_arrive(tc5::smem_u32(&sm.empty[(i + lane / arrivals) % SLOTS]));
+    }
+    __device__ __forceinline__ bool row_in_use(int m) const { return (live >> m & 1) != 0; }
 
     // One lane's look at one word that is not there yet, until it is: what a long wait costs the others is one sector a warp.
     __device__ __forceinline__ bool watch(const uint64_t* p, bool missing, uint32_t tag) {
@@ -318,7 +335,7 @@ struct Worker {
     __device__ __forceinline__ void row_scales(int helper, uint32_t tag) {
 #pragma unroll 1
         for (int m = helper; m < a.M; m += HELPERS) {
-            if (sm.hi[m] <= 0) continue;
+            if (!row_in_use(m)) continue;
             const uint64_t* p = a.squares + (size_t)m * (a.D / UR);
             float ss;
             for (uint32_t n = 0;; n++) {
@@ -331,7 +348,7 @@ struct Worker {
                     ss += __uint_as_float((uint32_t)v);
                 }
                 if (__all_sync(0xffffffffu, gone == nullptr)) break;
-                if (watch(gone, gone != nullptr, tag)) break;
+                if (n >= 4 && watch(gone, gone != nullptr, tag)) break;
             }
             ss = warp_sum(ss);
             if (lane == 0) sm.inv_rms[m] = 1.0f / sqrtf(ss / (float)a.D + a.eps);
@@ -376,89 +393,93 @@ struct Worker {
         uint32_t next;                                   // the tag of what comes out
     };
 
-    // The lane's words of a warp's share of one slot's columns: row lane / 4, as the product's B operand wants them.
-    __device__ __forceinline__ void peek_share(const Product& q, int k0, bool on, uint64_t (&v)[PIECES][4]) {
-        const int left = min(KC, q.K - k0) - warp * KW;  // columns of this share that exist (a multiple of 64)
-        const uint64_t* p = q.src + ((size_t)(lane >> 2) * q.K + k0 + warp * KW) / 2 + (lane & 3);
+    // A warp reads its shares of the rows a stage at a time: as many slots' columns as make eight rows in all (one slot's of
+    // eight rows, eight slots' of one row), four columns a lane. Row i of a stage is row i % (1 << lg_rows) of the step, of the
+    // stage's slot i >> lg_rows.
+    __device__ __forceinline__ const uint64_t* staged(const Product& q, int k0, int i) const {   // null: there is none
+        const int m = i & ((1 << a.lg_rows) - 1), k = k0 + (i >> a.lg_rows) * KC + warp * KW + lane * 4;
+        return k < q.K && row_in_use(m) ? q.src + ((uint32_t)(m * q.K + k) >> 1) : nullptr;
+    }
+    __device__ __forceinline__ void peek_stage(const Product& q, int k0, uint64_t (&v)[MAX_ROWS][2]) const {
 #pragma unroll
-        for (int c = 0; c < PIECES; c++)
-#pragma unroll
-            for (int e = 0; e < 4; e++) v[c][e] = on && c * 32 < left ? peek(p + c * 16 + e * 4) : (uint64_t)q.tag << 32;
+        for (int i = 0; i < MAX_ROWS; i++) {
+            const uint64_t* p = staged(q, k0, i);
+            v[i][0] = v[i][1] = (uint64_t)q.tag << 32;
+            if (p != nullptr) peek2(p, v[i][0], v[i][1]);
+        }
     }
 
     __device__ __forceinline__ void product(const Product& q) {
-        constexpr int PASS = CONSUMERS / (MAX_ROWS * UR), OUTS = (TG + PASS - 1) / PASS;
         const int cnt = my_units(q.n_units), per = q.res == TO_SWIGLU ? 2 : 1, ug = TG / per;
-        const int om = (tid / UR) % MAX_ROWS, ou = tid / (MAX_ROWS * UR);        // this thread's outputs: row om, units ou + PASS i
-        const bool mine = row_in_use(om), row_on = row_in_use(lane >> 2);
+        const int om = (tid / UR) & ((1 << a.lg_rows) - 1), ou = tid >> (3 + a.lg_rows);         // this thread's outputs: row om, units ou, ou + pass ...
+        const int pass = (CONSUMERS / UR) >> a.lg_rows, depth = MAX_ROWS >> a.lg_rows;           // (slots' columns in a stage)
+        const bool mine = row_in_use(om);
+        // 16-byte pieces j (and 4 + j) of a block of 64 columns: row lane % 8, swizzled by the row
+        const int r = lane & 7, j = lane >> 3;
+        const uint32_t off = warp * (UR * KW * 2) + r * 128 + ((j ^ r) << 4);
+        unsigned char* stage = sm.stage[warp];
 #pragma unroll 1
         for (int u0 = 0; u0 < cnt; u0 += ug) {
             const int nu = min(ug, cnt - u0), nst = nu * per;
-            float old[OUTS], gn[OUTS];
-            if (q.res == ADD_TO_STREAM) {                // asked for now, needed at the end
-#pragma unroll
-                for (int o = 0; o < OUTS; o++) {
-                    const int u = ou + o * PASS, n = (blockIdx.x + (u0 + u) * gridDim.x) * UR + tid % UR;
-                    const bool on = u < nu && mine;
-                    old[o] = on ? a.x[(size_t)om * a.D + n] : 0.f;               // (this thread wrote it, or the embedding)
-                    gn[o] = on && q.gain != nullptr ? VecRef{q.gain, a.gain_dtype}.at(n) : 0.f;
-                }
-            }
-            // 16-byte pieces j (and 4 + j) of a block of 64 columns: row lane % 8, swizzled by the row
-            const int r = lane & 7, j = lane >> 3;
-            const uint32_t off = warp * (UR * KW * 2) + r * 128 + ((j ^ r) << 4);
-            float acc[TG / 2][4] = {};
-            uint64_t v[PIECES][4];
-            peek_share(q, 0, row_on, v);
+            float old = 0.f, gn = 0.f;
+            auto ask = [&](int u) {                      // what an addition to the stream needs of it
+                const int n = (blockIdx.x + (u0 + u) * gridDim.x) * UR + tid % UR;
+                if (q.res != ADD_TO_STREAM || u >= nu || !mine) return;
+                old = a.x[(size_t)om * a.D + n];         // (this thread wrote it, or the embedding)
+                gn = q.gain != nullptr ? VecRef{q.gain, a.gain_dtype}.at(n) : 0.f;
+            };
+            ask(ou);                                     // (asked for now, needed at the end)
+            float acc[TG / 2][2][4] = {};                // two chains of products each
+            uint64_t v[MAX_ROWS][2];
+            peek_stage(q, 0, v);
 #pragma unroll 1
-            for (int k0 = 0; k0 < q.K; k0 += KC) {
-                uint32_t f[PIECES][4];
+            for (int ks0 = 0; ks0 < q.K; ks0 += depth * KC) {
                 for (uint32_t n = 0;; n++) {
                     int gone = -1;
 #pragma unroll
-                    for (int c = 0; c < PIECES; c++)
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            if (!has_tag(v[c][e], q.tag)) gone = c * 16 + e * 4;
-                            f[c][e] = (uint32_t)v[c][e];
-                        }
+                    for (int i = 0; i < MAX_ROWS; i++)
+                        if (!has_tag(v[i][0], q.tag) || !has_tag(v[i][1], q.tag)) gone = i;
                     if (__all_sync(0xffffffffu, gone < 0)) break;
-                    if (n >= 2 && watch(q.src + ((size_t)(lane >> 2) * q.K + k0 + warp * KW) / 2 + (lane & 3) + gone, gone >= 0, q.tag)) break;
-                    peek_share(q, k0, row_on, v);
-                }
-                bool ready[TG];
-#pragma unroll
-                for (int t = 0; t < TG; t++) ready[t] = t < nst && is_full(it + t);
-                if (k0 + KC < q.K) peek_share(q, k0 + KC, row_on, v);            // under way while this slot's columns are multiplied
-#pragma unroll
-                for (int t = 0; t < TG; t += 2) {
-                    if (t < nst) {
-                        const bool two = t + 1 < nst;
-                        uint32_t w0[PIECES][4], w1[PIECES][4] = {};
-                        if (!__all_sync(0xffffffffu, ready[t])) wait_full(it);
-                        const uint32_t s0 = tc5::smem_u32(sm.slots[it % SLOTS]) + off;
-#pragma unroll
-                        for (int c = 0; c < PIECES; c++) ldmatrix_x4(w0[c], (s0 + c / 2 * (UR * 128)) ^ (c % 2 * 64));
-                        if (two) {
-                            if (!__all_sync(0xffffffffu, ready[t + 1])) wait_full(it + 1);
-                            const uint32_t s1 = tc5::smem_u32(sm.slots[(it + 1) % SLOTS]) + off;
-#pragma unroll
-                            for (int c = 0; c < PIECES; c++) ldmatrix_x4(w1[c], (s1 + c / 2 * (UR * 128)) ^ (c % 2 * 64));
-                        }
-#pragma unroll
-                        for (int c = 0; c < PIECES; c++) {
-                            const uint32_t lo[4] = {w0[c][0], w1[c][0], w0[c][1], w1[c][1]}, hi[4] = {w0[c][2], w1[c][2], w0[c][3], w1[c][3]};
-                            mma_bf16(acc[t / 2], lo, f[c][0], f[c][1]);
-                            mma_bf16(acc[t / 2], hi, f[c][2], f[c][3]);
-                        }
-                        __syncwarp();
-                        if (lane == 0) {
-                            tc5::mbar_arrive(tc5::smem_u32(&sm.empty[it % SLOTS]));
-                            if (two) tc5::mbar_arrive(tc5::smem_u32(&sm.empty[(it + 1) % SLOTS]));
-                        }
-                        it += two ? 2 : 1;
+                    if (n >= 3) {
+                        const uint64_t* p = gone >= 0 ? staged(q, ks0, gone) : nullptr;
+                        if (gone >= 0 && has_tag(peek(p), q.tag)) p++;
+                        if (watch(p, gone >= 0, q.tag)) break;
                     }
+                    peek_stage(q, ks0, v);
                 }
+#pragma unroll
+                for (int i = 0; i < MAX_ROWS; i++)
+                    *reinterpret_cast<uint2*>(stage + i * STAGE_PITCH + lane * 8) = make_uint2((uint32_t)v[i][0], (uint32_t)v[i][1]);
+                __syncwarp();
+                if (ks0 + depth * KC < q.K) peek_stage(q, ks0 + depth * KC, v);  // under way while these are multiplied
+#pragma unroll 1
+                for (int ks = 0; ks < depth && ks0 + ks * KC < q.K; ks++) {
+                    uint32_t f[PIECES][4];               // (rows that the step does not have: some other row)
+                    const uint32_t s = tc5::smem_u32(stage) + ((ks << a.lg_rows) + min(r, (1 << a.lg_rows) - 1)) * STAGE_PITCH + j * 16;
+#pragma unroll
+                    for (int c = 0; c < PIECES; c++) ldmatrix_x4(f[c], s + c * 64);
+                    wait_full(it, nst);
+#pragma unroll
+                    for (int t = 0; t < TG; t += 2) {
+                        if (t < nst) {
+                            const uint32_t s0 = tc5::smem_u32(sm.slots[(it + t) % SLOTS]) + off;
+                            // (an odd unit is multiplied with itself: its second half is not looked at)
+                            const uint32_t s1 = tc5::smem_u32(sm.slots[(it + (t + 1 < nst ? t + 1 : t)) % SLOTS]) + off;
+#pragma unroll
+                            for (int c = 0; c < PIECES; c++) {
+                                uint32_t w0[4], w1[4];
+                                ldmatrix_x4(w0, (s0 + c / 2 * (UR * 128)) ^ (c % 2 * 64));
+                                ldmatrix_x4(w1, (s1 + c / 2 * (UR * 128)) ^ (c % 2 * 64));
+                                const uint32_t lo[4] = {w0[0], w1[0], w0[1], w1[1]}, hi[4] = {w0[2], w1[2], w0[3], w1[3]};
+                                mma_bf16(acc[t / 2][0], lo, f[c][0], f[c][1]);
+                                mma_bf16(acc[t / 2][1], hi, f[c][2], f[c][3]);
+                            }
+                        }
+                    }
+                    release(it, nst, 1);
+                    it += nst;
+                }
+                __syncwarp();                            // the staged rows have been read
             }
             float(*sums)[TG][UR * MAX_ROWS] = sm.sums[turn];
             turn ^= 1;
@@ -467,15 +488,16 @@ struct Worker {
                 if (t < nst) {
 #pragma unroll
                     for (int e = 0; e < 2; e++)          // a row of the step, a row of the weights
-                        sums[warp][t][((lane & 3) * 2 + e) * UR + (lane >> 2)] = acc[t / 2][(t & 1) * 2 + e];
+                        sums[warp][t][((lane & 3) * 2 + e) * UR + (lane >> 2)] = acc[t / 2][0][(t & 1) * 2 + e] + acc[t / 2][1][(t & 1) * 2 + e];
                 }
             if (q.normed && u0 == 0) sync_norm();
             else sync_all();
-#pragma unroll
-            for (int o = 0; o < OUTS; o++) {
-                const int u = ou + o * PASS, n = (blockIdx.x + (u0 + u) * gridDim.x) * UR + tid % UR;
+#pragma unroll 1
+            for (int u = ou; u - ou < nu; u += pass) {   // (as often in every thread)
+                const int n = (blockIdx.x + (u0 + u) * gridDim.x) * UR + tid % UR;
                 const bool on = u < nu && mine;
                 if (!__any_sync(0xffffffffu, on)) continue;
+                if (u != ou) ask(u);
                 float s = 0.f, s2 = 0.f;
                 if (on) {
                     const float* p = &sums[0][u * per][om * UR + tid % UR];
@@ -491,9 +513,9 @@ struct Worker {
                     }
                 }
                 if (q.res == ADD_TO_STREAM) {
-                    const float x = old[o] + s;
+                    const float x = old + s;
                     if (on) a.x[(size_t)om * a.D + n] = x;
-                    if (q.gain != nullptr) publish_stream(on, x, gn[o], om, n, q.next);
+                    if (q.gain != nullptr) publish_stream(on, x, gn, om, n, q.next);
                 } else {
                     if (per == 2) s = s / (1.0f + expf(-s)) * s2;
                     const float y1 = __shfl_down_sync(0xffffffffu, s, 1);
@@ -503,30 +525,10 @@ struct Worker {
         }
     }
 
-    // Where a page's result goes: tagged partial rows, or (a sequence of one visible page) the finished output.
-    struct PutPage {
-        uint64_t *o_row, *ml_row, *att;                  // of the group's first head
-        int S;
-        uint32_t tag;
-        bool whole;
-        const float (*red_l)[MAX_G];
-        __device__ __forceinline__ void o(int h, int d, float v0, float v1) const {
-            if (whole) {
-                const float inv = 1.0f / ((red_l[0][h] + red_l[1][h]) + (red_l[2][h] + red_l[3][h]));
-                publish(att + ((size_t)h * HD + d) / 2, pack2(v0 * inv, v1 * inv), tag);
-            } else {
-                publish2(o_row + (size_t)h * S * HD + d, __float_as_uint(v0), __float_as_uint(v1), tag);
-            }
-        }
-        __device__ __forceinline__ void ml(int h, float m, float l) const {
-            if (!whole) publish2(ml_row + (size_t)h * S * 2, __float_as_uint(m), __float_as_uint(l), tag);
-        }
-    };
-
-    // The n pages of one (sequence, kv head), by the four warps of a group: out[h] = sum_s w_s o_s / sum_s w_s l_s with
-    // w_s = exp(m_s - m). 4 / G warps a head (at least one), each adds every so many-th page; their sums are added in order.
+    // The n runs of one (sequence, kv head), by the four warps of a group: out[h] = sum_s w_s o_s / sum_s w_s l_s with
+    // w_s = 2^(m_s - m). 4 / G warps a head (at least one), each adds every so many-th run; their sums are added in order.
     __device__ __forceinline__ void merge(AttnWork<HD>& w, int b, int g, int n, uint32_t tag) {
-        constexpr int DL = HD / 32, BATCH = 8;           // a lane's columns; pages whose rows are under way together
+        constexpr int DL = HD / 32, BATCH = 4;           // a lane's columns; runs whose rows are under way together
         const int G = a.H / a.KV, lw = warp & 3;
         const int wph = G >= 3 ? 1 : 4 / G, hpt = 4 / wph, sub = lw % wph;       // warps a head, heads in one turn
 #pragma unroll 1
@@ -538,7 +540,7 @@ struct Worker {
                 const uint64_t* ml = a.part_ml + row * 2;
                 float m = -INFINITY;
 #pragma unroll 1
-                for (int s0 = 0; s0 < n; s0 += 32) {     // all pages' maxima and sums, a page a lane
+                for (int s0 = 0; s0 < n; s0 += 32) {     // all runs' maxima and sums, a run a lane
                     const int s = s0 + lane;
                     uint64_t vm = 0, vl = 0;
                     for (uint32_t k = 0;; k++) {
@@ -550,18 +552,18 @@ struct Worker {
                     const float pm = s < n ? __uint_as_float((uint32_t)vm) : -INFINITY, pl = __uint_as_float((uint32_t)vl);
                     if (pm > -INFINITY) {
                         const float nm = fmaxf(m, pm);
-                        lsum = lsum * expf(m - nm) + pl * expf(pm - nm);
+                        lsum = lsum * exp2f(m - nm) + pl * exp2f(pm - nm);
                         m = nm;
                     }
                 }
                 const float top = warp_max(m);
-                lsum = warp_sum(m > -INFINITY ? lsum * expf(m - top) : 0.f);
+                lsum = warp_sum(m > -INFINITY ? lsum * exp2f(m - top) : 0.f);
 #pragma unroll 1
                 for (int s0 = 0; s0 < n && top > -INFINITY; s0 += 32) {
                     uint64_t vm = 0, vl;
                     if (s0 + lane < n) peek2(ml + 2 * (s0 + lane), vm, vl);
                     const float pm = s0 + lane < n ? __uint_as_float((uint32_t)vm) : -INFINITY;
-                    const float e = pm > -INFINITY ? expf(pm - top) : 0.f;       // (0: a page that was not there has no row)
+                    const float e = pm > -INFINITY ? exp2f(pm - top) : 0.f;       // (0: nothing to add)
                     const int n1 = min(32, n - s0);
 #pragma unroll 1
                     for (int i0 = sub; i0 < n1; i0 += wph * BATCH) {
@@ -594,7 +596,7 @@ struct Worker {
                     }
                 }
             }
-            float* part = reinterpret_cast<float*>(w.p); // [4 warps][HD]
+            float* part = &w.o[0][0][0];                 // [4 warps][HD]
             if (wph > 1) {
                 SyncGroup::sync();
                 if (sub > 0) {
@@ -617,138 +619,206 @@ struct Worker {
     }
 
     __device__ __forceinline__ void attention(const LayerDesc& d, uint32_t tag) {
-        constexpr int KSTEPS = HD / 16, QLD = HD + 8;
+        constexpr int KSTEPS = HD / 16, NT = HD / 8, QLD = HD + 8;
         constexpr int LPH = HeadLanes<HD>::LPH, HPW = HeadLanes<HD>::HPW;
-        const int grp = (int)d.group, J = sm.cum[grp][a.M], G = a.H / a.KV;
+        const int grp = (int)d.group, J = sm.cum[grp][a.M], G = a.H / a.KV, window = a.window[grp];
         const int j0 = first_job(J, blockIdx.x), j1 = first_job(J, blockIdx.x + 1);
         const int gi = warp >> 2, lw = warp & 3, ltid = tid & 127, sub = lane / LPH, li = lane % LPH;
+        const int mat = lane >> 3, rr = lane & 7;
         AttnWork<HD>& w = sm.a[gi];
-        const TcArgs ta{a.H, a.KV, 0, a.window[grp], a.S, a.scale, 0, 1, 0.f};
         const int NQ = (a.H + 2 * a.KV) * HD;
         const bool rotate = a.cos_t != nullptr, has_gain = d.q_gain != nullptr;
         int pb = -1, pg = -1;                            // the (sequence, kv head) at hand
-        bool merges = false;                             // some job of this group is a newest page of several
+        bool merges = false;                             // some job of this group is a newest run of several
 #pragma unroll 1
-        for (int j = j0 + gi; j < j1; j += PAGE_GROUPS) {
-            int page;
-            const Job job = look_up(sm, a.pt[grp], grp, j, j0, a.M, page);
-            const int hi = sm.hi[job.b], pos = hi - 1, n_pages = sm.cnt[grp][job.b];
+        for (int j = j0; j < j1; j++) {
+            const Job job = look_up(sm, grp, j, j0, a.M, a.run);
+            if ((j - j0) % PAGE_GROUPS != gi) {          // the other group's
+                it += 2 * job.n;
+                continue;
+            }
+            const int hi = sm.hi[job.b], pos = hi - 1, runs = runs_of(sm.cnt[grp][job.b], a.run);
             const uint64_t* qrow = a.qkv + (size_t)job.b * NQ / 2;
-            const int p0 = (sm.pg0[grp][job.b] + job.s) * PAGE_TOKENS, lo = first_visible(hi, a.window[grp]);
-            const int r_new = pos >= p0 && pos < p0 + PAGE_TOKENS ? pos - p0 : -1;
+            const int first = (sm.pg0[grp][job.b] + job.r * a.run) * PAGE_TOKENS, lo = first_visible(hi, window);
             const bool pos_ok = !rotate || pos < a.n_pos;
             if (!pos_ok && ltid == 0) atomicOr(a.status, MYNAH_ST_POS_RANGE);
-            merges = merges || (job.s == n_pages - 1 && n_pages > 1);
-            // the new key and value, by the fourth warp of the group that has their page; the queries by the first ones
+            merges = merges || (job.r == runs - 1 && runs > 1);
+            // The queries (for the first job of a sequence and kv head) and the new key and value: a warp takes every fourth pass
+            // of heads, and the key if its place is among the warp's; whose that is begins with the queries last.
+            const int at_new = pos - first;
+            const bool newest = at_new >= 0 && at_new < job.n * PAGE_TOKENS, fresh = job.b != pb || job.g != pg;
+            const int w_new = newest ? (at_new % PAGE_TOKENS) / 16 : 3, i_new = newest && w_new == lw ? at_new / PAGE_TOKENS : -1;
             uint4 ko = make_uint4(0, 0, 0, 0), vn = ko;
-            if (r_new >= 0 && lw == 3) {
-                float kn[8], gain[8], rc[8], rs[8];
+            pb = job.b;
+            pg = job.g;
+#pragma unroll 1
+            for (int hb = fresh ? ((lw - w_new - 1) & 3) * HPW : G; hb < G || i_new >= 0; hb += 4 * HPW) {        // uniform over the warp
+                const bool is_k = hb >= G;
+                const int head = is_k ? a.H + job.g : job.g * G + hb + sub;
+                float v[8], gain[8], rc[8], rs[8];
                 if (rotate) load_rotation<HD>(a.cos_t, a.sin_t, pos_ok ? pos : 0, lane, rc, rs);
-                if (has_gain) load_gain8(VecRef{d.k_gain, a.qk_dtype}, li * 8, gain);
-                const uint64_t* p[2] = {qrow + ((size_t)(a.H + job.g) * HD + li * 8) / 2, qrow + ((size_t)(a.H + a.KV + job.g) * HD + li * 8) / 2};
-                const bool on[2] = {sub == 0, sub == 0};
+                if (has_gain) load_gain8(VecRef{is_k ? d.k_gain : d.q_gain, a.qk_dtype}, li * 8, gain);
+                const uint64_t* p[2] = {qrow + (head * HD + li * 8) / 2, qrow + ((a.H + a.KV + job.g) * HD + li * 8) / 2};
+                const bool on[2] = {is_k ? sub == 0 : hb + sub < G, is_k && sub == 0};
                 uint32_t raw[2][4];
                 read_tagged<2>(p, on, tag, raw);
                 Raw8<bf16> r8;
                 r8.q[0] = make_uint4(raw[0][0], raw[0][1], raw[0][2], raw[0][3]);
-                r8.to_f32(kn);
-                vn = make_uint4(raw[1][0], raw[1][1], raw[1][2], raw[1][3]);
-                head_norm_rotate<HD>(kn, has_gain, gain, a.qk_eps, rotate, rc, rs, lane);
-                ko = make_uint4(pack2(kn[0], kn[1]), pack2(kn[2], kn[3]), pack2(kn[4], kn[5]), pack2(kn[6], kn[7]));
+                r8.to_f32(v);
+                head_norm_rotate<HD>(v, has_gain, gain, a.qk_eps, rotate, rc, rs, lane);
+                const uint4 out = make_uint4(pack2(v[0], v[1]), pack2(v[2], v[3]), pack2(v[4], v[5]), pack2(v[6], v[7]));
+                if (is_k) {
+                    ko = out;
+                    vn = make_uint4(raw[1][0], raw[1][1], raw[1][2], raw[1][3]);
+                    break;
+                }
+                if (on[0]) *reinterpret_cast<uint4*>(w.q + (hb + sub) * QLD + li * 8) = out;
             }
-            if (job.b != pb || job.g != pg) {
-                pb = job.b;
-                pg = job.g;
-                if (lw * HPW < G) {                      // uniform over the warp
-                    float gain[8], rc[8], rs[8];
-                    if (rotate) load_rotation<HD>(a.cos_t, a.sin_t, pos_ok ? pos : 0, lane, rc, rs);
-                    if (has_gain) load_gain8(VecRef{d.q_gain, a.qk_dtype}, li * 8, gain);
+            if (fresh) SyncGroup::sync();
+            // ---- the run's pages: this warp's 16 keys of each
+            const uint32_t q32 = tc5::smem_u32(w.q) + ((lane & 15) * QLD + (lane >> 4) * 8) * 2;
+            float oc[NT][4] = {}, m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll 1
-                    for (int hb = lw * HPW; hb < G; hb += 4 * HPW) {
-                        const uint64_t* p[1] = {qrow + ((size_t)(job.g * G + hb + sub) * HD + li * 8) / 2};
-                        const bool on[1] = {hb + sub < G};
-                        uint32_t raw[1][4];
-                        read_tagged<1>(p, on, tag, raw);
-                        Raw8<bf16> r8;
-                        r8.q[0] = make_uint4(raw[0][0], raw[0][1], raw[0][2], raw[0][3]);
-                        float v[8];
-                        r8.to_f32(v);
-                        head_norm_rotate<HD>(v, has_gain, gain, a.qk_eps, rotate, rc, rs, lane);
-                        if (hb + sub < G) store8<bf16>(w.q + (hb + sub) * QLD + li * 8, v);
+            for (int i = 0; i < job.n; i++, it += 2) {
+                const int page = page_at(sm, a.pt[grp], grp, job, j, j0, a.run, i), p0 = first + i * PAGE_TOKENS;
+                const bool empty = page < 0 || !pos_ok;
+                if (page < 0 && ltid == 0) atomicOr(a.status, MYNAH_ST_PAGE_RANGE);
+                const int k_first = max(lo, p0) - p0, k_last = min(hi, p0 + PAGE_TOKENS) - 1 - p0;
+                const uint32_t ik = it % SLOTS, iv = (it + 1) % SLOTS;
+                unsigned char *kt = sm.slots[ik], *vt = sm.slots[iv];
+                wait_full(it, 2);
+                const bool mend = !empty && (lw * 16 < k_first || lw * 16 + 15 > k_last || i == i_new);      // uniform over the warp
+                if (mend) {
+                    // what a page holds outside the visible range may be anything: value rows that meet a probability of zero
+                    // are cleared (scores of such keys are replaced, not multiplied)
+                    for (int c = lane; c < 16 * (HD / 8); c += 32) {
+                        const int row = lw * 16 + c / (HD / 8);
+                        if (row < k_first || row > k_last) *reinterpret_cast<uint4*>(vt + TileTma<HD>::off(row, c % (HD / 8))) = make_uint4(0, 0, 0, 0);
+                    }
+                    if (i == i_new && sub == 0) {
+                        *reinterpret_cast<uint4*>(kt + TileTma<HD>::off(at_new % PAGE_TOKENS, li)) = ko;
+                        *reinterpret_cast<uint4*>(vt + TileTma<HD>::off(at_new % PAGE_TOKENS, li)) = vn;
+                    }
+                    __syncwarp();
+                }
+                if (!empty) {
+                    float sc[2][4] = {};                 // heads lane / 4 (+ 8 in elements 2, 3), keys 16 lw + 8 t + (lane % 4) * 2 + {0, 1}
+                    const uint32_t kb32 = tc5::smem_u32(kt), vb32 = tc5::smem_u32(vt);
+#pragma unroll
+                    for (int ks = 0; ks < KSTEPS; ks++) {
+                        uint32_t qa[4], kb[4];           // (query rows beyond the group's heads: whatever is there)
+                        ldmatrix_x4(qa, q32 + ks * 32);
+                        ldmatrix_x4(kb, kb32 + TileTma<HD>::off(lw * 16 + (mat >> 1) * 8 + rr, ks * 2 + (mat & 1)));
+                        mma_bf16(sc[0], qa, kb[0], kb[1]);
+                        mma_bf16(sc[1], qa, kb[2], kb[3]);
+                    }
+                    float top[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+                    for (int t = 0; t < 2; t++)
+#pragma unroll
+                        for (int e = 0; e < 4; e++) {
+                            const int key = lw * 16 + t * 8 + (lane & 3) * 2 + (e & 1);
+                            sc[t][e] = key >= k_first && key <= k_last ? sc[t][e] * a.scale : -INFINITY;
+                            top[e >> 1] = fmaxf(top[e >> 1], sc[t][e]);
+                        }
+                    float shrink[2];
+#pragma unroll
+                    for (int e = 0; e < 2; e++) {
+                        top[e] = fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 1));
+                        top[e] = fmaxf(m[e], fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 2)));
+                        shrink[e] = m[e] == top[e] ? 1.0f : exp2f(m[e] - top[e]);         // (nothing seen yet: 2^-inf = 0, of zeros)
+                        m[e] = top[e];
+                        l[e] *= shrink[e];
+                        if (top[e] == -INFINITY) top[e] = 0.f;       // no key of this warp is visible: every probability is 0
+                    }
+                    if (__any_sync(0xffffffffu, shrink[0] != 1.0f || shrink[1] != 1.0f)) {
+#pragma unroll
+                        for (int nt = 0; nt < NT; nt++)
+#pragma unroll
+                            for (int e = 0; e < 4; e++) oc[nt][e] *= shrink[e >> 1];
+                    }
+                    uint32_t pa[4];                      // probabilities: fp32 for the sum, bf16 for the product
+#pragma unroll
+                    for (int t = 0; t < 2; t++)
+#pragma unroll
+                        for (int e = 0; e < 2; e++) {
+                            const float u0 = exp2f(sc[t][2 * e] - top[e]), u1 = exp2f(sc[t][2 * e + 1] - top[e]);
+                            l[e] += u0 + u1;
+                            pa[t * 2 + e] = pack2(u0, u1);
+                        }
+#pragma unroll
+                    for (int nt = 0; nt < NT; nt += 2) {
+                        uint32_t vb[4];
+                        ldmatrix_x4_trans(vb, vb32 + TileTma<HD>::off(lw * 16 + (mat & 1) * 8 + rr, nt + (mat >> 1)));
+                        mma_bf16(oc[nt], pa, vb[0], vb[1]);
+                        mma_bf16(oc[nt + 1], pa, vb[2], vb[3]);
                     }
                 }
-                SyncGroup::sync();
-            }
-            const uint32_t ik = it + 2 * (uint32_t)(j - j0), iv = ik + 1;
-            unsigned char *kt = sm.slots[ik % SLOTS], *vt = sm.slots[iv % SLOTS];
-            PageJob pj;
-            pj.s = job.s; pj.g = job.g; pj.b = job.b; pj.page = page; pj.h_first = 1; pj.h_last = 0;
-            pj.k_first = max(lo, p0) - p0;
-            pj.k_last = min(hi, p0 + PAGE_TOKENS) - 1 - p0;
-            pj.row0 = ((size_t)job.b * a.H + (size_t)job.g * G) * a.S + job.s;
-            pj.empty = page < 0 || !pos_ok;
-            const bool mend = !pj.empty && (pj.k_first > 0 || pj.k_last < KEYS - 1 || r_new >= 0);      // uniform over the group
-            wait_full(ik);
-            wait_full(iv);
-            if (mend) {
-                // what a page holds outside the visible range may be anything: value rows that meet a probability of zero are
-                // cleared (scores of such keys are replaced, not multiplied)
-                for (int i = ltid; i < KEYS * (HD / 8); i += 128) {
-                    const int r = i / (HD / 8), c = i % (HD / 8);
-                    if (r < pj.k_first || r > pj.k_last) *reinterpret_cast<uint4*>(vt + TileTma<HD>::off(r, c)) = make_uint4(0, 0, 0, 0);
-                }
-                if (r_new >= 0 && lw == 3 && sub == 0) {
-                    *reinterpret_cast<uint4*>(kt + TileTma<HD>::off(r_new, li)) = ko;
-                    *reinterpret_cast<uint4*>(vt + TileTma<HD>::off(r_new, li)) = vn;
-                }
-                SyncGroup::sync();
-            }
-            const PutPage put{a.part_o + pj.row0 * HD, a.part_ml + pj.row0 * 2, a.att + ((size_t)job.b * a.H + (size_t)job.g * G) * HD / 2,
-                              a.S, tag, n_pages == 1, w.red_l};
-            if (pj.empty) {
-                if (page < 0 && ltid == 0) atomicOr(a.status, MYNAH_ST_PAGE_RANGE);
-                if (n_pages == 1) {
-                    for (int i = ltid; i < G * HD / 2; i += 128) publish(put.att + i, 0, tag);
-                } else {
-                    for (int i = ltid; i < G; i += 128) put.ml(i, -INFINITY, 0.f);
-                }
-            } else {
-                uint32_t qa[KSTEPS][4];
-                const uint32_t q32 = tc5::smem_u32(w.q) + ((lane & 15) * QLD + (lane >> 4) * 8) * 2;     // (rows beyond the group's heads: whatever is there)
-#pragma unroll
-                for (int ks = 0; ks < KSTEPS; ks++) ldmatrix_x4(qa[ks], q32 + ks * 32);
-                const uint32_t kb32 = tc5::smem_u32(kt), vb32 = tc5::smem_u32(vt);
-                compute_page_core<HD, HD, SyncGroup>(
-                    pj, qa, ta,
-                    [&](int ks, uint32_t (&kb)[4]) { load_k_frag<HD, TileTma<HD>>(kb32, ks, kb); },
-                    [&](int ks, int nt, uint32_t (&vb)[4]) { load_v_frag<HD, TileTma<HD>>(vb32, ks, nt, vb); },
-                    []() {}, []() { SyncGroup::sync(); }, w.p, w.red_m, w.red_l, put);
-                if (r_new >= 0 && lw == 3 && sub == 0) {             // the new position's place in the cache
-                    const size_t row = (((size_t)page * a.KV + job.g) * PAGE_TOKENS + r_new) * HD + li * 8;
+                if (mend) tc5::fence_async_smem();       // before a copy fills the slots again
+                release(it, 2, CWARPS / 4);              // (four warps make the arrivals of all)
+                if (i == i_new && !empty && sub == 0) {  // the new position's place in the cache
+                    const size_t row = (((size_t)page * a.KV + job.g) * PAGE_TOKENS + at_new % PAGE_TOKENS) * HD + li * 8;
                     *reinterpret_cast<uint4*>(d.k + row) = ko;
                     *reinterpret_cast<uint4*>(d.v + row) = vn;
                 }
             }
-            if (mend) tc5::fence_async_smem();           // before a copy fills the slots again
-            __syncwarp();
-            if (lane < CWARPS / 4) {                     // four warps make the arrivals of all that empty a slot
-                tc5::mbar_arrive(tc5::smem_u32(&sm.empty[ik % SLOTS]));
-                tc5::mbar_arrive(tc5::smem_u32(&sm.empty[iv % SLOTS]));
+            // ---- the four warps' shares together, CHUNK heads at a time
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1);
+                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2);
+                if ((lane & 3) == 0) {
+                    w.m[lw][(lane >> 2) + 8 * e] = m[e];
+                    w.l[lw][(lane >> 2) + 8 * e] = l[e];
+                }
             }
-            SyncGroup::sync();
+            const size_t row0 = ((size_t)job.b * a.H + (size_t)job.g * G) * a.S + job.r;
+#pragma unroll 1
+            for (int h0 = 0; h0 < G; h0 += CHUNK) {
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const int h = (lane >> 2) + 8 * e - h0;
+                    if (h >= 0 && h < CHUNK) {
+#pragma unroll
+                        for (int nt = 0; nt < NT; nt++)
+                            *reinterpret_cast<float2*>(&w.o[lw][h][nt * 8 + (lane & 3) * 2]) = make_float2(oc[nt][2 * e], oc[nt][2 * e + 1]);
+                    }
+                }
+                SyncGroup::sync();
+                const int hc = ltid / (HD / 2), h = h0 + hc, c = ltid % (HD / 2) * 2;
+                if (hc < CHUNK && h < G) {
+                    const float top = fmaxf(fmaxf(w.m[0][h], w.m[1][h]), fmaxf(w.m[2][h], w.m[3][h]));
+                    float o0 = 0.f, o1 = 0.f, sum = 0.f;
+#pragma unroll
+                    for (int p = 0; p < 4; p++) {
+                        const float mp = w.m[p][h], f = mp > -INFINITY ? exp2f(mp - top) : 0.f;
+                        const float2 o = *reinterpret_cast<const float2*>(&w.o[p][hc][c]);
+                        sum = fmaf(f, w.l[p][h], sum);
+                        o0 = fmaf(f, o.x, o0);
+                        o1 = fmaf(f, o.y, o1);
+                    }
+                    if (runs == 1) {                     // all that the sequence sees: finished
+                        const float inv = sum > 0.f ? 1.0f / sum : 0.f;
+                        publish(a.att + ((size_t)job.b * a.H * HD + (size_t)(job.g * G + h) * HD + c) / 2, pack2(o0 * inv, o1 * inv), tag);
+                    } else {
+                        const size_t row = row0 + (size_t)h * a.S;
+                        publish2(a.part_o + row * HD + c, __float_as_uint(o0), __float_as_uint(o1), tag);
+                        if (c == 0) publish2(a.part_ml + row * 2, __float_as_uint(top), __float_as_uint(sum), tag);
+                    }
+                }
+                SyncGroup::sync();
+            }
         }
-        it += 2 * (uint32_t)(j1 - j0);
         // Both groups are through with their pages before a warp asks for a slot behind them: a barrier's parity names the right
         // filling only to those who know that the one before has come.
         sync_all();
         if (!merges) return;
-        // A merge waits for pages with lower numbers only, and these wait for merges of still lower ones at most.
+        // A merge waits for runs with lower numbers only, and these wait for merges of still lower ones at most.
 #pragma unroll 1
         for (int j = j0 + gi; j < j1; j += PAGE_GROUPS) {
-            int page;
-            const Job job = look_up(sm, a.pt[grp], grp, j, j0, a.M, page);
-            const int n_pages = sm.cnt[grp][job.b];
-            if (job.s == n_pages - 1 && n_pages > 1) merge(w, job.b, job.g, n_pages, tag);
+            const Job job = look_up(sm, grp, j, j0, a.M, a.run);
+            const int runs = runs_of(sm.cnt[grp][job.b], a.run);
+            if (job.r == runs - 1 && runs > 1) merge(w, job.b, job.g, runs, tag);
         }
     }
 };
@@ -780,7 +850,7 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
             sm.pg0[tid][b] = vp.pg0;
             sm.cnt[tid][b] = min(vp.count(), a.S);
             sm.cum[tid][b] = sum;
-            sum += sm.cnt[tid][b] * a.KV;
+            sum += runs_of(sm.cnt[tid][b], a.run) * a.KV;
         }
         sm.cum[tid][a.M] = sum;
     }
@@ -788,9 +858,9 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
     for (int i = tid; i < MAX_GROUPS * TABLE; i += THREADS) {
         const int g = i / TABLE, J = sm.cum[g][a.M], j = first_job(J, blockIdx.x) + i % TABLE;
         if (a.pt[g].ids != nullptr && j < first_job(J, blockIdx.x + 1)) {
-            int page;
-            const Job job = find_job(sm, a.pt[g], g, j, a.M, page);
-            sm.table[g][i % TABLE] = make_int2((int)((unsigned)job.b << 28) | job.g << 20 | job.s, page);
+            sm.table[g][i % TABLE] = find_job(sm, g, j, a.M, a.run);
+            const Job job = look_up(sm, g, first_job(J, blockIdx.x) + i % TABLE, first_job(J, blockIdx.x), a.M, a.run);
+            for (int k = 0; k < job.n; k++) sm.pages[g][i % TABLE][k] = page_of(a.pt[g], job.b, (sm.pg0[g][job.b] + job.r * a.run + k) * PAGE_TOKENS);
         }
     }
     __syncthreads();
@@ -827,6 +897,7 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
         c.tid = tid;
         c.warp = warp;
         c.lane = lane;
+        for (int m = 0; m < a.M; m++) c.live |= sm.hi[m] > 0 ? 1u << m : 0u;
         if (warp > CWARPS) {
 #pragma unroll 1
             for (int l = 0; l < a.L; l++) {
@@ -932,7 +1003,10 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     a.M = M; a.D = D; a.H = H; a.KV = KV; a.F = F; a.L = L; a.S = S;
     a.gain_dtype = gain_dtype; a.qk_dtype = qk_dtype; a.n_pos = n_pos;
     a.eps = eps; a.qk_eps = qk_eps;
-    a.scale = 1.0f / sqrtf((float)HD);
+    a.scale = (float)(1.4426950408889634 / sqrt((double)HD));        // probabilities are powers of two: score times log2(e)
+    while ((1 << a.lg_rows) < M) a.lg_rows++;
+    // Few sequences: short runs, so that more warps share a long one; many: longer ones, with fewer partial results to merge.
+    a.run = M <= 2 ? 2 : RUN;
     a.layers = static_cast<const LayerDesc*>(layers);
     a.x = x;
     a.hid = static_cast<uint64_t*>(words);
