@@ -331,27 +331,40 @@ struct Worker {
         }
     }
 
-    // 1 / rms of every row from the shares of its columns' owners (by the helper warps, while the others multiply).
+    // 1 / rms of every row from the shares of its columns' owners (by the helper warps, while the others multiply): a helper
+    // takes every third row, all of its rows together. One word is watched while nothing has come yet; the rest follows within
+    // a microsecond and is looked for by all lanes.
     __device__ __forceinline__ void row_scales(int helper, uint32_t tag) {
+        constexpr int ROWS = (MAX_ROWS + HELPERS - 1) / HELPERS;
+        float ss[ROWS];
+        watch(a.squares + (size_t)helper * (a.D / UR), lane == 0 && row_in_use(helper), tag);
+        for (uint32_t n = 0;; n++) {
+            bool gone = false;
+#pragma unroll
+            for (int i = 0; i < ROWS; i++) ss[i] = 0.f;
 #pragma unroll 1
-        for (int m = helper; m < a.M; m += HELPERS) {
-            if (!row_in_use(m)) continue;
-            const uint64_t* p = a.squares + (size_t)m * (a.D / UR);
-            float ss;
-            for (uint32_t n = 0;; n++) {
-                const uint64_t* gone = nullptr;
-                ss = 0.f;
-#pragma unroll 4
-                for (int u = lane; u < a.D / UR; u += 32) {
-                    const uint64_t v = peek(p + u);
-                    if (!has_tag(v, tag)) gone = p + u;
-                    ss += __uint_as_float((uint32_t)v);
+            for (int u = lane * 4; u < a.D / UR; u += 128) {         // (a multiple of eight of them)
+#pragma unroll
+                for (int i = 0; i < ROWS; i++) {
+                    if (!row_in_use(helper + i * HELPERS)) continue;
+                    const uint64_t* p = a.squares + (size_t)(helper + i * HELPERS) * (a.D / UR) + u;
+                    uint64_t v[4];
+                    peek2(p, v[0], v[1]);
+                    peek2(p + 2, v[2], v[3]);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) {
+                        gone = gone || !has_tag(v[e], tag);
+                        ss[i] += __uint_as_float((uint32_t)v[e]);
+                    }
                 }
-                if (__all_sync(0xffffffffu, gone == nullptr)) break;
-                if (n >= 4 && watch(gone, gone != nullptr, tag)) break;
             }
-            ss = warp_sum(ss);
-            if (lane == 0) sm.inv_rms[m] = 1.0f / sqrtf(ss / (float)a.D + a.eps);
+            if (__all_sync(0xffffffffu, !gone)) break;
+            if (__any_sync(0xffffffffu, tired(n, WAIT_LOOKS))) break;
+        }
+#pragma unroll
+        for (int i = 0; i < ROWS; i++) {
+            const float sum = warp_sum(ss[i]);
+            if (lane == 0 && helper + i * HELPERS < MAX_ROWS) sm.inv_rms[helper + i * HELPERS] = 1.0f / sqrtf(sum / (float)a.D + a.eps);
         }
         sync_norm();                                     // (a wait, not an arrival: a helper without rows must not run ahead)
     }
@@ -372,6 +385,7 @@ struct Worker {
     // The stream as the step's embedding left it: every owner publishes its columns.
     __device__ __forceinline__ void first_stream(const void* gain, uint32_t tag) {
         const int n_out = my_units(a.D / UR) * MAX_ROWS * UR;
+#pragma unroll 1
         for (int i0 = 0; i0 < n_out; i0 += CONSUMERS) {
             const int i = i0 + tid, m = (i / UR) % MAX_ROWS, n = (blockIdx.x + i / (MAX_ROWS * UR) * gridDim.x) * UR + i % UR;
             const bool on = i < n_out && row_in_use(m);
@@ -440,7 +454,7 @@ struct Worker {
                     for (int i = 0; i < MAX_ROWS; i++)
                         if (!has_tag(v[i][0], q.tag) || !has_tag(v[i][1], q.tag)) gone = i;
                     if (__all_sync(0xffffffffu, gone < 0)) break;
-                    if (n >= 3) {
+                    if (n >= 2) {                        // (looking on with all lanes slows the others' copies down)
                         const uint64_t* p = gone >= 0 ? staged(q, ks0, gone) : nullptr;
                         if (gone >= 0 && has_tag(peek(p), q.tag)) p++;
                         if (watch(p, gone >= 0, q.tag)) break;
@@ -606,6 +620,7 @@ struct Worker {
                 SyncGroup::sync();
             }
             if (sub == 0 && h < G) {
+#pragma unroll 1
                 for (int p = 1; p < wph; p++)
 #pragma unroll
                     for (int d = 0; d < DL; d++) o[d] += part[(lw + p) * HD + lane * DL + d];
@@ -691,6 +706,7 @@ struct Worker {
                 if (mend) {
                     // what a page holds outside the visible range may be anything: value rows that meet a probability of zero
                     // are cleared (scores of such keys are replaced, not multiplied)
+#pragma unroll 1
                     for (int c = lane; c < 16 * (HD / 8); c += 32) {
                         const int row = lw * 16 + c / (HD / 8);
                         if (row < k_first || row > k_last) *reinterpret_cast<uint4*>(vt + TileTma<HD>::off(row, c % (HD / 8))) = make_uint4(0, 0, 0, 0);
@@ -902,8 +918,9 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
 #pragma unroll 1
             for (int l = 0; l < a.L; l++) {
                 const uint32_t t1 = base + 2 * l + 1;
-                if (my_units(NQ / UR) > 0) c.row_scales(warp - CWARPS - 1, t1);
-                if (my_units(a.F / UR) > 0) c.row_scales(warp - CWARPS - 1, t1 + 1);
+#pragma unroll 1
+                for (int i = 0; i < 2; i++)
+                    if (my_units((i == 0 ? NQ : a.F) / UR) > 0) c.row_scales(warp - CWARPS - 1, t1 + i);
             }
         } else {
             c.first_stream(sm.layers[0].gain1, base + 1);

@@ -21,9 +21,9 @@ KERNEL_ROWS = 8         # rows that the kernel takes at most
 # Rows up to which a step takes the one launch. 0: never.
 MAX_ROWS = 8
 # And rows times the widest product's columns: every CTA reads all of a product's rows, twice their size with the tags. One launch
-# against the layers one by one, ms a step: 0.6B shape (3,072 columns) 1 row 0.59 / 0.87, 3 rows 0.80 / 1.01, 8 rows 0.89 / 1.01;
-# 4B shape's first 8 layers (9,728 columns) 1 row 0.60 / 0.80, 4 rows 0.68 / 0.69, 8 rows 0.83 / 0.75.
-MAX_ROW_COLUMNS = 40000
+# against the layers one by one, ms a step: 0.6B shape (3,072 columns) 1 row 0.50 / 0.87, 3 rows 0.66 / 1.01, 8 rows 0.76 / 1.01;
+# 4B shape's first 8 layers (9,728 columns) 1 row 0.56 / 0.80, 4 rows 0.60 / 0.70, 8 rows 0.68 / 0.75. Wider ones are not measured.
+MAX_ROW_COLUMNS = 8 * 9728
 
 
 class DecodeLayers:
