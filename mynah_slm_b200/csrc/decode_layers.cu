@@ -82,11 +82,12 @@ struct StepMaps {
 };
 
 // a job's place to work
+constexpr int HEADS = 8;                                 // query heads per kv head at most: the columns of a product
 constexpr int CHUNK = 2;                                 // heads whose outputs the four warps add at a time
 template <int HD> struct alignas(16) AttnWork {
-    bf16 q[MAX_G * (HD + 8)];                            // the group's queries
+    bf16 q[HEADS * (HD + 8)];                            // the group's queries
     float o[4][CHUNK][HD];                               // the warps' outputs, and the merge's sums
-    float m[4][MAX_G], l[4][MAX_G];
+    float m[4][HEADS], l[4][HEADS];
 };
 constexpr int STAGE_PITCH = KW * 2 + 16;                 // bytes of a staged row: eight rows' pieces of 16 bytes in different banks
 
@@ -106,6 +107,11 @@ struct Smem {
     int abort;
 };
 
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t r) {       // of 16-bit elements, two a lane
+    uint32_t t;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(t) : "r"(r));
+    return t;
+}
 struct SyncGroup {
     static __device__ __forceinline__ void sync() { asm volatile("bar.sync %0, 128;" ::"r"(1 + (int)(threadIdx.x >> 7)) : "memory"); }
 };
@@ -542,7 +548,7 @@ struct Worker {
     // The n runs of one (sequence, kv head), by the four warps of a group: out[h] = sum_s w_s o_s / sum_s w_s l_s with
     // w_s = 2^(m_s - m). 4 / G warps a head (at least one), each adds every so many-th run; their sums are added in order.
     __device__ __forceinline__ void merge(AttnWork<HD>& w, int b, int g, int n, uint32_t tag) {
-        constexpr int DL = HD / 32, BATCH = 4;           // a lane's columns; runs whose rows are under way together
+        constexpr int DL = HD / 32, BATCH = 8;           // a lane's columns; runs whose rows are under way together
         const int G = a.H / a.KV, lw = warp & 3;
         const int wph = G >= 3 ? 1 : 4 / G, hpt = 4 / wph, sub = lw % wph;       // warps a head, heads in one turn
 #pragma unroll 1
@@ -634,7 +640,7 @@ struct Worker {
     }
 
     __device__ __forceinline__ void attention(const LayerDesc& d, uint32_t tag) {
-        constexpr int KSTEPS = HD / 16, NT = HD / 8, QLD = HD + 8;
+        constexpr int KSTEPS = HD / 16, NT = HD / 16, QLD = HD + 8;
         constexpr int LPH = HeadLanes<HD>::LPH, HPW = HeadLanes<HD>::HPW;
         const int grp = (int)d.group, J = sm.cum[grp][a.M], G = a.H / a.KV, window = a.window[grp];
         const int j0 = first_job(J, blockIdx.x), j1 = first_job(J, blockIdx.x + 1);
@@ -691,7 +697,7 @@ struct Worker {
             }
             if (fresh) SyncGroup::sync();
             // ---- the run's pages: this warp's 16 keys of each
-            const uint32_t q32 = tc5::smem_u32(w.q) + ((lane & 15) * QLD + (lane >> 4) * 8) * 2;
+            const uint32_t q32 = tc5::smem_u32(w.q) + rr * QLD * 2 + mat * 16;
             float oc[NT][4] = {}, m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll 1
             for (int i = 0; i < job.n; i++, it += 2) {
@@ -718,31 +724,33 @@ struct Worker {
                     __syncwarp();
                 }
                 if (!empty) {
-                    float sc[2][4] = {};                 // heads lane / 4 (+ 8 in elements 2, 3), keys 16 lw + 8 t + (lane % 4) * 2 + {0, 1}
+                    // keys times queries: the warp's 16 keys are the rows, the heads the columns (those beyond the group's hold
+                    // whatever is there); element e: key 16 lw + lane / 4 (+ 8 from e = 2 on), head (lane % 4) * 2 + e % 2
+                    float sc[2][4] = {};
                     const uint32_t kb32 = tc5::smem_u32(kt), vb32 = tc5::smem_u32(vt);
 #pragma unroll
-                    for (int ks = 0; ks < KSTEPS; ks++) {
-                        uint32_t qa[4], kb[4];           // (query rows beyond the group's heads: whatever is there)
-                        ldmatrix_x4(qa, q32 + ks * 32);
-                        ldmatrix_x4(kb, kb32 + TileTma<HD>::off(lw * 16 + (mat >> 1) * 8 + rr, ks * 2 + (mat & 1)));
-                        mma_bf16(sc[0], qa, kb[0], kb[1]);
-                        mma_bf16(sc[1], qa, kb[2], kb[3]);
+                    for (int ks = 0; ks < KSTEPS; ks += 2) {
+                        uint32_t qb[4], k0[4], k1[4];
+                        ldmatrix_x4(qb, q32 + ks * 32);
+                        ldmatrix_x4(k0, kb32 + TileTma<HD>::off(lw * 16 + (mat & 1) * 8 + rr, ks * 2 + (mat >> 1)));
+                        ldmatrix_x4(k1, kb32 + TileTma<HD>::off(lw * 16 + (mat & 1) * 8 + rr, ks * 2 + 2 + (mat >> 1)));
+                        mma_bf16(sc[0], k0, qb[0], qb[1]);
+                        mma_bf16(sc[1], k1, qb[2], qb[3]);
                     }
                     float top[2] = {-INFINITY, -INFINITY};
 #pragma unroll
-                    for (int t = 0; t < 2; t++)
-#pragma unroll
-                        for (int e = 0; e < 4; e++) {
-                            const int key = lw * 16 + t * 8 + (lane & 3) * 2 + (e & 1);
-                            sc[t][e] = key >= k_first && key <= k_last ? sc[t][e] * a.scale : -INFINITY;
-                            top[e >> 1] = fmaxf(top[e >> 1], sc[t][e]);
-                        }
+                    for (int e = 0; e < 4; e++) {
+                        const int key = lw * 16 + (lane >> 2) + (e >> 1) * 8;
+                        sc[0][e] = key >= k_first && key <= k_last ? (sc[0][e] + sc[1][e]) * a.scale : -INFINITY;
+                        top[e & 1] = fmaxf(top[e & 1], sc[0][e]);
+                    }
                     float shrink[2];
 #pragma unroll
                     for (int e = 0; e < 2; e++) {
-                        top[e] = fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 1));
-                        top[e] = fmaxf(m[e], fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 2)));
-                        shrink[e] = m[e] == top[e] ? 1.0f : exp2f(m[e] - top[e]);         // (nothing seen yet: 2^-inf = 0, of zeros)
+                        top[e] = fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 4));
+                        top[e] = fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 8));
+                        top[e] = fmaxf(m[e], fmaxf(top[e], __shfl_xor_sync(0xffffffffu, top[e], 16)));
+                        shrink[e] = m[e] == top[e] ? 1.0f : exp2f(m[e] - top[e]);        // (nothing seen yet: 2^-inf = 0, of zeros)
                         m[e] = top[e];
                         l[e] *= shrink[e];
                         if (top[e] == -INFINITY) top[e] = 0.f;       // no key of this warp is visible: every probability is 0
@@ -751,23 +759,23 @@ struct Worker {
 #pragma unroll
                         for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-                            for (int e = 0; e < 4; e++) oc[nt][e] *= shrink[e >> 1];
+                            for (int e = 0; e < 4; e++) oc[nt][e] *= shrink[e & 1];
                     }
-                    uint32_t pa[4];                      // probabilities: fp32 for the sum, bf16 for the product
+                    // probabilities: fp32 for the sum, bf16 and transposed (a head's keys in a row) for the product
+                    uint32_t pr[2];
 #pragma unroll
-                    for (int t = 0; t < 2; t++)
+                    for (int t = 0; t < 2; t++) {
+                        const float u0 = exp2f(sc[0][2 * t] - top[0]), u1 = exp2f(sc[0][2 * t + 1] - top[1]);
+                        l[0] += u0;
+                        l[1] += u1;
+                        pr[t] = transpose8x8(pack2(u0, u1));
+                    }
+                    // values (transposed as they are loaded) times probabilities: 16 columns of the heads a product
 #pragma unroll
-                        for (int e = 0; e < 2; e++) {
-                            const float u0 = exp2f(sc[t][2 * e] - top[e]), u1 = exp2f(sc[t][2 * e + 1] - top[e]);
-                            l[e] += u0 + u1;
-                            pa[t * 2 + e] = pack2(u0, u1);
-                        }
-#pragma unroll
-                    for (int nt = 0; nt < NT; nt += 2) {
-                        uint32_t vb[4];
-                        ldmatrix_x4_trans(vb, vb32 + TileTma<HD>::off(lw * 16 + (mat & 1) * 8 + rr, nt + (mat >> 1)));
-                        mma_bf16(oc[nt], pa, vb[0], vb[1]);
-                        mma_bf16(oc[nt + 1], pa, vb[2], vb[3]);
+                    for (int nt = 0; nt < NT; nt++) {
+                        uint32_t va[4];
+                        ldmatrix_x4_trans(va, vb32 + TileTma<HD>::off(lw * 16 + (mat >> 1) * 8 + rr, nt * 2 + (mat & 1)));
+                        mma_bf16(oc[nt], va, pr[0], pr[1]);
                     }
                 }
                 if (mend) tc5::fence_async_smem();       // before a copy fills the slots again
@@ -781,24 +789,22 @@ struct Worker {
             // ---- the four warps' shares together, CHUNK heads at a time
 #pragma unroll
             for (int e = 0; e < 2; e++) {
-                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 1);
-                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 2);
-                if ((lane & 3) == 0) {
-                    w.m[lw][(lane >> 2) + 8 * e] = m[e];
-                    w.l[lw][(lane >> 2) + 8 * e] = l[e];
+                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 4);
+                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 8);
+                l[e] += __shfl_xor_sync(0xffffffffu, l[e], 16);
+                if (lane < 4) {
+                    w.m[lw][lane * 2 + e] = m[e];
+                    w.l[lw][lane * 2 + e] = l[e];
                 }
             }
             const size_t row0 = ((size_t)job.b * a.H + (size_t)job.g * G) * a.S + job.r;
 #pragma unroll 1
             for (int h0 = 0; h0 < G; h0 += CHUNK) {
+                if ((lane & 3) == h0 / CHUNK) {
 #pragma unroll
-                for (int e = 0; e < 2; e++) {
-                    const int h = (lane >> 2) + 8 * e - h0;
-                    if (h >= 0 && h < CHUNK) {
+                    for (int nt = 0; nt < NT; nt++)
 #pragma unroll
-                        for (int nt = 0; nt < NT; nt++)
-                            *reinterpret_cast<float2*>(&w.o[lw][h][nt * 8 + (lane & 3) * 2]) = make_float2(oc[nt][2 * e], oc[nt][2 * e + 1]);
-                    }
+                        for (int e = 0; e < 4; e++) w.o[lw][e & 1][nt * 16 + (e >> 1) * 8 + (lane >> 2)] = oc[nt][e];
                 }
                 SyncGroup::sync();
                 const int hc = ltid / (HD / 2), h = h0 + hc, c = ltid % (HD / 2) * 2;
@@ -999,7 +1005,7 @@ int weight_map(CUtensorMap* map, const void* base, long long rows, int K) {
 MYNAH_API int mynah_decode_layers_supported(int M, int D, int H, int KV, int HD, int F, int L, int n_groups) {
     if (M < 1 || M > MAX_ROWS || L < 1 || L > MAX_LAYERS || n_groups < 1 || n_groups > MAX_GROUPS) return 0;
     if (HD != 64 && HD != 128) return 0;
-    if (KV < 1 || KV > 255 || H < 1 || H % KV != 0 || H / KV > MAX_G) return 0;
+    if (KV < 1 || KV > 255 || H < 1 || H % KV != 0 || H / KV > HEADS) return 0;
     if (D < 64 || F < 64 || D % 64 != 0 || F % 64 != 0) return 0;
     return 1;
 }

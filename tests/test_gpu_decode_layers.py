@@ -20,12 +20,12 @@ def _cfg(layers, hidden, heads, kv, dim, ffn, window=None):
 
 # one sequence of a single page and several rows that are not a power of two; pages that end where the step begins or ends
 # (63 -> 64 -> 65); more units a CTA than are summed at a time (feed-forwards of 8,192); columns that are no multiple of a
-# slot's 1,024 or of a warp's 128; groups of 1, 2, 3, 4 and 16 query heads; windows shorter than a page and longer; more page
+# slot's 1,024 or of a warp's 128; groups of 1, 2, 3, 4 and 8 query heads; windows shorter than a page and longer; more page
 # jobs a CTA than its table holds is beyond a test's memory: 17 kv heads of 64 with 700 positions come to 1.4 a CTA
 CASES = [
     (_cfg(2, 64, 1, 1, 64, 64), [5]),
     (_cfg(2, 192, 6, 2, 64, 320), [63, 1, 130]),
-    (_cfg(3, 1088, 16, 1, 64, 1216), [64, 3, 700, 65, 128, 62, 191]),
+    (_cfg(3, 1088, 8, 1, 64, 1216), [64, 3, 700, 65, 128, 62, 191]),
     (_cfg(2, 1024, 16, 8, 128, 3072), [62, 126, 500, 1, 1000, 333, 64, 129]),
     (_cfg(2, 2560, 8, 2, 128, 8192), [200, 31]),
     (_cfg(3, 256, 4, 4, 128, 8192, window=20), [300, 19, 70]),
