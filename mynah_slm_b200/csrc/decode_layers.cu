@@ -64,7 +64,7 @@ struct StepArgs {
     int run;                                             // pages of a job
     int lg_rows;                                         // M, rounded up to a power of two: its logarithm
     int gain_dtype, qk_dtype, n_pos;
-    float eps, qk_eps, scale;
+    float eps, qk_eps, scale, inv_d;                     // inv_d: 1 / D
     int window[MAX_GROUPS];
     PageTable pt[MAX_GROUPS];
     const LayerDesc* layers;
@@ -343,9 +343,11 @@ struct Worker {
     __device__ __forceinline__ void row_scales(int helper, uint32_t tag) {
         constexpr int ROWS = (MAX_ROWS + HELPERS - 1) / HELPERS;
         float ss[ROWS];
+        // (What runs between the last share's arrival and the barrier keeps everybody waiting, and after the attention its code
+        // comes from far away: it is kept short.)
         watch(a.squares + (size_t)helper * (a.D / UR), lane == 0 && row_in_use(helper), tag);
         for (uint32_t n = 0;; n++) {
-            bool gone = false;
+            uint32_t gone = 0;
 #pragma unroll
             for (int i = 0; i < ROWS; i++) ss[i] = 0.f;
 #pragma unroll 1
@@ -353,25 +355,32 @@ struct Worker {
 #pragma unroll
                 for (int i = 0; i < ROWS; i++) {
                     if (!row_in_use(helper + i * HELPERS)) continue;
-                    const uint64_t* p = a.squares + (size_t)(helper + i * HELPERS) * (a.D / UR) + u;
+                    const uint64_t* p = a.squares + (uint32_t)((helper + i * HELPERS) * (a.D / UR) + u);
                     uint64_t v[4];
                     peek2(p, v[0], v[1]);
                     peek2(p + 2, v[2], v[3]);
 #pragma unroll
                     for (int e = 0; e < 4; e++) {
-                        gone = gone || !has_tag(v[e], tag);
+                        gone |= (uint32_t)(v[e] >> 32) ^ tag;
                         ss[i] += __uint_as_float((uint32_t)v[e]);
                     }
                 }
             }
-            if (__all_sync(0xffffffffu, !gone)) break;
+            if (__all_sync(0xffffffffu, gone == 0)) break;
             if (__any_sync(0xffffffffu, tired(n, WAIT_LOOKS))) break;
         }
 #pragma unroll
-        for (int i = 0; i < ROWS; i++) {
-            const float sum = warp_sum(ss[i]);
-            if (lane == 0 && helper + i * HELPERS < MAX_ROWS) sm.inv_rms[helper + i * HELPERS] = 1.0f / sqrtf(sum / (float)a.D + a.eps);
-        }
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int i = 0; i < ROWS; i++) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
+        // lane i takes the helper's row i; 1 / sqrt by the hardware's estimate and one Newton step
+        float x = ss[0];
+#pragma unroll
+        for (int i = 1; i < ROWS; i++) x = lane == i ? ss[i] : x;
+        x = fmaf(x, a.inv_d, a.eps);
+        float y = rsqrtf(x);
+        y = fmaf(0.5f * y, fmaf(-x * y, y, 1.0f), y);
+        if (lane < ROWS && row_in_use(helper + lane * HELPERS)) sm.inv_rms[helper + lane * HELPERS] = y;
         sync_norm();                                     // (a wait, not an arrival: a helper without rows must not run ahead)
     }
 
@@ -1025,7 +1034,7 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     StepArgs a = {};
     a.M = M; a.D = D; a.H = H; a.KV = KV; a.F = F; a.L = L; a.S = S;
     a.gain_dtype = gain_dtype; a.qk_dtype = qk_dtype; a.n_pos = n_pos;
-    a.eps = eps; a.qk_eps = qk_eps;
+    a.eps = eps; a.qk_eps = qk_eps; a.inv_d = 1.0f / (float)D;
     a.scale = (float)(1.4426950408889634 / sqrt((double)HD));        // probabilities are powers of two: score times log2(e)
     while ((1 << a.lg_rows) < M) a.lg_rows++;
     // Few sequences: short runs, so that more warps share a long one; many: longer ones, with fewer partial results to merge.
