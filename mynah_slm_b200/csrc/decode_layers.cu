@@ -43,6 +43,7 @@ constexpr int SLOT_BYTES = UR * KC * 2;                  // eight rows in blocks
 constexpr int SLOTS = 10;                                // as many as the rest leaves room for
 constexpr int TG = 6;                                    // units whose sums a warp holds at a time
 constexpr int MAX_LAYERS = 48, MAX_GROUPS = 4, MAX_ROWS = 8;
+constexpr int COPIES = 4, SQUARE_COPIES = 8;             // of what every CTA reads: see publish_pair
 constexpr uint32_t WAIT_LOOKS = 1u << 22;                // trips to L2 after which a wait is given up (a second and more)
 constexpr int RUN = 4;                                   // pages of a job at most
 constexpr int TABLE = 32;                                // jobs of a CTA that are looked up once for all layers
@@ -69,7 +70,7 @@ struct StepArgs {
     PageTable pt[MAX_GROUPS];
     const LayerDesc* layers;
     float* x;
-    uint64_t *hid, *squares, *qkv, *att, *act;           // tagged words: [rows][columns / 2], squares [rows][D / 8]
+    uint64_t *hid, *squares, *qkv, *att, *act;           // tagged words: [copies][rows][columns / 2], squares [copies][rows][D / 8]
     uint64_t *part_o, *part_ml;                          // pages' partial results, tagged: [rows][heads][S][HD], [..][2]
     unsigned* sync;                                      // [0] the last step's tag, [1] CTAs that have left
     const int* kv_len;
@@ -173,6 +174,26 @@ __device__ __forceinline__ bool has_tag(uint64_t v, uint32_t tag) { return (uint
 __device__ __forceinline__ uint32_t pack2(float lo, float hi) {
     const __nv_bfloat162 b = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<const uint32_t*>(&b);
+}
+
+// A word that every CTA reads is published in several copies, and a CTA reads copy number blockIdx modulo their count: 148 SMs
+// at one line of one L2 slice queue for it (a few rows are a few lines, and where these fell decided up to 25% of a step: 0.48
+// or 0.58 ms at one row on two GPUs).
+__device__ __forceinline__ void publish_copies(uint64_t* p, size_t copy, uint32_t data, uint32_t tag) {
+#pragma unroll
+    for (int i = 0; i < COPIES; i++) publish(p + i * copy, data, tag);
+}
+// The same of two neighbouring lanes' values, a lane half of the copies (copy 0: there is one only).
+__device__ __forceinline__ void publish_pair(uint64_t* p, size_t copy, bool on, float mine, float other, uint32_t tag) {
+    const bool odd = threadIdx.x & 1;
+    const uint32_t data = odd ? pack2(other, mine) : pack2(mine, other);
+    if (!on || (odd && copy == 0)) return;
+    p += odd ? copy : 0;
+    publish(p, data, tag);
+    if (copy != 0) {
+#pragma unroll
+        for (int i = 2; i < COPIES; i += 2) publish(p + i * copy, data, tag);
+    }
 }
 
 // ---------------------------------------------------------------- the producer warp
@@ -345,7 +366,8 @@ struct Worker {
         float ss[ROWS];
         // (What runs between the last share's arrival and the barrier keeps everybody waiting, and after the attention its code
         // comes from far away: it is kept short.)
-        watch(a.squares + (size_t)helper * (a.D / UR), lane == 0 && row_in_use(helper), tag);
+        const uint64_t* squares = a.squares + (size_t)(blockIdx.x % SQUARE_COPIES) * MAX_ROWS * (a.D / UR);
+        watch(squares + (size_t)helper * (a.D / UR), lane == 0 && row_in_use(helper), tag);
         for (uint32_t n = 0;; n++) {
             uint32_t gone = 0;
 #pragma unroll
@@ -355,7 +377,7 @@ struct Worker {
 #pragma unroll
                 for (int i = 0; i < ROWS; i++) {
                     if (!row_in_use(helper + i * HELPERS)) continue;
-                    const uint64_t* p = a.squares + (uint32_t)((helper + i * HELPERS) * (a.D / UR) + u);
+                    const uint64_t* p = squares + (uint32_t)((helper + i * HELPERS) * (a.D / UR) + u);
                     uint64_t v[4];
                     peek2(p, v[0], v[1]);
                     peek2(p + 2, v[2], v[3]);
@@ -387,14 +409,14 @@ struct Worker {
     // The owner's new values of the stream for the next norm: x times the gain in bf16 (pairs of neighbouring lanes) and the
     // squares of a unit's eight columns (lanes of one row). All lanes of a warp call it.
     __device__ __forceinline__ void publish_stream(bool on, float x, float gain, int m, int n, uint32_t tag) {
-        const float y = x * gain, y1 = __shfl_down_sync(0xffffffffu, y, 1);
+        const float y = x * gain, other = __shfl_xor_sync(0xffffffffu, y, 1);
         float q = x * x;
         q += __shfl_xor_sync(0xffffffffu, q, 1);
         q += __shfl_xor_sync(0xffffffffu, q, 2);
         q += __shfl_xor_sync(0xffffffffu, q, 4);
-        if (!on) return;
-        if ((lane & 1) == 0) publish(a.hid + ((size_t)m * a.D + n) / 2, pack2(y, y1), tag);
-        if ((lane & 7) == 0) publish(a.squares + ((size_t)m * a.D + n) / UR, __float_as_uint(q), tag);
+        publish_pair(a.hid + ((uint32_t)(m * a.D + n) >> 1), (size_t)MAX_ROWS * (a.D / 2), on, y, other, tag);
+        static_assert(SQUARE_COPIES == UR, "a lane a copy");
+        if (on) publish(a.squares + (uint32_t)(((lane & 7) * MAX_ROWS + m) * (a.D / UR) + n / UR), __float_as_uint(q), tag);
     }
 
     // The stream as the step's embedding left it: every owner publishes its columns.
@@ -416,7 +438,8 @@ struct Worker {
         int n_units, K;
         bool normed;                                     // the sums are scaled by the row's 1 / rms
         Result res;
-        uint64_t* dst;                                   // tagged rows of width ld; ADD_TO_STREAM: the stream, published
+        uint64_t* dst;                                   // tagged rows of width ld, `copy` words from copy to copy (0: one
+        size_t copy;                                     // copy); ADD_TO_STREAM: the stream, published
         int ld;                                          // with `gain` unless that is null
         const void* gain;
         uint32_t next;                                   // the tag of what comes out
@@ -547,8 +570,8 @@ struct Worker {
                     if (q.gain != nullptr) publish_stream(on, x, gn, om, n, q.next);
                 } else {
                     if (per == 2) s = s / (1.0f + expf(-s)) * s2;
-                    const float y1 = __shfl_down_sync(0xffffffffu, s, 1);
-                    if (on && (lane & 1) == 0) publish(q.dst + ((size_t)om * q.ld + n) / 2, pack2(s, y1), q.next);
+                    const float other = __shfl_xor_sync(0xffffffffu, s, 1);
+                    publish_pair(q.dst + ((uint32_t)(om * q.ld + n) >> 1), q.copy, on, s, other, q.next);
                 }
             }
         }
@@ -642,7 +665,7 @@ struct Worker {
                 const float inv = lsum > 0.f ? 1.0f / lsum : 0.f;
                 uint64_t* dst = a.att + ((size_t)b * a.H * HD + (size_t)(g * G + h) * HD + lane * DL) / 2;
 #pragma unroll
-                for (int d = 0; d < DL; d += 2) publish(dst + d / 2, pack2(o[d] * inv, o[d + 1] * inv), tag);
+                for (int d = 0; d < DL; d += 2) publish_copies(dst + d / 2, (size_t)MAX_ROWS * (a.H * HD / 2), pack2(o[d] * inv, o[d + 1] * inv), tag);
             }
         }
         SyncGroup::sync();
@@ -830,7 +853,8 @@ struct Worker {
                     }
                     if (runs == 1) {                     // all that the sequence sees: finished
                         const float inv = sum > 0.f ? 1.0f / sum : 0.f;
-                        publish(a.att + ((size_t)job.b * a.H * HD + (size_t)(job.g * G + h) * HD + c) / 2, pack2(o0 * inv, o1 * inv), tag);
+                        publish_copies(a.att + ((size_t)job.b * a.H * HD + (size_t)(job.g * G + h) * HD + c) / 2, (size_t)MAX_ROWS * (a.H * HD / 2),
+                                       pack2(o0 * inv, o1 * inv), tag);
                     } else {
                         const size_t row = row0 + (size_t)h * a.S;
                         publish2(a.part_o + row * HD + c, __float_as_uint(o0), __float_as_uint(o1), tag);
@@ -947,12 +971,14 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
                 for (int i = 0; i < 4; i++) {
                     typename Worker<HD>::Product q;
                     q.src = i == 1 ? a.att : (i == 3 ? a.act : a.hid);
+                    q.src += (size_t)(blockIdx.x % COPIES) * MAX_ROWS * ((i == 1 ? NO : (i == 3 ? a.F : a.D)) / 2);
                     q.tag = i < 2 ? t1 : t2;
                     q.n_units = (i == 0 ? NQ : (i == 2 ? a.F : a.D)) / UR;
                     q.K = i == 1 ? NO : (i == 3 ? a.F : a.D);
                     q.normed = i % 2 == 0;
                     q.res = i == 0 ? TO_BF16 : (i == 2 ? TO_SWIGLU : ADD_TO_STREAM);
                     q.dst = i == 0 ? a.qkv : a.act;
+                    q.copy = i == 0 ? 0 : (size_t)MAX_ROWS * (a.F / 2);          // (the queries, keys and values of a head have few readers)
                     q.ld = i == 0 ? NQ : a.F;
                     q.gain = i == 1 ? d.gain2 : (l + 1 < a.L ? sm.layers[l + 1].gain1 : nullptr);
                     q.next = i == 0 ? t1 : (i == 3 ? t2 + 1 : t2);
@@ -1021,7 +1047,7 @@ MYNAH_API int mynah_decode_layers_supported(int M, int D, int H, int KV, int HD,
 
 // One decode step through all layers. layers: L descriptors of 96 bytes on the device; host_layers: the same on the host.
 // Per cache group (n_groups of them) eight words: k and v bases, their rows (entries * pages * kv heads * 64), window, and the
-// page lists. words: 64-bit words for 8 rows of D / 2 + D / 8 + ((H + 2 KV) HD + H HD + F) / 2; part: 64-bit words for
+// page lists. words: 64-bit words for 8 rows of 4 (D + H HD + F) / 2 + D + (H + 2 KV) HD / 2; part: 64-bit words for
 // 8 * H * S * (HD + 2); sync: two 32-bit words. All three zero before the first launch and kept from step to step.
 MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, int L, int M, int D, int H, int KV, int HD, int F, int S,
                                   float* x, void* words, void* part, unsigned* sync,
@@ -1042,10 +1068,10 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     a.layers = static_cast<const LayerDesc*>(layers);
     a.x = x;
     a.hid = static_cast<uint64_t*>(words);
-    a.squares = a.hid + (size_t)MAX_ROWS * (D / 2);
-    a.qkv = a.squares + (size_t)MAX_ROWS * (D / UR);
+    a.squares = a.hid + (size_t)COPIES * MAX_ROWS * (D / 2);
+    a.qkv = a.squares + (size_t)SQUARE_COPIES * MAX_ROWS * (D / UR);
     a.att = a.qkv + (size_t)MAX_ROWS * ((H + 2 * KV) * HD / 2);
-    a.act = a.att + (size_t)MAX_ROWS * (H * HD / 2);
+    a.act = a.att + (size_t)COPIES * MAX_ROWS * (H * HD / 2);
     a.part_o = static_cast<uint64_t*>(part);
     a.part_ml = a.part_o + (size_t)MAX_ROWS * H * S * HD;
     a.sync = sync; a.kv_len = kv_len;

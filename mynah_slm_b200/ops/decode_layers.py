@@ -33,7 +33,7 @@ class DecodeLayers:
         self.sizes = sizes
         self.groups = groups                       # (K cache, V cache, window) of every storage group
         z = sizes
-        self.words = torch.zeros((KERNEL_ROWS * (z["D"] // 2 + z["D"] // 8 + ((z["H"] + z["KV"]) * z["HD"] * 2 + z["F"]) // 2),),
+        self.words = torch.zeros((KERNEL_ROWS * (2 * (z["D"] + z["H"] * z["HD"] + z["F"]) + z["D"] + (z["H"] + 2 * z["KV"]) * z["HD"] // 2),),
                                  dtype=torch.int64, device=device)
         self.sync = torch.zeros((2,), dtype=torch.int32, device=device)
         self.part: Optional[torch.Tensor] = None
