@@ -49,7 +49,7 @@ constexpr int RUN = 4;                                   // pages of a job at mo
 constexpr int TABLE = 32;                                // jobs of a CTA that are looked up once for all layers
 constexpr int BAR_ALL = 5, BAR_NORM = 6;                 // named barriers of the eight warps, and with the helpers (1, 2: a page's four warps)
 static_assert(KEYS * 128 * 2 <= SLOT_BYTES && KW % 64 == 0, "a slot holds either kind of tile; a warp takes whole blocks of columns");
-static_assert(SLOTS > 2 * RUN, "a warp that passes over the other group's job has seen a filling of every slot since the one before");
+static_assert(SLOTS >= TG, "what is waited for together fits the ring");
 
 struct LayerDesc {                                       // as the host lays them out: 12 words of 64 bits
     const bf16 *w_qkv, *w_o, *w_gu, *w_down;
@@ -102,6 +102,7 @@ struct Smem {
     int table[MAX_GROUPS][TABLE];                        // a job's sequence, kv head and run
     int pages[MAX_GROUPS][TABLE][RUN];                   // the places of its pages, -1: none
     unsigned long long full[SLOTS], empty[SLOTS];
+    uint32_t issued;                                     // fillings that the producer has come to: see page_is_full
     int pg0[MAX_GROUPS][MAX_ROWS], cnt[MAX_GROUPS][MAX_ROWS], cum[MAX_GROUPS][MAX_ROWS + 1];   // pages seen by a sequence, jobs before it
     float inv_rms[MAX_ROWS];
     int hi[MAX_ROWS];
@@ -254,6 +255,7 @@ struct Producer {
                         } else {
                             tc5::mbar_arrive(bar);       // a page that is not there: the slot keeps its turn
                         }
+                        asm volatile("st.release.cta.shared.u32 [%0], %1;" ::"r"(tc5::smem_u32(&sm.issued)), "r"(it + 1) : "memory");
                     }
                     __syncwarp();
                 }
@@ -303,11 +305,23 @@ struct Worker {
             : "=r"(done) : "r"(tc5::smem_u32(&sm.full[i % SLOTS])), "r"((i / SLOTS) & 1) : "memory");
         return done != 0;
     }
+    // A barrier's parity tells a filling from the next one, not from the one before: it may be asked only by those who know that
+    // the one before is complete. In the products every warp has seen every filling. Among pages a group passes over the other's
+    // fillings (which may be still on their way when its own, asked for later, have come), so it first looks whether the producer
+    // has come to filling i: the producer has by then seen the slot's last filling read and handed back. (The filling after i
+    // cannot come before this group has handed i back. To look at the other group's fillings as well would not do: they may be
+    // two fillings past by then.)
+    __device__ __forceinline__ bool page_is_full(uint32_t i) const {
+        uint32_t n;
+        asm volatile("ld.acquire.cta.shared.u32 %0, [%1];" : "=r"(n) : "r"(tc5::smem_u32(&sm.issued)) : "memory");
+        return n > i && is_full(i);
+    }
     // Until the n slots from number i on are full; a lane looks after a slot (a look may take a hardware wait of its own, so this
     // limit is a clock, not a count).
+    template <bool PAGES = false>
     __device__ __forceinline__ void wait_full(uint32_t i, int n) {
         unsigned long long t0 = 0;
-        while (!__all_sync(0xffffffffu, lane >= n || is_full(i + lane))) {
+        while (!__all_sync(0xffffffffu, lane >= n || (PAGES ? page_is_full(i + lane) : is_full(i + lane)))) {
             const unsigned long long now = tc5::now_ns();
             if (t0 == 0) t0 = now;
             else if (now - t0 > tc5::WAIT_LIMIT_NS) tired(~0u, 0);
@@ -739,7 +753,7 @@ struct Worker {
                 const int k_first = max(lo, p0) - p0, k_last = min(hi, p0 + PAGE_TOKENS) - 1 - p0;
                 const uint32_t ik = it % SLOTS, iv = (it + 1) % SLOTS;
                 unsigned char *kt = sm.slots[ik], *vt = sm.slots[iv];
-                wait_full(it, 2);
+                wait_full<true>(it, 2);
                 const bool mend = !empty && (lw * 16 < k_first || lw * 16 + 15 > k_last || i == i_new);      // uniform over the warp
                 if (mend) {
                     // what a page holds outside the visible range may be anything: value rows that meet a probability of zero
@@ -890,6 +904,7 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
             tc5::mbar_init(tc5::smem_u32(&sm.empty[i]), CWARPS);
         }
         sm.abort = 0;
+        sm.issued = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc5::fence_async_smem();
     }

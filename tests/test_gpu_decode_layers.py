@@ -20,8 +20,8 @@ def _cfg(layers, hidden, heads, kv, dim, ffn, window=None):
 
 # one sequence of a single page and several rows that are not a power of two; pages that end where the step begins or ends
 # (63 -> 64 -> 65); more units a CTA than are summed at a time (feed-forwards of 8,192); columns that are no multiple of a
-# slot's 1,024 or of a warp's 128; groups of 1, 2, 3, 4 and 8 query heads; windows shorter than a page and longer; more page
-# jobs a CTA than its table holds is beyond a test's memory: 17 kv heads of 64 with 700 positions come to 1.4 a CTA
+# slot's 1,024 or of a warp's 128; groups of 1, 2, 3, 4 and 8 query heads; windows shorter than a page and longer; 768 runs of
+# pages, five a CTA
 CASES = [
     (_cfg(2, 64, 1, 1, 64, 64), [5]),
     (_cfg(2, 192, 6, 2, 64, 320), [63, 1, 130]),
@@ -30,11 +30,15 @@ CASES = [
     (_cfg(2, 2560, 8, 2, 128, 8192), [200, 31]),
     (_cfg(3, 256, 4, 4, 128, 8192, window=20), [300, 19, 70]),
     (_cfg(3, 512, 34, 17, 64, 704, window=100), [700, 99, 101, 230]),
+    (_cfg(2, 512, 32, 32, 64, 512), [620, 610, 600, 590, 580, 570, 639, 560]),
 ]
+# And with few CTAs, so that each has several of everything: both groups of warps at work and passing over each other's pages, more
+# jobs than the table holds (102 on three CTAs), queries kept from job to job, several merges, units in several turns.
+FEW = [(1, 3), (2, 3), (2, 20), (3, 20), (5, 3), (6, 3), (6, 20), (7, 20)]
 
 
-@pytest.mark.parametrize("i", range(len(CASES)))
-def test_one_launch_a_step(tmp_path, i):
+@pytest.mark.parametrize("i,ctas", [(i, None) for i in range(len(CASES))] + FEW)
+def test_one_launch_a_step(tmp_path, i, ctas):
     from mynah_slm_b200.engine.engine import Engine, StepEntry
     cfg, lens = CASES[i]
     folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=i)
@@ -48,6 +52,8 @@ def test_one_launch_a_step(tmp_path, i):
     for one in (True, False):
         eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=room + 64, max_seqs=len(lens) + 1)
         assert eng.decode_layers is not None
+        if ctas is not None:
+            eng.runtime.sm_count = ctas
         took = []
         takes = eng.decode_layers.takes
         eng.decode_layers.takes = lambda ctx: took.append(takes(ctx) and one) or took[-1]
