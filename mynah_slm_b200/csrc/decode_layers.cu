@@ -910,15 +910,24 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
     }
     for (int i = tid; i < a.L * (int)(sizeof(LayerDesc) / 8); i += THREADS)
         reinterpret_cast<unsigned long long*>(sm.layers)[i] = reinterpret_cast<const unsigned long long*>(a.layers)[i];
-    if (tid < MAX_ROWS) sm.hi[tid] = tid < a.M ? a.kv_len[tid] : 0;
+    if (tid < MAX_ROWS) {
+        int hi = tid < a.M ? a.kv_len[tid] : 0;
+        // A row that sees more pages than the launch has splits for is reported and left alone, as a padding row is. (Without its
+        // last pages nobody would read its new key and value, and the waits count on everything being read.)
+        for (int g = 0; g < MAX_GROUPS; g++)
+            if (a.pt[g].ids != nullptr && visible_pages(hi, a.window[g], 0).count() > a.S) {
+                if (blockIdx.x == 0) atomicOr(a.status, MYNAH_ST_SPLIT_RANGE);
+                hi = 0;
+            }
+        sm.hi[tid] = hi;
+    }
     __syncthreads();
     if (tid < MAX_GROUPS) {                              // the pages that every sequence sees in each cache group
         int sum = 0;
         for (int b = 0; b < a.M; b++) {
             const VisiblePages vp = visible_pages(sm.hi[b], a.window[tid], 0);
-            if (vp.count() > a.S && blockIdx.x == 0 && a.pt[tid].ids != nullptr) atomicOr(a.status, MYNAH_ST_SPLIT_RANGE);
             sm.pg0[tid][b] = vp.pg0;
-            sm.cnt[tid][b] = min(vp.count(), a.S);
+            sm.cnt[tid][b] = vp.count();
             sm.cum[tid][b] = sum;
             sum += runs_of(sm.cnt[tid][b], a.run) * a.KV;
         }

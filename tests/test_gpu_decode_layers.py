@@ -77,3 +77,25 @@ def test_one_launch_a_step(tmp_path, i, ctas):
         for b, n in enumerate(lens):
             assert_close(refs[b][n + t][None], rows[True][t][b][None], BF16_REL, f"one launch, sequence {b}, step {t}")
             assert_close(refs[b][n + t][None], rows[False][t][b][None], BF16_REL, f"layer by layer, sequence {b}, step {t}")
+
+
+def test_a_row_beyond_the_splits_is_left_alone(tmp_path, monkeypatch):
+    """A sequence with more pages than the launch was given splits: reported at once, its neighbour as ever."""
+    from mynah_slm_b200.engine.engine import Engine, EngineError, StepEntry
+    cfg = _cfg(2, 256, 4, 2, 64, 320)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=3)
+    seqs = [np.random.default_rng(n).integers(0, cfg["vocab_size"], size=n + 1).tolist() for n in (300, 40)]
+    rows = []
+    for splits in (5, 1):
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=512, max_seqs=2, use_graphs=False)
+        slots = [eng.open_sequence() for _ in seqs]
+        eng.step([StepEntry(s, q[:-1], ()) for s, q in zip(slots, seqs)])
+        eng.check_status()
+        monkeypatch.setattr(Engine, "_decode_pages", staticmethod(lambda n, splits=splits: splits))
+        rows.append(eng.step([StepEntry(s, q[-1:], (0,)) for s, q in zip(slots, seqs)]).cpu().numpy()[1])
+        if splits == 5:
+            eng.check_status()
+        else:
+            with pytest.raises(EngineError, match="refused an index: a decode launch too small for a sequence$"):
+                eng.check_status()
+    assert np.array_equal(*rows)
