@@ -15,6 +15,7 @@ import torch
 
 from ..cache.pages import PAGE_TOKENS
 from . import lib
+from .kernels import _chk
 from .lib import KernelError, call, code, ptr, stream_ptr
 
 KERNEL_ROWS = 8         # rows that the kernel takes at most
@@ -115,6 +116,9 @@ class DecodeLayers:
     def forward(self, x: torch.Tensor, ctx, runtime) -> torch.Tensor:
         """The residual stream x [T, D] (fp32, updated in place) behind all layers."""
         z, M, S = self.sizes, ctx.T, ctx.decode_splits
+        _chk(x, "residual", torch.float32, 2)
+        if tuple(x.shape) != (M, z["D"]):
+            raise KernelError(f"decode_layers: the residual is {tuple(x.shape)}, the step has {(M, z['D'])}")
         words = []
         for (k, v, window), p in zip(self.groups, ctx.pages):
             words += [k.data_ptr(), v.data_ptr(), k.numel() // z["HD"], window, p.indptr.data_ptr(), p.ids.data_ptr(), p.base.data_ptr(), p.n_pages]

@@ -1,0 +1,56 @@
+"""The host's side of the one-launch decode step (ops/decode_layers.py), without a GPU."""
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from mynah_slm_b200.ops import decode_layers
+from mynah_slm_b200.ops.lib import KernelError
+
+
+class Rows:
+    """Stands for a tensor on the device."""
+    def __init__(self, shape, dtype=torch.float32, is_cuda=True, contiguous=True):
+        self.shape, self.dtype, self.is_cuda, self.contiguous = torch.Size(shape), dtype, is_cuda, contiguous
+
+    def is_contiguous(self):
+        return self.contiguous
+
+    def dim(self):
+        return len(self.shape)
+
+    def data_ptr(self):
+        return 0
+
+
+@pytest.fixture
+def steps(monkeypatch):
+    """A plan of two layers of 64 whose launches are noted instead of made."""
+    made = []
+    monkeypatch.setattr(decode_layers, "call", lambda name, *args: made.append((name, args)))
+    monkeypatch.setattr(decode_layers, "stream_ptr", lambda: 0)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    sizes = dict(D=64, H=1, KV=1, HD=64, F=64, eps=1e-6, qk_eps=1e-6, gain_dtype=0, qk_dtype=0, cos=None, sin=None)
+    cache = torch.zeros((2, 4, 1, 64, 64), dtype=torch.bfloat16)
+    plan = decode_layers.DecodeLayers([[0] * 12] * 2, sizes, [(cache, cache, 0)], torch.device("cpu"))
+    return plan, made
+
+
+def _ctx(rows, splits=1):
+    pages = SimpleNamespace(indptr=Rows([rows + 1]), ids=Rows([4]), base=Rows([rows]), n_pages=4)
+    return SimpleNamespace(T=rows, is_decode=True, decode_splits=splits, pages=[pages], kv_len=Rows([rows]), status=Rows([1]))
+
+
+RUNTIME = SimpleNamespace(sm_count=148)
+
+
+@pytest.mark.parametrize("x", [Rows([2, 64], torch.bfloat16), Rows([2, 64], is_cuda=False), Rows([2, 64], contiguous=False), Rows([128]),
+                               Rows([2, 32]), Rows([1, 64]), Rows([2, 128])])
+def test_other_rows_are_refused(steps, x):
+    """What an embedding returns is checked before the kernel writes to it."""
+    plan, made = steps
+    with pytest.raises(KernelError, match="residual"):
+        plan.forward(x, _ctx(2), RUNTIME)
+    assert not made
+    plan.forward(Rows([2, 64]), _ctx(2), RUNTIME)
+    assert [name for name, _ in made] == ["mynah_decode_layers"]
