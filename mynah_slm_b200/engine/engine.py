@@ -608,7 +608,10 @@ class Engine:
             g.graphs[mode] = (graph, res, n_kernels)
             replays -= 1
         graph, res, n_kernels = g.graphs[mode]
+        one_launch = self.decode_layers is not None and self.decode_layers.takes(g.ctx)
         for _ in range(replays):
+            if one_launch:
+                self.decode_layers.count_launch()
             graph.replay()
         lib.add_launches(n_kernels * replays)
         return res

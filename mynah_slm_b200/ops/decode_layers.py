@@ -28,6 +28,10 @@ MAX_ROW_COLUMNS = 8 * 9728
 
 
 class DecodeLayers:
+    # Tags that launches may use before the words are cleared and the tags begin again at 1: a tag names one stage of one launch as
+    # long as 32 bits do not wrap (74 million steps of 28 layers, ten hours of steps of 0.5 ms).
+    TAG_LIMIT = 2 ** 32 - 1
+
     def __init__(self, rows, sizes: dict, groups: list, device):
         self.host_table = torch.tensor(rows, dtype=torch.int64)                 # [layers, 12]
         self.table = self.host_table.to(device)
@@ -39,6 +43,7 @@ class DecodeLayers:
         self.sync = torch.zeros((2,), dtype=torch.int32, device=device)
         self.part: Optional[torch.Tensor] = None
         self._retired: list[torch.Tensor] = []     # outgrown buffers stay alive: a captured graph may still hold their address
+        self._tags = 0                             # tags used since the words were cleared
 
     @classmethod
     def plan(cls, model, cache, runtime) -> Optional["DecodeLayers"]:
@@ -103,6 +108,17 @@ class DecodeLayers:
         z = self.sizes
         return ctx.is_decode and ctx.T <= min(MAX_ROWS, KERNEL_ROWS) and ctx.T * max(z["D"], z["H"] * z["HD"], z["F"]) <= MAX_ROW_COLUMNS
 
+    def count_launch(self) -> None:
+        """To be called before every launch, replayed ones too, on the launch's stream: keeps the tags from wrapping, after which
+        words that were written long ago, or never, would pass for new ones."""
+        n = 2 * self.table.shape[0] + 2            # as the kernel moves its tags on
+        if self._tags + n > self.TAG_LIMIT:
+            for t in (self.sync, self.words, self.part, *self._retired):
+                if t is not None:
+                    t.zero_()
+            self._tags = 0
+        self._tags += n
+
     def _partials(self, splits: int) -> torch.Tensor:
         need = KERNEL_ROWS * self.sizes["H"] * splits * (self.sizes["HD"] + 2)
         if self.part is None or self.part.numel() < need:
@@ -123,6 +139,8 @@ class DecodeLayers:
         for (k, v, window), p in zip(self.groups, ctx.pages):
             words += [k.data_ptr(), v.data_ptr(), k.numel() // z["HD"], window, p.indptr.data_ptr(), p.ids.data_ptr(), p.base.data_ptr(), p.n_pages]
         cos, sin = z["cos"], z["sin"]
+        if not torch.cuda.is_current_stream_capturing():
+            self.count_launch()                    # (a recorded launch counts when it is replayed)
         call("mynah_decode_layers", ptr(self.table), ptr(self.host_table), self.table.shape[0], M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S,
              ptr(x), ptr(self.words), ptr(self._partials(S)), ptr(self.sync),
              z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,

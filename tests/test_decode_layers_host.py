@@ -54,3 +54,27 @@ def test_other_rows_are_refused(steps, x):
     assert not made
     plan.forward(Rows([2, 64]), _ctx(2), RUNTIME)
     assert [name for name, _ in made] == ["mynah_decode_layers"]
+
+
+def test_tags_begin_again_before_they_wrap(steps):
+    """Six tags a launch of two layers. Before a launch would pass the limit, everything that carries tags is cleared: the words,
+    the partial results at hand and those that an older captured step still uses, and the count in the kernel's own keeping."""
+    plan, made = steps
+    plan.TAG_LIMIT = 20
+    plan.forward(Rows([1, 64]), _ctx(1, splits=2), RUNTIME)
+    small = plan.part
+    plan.forward(Rows([1, 64]), _ctx(1, splits=64), RUNTIME)
+    assert plan.part is not small
+    tagged = (plan.sync, plan.words, plan.part, small)
+    for t in tagged:
+        t.fill_(7)
+    plan.forward(Rows([1, 64]), _ctx(1), RUNTIME)                    # tags 13 to 18
+    assert all(bool((t == 7).all()) for t in tagged)
+    plan.count_launch()                                              # 24 would be too many
+    assert not any(bool(t.any()) for t in tagged)
+    plan.sync.fill_(7)
+    plan.count_launch()
+    plan.count_launch()
+    assert bool((plan.sync == 7).all())
+    plan.count_launch()
+    assert not bool(plan.sync.any())

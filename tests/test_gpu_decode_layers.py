@@ -99,3 +99,25 @@ def test_a_row_beyond_the_splits_is_left_alone(tmp_path, monkeypatch):
             with pytest.raises(EngineError, match="refused an index: a decode launch too small for a sequence$"):
                 eng.check_status()
     assert np.array_equal(*rows)
+
+
+def test_tags_begin_again(tmp_path):
+    """Steps across the point where the tags begin again, captured, looped and launched: the same bits."""
+    from mynah_slm_b200.engine.engine import Engine, StepEntry
+    cfg = _cfg(2, 256, 4, 2, 64, 320)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=3)
+    toks = np.random.default_rng(0).integers(0, cfg["vocab_size"], size=330).tolist()
+    rows = []
+    for graphs, limit in ((True, None), (True, 20), (False, 20)):
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=512, max_seqs=2, use_graphs=graphs)
+        if limit is not None:
+            eng.decode_layers.TAG_LIMIT = limit                      # three launches of six tags
+        slot = eng.open_sequence()
+        eng.step([StepEntry(slot, toks[:310], ())])
+        rows.append([eng.step([StepEntry(slot, [t], (0,))]).cpu().numpy() for t in toks[310:]])
+        if graphs:
+            rows[-1].append(eng.decode_loop([slot], [5], 9).cpu().numpy())
+            assert (int(eng.decode_layers.sync[0]) <= 18) == (limit is not None)
+        eng.check_status()
+    for a, b in ((rows[0], rows[1]), (rows[0][:20], rows[2])):
+        assert len(a) == len(b) and all(np.array_equal(u, v) for u, v in zip(a, b))
