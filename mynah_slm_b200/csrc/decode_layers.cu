@@ -17,11 +17,11 @@
 // A product's unit is eight output rows of the weights: 1,024 outputs make 128 units, so the narrow products still use 128
 // SMs without splitting a sum across CTAs. Within the CTA every warp multiplies its 128 of a slot's 1,024 columns
 // (mma.sync m16n8k16, two units as the 16 rows, the step's rows as the 8 columns, fp32 sums) and the eight partial sums are
-// added in a fixed order. A row's bits do not depend on the other rows. Who owns a column of the residual stream publishes it
+// added in a fixed order. A row's bits do not depend on the other rows of the launch. Who owns a column of the residual stream publishes it
 // times the norm's gain, and its share of the row's squares; 1/rms is a factor on the finished sums.
 //
-// Attention's jobs are runs of up to four pages of a (sequence, kv head), cut by the sequence alone, four warps a job: each warp
-// keeps its own 16 keys of every page, with a running maximum, and meets the others once a run. The warps that have a
+// Attention's jobs are runs of two or four pages of a (sequence, kv head), cut by the sequence's own page count, four warps a job:
+// each warp keeps its own 16 keys of every page, with a running maximum, and meets the others once a run. The warps that have a
 // sequence's newest run merge all of its runs when their own jobs are done, in an order that depends on their number only.
 //
 // All CTAs must be resident at once: the launch is cooperative, and every wait is bounded (status bit 16). Registers: twelve
@@ -45,7 +45,12 @@ constexpr int TG = 6;                                    // units whose sums a w
 constexpr int MAX_LAYERS = 48, MAX_GROUPS = 4, MAX_ROWS = 8;
 constexpr int COPIES = 4, SQUARE_COPIES = 8;             // of what every CTA reads: see publish_pair
 constexpr uint32_t WAIT_LOOKS = 1u << 22;                // trips to L2 after which a wait is given up (a second and more)
-constexpr int RUN = 4;                                   // pages of a job at most
+// Pages of a job, by the pages that its sequence sees (by nothing else: a sequence's bits must not depend on its company). Short
+// runs spread a sequence over more warps, long ones leave fewer partial results to merge. 0.6B shape, us a step with runs of 2 / of
+// 4: 5 pages, 1 row 558 / 593, 4 rows 613 / 653; 8 pages, 8 rows 770 / 738; 16 pages, 1 row 588 / 609, 4 rows 648 / 690, 8 rows
+// 794 / 844; 24 pages, 1 row 576 / 602, 4 rows 739 / 713, 8 rows 901 / 860; 33 pages, 8 rows 1,029 / 952; 63 pages, 1 row 638 / 635,
+// 2 rows 764 / 695; 250 pages, 1 row 1,154 / 958.
+constexpr int RUN = 4, RUN_SHIFT = 2, SHORT_RUN_SHIFT = 1, SHORT_PAGES = 16;
 constexpr int TABLE = 32;                                // jobs of a CTA that are looked up once for all layers
 constexpr int BAR_ALL = 5, BAR_NORM = 6;                 // named barriers of the eight warps, and with the helpers (1, 2: a page's four warps)
 static_assert(KEYS * 128 * 2 <= SLOT_BYTES && KW % 64 == 0, "a slot holds either kind of tile; a warp takes whole blocks of columns");
@@ -62,7 +67,6 @@ static_assert(sizeof(LayerDesc) == 96, "the host's layout");
 
 struct StepArgs {
     int M, D, H, KV, F, L, S;
-    int run;                                             // pages of a job
     int lg_rows;                                         // M, rounded up to a power of two: its logarithm
     int gain_dtype, qk_dtype, n_pos;
     float eps, qk_eps, scale, inv_d;                     // inv_d: 1 / D
@@ -131,27 +135,33 @@ __device__ __forceinline__ int my_units(int n_units) {
 
 // Jobs are numbered sequence by sequence, kv head by kv head, run by run; a CTA takes consecutive ones.
 struct Job {
-    int b, g, r, n;                                      // run r of n pages
+    int b, g, r, p, n;                                   // run r: n pages, from the sequence's visible page p on
 };
-__device__ __forceinline__ int runs_of(int pages, int run) { return (pages + run - 1) / run; }
+__device__ __forceinline__ int run_shift(int pages) { return pages <= SHORT_PAGES ? SHORT_RUN_SHIFT : RUN_SHIFT; }
+__device__ __forceinline__ int runs_of(int pages) {
+    const int s = run_shift(pages);
+    return (pages + (1 << s) - 1) >> s;
+}
 template <class SM>
-__device__ __noinline__ int find_job(const SM& sm, int grp, int j, int M, int run) {
+__device__ __noinline__ int find_job(const SM& sm, int grp, int j, int M) {
     int b = 0;
     while (b + 1 < M && j >= sm.cum[grp][b + 1]) b++;
-    const int r = j - sm.cum[grp][b], n = runs_of(sm.cnt[grp][b], run);
+    const int r = j - sm.cum[grp][b], n = runs_of(sm.cnt[grp][b]);
     return (int)((unsigned)b << 28) | (r / n) << 20 | r % n;
 }
 template <class SM>
-__device__ __forceinline__ Job look_up(const SM& sm, int grp, int j, int j0, int M, int run) {
-    const int e = j - j0 < TABLE ? sm.table[grp][j - j0] : find_job(sm, grp, j, M, run);
-    Job job{(int)((unsigned)e >> 28), (e >> 20) & 255, e & 0xfffff, 0};
-    job.n = min(run, sm.cnt[grp][job.b] - job.r * run);
+__device__ __forceinline__ Job look_up(const SM& sm, int grp, int j, int j0, int M) {
+    const int e = j - j0 < TABLE ? sm.table[grp][j - j0] : find_job(sm, grp, j, M);
+    Job job{(int)((unsigned)e >> 28), (e >> 20) & 255, e & 0xfffff, 0, 0};
+    const int pages = sm.cnt[grp][job.b], s = run_shift(pages);
+    job.p = job.r << s;
+    job.n = min(1 << s, pages - job.p);
     return job;
 }
 // The physical page of a run's page i, -1: none.
 template <class SM>
-__device__ __forceinline__ int page_at(const SM& sm, const PageTable& pt, int grp, const Job& job, int j, int j0, int run, int i) {
-    return j - j0 < TABLE ? sm.pages[grp][j - j0][i] : page_of(pt, job.b, (sm.pg0[grp][job.b] + job.r * run + i) * PAGE_TOKENS);
+__device__ __forceinline__ int page_at(const SM& sm, const PageTable& pt, int grp, const Job& job, int j, int j0, int i) {
+    return j - j0 < TABLE ? sm.pages[grp][j - j0][i] : page_of(pt, job.b, (sm.pg0[grp][job.b] + job.p + i) * PAGE_TOKENS);
 }
 __device__ __forceinline__ int first_job(int jobs, int cta) { return (int)((long long)jobs * cta / gridDim.x); }
 
@@ -238,9 +248,9 @@ struct Producer {
         const int grp = (int)d.group, J = sm.cum[grp][a.M];
         const int j0 = first_job(J, blockIdx.x), j1 = first_job(J, blockIdx.x + 1);
         for (int j = j0; j < j1; j++) {
-            const Job job = look_up(sm, grp, j, j0, a.M, a.run);
+            const Job job = look_up(sm, grp, j, j0, a.M);
             for (int i = 0; i < job.n; i++) {
-                const int page = page_at(sm, a.pt[grp], grp, job, j, j0, a.run, i);
+                const int page = page_at(sm, a.pt[grp], grp, job, j, j0, i);
                 const int r = (int)d.map_row0 + (page * a.KV + job.g) * PAGE_TOKENS;
 #pragma unroll
                 for (int kv = 0; kv < 2; kv++, it++) {
@@ -699,14 +709,14 @@ struct Worker {
         bool merges = false;                             // some job of this group is a newest run of several
 #pragma unroll 1
         for (int j = j0; j < j1; j++) {
-            const Job job = look_up(sm, grp, j, j0, a.M, a.run);
+            const Job job = look_up(sm, grp, j, j0, a.M);
             if ((j - j0) % PAGE_GROUPS != gi) {          // the other group's
                 it += 2 * job.n;
                 continue;
             }
-            const int hi = sm.hi[job.b], pos = hi - 1, runs = runs_of(sm.cnt[grp][job.b], a.run);
+            const int hi = sm.hi[job.b], pos = hi - 1, runs = runs_of(sm.cnt[grp][job.b]);
             const uint64_t* qrow = a.qkv + (size_t)job.b * NQ / 2;
-            const int first = (sm.pg0[grp][job.b] + job.r * a.run) * PAGE_TOKENS, lo = first_visible(hi, window);
+            const int first = (sm.pg0[grp][job.b] + job.p) * PAGE_TOKENS, lo = first_visible(hi, window);
             const bool pos_ok = !rotate || pos < a.n_pos;
             if (!pos_ok && ltid == 0) atomicOr(a.status, MYNAH_ST_POS_RANGE);
             merges = merges || (job.r == runs - 1 && runs > 1);
@@ -747,7 +757,7 @@ struct Worker {
             float oc[NT][4] = {}, m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll 1
             for (int i = 0; i < job.n; i++, it += 2) {
-                const int page = page_at(sm, a.pt[grp], grp, job, j, j0, a.run, i), p0 = first + i * PAGE_TOKENS;
+                const int page = page_at(sm, a.pt[grp], grp, job, j, j0, i), p0 = first + i * PAGE_TOKENS;
                 const bool empty = page < 0 || !pos_ok;
                 if (page < 0 && ltid == 0) atomicOr(a.status, MYNAH_ST_PAGE_RANGE);
                 const int k_first = max(lo, p0) - p0, k_last = min(hi, p0 + PAGE_TOKENS) - 1 - p0;
@@ -885,8 +895,8 @@ struct Worker {
         // A merge waits for runs with lower numbers only, and these wait for merges of still lower ones at most.
 #pragma unroll 1
         for (int j = j0 + gi; j < j1; j += PAGE_GROUPS) {
-            const Job job = look_up(sm, grp, j, j0, a.M, a.run);
-            const int runs = runs_of(sm.cnt[grp][job.b], a.run);
+            const Job job = look_up(sm, grp, j, j0, a.M);
+            const int runs = runs_of(sm.cnt[grp][job.b]);
             if (job.r == runs - 1 && runs > 1) merge(w, job.b, job.g, runs, tag);
         }
     }
@@ -929,7 +939,7 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
             sm.pg0[tid][b] = vp.pg0;
             sm.cnt[tid][b] = vp.count();
             sm.cum[tid][b] = sum;
-            sum += runs_of(sm.cnt[tid][b], a.run) * a.KV;
+            sum += runs_of(sm.cnt[tid][b]) * a.KV;
         }
         sm.cum[tid][a.M] = sum;
     }
@@ -937,9 +947,9 @@ decode_layers_kernel(const __grid_constant__ StepMaps maps, const __grid_constan
     for (int i = tid; i < MAX_GROUPS * TABLE; i += THREADS) {
         const int g = i / TABLE, J = sm.cum[g][a.M], j = first_job(J, blockIdx.x) + i % TABLE;
         if (a.pt[g].ids != nullptr && j < first_job(J, blockIdx.x + 1)) {
-            sm.table[g][i % TABLE] = find_job(sm, g, j, a.M, a.run);
-            const Job job = look_up(sm, g, first_job(J, blockIdx.x) + i % TABLE, first_job(J, blockIdx.x), a.M, a.run);
-            for (int k = 0; k < job.n; k++) sm.pages[g][i % TABLE][k] = page_of(a.pt[g], job.b, (sm.pg0[g][job.b] + job.r * a.run + k) * PAGE_TOKENS);
+            sm.table[g][i % TABLE] = find_job(sm, g, j, a.M);
+            const Job job = look_up(sm, g, j, first_job(J, blockIdx.x), a.M);
+            for (int k = 0; k < job.n; k++) sm.pages[g][i % TABLE][k] = page_of(a.pt[g], job.b, (sm.pg0[g][job.b] + job.p + k) * PAGE_TOKENS);
         }
     }
     __syncthreads();
@@ -1087,8 +1097,6 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     a.eps = eps; a.qk_eps = qk_eps; a.inv_d = 1.0f / (float)D;
     a.scale = (float)(1.4426950408889634 / sqrt((double)HD));        // probabilities are powers of two: score times log2(e)
     while ((1 << a.lg_rows) < M) a.lg_rows++;
-    // Few sequences: short runs, so that more warps share a long one; many: longer ones, with fewer partial results to merge.
-    a.run = M <= 2 ? 2 : RUN;
     a.layers = static_cast<const LayerDesc*>(layers);
     a.x = x;
     a.hid = static_cast<uint64_t*>(words);

@@ -66,7 +66,7 @@ def test_one_launch_a_step(tmp_path, i, ctas):
         eng.check_status()
         assert any(took) == one
         if one:
-            # a step again, with the rows in another order: a sequence's bits do not depend on its row or its company
+            # a step again, with the rows in another order: a sequence's bits do not depend on its row
             for s in slots:
                 eng.close_sequence(s)
             slots = [eng.open_sequence() for _ in lens]
@@ -121,3 +121,30 @@ def test_tags_begin_again(tmp_path):
         eng.check_status()
     for a, b in ((rows[0], rows[1]), (rows[0][:20], rows[2])):
         assert len(a) == len(b) and all(np.array_equal(u, v) for u, v in zip(a, b))
+
+
+def test_a_sequence_has_the_same_bits_in_every_batch_of_the_one_launch(tmp_path, monkeypatch):
+    """Alone and with one, two, three and seven others, captured (padded to a bucket) and launched, among them sequences on both
+    sides of the page count that decides how long the attention's runs are. What is compared are the logits behind the layers:
+    the head's product is the same for every number of rows up to 16."""
+    from mynah_slm_b200.engine import engine as engine_module
+    from mynah_slm_b200.engine.engine import Engine, StepEntry
+    monkeypatch.setattr(engine_module, "PROMPT_GRAPH_MAX_ROWS", 0)   # every prompt by the same launches
+    cfg = _cfg(2, 512, 8, 4, 128, 704)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=5)
+    lens = [700, 1500, 1024, 1023, 3, 64, 200, 1100]                 # (1,024 + 1 positions are the first of seventeen pages)
+    rng = np.random.default_rng(0)
+    seqs = [rng.integers(0, cfg["vocab_size"], size=n + 1).tolist() for n in lens]
+    got = {}
+    for graphs in (True, False):
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=7168, max_seqs=8, use_graphs=graphs)
+        for who in ([0], [1], [2], [3], [4], [0, 1], [2, 0, 3], [7, 1, 4, 0], list(range(8)), [3, 2, 1, 0, 6], [2, 1]):
+            slots = [eng.open_sequence() for _ in who]
+            for s, i in zip(slots, who):                             # (one by one: a prompt's bits may depend on its batch)
+                eng.step([StepEntry(s, seqs[i][:-1], ())])
+            rows = eng.step([StepEntry(s, seqs[i][-1:], (0,)) for s, i in zip(slots, who)]).cpu().numpy()
+            for i, row in zip(who, rows):
+                assert np.array_equal(got.setdefault(i, row), row), (graphs, who, i)
+            for s in slots:
+                eng.close_sequence(s)
+        eng.check_status()
