@@ -67,6 +67,7 @@ static_assert(sizeof(LayerDesc) == 96, "the host's layout");
 
 struct StepArgs {
     int M, D, H, KV, F, L, S;
+    int R;                                               // runs of a sequence at most: the pitch of the partial results
     int lg_rows;                                         // M, rounded up to a power of two: its logarithm
     int gain_dtype, qk_dtype, n_pos;
     float eps, qk_eps, scale, inv_d;                     // inv_d: 1 / D
@@ -75,7 +76,7 @@ struct StepArgs {
     const LayerDesc* layers;
     float* x;
     uint64_t *hid, *squares, *qkv, *att, *act;           // tagged words: [copies][rows][columns / 2], squares [copies][rows][D / 8]
-    uint64_t *part_o, *part_ml;                          // pages' partial results, tagged: [rows][heads][S][HD], [..][2]
+    uint64_t *part_o, *part_ml;                          // pages' partial results, tagged: [rows][heads][R][HD], [..][2]
     unsigned* sync;                                      // [0] the last step's tag, [1] CTAs that have left
     const int* kv_len;
     const float *cos_t, *sin_t;
@@ -137,8 +138,8 @@ __device__ __forceinline__ int my_units(int n_units) {
 struct Job {
     int b, g, r, p, n;                                   // run r: n pages, from the sequence's visible page p on
 };
-__device__ __forceinline__ int run_shift(int pages) { return pages <= SHORT_PAGES ? SHORT_RUN_SHIFT : RUN_SHIFT; }
-__device__ __forceinline__ int runs_of(int pages) {
+__host__ __device__ __forceinline__ int run_shift(int pages) { return pages <= SHORT_PAGES ? SHORT_RUN_SHIFT : RUN_SHIFT; }
+__host__ __device__ __forceinline__ int runs_of(int pages) {
     const int s = run_shift(pages);
     return (pages + (1 << s) - 1) >> s;
 }
@@ -163,6 +164,8 @@ template <class SM>
 __device__ __forceinline__ int page_at(const SM& sm, const PageTable& pt, int grp, const Job& job, int j, int j0, int i) {
     return j - j0 < TABLE ? sm.pages[grp][j - j0][i] : page_of(pt, job.b, (sm.pg0[grp][job.b] + job.p + i) * PAGE_TOKENS);
 }
+// Runs that a sequence of at most so many visible pages is cut into at most.
+inline int most_runs(int pages) { return max(runs_of(min(pages, SHORT_PAGES)), runs_of(pages)); }
 __device__ __forceinline__ int first_job(int jobs, int cta) { return (int)((long long)jobs * cta / gridDim.x); }
 
 // ---- tagged words
@@ -612,7 +615,7 @@ struct Worker {
             const int h = h0 + lw / wph;
             float o[DL] = {}, lsum = 0.f;
             if (h < G) {
-                const size_t row = ((size_t)b * a.H + g * G + h) * a.S;
+                const size_t row = ((size_t)b * a.H + g * G + h) * a.R;
                 const uint64_t* ml = a.part_ml + row * 2;
                 float m = -INFINITY;
 #pragma unroll 1
@@ -853,7 +856,7 @@ struct Worker {
                     w.l[lw][lane * 2 + e] = l[e];
                 }
             }
-            const size_t row0 = ((size_t)job.b * a.H + (size_t)job.g * G) * a.S + job.r;
+            const size_t row0 = ((size_t)job.b * a.H + (size_t)job.g * G) * a.R + job.r;
 #pragma unroll 1
             for (int h0 = 0; h0 < G; h0 += CHUNK) {
                 if ((lane & 3) == h0 / CHUNK) {
@@ -880,7 +883,7 @@ struct Worker {
                         publish_copies(a.att + ((size_t)job.b * a.H * HD + (size_t)(job.g * G + h) * HD + c) / 2, (size_t)MAX_ROWS * (a.H * HD / 2),
                                        pack2(o0 * inv, o1 * inv), tag);
                     } else {
-                        const size_t row = row0 + (size_t)h * a.S;
+                        const size_t row = row0 + (size_t)h * a.R;
                         publish2(a.part_o + row * HD + c, __float_as_uint(o0), __float_as_uint(o1), tag);
                         if (c == 0) publish2(a.part_ml + row * 2, __float_as_uint(top), __float_as_uint(sum), tag);
                     }
@@ -1082,9 +1085,9 @@ MYNAH_API int mynah_decode_layers_supported(int M, int D, int H, int KV, int HD,
 // One decode step through all layers. layers: L descriptors of 96 bytes on the device; host_layers: the same on the host.
 // Per cache group (n_groups of them) eight words: k and v bases, their rows (entries * pages * kv heads * 64), window, and the
 // page lists. words: 64-bit words for 8 rows of 4 (D + H HD + F) / 2 + D + (H + 2 KV) HD / 2; part: 64-bit words for
-// 8 * H * S * (HD + 2); sync: two 32-bit words. All three zero before the first launch and kept from step to step.
+// M * H * R * (HD + 2), R = most_runs(S), of which there are part_words; sync: two 32-bit words. All three zero before the first launch and kept from step to step.
 MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, int L, int M, int D, int H, int KV, int HD, int F, int S,
-                                  float* x, void* words, void* part, unsigned* sync,
+                                  float* x, void* words, void* part, long long part_words, unsigned* sync,
                                   int gain_dtype, float eps, int qk_dtype, float qk_eps, const float* cos_t, const float* sin_t, int n_pos,
                                   const int* kv_len, int n_groups, const long long* group_words, int* status, int sms, cudaStream_t stream) {
     MYNAH_REQUIRE(mynah_decode_layers_supported(M, D, H, KV, HD, F, L, n_groups), "decode_layers: sizes are not supported");
@@ -1092,7 +1095,8 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     MYNAH_REQUIRE(sms >= 1 && sms <= mynah_sm_count(), "decode_layers: bad CTA count");
     StepMaps maps = {};
     StepArgs a = {};
-    a.M = M; a.D = D; a.H = H; a.KV = KV; a.F = F; a.L = L; a.S = S;
+    a.M = M; a.D = D; a.H = H; a.KV = KV; a.F = F; a.L = L; a.S = S; a.R = most_runs(S);
+    MYNAH_REQUIRE((long long)M * H * a.R * (HD + 2) <= part_words, "decode_layers: %lld words of partial results are too few", part_words);
     a.gain_dtype = gain_dtype; a.qk_dtype = qk_dtype; a.n_pos = n_pos;
     a.eps = eps; a.qk_eps = qk_eps; a.inv_d = 1.0f / (float)D;
     a.scale = (float)(1.4426950408889634 / sqrt((double)HD));        // probabilities are powers of two: score times log2(e)
@@ -1105,7 +1109,7 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     a.att = a.qkv + (size_t)MAX_ROWS * ((H + 2 * KV) * HD / 2);
     a.act = a.att + (size_t)COPIES * MAX_ROWS * (H * HD / 2);
     a.part_o = static_cast<uint64_t*>(part);
-    a.part_ml = a.part_o + (size_t)MAX_ROWS * H * S * HD;
+    a.part_ml = a.part_o + (size_t)M * H * a.R * HD;
     a.sync = sync; a.kv_len = kv_len;
     a.cos_t = cos_t; a.sin_t = sin_t; a.status = status;
     for (int g = 0; g < n_groups; g++) {

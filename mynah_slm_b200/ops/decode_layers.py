@@ -27,6 +27,11 @@ MAX_ROWS = 8
 MAX_ROW_COLUMNS = 8 * 9728
 
 
+def most_runs(pages: int) -> int:
+    """Runs of pages that a sequence of at most so many is cut into at most: twos up to 16 pages, fours beyond (csrc/decode_layers.cu)."""
+    return max(-(-min(pages, 16) // 2), -(-pages // 4) if pages > 16 else 0)
+
+
 class DecodeLayers:
     # Tags that launches may use before the words are cleared and the tags begin again at 1: a tag names one stage of one launch as
     # long as 32 bits do not wrap (74 million steps of 28 layers, ten hours of steps of 0.5 ms).
@@ -119,13 +124,14 @@ class DecodeLayers:
             self._tags = 0
         self._tags += n
 
-    def _partials(self, splits: int) -> torch.Tensor:
-        need = KERNEL_ROWS * self.sizes["H"] * splits * (self.sizes["HD"] + 2)
+    def _partials(self, rows: int, splits: int) -> torch.Tensor:
+        need = rows * self.sizes["H"] * most_runs(splits) * (self.sizes["HD"] + 2)
         if self.part is None or self.part.numel() < need:
             if torch.cuda.is_current_stream_capturing():
                 raise KernelError("decode_layers: the pages' partial results would have to grow during graph capture")
             if self.part is not None:
                 self._retired.append(self.part)
+                need = max(need, 2 * self.part.numel())          # (what has been outgrown is never more than what is in use)
             self.part = torch.zeros((need,), dtype=torch.int64, device=self.words.device)
         return self.part
 
@@ -141,8 +147,9 @@ class DecodeLayers:
         cos, sin = z["cos"], z["sin"]
         if not torch.cuda.is_current_stream_capturing():
             self.count_launch()                    # (a recorded launch counts when it is replayed)
+        part = self._partials(M, S)
         call("mynah_decode_layers", ptr(self.table), ptr(self.host_table), self.table.shape[0], M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S,
-             ptr(x), ptr(self.words), ptr(self._partials(S)), ptr(self.sync),
+             ptr(x), ptr(self.words), ptr(part), part.numel(), ptr(self.sync),
              z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,
              ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, stream_ptr())
         return x

@@ -63,7 +63,7 @@ def test_tags_begin_again_before_they_wrap(steps):
     plan.TAG_LIMIT = 20
     plan.forward(Rows([1, 64]), _ctx(1, splits=2), RUNTIME)
     small = plan.part
-    plan.forward(Rows([1, 64]), _ctx(1, splits=64), RUNTIME)
+    plan.forward(Rows([1, 64]), _ctx(1, splits=640), RUNTIME)
     assert plan.part is not small
     tagged = (plan.sync, plan.words, plan.part, small)
     for t in tagged:
@@ -78,3 +78,21 @@ def test_tags_begin_again_before_they_wrap(steps):
     assert bool((plan.sync == 7).all())
     plan.count_launch()
     assert not bool(plan.sync.any())
+
+
+def test_partial_results_take_room_by_runs_and_rows(steps):
+    """One sequence decoded from its first page to its 640th, then a batch of eight: what is held, outgrown buffers included, stays
+    within four times what the last step needs (16 times that, and 80 times as much outgrown, with a row a page for eight rows)."""
+    plan, made = steps
+    for splits in range(1, 641):
+        plan.forward(Rows([1, 64]), _ctx(1, splits=splits), RUNTIME)
+    held = lambda: plan.part.numel() + sum(t.numel() for t in plan._retired)       # noqa: E731
+    assert 160 * 66 <= plan.part.numel() <= held() <= 4 * 160 * 66
+    plan.forward(Rows([8, 64]), _ctx(8, splits=640), RUNTIME)
+    assert 8 * 160 * 66 <= plan.part.numel() <= held() <= 4 * 8 * 160 * 66
+
+
+def test_runs_of_every_page_count_fit():
+    """A sequence of up to 16 pages is cut in twos, a longer one in fours; none has more runs than a step of its splits holds."""
+    for s in range(1, 700):
+        assert decode_layers.most_runs(s) == max(-(-n // (2 if n <= 16 else 4)) for n in range(1, s + 1))
