@@ -349,14 +349,26 @@ class Engine:
         """embedding -> layers in schedule order -> final norm of the wanted
         rows -> head. Returns fp32 logits [rows, vocab]. `taps`, a dictionary,
         receives copies of the residual stream on the way (see `step`)."""
-        x = self._embed(ctx)
-        stream = Residual(x)
-        if taps is None and self.decode_layers is not None and self.decode_layers.takes(ctx):
-            self.decode_layers.forward(x, ctx, self.runtime)
-            return self.model.head.forward(self.model.final_norm.apply(stream, rows=want_rows, lazy=want_rows is None))
+        stream = Residual(self._embed(ctx))
         if taps is not None:
-            taps["embed"] = x.clone()
-        x0 = x.clone() if self._feeds_embedding else None      # the stream itself is added to in place
+            taps["embed"] = stream.x.clone()
+        self._layers(stream, ctx, taps)
+        h = self.model.final_norm.apply(stream, rows=want_rows, lazy=want_rows is None and taps is None)
+        if taps is not None:
+            taps["final_norm"] = h.float()
+        return self.model.head.forward(h)
+
+    def _layers(self, stream: Residual, ctx: StepContext, taps: Optional[dict] = None) -> None:
+        """The stream behind all layers. Whether a step's logits are wanted or tapped changes nothing in what it computes: what
+        it leaves in the cache has the same bits."""
+        if self.decode_layers is not None and self.decode_layers.takes(ctx):
+            if taps is None:
+                self.decode_layers.forward(stream.x, ctx, self.runtime)
+            for i in range(len(self.model.schedule) if taps is not None else 0):
+                self.decode_layers.forward(stream.x, ctx, self.runtime, range(i, i + 1))
+                taps[f"layer{i}"] = stream.x.clone()
+            return
+        x0 = stream.x.clone() if self._feeds_embedding else None      # the stream itself is added to in place
         views = self.cache.views
         ahead = self._ahead if self._prefetching else None
         for i, e in enumerate(self.model.schedule):
@@ -372,10 +384,6 @@ class Engine:
                 taps[f"layer{i}"] = stream.flush().clone()
         if ahead is not None:
             ahead.join()
-        h = self.model.final_norm.apply(stream, rows=want_rows, lazy=want_rows is None and taps is None)
-        if taps is not None:
-            taps["final_norm"] = h.float()
-        return self.model.head.forward(h)
 
     # ---------------------------------------------------------------- step
     def step(self, entries: Sequence[StepEntry], taps: Optional[dict] = None) -> torch.Tensor:
@@ -504,24 +512,13 @@ class Engine:
         self._host_fields(ctx, entries)
         if n_want == 0:
             # nothing wanted: the cache is still filled; skip norm and head
-            self._forward_layers_only(ctx)
+            self._layers(Residual(self._embed(ctx)), ctx)
             return torch.empty((0, self.spec.vocab_size), dtype=torch.float32, device=self.device)
         rows = ctx.want[:len(uniq)]
         logits = self._forward(ctx, rows, taps)
         if len(uniq) != n_want or not np.array_equal(inverse, np.arange(n_want)):
             logits = logits[torch.from_numpy(inverse.astype(np.int64)).to(self.device)]
         return logits
-
-    def _forward_layers_only(self, ctx: StepContext) -> None:
-        stream = Residual(self._embed(ctx))
-        x0 = stream.x.clone() if self._feeds_embedding else None
-        for i, e in enumerate(self.model.schedule):
-            if e.add_embedding:
-                stream.add_f32(x0)
-            if e.add_vector is not None:
-                kernels.residual_add_row(stream.flush(), self.model.stream_vectors.rows[e.add_vector])
-                stream.rounded = None
-            self.model.layers[e.layer].forward(stream, ctx, self.cache.views[i])
 
     def _embed(self, ctx: StepContext) -> torch.Tensor:
         emb = self.model.embedding

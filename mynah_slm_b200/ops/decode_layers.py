@@ -110,13 +110,13 @@ class DecodeLayers:
         return cls(rows, sizes, groups, runtime.device)
 
     def takes(self, ctx) -> bool:
-        z = self.sizes
-        return ctx.is_decode and ctx.T <= min(MAX_ROWS, KERNEL_ROWS) and ctx.T * max(z["D"], z["H"] * z["HD"], z["F"]) <= MAX_ROW_COLUMNS
+        z, rows = self.sizes, 1 << (ctx.T - 1).bit_length()          # (as a captured step pads them: both take the same route)
+        return ctx.is_decode and rows <= min(MAX_ROWS, KERNEL_ROWS) and rows * max(z["D"], z["H"] * z["HD"], z["F"]) <= MAX_ROW_COLUMNS
 
-    def count_launch(self) -> None:
+    def count_launch(self, layers: Optional[int] = None) -> None:
         """To be called before every launch, replayed ones too, on the launch's stream: keeps the tags from wrapping, after which
         words that were written long ago, or never, would pass for new ones."""
-        n = 2 * self.table.shape[0] + 2            # as the kernel moves its tags on
+        n = 2 * (layers or self.table.shape[0]) + 2   # as the kernel moves its tags on
         if self._tags + n > self.TAG_LIMIT:
             for t in (self.sync, self.words, self.part, *self._retired):
                 if t is not None:
@@ -135,9 +135,11 @@ class DecodeLayers:
             self.part = torch.zeros((need,), dtype=torch.int64, device=self.words.device)
         return self.part
 
-    def forward(self, x: torch.Tensor, ctx, runtime) -> torch.Tensor:
-        """The residual stream x [T, D] (fp32, updated in place) behind all layers."""
+    def forward(self, x: torch.Tensor, ctx, runtime, layers: Optional[range] = None) -> torch.Tensor:
+        """The residual stream x [T, D] (fp32, updated in place) behind all layers, or behind those of a range of them. A launch for
+        every layer gives the bits that one for all of them gives: what is handed on from layer to layer is the stream."""
         z, M, S = self.sizes, ctx.T, ctx.decode_splits
+        layers = range(self.table.shape[0]) if layers is None else layers
         _chk(x, "residual", torch.float32, 2)
         if tuple(x.shape) != (M, z["D"]):
             raise KernelError(f"decode_layers: the residual is {tuple(x.shape)}, the step has {(M, z['D'])}")
@@ -146,9 +148,9 @@ class DecodeLayers:
             words += [k.data_ptr(), v.data_ptr(), k.numel() // z["HD"], window, p.indptr.data_ptr(), p.ids.data_ptr(), p.base.data_ptr(), p.n_pages]
         cos, sin = z["cos"], z["sin"]
         if not torch.cuda.is_current_stream_capturing():
-            self.count_launch()                    # (a recorded launch counts when it is replayed)
+            self.count_launch(len(layers))         # (a recorded launch counts when it is replayed)
         part = self._partials(M, S)
-        call("mynah_decode_layers", ptr(self.table), ptr(self.host_table), self.table.shape[0], M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S,
+        call("mynah_decode_layers", ptr(self.table[layers.start]), ptr(self.host_table[layers.start]), len(layers), M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S,
              ptr(x), ptr(self.words), ptr(part), part.numel(), ptr(self.sync),
              z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,
              ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, stream_ptr())

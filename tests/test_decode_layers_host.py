@@ -96,3 +96,12 @@ def test_runs_of_every_page_count_fit():
     """A sequence of up to 16 pages is cut in twos, a longer one in fours; none has more runs than a step of its splits holds."""
     for s in range(1, 700):
         assert decode_layers.most_runs(s) == max(-(-n // (2 if n <= 16 else 4)) for n in range(1, s + 1))
+
+
+def test_padded_and_unpadded_steps_take_the_same_route(steps):
+    """A captured step has its rows padded to a power of two; the rule looks at that number for an uncaptured one as well."""
+    plan, made = steps
+    for columns in (64, 9728, 12288, 20000):
+        plan.sizes["F"] = columns
+        for rows in range(1, 20):
+            assert plan.takes(_ctx(rows)) == plan.takes(_ctx(1 << (rows - 1).bit_length()))

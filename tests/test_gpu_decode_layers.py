@@ -148,3 +148,33 @@ def test_a_sequence_has_the_same_bits_in_every_batch_of_the_one_launch(tmp_path,
             for s in slots:
                 eng.close_sequence(s)
         eng.check_status()
+
+
+def test_what_a_step_leaves_does_not_depend_on_what_is_asked_of_it(tmp_path):
+    """The same tokens with logits wanted, with none wanted and with taps: the same bits in the cache, and the logits' too."""
+    from mynah_slm_b200.engine.engine import Engine, StepEntry
+    cfg = _cfg(3, 512, 8, 4, 64, 704, window=100)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=6)
+    lens, steps = [130, 700, 64, 3, 5], 6
+    seqs = [np.random.default_rng(n).integers(0, cfg["vocab_size"], size=n + steps).tolist() for n in lens]
+    caches, rows = [], []
+    for how in ("captured", "taps", "nothing wanted"):
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=1280, max_seqs=5, use_graphs=how == "captured")
+        for t in eng.cache.keys + eng.cache.values:
+            t.zero_()
+        slots = [eng.open_sequence() for _ in seqs]
+        for s, q, n in zip(slots, seqs, lens):
+            eng.step([StepEntry(s, q[:n], ())])
+        for i in range(steps):
+            taps = {} if how == "taps" else None
+            want = () if how == "nothing wanted" and i < steps - 1 else (0,)
+            out = eng.step([StepEntry(s, [q[n + i]], want) for s, q, n in zip(slots, seqs, lens)], taps=taps)
+            if taps is not None:
+                assert sorted(taps) == ["embed", "final_norm", "layer0", "layer1", "layer2"]
+                assert not torch.equal(taps["layer0"], taps["layer1"])
+        eng.check_status()
+        rows.append(out.cpu().numpy())
+        caches.append([t.cpu() for t in eng.cache.keys + eng.cache.values])
+    for r, c in zip(rows[1:], caches[1:]):
+        assert np.array_equal(rows[0], r)
+        assert all(torch.equal(a, b) for a, b in zip(caches[0], c))
