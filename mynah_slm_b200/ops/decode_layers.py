@@ -15,6 +15,7 @@ import torch
 
 from ..cache.pages import PAGE_TOKENS
 from . import lib
+from .attention_dispatch import _tc_fits
 from .kernels import _chk
 from .lib import KernelError, call, code, ptr, stream_ptr
 
@@ -25,6 +26,11 @@ MAX_ROWS = 8
 # against the layers one by one, ms a step: 0.6B shape (3,072 columns) 1 row 0.50 / 0.87, 3 rows 0.66 / 1.01, 8 rows 0.76 / 1.01;
 # 4B shape's first 8 layers (9,728 columns) 1 row 0.56 / 0.80, 4 rows 0.60 / 0.70, 8 rows 0.68 / 0.75. Wider ones are not measured.
 MAX_ROW_COLUMNS = 8 * 9728
+# And rows times the longest sequence's pages, by head size: behind long caches the page loop and the merge of the runs bound a
+# layer, where the layers one by one stream pages with three CTAs an SM. ms a step, one launch / one by one, 0.6B shape: heads of 128,
+# 8 rows x 250 pages 3.13 / 3.51, x 313 3.92 / 4.12, x 438 5.55 / 5.33, x 625 8.12 / 7.23; 4 rows x 625 3.99 / 4.35; 1 row x 625
+# 1.70 / 2.23, x 1,016 2.46 / 3.03. Heads of 64, 8 rows x 250 2.62 / 2.70, x 625 6.98 / 5.26; 2 rows x 625 2.05 / 2.34.
+MAX_ROW_PAGES = {64: 2048, 128: 2944}
 
 
 def most_runs(pages: int) -> int:
@@ -111,7 +117,11 @@ class DecodeLayers:
 
     def takes(self, ctx) -> bool:
         z, rows = self.sizes, 1 << (ctx.T - 1).bit_length()          # (as a captured step pads them: both take the same route)
-        return ctx.is_decode and rows <= min(MAX_ROWS, KERNEL_ROWS) and rows * max(z["D"], z["H"] * z["HD"], z["F"]) <= MAX_ROW_COLUMNS
+        if not ctx.is_decode or rows > min(MAX_ROWS, KERNEL_ROWS) or rows * max(z["D"], z["H"] * z["HD"], z["F"]) > MAX_ROW_COLUMNS:
+            return False
+        # (Beyond what the tensor-core kernels' merge takes the layers one by one have the general kernel only: 4B shape's first 8
+        # layers, 8 rows x 625 pages 2.80 / 12.75.)
+        return rows * ctx.decode_splits <= MAX_ROW_PAGES[z["HD"]] or not _tc_fits(z["H"], z["KV"], ctx.decode_splits)
 
     def count_launch(self, layers: Optional[int] = None) -> None:
         """To be called before every launch, replayed ones too, on the launch's stream: keeps the tags from wrapping, after which

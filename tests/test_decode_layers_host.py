@@ -99,9 +99,20 @@ def test_runs_of_every_page_count_fit():
 
 
 def test_padded_and_unpadded_steps_take_the_same_route(steps):
-    """A captured step has its rows padded to a power of two; the rule looks at that number for an uncaptured one as well."""
+    """A captured step has its rows padded to a power of two and its page splits to one or to a multiple of sixteen; the rule
+    gives the same answer for the uncaptured step."""
+    from mynah_slm_b200.engine.engine import Engine
     plan, made = steps
-    for columns in (64, 9728, 12288, 20000):
-        plan.sizes["F"] = columns
+    for columns, dim, pages in [(c, 64, 1) for c in (64, 9728, 12288, 20000)] + [(64, d, p) for d in (64, 128) for p in range(1, 800, 3)]:
+        plan.sizes["F"], plan.sizes["HD"] = columns, dim
         for rows in range(1, 20):
-            assert plan.takes(_ctx(rows)) == plan.takes(_ctx(1 << (rows - 1).bit_length()))
+            assert plan.takes(_ctx(rows, pages)) == plan.takes(_ctx(Engine._bucket(rows), max(4, Engine._pages_bucket(pages))))
+
+
+def test_long_caches_take_the_layers_one_by_one(steps):
+    """Where the one launch measured slower; not where the layers one by one would have the general attention kernel only."""
+    plan, made = steps
+    for heads, dim, rows, pages, one in [(16, 128, 8, 368, True), (16, 128, 8, 384, False), (16, 128, 4, 736, True), (16, 128, 1, 1008, True),
+                                         (16, 64, 8, 256, True), (16, 64, 8, 272, False), (32, 128, 8, 512, False), (32, 128, 8, 528, True)]:
+        plan.sizes.update(H=heads, KV=8, HD=dim)
+        assert plan.takes(_ctx(rows, pages)) is one
