@@ -178,3 +178,25 @@ def test_what_a_step_leaves_does_not_depend_on_what_is_asked_of_it(tmp_path):
     for r, c in zip(rows[1:], caches[1:]):
         assert np.array_equal(rows[0], r)
         assert all(torch.equal(a, b) for a, b in zip(caches[0], c))
+
+
+def test_a_row_whose_squares_overflow(tmp_path):
+    """1 / rms of an infinite mean square is 0: such a row's logits are those of a row of zeros, as layer by layer, and its
+    neighbour's are as ever."""
+    from mynah_slm_b200.engine.engine import Engine, StepEntry
+    cfg = dict(_cfg(2, 256, 4, 2, 64, 320), tie_word_embeddings=False)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=3)
+    out = {}
+    for one in (True, False):
+        for big in (True, False):
+            eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=256, max_seqs=2)
+            if not one:
+                eng.decode_layers = None
+            if big:
+                eng.model.embedding.table[7] *= 1e21
+            slots = [eng.open_sequence() for _ in range(2)]
+            out[one, big] = eng.step([StepEntry(slots[0], [7], (0,)), StepEntry(slots[1], [9], (0,))]).cpu().numpy()
+            eng.check_status()
+    for one in (True, False):
+        assert not out[one, True][0].any() and out[one, False][0].any()
+        assert np.array_equal(out[one, True][1], out[one, False][1])
