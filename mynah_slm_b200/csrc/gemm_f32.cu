@@ -81,6 +81,7 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
 // Bound by the FFMA pipes where the tiles fill the SMs. A prompt of 161 rows through the 0.6B shape (products of 1,024 to
 // 6,144 outputs): 163 us a product with the scalar kernel above for every size, 70 us with these.
 
+constexpr int GRID_ROWS = 65535;                                     // tiles of rows that a launch's grid can name
 constexpr int SLAB = 32, PITCH = SLAB + 4, TILE_STAGES = 3;
 
 template <int BM, int BN, int TM, int TN>
@@ -166,9 +167,7 @@ int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, i
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return mynah_fail("gemm_f32: %s", cudaGetErrorString(e));
     }
-    const int gy = ceil_div(M, BM);
-    MYNAH_REQUIRE(gy <= 65535, "gemm_f32: %d rows exceed one launch (%d)", M, 65535 * BM);
-    mynah_launch(kern, dim3(ceil_div(N, BN), gy), dim3((BM / TM) * (BN / TN)), smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
+    mynah_launch(kern, dim3(ceil_div(N, BN), ceil_div(M, BM)), dim3((BM / TM) * (BN / TN)), smem, stream, A, W, C, M, N, K, lda, ldw, ldc);
     return mynah_check_launch("gemm_f32");
 }
 
@@ -281,11 +280,10 @@ MYNAH_API int mynah_gemm_f32(const float* A, const float* W, float* C, int M, in
     if (M == 0 || N == 0) return 0;
     MYNAH_REQUIRE(M > 0 && N > 0 && K > 0, "gemm_f32: bad sizes M=%d N=%d K=%d", M, N, K);
     MYNAH_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32: a leading dimension is smaller than its row");
+    MYNAH_REQUIRE(ceil_div(M, BM) <= GRID_ROWS, "gemm_f32: %d rows exceed one launch (%d)", M, GRID_ROWS * BM);
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
     if (!vec) {
-        const int gy = ceil_div(M, BM);
-        MYNAH_REQUIRE(gy <= 65535, "gemm_f32: %d rows exceed one launch (%d)", M, 65535 * BM);
-        const dim3 grid(ceil_div(N, BN), gy);
+        const dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
         gemm_f32_kernel<<<grid, 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc);
         return mynah_check_launch("gemm_f32");
     }
@@ -305,6 +303,6 @@ MYNAH_API int mynah_gemm_f32(const float* A, const float* W, float* C, int M, in
     };
     const double c128 = cost(128, 128, 0.85), c64 = cost(64, 64, 0.60), c32 = cost(32, 32, 0.35);
     if (c128 <= c64 && c128 <= c32) return launch_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    if (c64 <= c32) return launch_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (c64 <= c32 || ceil_div(M, 32) > GRID_ROWS) return launch_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     return launch_tile<32, 32, 4, 2>(A, W, C, M, N, K, lda, ldw, ldc, stream);
 }

@@ -150,6 +150,21 @@ def test_gemm_f32_kernels_walk_the_same_chain(M, N, K):
     assert torch.equal(k.linear(wide[:, :K].contiguous(), w), general)
 
 
+def test_gemm_f32_of_very_many_rows():
+    """More rows than the smallest tile's grid can name (65,535 tiles of 32), for outputs so few that it would be chosen; the limit
+    is that of tiles of 64, as for rows at an odd pitch."""
+    k = _k()
+    from mynah_slm_b200.ops.lib import KernelError
+    M = 65535 * 32 + 5
+    g = torch.Generator(device=DEV).manual_seed(0)
+    x, w = torch.randn((M, 4), generator=g, device=DEV), torch.randn((3, 4), generator=g, device=DEV)
+    c = k.linear(x, w)
+    bound = 4 * 2.0 ** -24 * 1.001 * (x.double().abs() @ w.double().abs().T)       # four roundings an output
+    assert bool(((c.double() - x.double() @ w.double().T).abs() <= bound).all())
+    with pytest.raises(KernelError, match="rows exceed one launch"):
+        k.linear(torch.zeros((1, 4), device=DEV).expand(65535 * 64 + 1, 4).contiguous(), w)
+
+
 def _paged(kv: np.ndarray, page_ids, n_pages, dt, poison=None):
     """Scatter [T, KV, HD] into pages [n_pages, KV, 64, HD]."""
     T, KV, HD = kv.shape
