@@ -1056,6 +1056,10 @@ int launch_step(const StepMaps& maps, const StepArgs& a, int sms, cudaStream_t s
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, kern, maps, a);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {       // fewer SMs than CTAs are this process's (or context's) to use
+        (void)cudaGetLastError();
+        return 1;
+    }
     if (e != cudaSuccess) return mynah_fail("decode_layers: %s", cudaGetErrorString(e));
     return mynah_check_launch("decode_layers");
 }
@@ -1088,6 +1092,7 @@ MYNAH_API int mynah_decode_layers_supported(int M, int D, int H, int KV, int HD,
 // Per cache group (n_groups of them) eight words: k and v bases, their rows (entries * pages * kv heads * 64), window, and the
 // page lists. words: 64-bit words for 8 rows of 4 (D + H HD + F) / 2 + D + (H + 2 KV) HD / 2; part: 64-bit words for
 // M * H * R * (HD + 2), R = most_runs(S), of which there are part_words; sync: two 32-bit words. All three zero before the first launch and kept from step to step.
+// 1: declined, nothing was launched (its CTAs would not all be resident).
 MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, int L, int M, int D, int H, int KV, int HD, int F, int S,
                                   float* x, void* words, void* part, long long part_words, unsigned* sync,
                                   int gain_dtype, float eps, int qk_dtype, float qk_eps, const float* cos_t, const float* sin_t, int n_pos,

@@ -362,12 +362,14 @@ class Engine:
         """The stream behind all layers. Whether a step's logits are wanted or tapped changes nothing in what it computes: what
         it leaves in the cache has the same bits."""
         if self.decode_layers is not None and self.decode_layers.takes(ctx):
-            if taps is None:
-                self.decode_layers.forward(stream.x, ctx, self.runtime)
-            for i in range(len(self.model.schedule) if taps is not None else 0):
-                self.decode_layers.forward(stream.x, ctx, self.runtime, range(i, i + 1))
-                taps[f"layer{i}"] = stream.x.clone()
-            return
+            n = len(self.model.schedule)
+            for part in [range(n)] if taps is None else [range(i, i + 1) for i in range(n)]:
+                if not self.decode_layers.forward(stream.x, ctx, self.runtime, part):
+                    break
+                if taps is not None:
+                    taps[f"layer{part.start}"] = stream.x.clone()
+            else:
+                return
         x0 = stream.x.clone() if self._feeds_embedding else None      # the stream itself is added to in place
         views = self.cache.views
         ahead = self._ahead if self._prefetching else None

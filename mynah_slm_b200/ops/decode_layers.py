@@ -17,7 +17,7 @@ from ..cache.pages import PAGE_TOKENS
 from . import lib
 from .attention_dispatch import _tc_fits
 from .kernels import _chk
-from .lib import KernelError, call, code, ptr, stream_ptr
+from .lib import KernelError, code, offer, ptr, stream_ptr
 
 KERNEL_ROWS = 8         # rows that the kernel takes at most
 # Rows up to which a step takes the one launch. 0: never.
@@ -54,6 +54,7 @@ class DecodeLayers:
         self.sync = torch.zeros((2,), dtype=torch.int32, device=device)
         self.part: Optional[torch.Tensor] = None
         self._retired: list[torch.Tensor] = []     # outgrown buffers stay alive: a captured graph may still hold their address
+        self.declined = False                      # the launch's CTAs cannot all be resident here: the layers run one by one
         self._tags = 0                             # tags used since the words were cleared
 
     @classmethod
@@ -117,7 +118,7 @@ class DecodeLayers:
 
     def takes(self, ctx) -> bool:
         z, rows = self.sizes, 1 << (ctx.T - 1).bit_length()          # (as a captured step pads them: both take the same route)
-        if not ctx.is_decode or rows > min(MAX_ROWS, KERNEL_ROWS) or rows * max(z["D"], z["H"] * z["HD"], z["F"]) > MAX_ROW_COLUMNS:
+        if self.declined or not ctx.is_decode or rows > min(MAX_ROWS, KERNEL_ROWS) or rows * max(z["D"], z["H"] * z["HD"], z["F"]) > MAX_ROW_COLUMNS:
             return False
         # (Beyond what the tensor-core kernels' merge takes the layers one by one have the general kernel only: 4B shape's first 8
         # layers, 8 rows x 625 pages 2.80 / 12.75.)
@@ -145,9 +146,10 @@ class DecodeLayers:
             self.part = torch.zeros((need,), dtype=torch.int64, device=self.words.device)
         return self.part
 
-    def forward(self, x: torch.Tensor, ctx, runtime, layers: Optional[range] = None) -> torch.Tensor:
+    def forward(self, x: torch.Tensor, ctx, runtime, layers: Optional[range] = None) -> bool:
         """The residual stream x [T, D] (fp32, updated in place) behind all layers, or behind those of a range of them. A launch for
-        every layer gives the bits that one for all of them gives: what is handed on from layer to layer is the stream."""
+        every layer gives the bits that one for all of them gives: what is handed on from layer to layer is the stream. False:
+        declined, nothing was done (where the process may use fewer SMs than the device has); `takes` says no from then on."""
         z, M, S = self.sizes, ctx.T, ctx.decode_splits
         layers = range(self.table.shape[0]) if layers is None else layers
         _chk(x, "residual", torch.float32, 2)
@@ -160,8 +162,11 @@ class DecodeLayers:
         if not torch.cuda.is_current_stream_capturing():
             self.count_launch(len(layers))         # (a recorded launch counts when it is replayed)
         part = self._partials(M, S)
-        call("mynah_decode_layers", ptr(self.table[layers.start]), ptr(self.host_table[layers.start]), len(layers), M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S,
-             ptr(x), ptr(self.words), ptr(part), part.numel(), ptr(self.sync),
-             z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,
-             ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, stream_ptr())
-        return x
+        self.declined = not offer(
+            "mynah_decode_layers", ptr(self.table[layers.start]), ptr(self.host_table[layers.start]), len(layers),
+            M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S, ptr(x), ptr(self.words), ptr(part), part.numel(), ptr(self.sync),
+            z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,
+            ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, stream_ptr())
+        if self.declined and layers.start > 0:
+            raise KernelError("decode_layers: declined behind the first layers of a step")
+        return not self.declined

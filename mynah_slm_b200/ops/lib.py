@@ -266,6 +266,17 @@ def add_launches(n: int) -> None:
     _launches += n
 
 
+def offer(name: str, *args) -> bool:
+    """Call an entry point that may decline with the code 1, having launched nothing: False then."""
+    global _launches
+    lib = load()
+    rc = getattr(lib, name)(*args)
+    if rc not in (0, 1):
+        raise KernelError(lib.mynah_last_error().decode(errors="replace"))
+    _launches += rc == 0
+    return rc == 0
+
+
 def call(name: str, *args) -> None:
     global _launches
     lib = load()

@@ -27,7 +27,7 @@ class Rows:
 def steps(monkeypatch):
     """A plan of two layers of 64 whose launches are noted instead of made."""
     made = []
-    monkeypatch.setattr(decode_layers, "call", lambda name, *args: made.append((name, args)))
+    monkeypatch.setattr(decode_layers, "offer", lambda name, *args: made.append((name, args)) is None)
     monkeypatch.setattr(decode_layers, "stream_ptr", lambda: 0)
     monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
     sizes = dict(D=64, H=1, KV=1, HD=64, F=64, eps=1e-6, qk_eps=1e-6, gain_dtype=0, qk_dtype=0, cos=None, sin=None)
@@ -116,3 +116,27 @@ def test_long_caches_take_the_layers_one_by_one(steps):
                                          (16, 64, 8, 256, True), (16, 64, 8, 272, False), (32, 128, 8, 512, False), (32, 128, 8, 528, True)]:
         plan.sizes.update(H=heads, KV=8, HD=dim)
         assert plan.takes(_ctx(rows, pages)) is one
+
+
+def test_a_declined_launch_is_not_offered_again(steps, monkeypatch):
+    """Fewer SMs to use than the device has: the step goes on layer by layer, and so do those after it."""
+    plan, made = steps
+    assert plan.takes(_ctx(1)) and plan.forward(Rows([1, 64]), _ctx(1), RUNTIME) is True
+    monkeypatch.setattr(decode_layers, "offer", lambda name, *args: False)
+    assert plan.takes(_ctx(1)) and plan.forward(Rows([1, 64]), _ctx(1), RUNTIME) is False
+    assert not plan.takes(_ctx(1))
+    with pytest.raises(KernelError, match="declined behind"):
+        plan.forward(Rows([1, 64]), _ctx(1), RUNTIME, range(1, 2))
+
+
+def test_what_an_entry_point_may_answer(monkeypatch):
+    """0: launched; 1: declined, not counted as a launch; anything else is an error."""
+    from mynah_slm_b200.ops import lib
+    answers = SimpleNamespace(entry=lambda rc: rc, mynah_last_error=lambda: b"sizes are not supported")
+    monkeypatch.setattr(lib, "load", lambda: answers)
+    before = lib.launch_count()
+    assert lib.offer("entry", 0) is True and lib.launch_count() == before + 1
+    assert lib.offer("entry", 1) is False and lib.launch_count() == before + 1
+    with pytest.raises(KernelError, match="not supported"):
+        lib.offer("entry", -1)
+    lib.add_launches(-1)

@@ -200,3 +200,25 @@ def test_a_row_whose_squares_overflow(tmp_path):
     for one in (True, False):
         assert not out[one, True][0].any() and out[one, False][0].any()
         assert np.array_equal(out[one, True][1], out[one, False][1])
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_a_declined_launch_leaves_the_layers_one_by_one(tmp_path, monkeypatch, graphs):
+    """Where the one launch cannot be made, steps with and without taps go on as in an engine without it."""
+    from mynah_slm_b200.engine.engine import Engine, StepEntry
+    from mynah_slm_b200.ops import decode_layers
+    cfg = _cfg(2, 256, 4, 2, 64, 320)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=3)
+    toks = np.random.default_rng(0).integers(0, cfg["vocab_size"], size=76).tolist()
+    offered = []
+    monkeypatch.setattr(decode_layers, "offer", lambda name, *args: offered.append(name) is not None)
+    rows = []
+    for has in (True, False):
+        eng = Engine.from_folder(folder, dtype="bfloat16", max_tokens=256, max_seqs=1, use_graphs=graphs)
+        if not has:
+            eng.decode_layers = None
+        slot = eng.open_sequence()
+        eng.step([StepEntry(slot, toks[:70], ())])
+        rows.append([eng.step([StepEntry(slot, [t], (0,))], taps={} if i == 3 else None).cpu().numpy() for i, t in enumerate(toks[70:])])
+        eng.check_status()
+    assert len(offered) == 1 and all(np.array_equal(a, b) for a, b in zip(*rows))
