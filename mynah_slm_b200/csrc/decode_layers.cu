@@ -44,7 +44,6 @@ constexpr int SLOTS = 10;                                // as many as the rest 
 constexpr int TG = 6;                                    // units whose sums a warp holds at a time
 constexpr int MAX_LAYERS = 48, MAX_GROUPS = 4, MAX_ROWS = 8;
 constexpr int COPIES = 4, SQUARE_COPIES = 8;             // of what every CTA reads: see publish_pair
-constexpr uint32_t WAIT_LOOKS = 1u << 22;                // trips to L2 after which a wait is given up (a second and more)
 // Pages of a job, by the pages that its sequence sees (by nothing else: a sequence's bits must not depend on its company). Short
 // runs spread a sequence over more warps, long ones leave fewer partial results to merge. 0.6B shape, us a step with runs of 2 / of
 // 4: 5 pages, 1 row 558 / 593, 4 rows 613 / 653; 8 pages, 8 rows 770 / 738; 16 pages, 1 row 588 / 609, 4 rows 648 / 690, 8 rows
@@ -77,6 +76,7 @@ struct StepArgs {
     float* x;
     uint64_t *hid, *squares, *qkv, *att, *act;           // tagged words: [copies][rows][columns / 2], squares [copies][rows][D / 8]
     uint64_t *part_o, *part_ml;                          // pages' partial results, tagged: [rows][heads][R][HD], [..][2]
+    uint32_t looks, look_mask;                           // trips to L2 after which a wait is given up, and when they are counted
     unsigned* sync;                                      // [0] the last step's tag, [1] CTAs that have left
     const int* kv_len;
     const float *cos_t, *sin_t;
@@ -299,14 +299,15 @@ struct Worker {
     uint32_t live = 0;                                   // the rows in use, a bit each
     int tid, warp, lane;
 
-    // After `n` fruitless looks (of `limit`): whether to stop waiting, because the limit ran out here or somewhere in this CTA
-    // before. (A count, not a clock: it keeps these loops' registers few.)
-    __device__ __forceinline__ bool tired(uint32_t n, uint32_t limit) {
-        if ((n & 255u) != 255u) return false;
-        if (n >= limit) {
-            *(volatile int*)&sm.abort = 1;
-            atomicOr(a.status, MYNAH_ST_TIMEOUT);
-        }
+    __device__ __forceinline__ void give_up() {
+        *(volatile int*)&sm.abort = 1;
+        atomicOr(a.status, MYNAH_ST_TIMEOUT);
+    }
+    // After `n` fruitless looks: whether to stop waiting, because the limit ran out here or somewhere in this CTA before. (A
+    // count, not a clock: it keeps these loops' registers few.)
+    __device__ __forceinline__ bool tired(uint32_t n) {
+        if ((n & a.look_mask) != a.look_mask) return false;
+        if (n >= a.looks) give_up();
         return *(volatile int*)&sm.abort != 0;
     }
     __device__ __forceinline__ bool is_full(uint32_t i) const {
@@ -337,7 +338,7 @@ struct Worker {
         while (!__all_sync(0xffffffffu, lane >= n || (PAGES ? page_is_full(i + lane) : is_full(i + lane)))) {
             const unsigned long long now = tc5::now_ns();
             if (t0 == 0) t0 = now;
-            else if (now - t0 > tc5::WAIT_LIMIT_NS) tired(~0u, 0);
+            else if (now - t0 > tc5::WAIT_LIMIT_NS) give_up();
             if (__any_sync(0xffffffffu, *(volatile int*)&sm.abort != 0)) break;
         }
     }
@@ -354,7 +355,7 @@ struct Worker {
         bool stop = false;
         if (who != 0 && lane == __ffs(who) - 1)
             for (uint32_t n = 0; !has_tag(peek(p), tag); n++)
-                if (tired(n, WAIT_LOOKS)) {
+                if (tired(n)) {
                     stop = true;
                     break;
                 }
@@ -416,7 +417,7 @@ struct Worker {
                 }
             }
             if (__all_sync(0xffffffffu, gone == 0)) break;
-            if (__any_sync(0xffffffffu, tired(n, WAIT_LOOKS))) break;
+            if (__any_sync(0xffffffffu, tired(n))) break;
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
@@ -1092,13 +1093,16 @@ MYNAH_API int mynah_decode_layers_supported(int M, int D, int H, int KV, int HD,
 // Per cache group (n_groups of them) eight words: k and v bases, their rows (entries * pages * kv heads * 64), window, and the
 // page lists. words: 64-bit words for 8 rows of 4 (D + H HD + F) / 2 + D + (H + 2 KV) HD / 2; part: 64-bit words for
 // M * H * R * (HD + 2), R = most_runs(S), of which there are part_words; sync: two 32-bit words. All three zero before the first launch and kept from step to step.
+// looks: trips to L2 that a wait may take (a few tenths of a microsecond each) before it is given up, with MYNAH_ST_TIMEOUT in the
+// status, and with it all that its CTA still waits for; the others find what they wait for, if not its values.
 // 1: declined, nothing was launched (its CTAs would not all be resident).
 MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, int L, int M, int D, int H, int KV, int HD, int F, int S,
                                   float* x, void* words, void* part, long long part_words, unsigned* sync,
                                   int gain_dtype, float eps, int qk_dtype, float qk_eps, const float* cos_t, const float* sin_t, int n_pos,
-                                  const int* kv_len, int n_groups, const long long* group_words, int* status, int sms, cudaStream_t stream) {
+                                  const int* kv_len, int n_groups, const long long* group_words, int* status, int sms, int looks, cudaStream_t stream) {
     MYNAH_REQUIRE(mynah_decode_layers_supported(M, D, H, KV, HD, F, L, n_groups), "decode_layers: sizes are not supported");
     MYNAH_REQUIRE(S >= 1 && S <= 0xfffff, "decode_layers: %d page splits", S);
+    MYNAH_REQUIRE(looks >= 0, "decode_layers: a wait of %d looks", looks);
     MYNAH_REQUIRE(sms >= 1 && sms <= mynah_sm_count(), "decode_layers: bad CTA count");
     StepMaps maps = {};
     StepArgs a = {};
@@ -1117,6 +1121,7 @@ MYNAH_API int mynah_decode_layers(const void* layers, const void* host_layers, i
     a.act = a.att + (size_t)COPIES * MAX_ROWS * (H * HD / 2);
     a.part_o = static_cast<uint64_t*>(part);
     a.part_ml = a.part_o + (size_t)M * H * a.R * HD;
+    a.looks = (uint32_t)looks; a.look_mask = looks >= 255 ? 255 : 0;
     a.sync = sync; a.kv_len = kv_len;
     a.cos_t = cos_t; a.sin_t = sin_t; a.status = status;
     for (int g = 0; g < n_groups; g++) {

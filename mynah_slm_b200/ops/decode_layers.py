@@ -42,6 +42,8 @@ class DecodeLayers:
     # Tags that launches may use before the words are cleared and the tags begin again at 1: a tag names one stage of one launch as
     # long as 32 bits do not wrap (74 million steps of 28 layers, ten hours of steps of 0.5 ms).
     TAG_LIMIT = 2 ** 32 - 1
+    # Looks at a word that has not come after which a wait is given up (a second and more).
+    WAIT_LOOKS = 1 << 22
 
     def __init__(self, rows, sizes: dict, groups: list, device):
         self.host_table = torch.tensor(rows, dtype=torch.int64)                 # [layers, 12]
@@ -166,7 +168,8 @@ class DecodeLayers:
             "mynah_decode_layers", ptr(self.table[layers.start]), ptr(self.host_table[layers.start]), len(layers),
             M, z["D"], z["H"], z["KV"], z["HD"], z["F"], S, ptr(x), ptr(self.words), ptr(part), part.numel(), ptr(self.sync),
             z["gain_dtype"], z["eps"], z["qk_dtype"], z["qk_eps"], ptr(cos), ptr(sin), cos.shape[0] if cos is not None else 0,
-            ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, stream_ptr())
+            ptr(ctx.kv_len), len(self.groups), (ctypes.c_longlong * len(words))(*words), ptr(ctx.status), runtime.sm_count, self.WAIT_LOOKS,
+            stream_ptr())
         if self.declined and layers.start > 0:
             raise KernelError("decode_layers: declined behind the first layers of a step")
         return not self.declined

@@ -74,7 +74,7 @@ _SIGNATURES: dict[str, list] = {
     "mynah_decode_layers_supported": [c_int] * 8,
     "mynah_decode_layers": [P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                             P, P, P, c_longlong, P, c_int, c_float, c_int, c_float, P, P, c_int,
-                            P, c_int, P, P, c_int, P],
+                            P, c_int, P, P, c_int, c_int, P],
     "mynah_gemv_decode": [P, c_int, c_int, c_int, P, P, P, P, P, c_int, c_float, P, c_int, c_int, c_int, P],
     "mynah_gemm_tcgen05": [P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
     "mynah_argmax": [P, c_int, c_int, c_int, P, P],

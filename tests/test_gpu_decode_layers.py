@@ -222,3 +222,36 @@ def test_a_declined_launch_leaves_the_layers_one_by_one(tmp_path, monkeypatch, g
         rows.append([eng.step([StepEntry(slot, [t], (0,))], taps={} if i == 3 else None).cpu().numpy() for i, t in enumerate(toks[70:])])
         eng.check_status()
     assert len(offered) == 1 and all(np.array_equal(a, b) for a, b in zip(*rows))
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_a_wait_that_is_given_up_is_reported_and_over(tmp_path, graphs):
+    """With no patience at all a step gives up the first wait for another CTA's words: it ends, says so, and the steps after it are
+    as ever (the tags have moved on, nothing that it left passes for a later step's)."""
+    from mynah_slm_b200.engine.engine import Engine, EngineError, StepEntry
+    cfg = _cfg(2, 1024, 16, 8, 128, 3072)
+    folder = make_folder(tmp_path, "one", torch.bfloat16, config=cfg, seed=3)
+    lens = [300, 20, 700]
+    seqs = [np.random.default_rng(n).integers(0, cfg["vocab_size"], size=n + 2).tolist() for n in lens]
+
+    def steps(eng):
+        slots = [eng.open_sequence() for _ in lens]
+        for s, q in zip(slots, seqs):
+            eng.step([StepEntry(s, q[:-2], ())])
+        out = [eng.step([StepEntry(s, [q[i]], (0,)) for s, q in zip(slots, seqs)]).cpu().numpy() for i in (-2, -1)]
+        for s in slots:
+            eng.close_sequence(s)
+        return out
+    engines = [Engine.from_folder(folder, dtype="bfloat16", max_tokens=1280, max_seqs=3, use_graphs=graphs) for _ in range(2)]
+    want = steps(engines[0])
+    want = steps(engines[0])                             # (the second time prompts are captured, too)
+    engines[0].check_status()
+    eng = engines[1]
+    eng.decode_layers.WAIT_LOOKS = 0
+    steps(eng)
+    with pytest.raises(EngineError, match="a bounded wait inside a kernel ran out"):
+        eng.check_status()
+    eng.decode_layers.WAIT_LOOKS = type(eng.decode_layers).WAIT_LOOKS
+    eng._graphs.clear()                                  # (they were captured with no patience)
+    assert all(np.array_equal(a, b) for a, b in zip(want, steps(eng)))
+    eng.check_status()
