@@ -5,7 +5,7 @@
 // What bounds such a step is the one pass over the weights and the cache (31 MB and up a layer at the 0.6B shape: 5 us),
 // but as seven launches a layer it took 29 us at one row: each kernel ends, drains and starts before the next one's loads
 // begin. Here one CTA an SM stays for the whole step. A producer warp walks all of the CTA's weights and cache pages in the
-// order they are used, copying them by TMA into a ring of shared-memory slots, never waiting for activations: 176 KB an SM
+// order they are used, copying them by TMA into a ring of shared-memory slots, never waiting for activations: 160 KB an SM
 // are under way while the other warps exchange activations.
 //
 // What the CTAs exchange (a few KB a row and stage) goes through L2 in words of 64 bits, 32 of data and 32 of a tag that
@@ -17,8 +17,8 @@
 // A product's unit is eight output rows of the weights: 1,024 outputs make 128 units, so the narrow products still use 128
 // SMs without splitting a sum across CTAs. Within the CTA every warp multiplies its 128 of a slot's 1,024 columns
 // (mma.sync m16n8k16, two units as the 16 rows, the step's rows as the 8 columns, fp32 sums) and the eight partial sums are
-// added in a fixed order. A row's bits do not depend on the other rows of the launch. Who owns a column of the residual stream publishes it
-// times the norm's gain, and its share of the row's squares; 1/rms is a factor on the finished sums.
+// added in a fixed order. A row's bits do not depend on the other rows of the launch. Who owns a column of the residual stream
+// publishes it times the norm's gain, and its share of the row's squares; 1/rms is a factor on the finished sums.
 //
 // Attention's jobs are runs of two or four pages of a (sequence, kv head), cut by the sequence's own page count, four warps a job:
 // each warp keeps its own 16 keys of every page, with a running maximum, and meets the others once a run. The warps that have a
@@ -28,6 +28,8 @@
 // warps leave 168 a thread. (Sixteen multiplying warps at 96 spilled, and beside this much shared memory L1 holds no spills:
 // 28 us a layer.)
 #include "attn_page.cuh"
+#include "head_prep.cuh"
+#include "tcgen05.cuh"
 
 #include <cuda.h>
 
