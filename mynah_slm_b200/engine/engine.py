@@ -172,7 +172,8 @@ class _PromptGraph:
 # Measured at 33 pages a sequence: splits of 64 / 48 / 40 give 1.371 / 1.364 / 1.355 ms a step at batch 8 and
 # 3.97 / 3.88 / 3.84 at batch 64; every new size is a capture (a step run twice), so not finer than 16.
 PAGE_BUCKET_STEP = int(os.environ.get("MYNAH_PAGE_BUCKET_STEP", "16"))
-# Captured decode steps of at most this many rows ask for the next layer's weights ahead of time (0: never).
+# Captured decode steps of at most this many rows whose layers run one by one ask for the next layer's weights ahead of time
+# (0: never).
 # Measured at the 0.6B shape: one row 0.988 -> 0.969 ms a step; eight rows 1.355 -> 1.569 ms (the second stream's
 # edges into the chain cost more than the L2 hits save, and the attention's pages push the weights out again).
 L2_PREFETCH_MAX_ROWS = int(os.environ.get("MYNAH_L2_PREFETCH_MAX_ROWS", "2"))
@@ -396,7 +397,8 @@ class Engine:
         results, the debugging taps of the reference (mynah-slm src/arch_qwen3.h:15-18, 46-49: on_embed,
         on_layer, on_final): "embed" [T, hidden], "layer<i>" [T, hidden] for run i of the schedule (the residual
         stream behind it), "final_norm" [wanted rows, hidden] (each wanted row once, ascending). Such a step
-        runs kernel by kernel, not from a captured graph, and needs at least one wanted place."""
+        runs launch by launch, not from a captured graph, and needs at least one wanted place. A decode step that would run all
+        layers in one launch makes one for every layer then, with the same bits."""
         self._validate(entries)
         if taps is not None and not any(len(e.want) for e in entries):
             raise EngineError("a step with taps needs at least one wanted place")

@@ -23,8 +23,9 @@ KERNEL_ROWS = 8         # rows that the kernel takes at most
 # Rows up to which a step takes the one launch. 0: never.
 MAX_ROWS = 8
 # And rows times the widest product's columns: every CTA reads all of a product's rows, twice their size with the tags. One launch
-# against the layers one by one, ms a step: 0.6B shape (3,072 columns) 1 row 0.50 / 0.87, 3 rows 0.66 / 1.01, 8 rows 0.76 / 1.01;
-# 4B shape's first 8 layers (9,728 columns) 1 row 0.56 / 0.80, 4 rows 0.60 / 0.70, 8 rows 0.68 / 0.75. Wider ones are not measured.
+# against the layers one by one, ms a step behind 200 positions with a vocabulary of 8,192: 0.6B shape (3,072 columns) 1 row
+# 0.56 / 0.80, 3 rows 0.61 / 0.99, 8 rows 0.67 / 1.02; 4B shape's first 8 layers (9,728 columns) 1 row 0.45 / 0.70, 4 rows
+# 0.47 / 0.57, 8 rows 0.51 / 0.59. Wider ones are not measured.
 MAX_ROW_COLUMNS = 8 * 9728
 # And rows times the longest sequence's pages, by head size: behind long caches the page loop and the merge of the runs bound a
 # layer, where the layers one by one stream pages with three CTAs an SM. ms a step, one launch / one by one, 0.6B shape: heads of 128,
