@@ -282,7 +282,12 @@ MYNAH_API int mynah_gemm_f32(const float* A, const float* W, float* C, int M, in
     MYNAH_REQUIRE(lda >= K && ldw >= K && ldc >= N, "gemm_f32: a leading dimension is smaller than its row");
     MYNAH_REQUIRE(ceil_div(M, BM) <= GRID_ROWS, "gemm_f32: %d rows exceed one launch (%d)", M, GRID_ROWS * BM);
     const bool vec = K % 4 == 0 && lda % 4 == 0 && ldw % 4 == 0 && ((uintptr_t)A | (uintptr_t)W) % 16 == 0;
-    if (!vec) {
+    // A single slab of 32 k or less: a step's rows would be multiplied with four times as many zeros. us a product of K = 32, general
+    // kernel / few rows: 16 x 16,384 4.8 / 8.1, 12 x 3,072 3.6 / 4.0, 8 x 3,072 3.6 / 3.9, 5 x 16,384 4.7 / 5.4, 4 x 16,384 4.7 / 5.0;
+    // 5 x 6,144 3.6 / 3.4, 4 x 6,144 3.6 / 3.3, 2 x 16,384 4.6 / 4.0. (Leaving the zeros out in that kernel costs one row of
+    // K = 1,024 to 3,072 10%.)
+    const bool thin = K <= 32 && M <= ROW_MAX_M && (M >= 8 ? N >= 3072 : (long long)M * N > 32768);
+    if (!vec || thin) {
         const dim3 grid(ceil_div(N, BN), ceil_div(M, BM));
         gemm_f32_kernel<<<grid, 256, 0, stream>>>(A, W, C, M, N, K, lda, ldw, ldc);
         return mynah_check_launch("gemm_f32");
