@@ -25,13 +25,16 @@ MAX_ROWS = 8
 # And rows times the widest product's columns: every CTA reads all of a product's rows, twice their size with the tags. One launch
 # against the layers one by one, ms a step behind 200 positions with a vocabulary of 8,192: 0.6B shape (3,072 columns) 1 row
 # 0.56 / 0.80, 3 rows 0.61 / 0.99, 8 rows 0.67 / 1.02; 4B shape's first 8 layers (9,728 columns) 1 row 0.45 / 0.70, 4 rows
-# 0.47 / 0.57, 8 rows 0.51 / 0.59. Wider ones are not measured.
+# 0.47 / 0.57, 8 rows 0.51 / 0.59; 8B shape's first 6 layers (12,288 columns) 1 row 0.51 / 0.84, 4 rows 0.53 / 0.69; 4 layers of 5,120
+# with 25,600 columns 1 row 0.74 / 1.24, 2 rows 0.75 / 1.27; 4 layers of 2,048 with 32,768 columns 2 rows 0.37 / 0.53.
 MAX_ROW_COLUMNS = 8 * 9728
-# And rows times the longest sequence's pages, by head size: behind long caches the page loop and the merge of the runs bound a
+# And rows times the longest sequence's pages times kv heads (at least 8), by head size: behind long caches the page loop and the merge of the runs bound a
 # layer, where the layers one by one stream pages with three CTAs an SM. ms a step, one launch / one by one, 0.6B shape: heads of 128,
 # 8 rows x 250 pages 3.13 / 3.51, x 313 3.92 / 4.12, x 438 5.55 / 5.33, x 625 8.12 / 7.23; 4 rows x 625 3.99 / 4.35; 1 row x 625
-# 1.70 / 2.23, x 1,016 2.46 / 3.03. Heads of 64, 8 rows x 250 2.62 / 2.70, x 625 6.98 / 5.26; 2 rows x 625 2.05 / 2.34.
-MAX_ROW_PAGES = {64: 2048, 128: 2944}
+# 1.70 / 2.23, x 1,016 2.46 / 3.03. Heads of 64, 8 rows x 250 2.62 / 2.70, x 625 6.98 / 5.26; 2 rows x 625 2.05 / 2.34. 12 layers of 32
+# kv heads of 64, 8 rows x 33 0.89 / 1.07, x 64 1.30 / 1.20, x 250 4.82 / 2.88. Two kv heads, 8 rows x 250: 1.34 / 1.46. (Heads of
+# 128 with more than 8 kv heads go by the same count and are not measured.)
+MAX_PAGE_TILES = {64: 14336, 128: 23552}
 
 
 def most_runs(pages: int) -> int:
@@ -125,7 +128,7 @@ class DecodeLayers:
             return False
         # (Beyond what the tensor-core kernels' merge takes the layers one by one have the general kernel only: 4B shape's first 8
         # layers, 8 rows x 625 pages 2.80 / 12.75.)
-        return rows * ctx.decode_splits <= MAX_ROW_PAGES[z["HD"]] or not _tc_fits(z["H"], z["KV"], ctx.decode_splits)
+        return rows * ctx.decode_splits * max(z["KV"], 8) <= MAX_PAGE_TILES[z["HD"]] or not _tc_fits(z["H"], z["KV"], ctx.decode_splits)
 
     def count_launch(self, layers: Optional[int] = None) -> None:
         """To be called before every launch, replayed ones too, on the launch's stream: keeps the tags from wrapping, after which

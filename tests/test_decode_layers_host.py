@@ -112,9 +112,10 @@ def test_padded_and_unpadded_steps_take_the_same_route(steps):
 def test_long_caches_take_the_layers_one_by_one(steps):
     """Where the one launch measured slower; not where the layers one by one would have the general attention kernel only."""
     plan, made = steps
-    for heads, dim, rows, pages, one in [(16, 128, 8, 368, True), (16, 128, 8, 384, False), (16, 128, 4, 736, True), (16, 128, 1, 1008, True),
-                                         (16, 64, 8, 256, True), (16, 64, 8, 272, False), (32, 128, 8, 512, False), (32, 128, 8, 528, True)]:
-        plan.sizes.update(H=heads, KV=8, HD=dim)
+    for heads, dim, rows, pages, one in [(4, 128, 8, 368, True), (4, 128, 8, 384, False), (16, 128, 8, 368, True), (16, 128, 8, 384, False), (16, 128, 4, 736, True), (16, 128, 1, 1008, True),
+                                         (16, 64, 8, 224, True), (16, 64, 8, 240, False), (32, 128, 8, 512, False), (32, 128, 8, 528, True),
+                                         (64, 64, 8, 48, True), (64, 64, 8, 64, False), (64, 64, 4, 112, True), (64, 64, 1, 448, True)]:
+        plan.sizes.update(H=heads, KV={4: 2, 64: 32}.get(heads, 8), HD=dim)
         assert plan.takes(_ctx(rows, pages)) is one
 
 
