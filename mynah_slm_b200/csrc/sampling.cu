@@ -11,6 +11,10 @@
 // Mass is summed as 2^-60 fixed point in 64-bit integers: integer sums do not
 // depend on the order of the additions, so the same logits and the same
 // generator state give the same token in every run.
+//
+// What bounds a draw is latency: a row of 151,936 logits is 0.6 MB, and what follows its one read is a chain of block and
+// cluster barriers. So a draw is one launch (penalties, maximum, exponentials, selection, the walk and the ring), a row is
+// read once, into the shared memory of its cluster's CTAs, and every later pass goes over that copy.
 #include "common.cuh"
 
 #include <cooperative_groups.h>
@@ -19,13 +23,21 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr int THREADS = 1024;
+constexpr int THREADS = 512;
+constexpr int WARPS = THREADS / 32;
 constexpr int ROW_CTAS = 8;            // CTAs (one cluster) that share a row of a large vocabulary
 constexpr int LOADS = 8;               // loads of a row that a thread keeps in flight
 constexpr int BINS = 2048;
+constexpr int MAX_CAND = 256;          // a top-k of at most this many entries is drawn from a list of candidates
 
+// floor(p * 2^60): for a probability (0 <= p <= 1) a shift of its mantissa, exactly what the product in double gives
 __device__ __forceinline__ unsigned long long mass_of(float p) {
-    return __double2ull_rd((double)p * 1152921504606846976.0);     // p * 2^60
+    const unsigned int bits = __float_as_uint(p);
+    const int e = (int)(bits >> 23);
+    if (e > 127) return __double2ull_rd((double)p * 1152921504606846976.0);       // (not a probability: infinite or no number)
+    const unsigned long long m = e > 0 ? (bits & 0x7fffffu) | 0x800000u : 0u;      // (a subnormal's product lies below 1)
+    const int s = e - 90;                                                          // p = m * 2^(e - 150)
+    return s >= 0 ? m << s : (s > -24 ? m >> -s : 0ull);
 }
 
 struct Prefix {            // a prefix of the sorted order
@@ -35,38 +47,62 @@ struct Prefix {            // a prefix of the sorted order
     unsigned long long mass;   // its total mass
 };
 
-struct Shared {
-    unsigned int count[BINS];
-    // a digit's mass (2^-60 fixed point) as two 32-bit words: 32-bit adds are native atomics in shared memory,
-    // 64-bit ones are compare-and-swap loops that crawl when many warps hit one digit
-    unsigned int mass_lo[BINS], mass_hi[BINS];
-    unsigned int warp_count[32];
-    unsigned long long warp_mass[32];
-    // results handed from the finding thread to the block (and, in a cluster, read by the other CTAs); two
-    // sets used in turn, so that one pass's results can still be read while the next pass starts
-    unsigned int found_digit[2], found_above[2], found_count[2];
-    unsigned long long found_mass[2];
-    unsigned int turn;                 // passes done so far (selects the set)
-    double part_d;                     // this CTA's share of a sum over the row
-    unsigned long long part_m;         // this CTA's share of the row's mass
-    unsigned int part_u;
-    float red_f[32];
-    int red_i[32];
-    double red_d[32];
-    unsigned int scan_u[32];
+struct Found {
+    unsigned int digit, above, count;                       // the digit, the elements in larger digits, those in it
+    unsigned long long mass;                                // mass of the elements in larger digits
 };
 
-__device__ __forceinline__ void add_mass(Shared& sh, unsigned int d, unsigned long long m) {
+// Elements of one digit share every bit from `shift` up, their exponent E among them, so where mass_of shifts a mantissa up
+// (E >= 90) a digit's mass follows from its count and the sum of the bits below `shift`. That sum is kept in two words, its
+// elements' low eleven bits and the rest: adds whose result nobody reads, and none that carries. Where mass_of shifts down,
+// or for what is no probability, the words are the low and high half of the masses' own sum (2^-60 fixed point). 64-bit adds
+// in shared memory would be compare-and-swap loops that crawl when many warps hit one digit.
+struct Histogram {
+    unsigned int count[BINS];
+    unsigned int lo[BINS], hi[BINS];
+};
+constexpr int LOW_BITS = 11;
+__device__ __forceinline__ bool mass_by_count(unsigned int bits) { return (bits >> 23) - 90u <= 127u - 90u; }
+
+template <int NC>
+struct Shared {
+    // The row's first maxima a group of threads, of all CTAs: their largest is the row's maximum, and the k-th largest of
+    // them is a lower bound of the row's k-th largest element.
+    static constexpr int GROUPS = 256, LANES = NC * THREADS / GROUPS;
+    __align__(16) float group_v[GROUPS];
+    int group_i[GROUPS];
+    union {
+        Histogram h;
+        unsigned long long list[NC][MAX_CAND];              // leading CTA: the candidates of every CTA
+    };
+    unsigned long long mine[MAX_CAND];                      // this CTA's candidates
+    unsigned long long key[MAX_CAND], sorted[MAX_CAND];
+    double part_d[NC];                                      // every CTA's sum of exponentials
+    unsigned long long part_m[NC];                          // a value a CTA: masses
+    unsigned int part_u[NC], part_v[NC];                    // a value a CTA: counts
+    Found found;
+    unsigned int n_mine, n_key;
+    float mx, bound;
+    int best, id;
+    double red_d[WARPS];
+    unsigned long long warp_mass[WARPS];
+    unsigned int warp_count[WARPS], scan_u[WARPS];
+    int ring[256];
+};
+
+struct ArgmaxShared {
+    float red_f[32];
+    int red_i[32];
+};
+
+__device__ __forceinline__ void add_mass(Histogram& h, unsigned int d, unsigned long long m) {
     const unsigned int lo = (unsigned int)m;
     unsigned int hi = (unsigned int)(m >> 32);
     if (lo != 0) {
-        const unsigned int old = atomicAdd(&sh.mass_lo[d], lo);
+        const unsigned int old = atomicAdd(&h.lo[d], lo);
         hi += old > 0xffffffffu - lo;                      // the low word wrapped: carry
     }
-    if (hi != 0) atomicAdd(&sh.mass_hi[d], hi);
-}
-__device__ __forceinline__ unsigned long long mass_at(const Shared& sh, int d) {
-    return ((unsigned long long)sh.mass_hi[d] << 32) | sh.mass_lo[d];
+    if (hi != 0) atomicAdd(&h.hi[d], hi);
 }
 
 // A row is shared by NC CTAs (NC = 1, or the ROW_CTAS CTAs of a cluster): CTA r works on the elements
@@ -74,16 +110,13 @@ __device__ __forceinline__ unsigned long long mass_at(const Shared& sh, int d) {
 // the same code with the same decisions, so the cluster barriers below are reached by all of them.
 template <int NC>
 struct RowShare {
-    int rank, begin, end;                                   // this CTA's elements
-    __device__ RowShare(int V) {
-        if (NC == 1) {
-            rank = 0; begin = 0; end = V;
-        } else {
-            rank = (int)cg::this_cluster().block_rank();
-            const int chunk = ((V + NC - 1) / NC + 3) & ~3;
-            begin = min(V, rank * chunk);
-            end = min(V, begin + chunk);
-        }
+    int rank, begin, n;                                     // this CTA's elements: `n` from `begin` on
+    float* p;                                               // where it keeps them: shared memory, or the row itself if too long
+    __device__ static int chunk(int V) { return NC == 1 ? V : ((V + NC - 1) / NC + 3) & ~3; }
+    __device__ explicit RowShare(int V) {
+        rank = NC == 1 ? 0 : (int)cg::this_cluster().block_rank();
+        begin = min(V, rank * chunk(V));
+        n = min(V, begin + chunk(V)) - begin;
     }
     __device__ __forceinline__ void sync() const {
         if (NC == 1) __syncthreads();
@@ -94,233 +127,250 @@ struct RowShare {
     }
 };
 
-struct Found {
-    unsigned int digit, above, count;                       // the digit, the elements in larger digits, those in it
-    unsigned long long mass;                                // mass of the elements in larger digits
+// What a pass of the search goes by: the elements p[i] * scale whose bits under `mask` are `bits`, by their next digit, the bits
+// [shift, shift + log2(n_bins)). Three passes: 11, 11 and 10 bits.
+struct Digit {
+    unsigned int bits, mask;
+    int shift, n_bins;
 };
 
-// Finds the digit where the running (count, mass), taken from the largest digit down, first satisfies the
-// target, among elements whose higher bits equal `prefix_bits` under `prefix_mask`. by_mass: cum_mass >=
-// target_mass; else cum_count >= target_count. The carried count and mass are those of the elements in larger
-// digits of earlier passes. Every thread of every CTA of the row gets the result.
+// A CTA's slice of the digits over all CTAs of the row: rank r has the r-th slice from the top, its thread t the digits
+// [hi - PER + 1, hi], taken from the largest down.
 template <int NC>
-__device__ Found radix_pass(const float* __restrict__ p, const RowShare<NC>& rs, unsigned int prefix_bits, unsigned int prefix_mask,
-                            int shift, int n_bins, bool by_mass, unsigned int target_count,
-                            unsigned long long target_mass, unsigned int carry_count, unsigned long long carry_mass,
-                            Shared& sh, float scale = 1.0f) {                // the elements are p[i] * scale (1: as stored)
+struct Slice {
+    static constexpr int WIDE = BINS / NC, PER = (WIDE + THREADS - 1) / THREADS;
+    int hi;
+    unsigned int c[PER];
+    unsigned long long m[PER];
+};
+
+// Counts and masses of a pass. Probabilities crowd into a few digits where the logits do: a warp whose 32 elements fall into
+// at most four digits adds each digit up over the warp and lets one lane do the atomics. Counts and masses are integers, so
+// the order of the additions does not matter.
+template <int NC>
+__device__ __noinline__ void fill_histogram(const RowShare<NC>& rs, const Digit dg, float scale, Shared<NC>& sh) {
     for (int i = threadIdx.x; i < BINS; i += THREADS) {
-        sh.count[i] = 0;
-        sh.mass_lo[i] = 0;
-        sh.mass_hi[i] = 0;
+        sh.h.count[i] = 0;
+        sh.h.lo[i] = 0;
+        sh.h.hi[i] = 0;
     }
-    __syncthreads();                                        // (the previous pass's advance of `turn` is visible from here on)
-    const unsigned int set = sh.turn & 1u;                  // advanced only after this pass's last barrier
-    if (threadIdx.x == 0) {
-        sh.found_digit[set] = 0;                            // the smallest digit, when the target is never met
-        sh.found_above[set] = 0xffffffffu;
-    }
-    // Probabilities crowd into a few digits where the digit is the exponent (the first pass): a warp whose 32
-    // elements fall into at most four digits adds each digit's count and mass up with shuffles and lets one lane
-    // do the atomics; a warp whose elements are spread out (the mantissa passes) uses plain atomics. Counts
-    // and masses are integers, so the order of the additions does not matter. A row of a large vocabulary
-    // comes from L2, a round trip a load: eight loads a thread are issued together.
-    const int lane_h = threadIdx.x & 31;
-    for (int base0 = rs.begin; base0 < rs.end; base0 += THREADS * LOADS) {    // the same number of turns for every thread
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const unsigned int low_mask = (1u << dg.shift) - 1u;
+    for (int base0 = 0; base0 < rs.n; base0 += THREADS * LOADS) {             // the same number of turns for every thread
         float vals[LOADS];
 #pragma unroll
         for (int u = 0; u < LOADS; u++) {
             const int i = base0 + u * THREADS + (int)threadIdx.x;
-            vals[u] = i < rs.end ? p[i] : 0.f;
+            vals[u] = i < rs.n ? rs.p[i] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < LOADS; u++) {
             const int i = base0 + u * THREADS + (int)threadIdx.x;
-            if (base0 + u * THREADS >= rs.end) break;             // uniform
-            bool on = false;
-            unsigned int d = 0xffffffffu;
-            unsigned long long ms = 0;
-            if (i < rs.end) {
-                const float v = vals[u] * scale;
-                const unsigned int bits = __float_as_uint(v);
-                if ((bits & prefix_mask) == prefix_bits) {
-                    on = true;
-                    d = (bits >> shift) & (n_bins - 1);
-                    ms = mass_of(v);
-                }
-            }
-            const unsigned int peers = __match_any_sync(0xffffffffu, d);
-            const bool leader = on && lane_h == __ffs(peers) - 1;
-            const unsigned int leaders = __ballot_sync(0xffffffffu, leader);
-            if (__popc(leaders) <= 4) {
-                unsigned int rem = leaders;
-                while (rem) {                                     // uniform over the warp
-                    const int src = __ffs(rem) - 1;
-                    rem &= rem - 1;
-                    const unsigned int grp = __shfl_sync(0xffffffffu, peers, src);
-                    unsigned long long m = ((grp >> lane_h) & 1u) ? ms : 0ull;
+            if (base0 + u * THREADS >= rs.n) break;               // uniform
+            const float v = vals[u] * scale;
+            const unsigned int bits = __float_as_uint(v);
+            const bool on = i < rs.n && (bits & dg.mask) == dg.bits;
+            const unsigned int active = __ballot_sync(0xffffffffu, on);
+            if (active == 0u) continue;                           // (most warps, once a prefix is known)
+            const unsigned int d = (bits >> dg.shift) & (dg.n_bins - 1);
+            // the first element's digit, then the first of what is left: two turns tell a crowd from a spread
+            unsigned int left = active;
 #pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) m += __shfl_xor_sync(0xffffffffu, m, o);
-                    if (lane_h == src) {
-                        atomicAdd(&sh.count[d], (unsigned int)__popc(grp));
-                        add_mass(sh, d, m);
+            for (int t = 0; t < 2; t++) {
+                if (__popc(left) >= 8) {                          // uniform
+                    const int src = __ffs(left) - 1;
+                    const unsigned int ds = __shfl_sync(0xffffffffu, d, src);
+                    const bool same = ((left >> lane) & 1u) && d == ds;
+                    const unsigned int grp = __ballot_sync(0xffffffffu, same);
+                    const unsigned int bs = __shfl_sync(0xffffffffu, bits, src);
+                    if (__popc(grp) >= 8 && (mass_by_count(bs))) {
+                        const unsigned int low = same ? bits & low_mask : 0u;
+                        const unsigned int lo = __reduce_add_sync(0xffffffffu, low & ((1u << LOW_BITS) - 1u));
+                        const unsigned int hi = __reduce_add_sync(0xffffffffu, low >> LOW_BITS);
+                        if (lane == src) {
+                            atomicAdd(&sh.h.count[ds], (unsigned int)__popc(grp));
+                            if (lo) atomicAdd(&sh.h.lo[ds], lo);
+                            if (hi) atomicAdd(&sh.h.hi[ds], hi);
+                        }
+                        left &= ~grp;
                     }
                 }
-            } else if (on) {
-                atomicAdd(&sh.count[d], 1u);
-                add_mass(sh, d, ms);
+            }
+            if ((left >> lane) & 1u) {
+                atomicAdd(&sh.h.count[d], 1u);
+                if (mass_by_count(bits)) {
+                    const unsigned int low = bits & low_mask, lo = low & ((1u << LOW_BITS) - 1u), hi = low >> LOW_BITS;
+                    if (lo) atomicAdd(&sh.h.lo[d], lo);
+                    if (hi) atomicAdd(&sh.h.hi[d], hi);
+                } else {
+                    add_mass(sh.h, d, mass_of(v));
+                }
             }
         }
     }
+}
+
+// This CTA's slice of a pass over the row. The histograms may be filled again behind find_digit's first barrier.
+template <int NC>
+__device__ __forceinline__ Slice<NC> add_up(const RowShare<NC>& rs, const Digit dg, float scale, Shared<NC>& sh) {
+    fill_histogram<NC>(rs, dg, scale, sh);
     rs.sync();                                              // every CTA's histogram is complete
-    if (NC > 1) {
-        // the histograms are added up a slice of digits a CTA (all CTAs at once), the totals go to the leading CTA
-        const int per_cta = (n_bins + NC - 1) / NC;
-        const int i = rs.rank * per_cta + (int)threadIdx.x;
-        const bool mine = (int)threadIdx.x < per_cta && i < n_bins;
-        unsigned int ct = 0;
-        unsigned long long mt = 0;
-        if (mine) {
+    Slice<NC> s;
+    s.hi = dg.n_bins - 1 - (rs.rank * Slice<NC>::WIDE + (int)threadIdx.x * Slice<NC>::PER);
+#pragma unroll
+    for (int q = 0; q < Slice<NC>::PER; q++) {
+        const int d = s.hi - q;
+        s.c[q] = 0;
+        s.m[q] = 0;
+        if ((int)threadIdx.x * Slice<NC>::PER < Slice<NC>::WIDE && d >= 0) {
             unsigned int c[NC], lo[NC], hi[NC];
 #pragma unroll
             for (int r = 0; r < NC; r++) {                  // the loads first, all in flight together
-                c[r] = *rs.at(&sh.count[i], r);
-                lo[r] = *rs.at(&sh.mass_lo[i], r);
-                hi[r] = *rs.at(&sh.mass_hi[i], r);
+                c[r] = *rs.at(&sh.h.count[d], r);
+                lo[r] = *rs.at(&sh.h.lo[d], r);
+                hi[r] = *rs.at(&sh.h.hi[d], r);
             }
+            unsigned long long lows = 0, masses = 0;
 #pragma unroll
             for (int r = 0; r < NC; r++) {
-                ct += c[r];
-                mt += ((unsigned long long)hi[r] << 32) | lo[r];
+                s.c[q] += c[r];
+                lows += lo[r] + ((unsigned long long)hi[r] << LOW_BITS);
+                masses += ((unsigned long long)hi[r] << 32) | lo[r];
             }
-        }
-        rs.sync();                                          // every digit of every CTA has been read: they may be overwritten
-        if (mine) {
-            *rs.at(&sh.count[i], 0) = ct;
-            *rs.at(&sh.mass_lo[i], 0) = (unsigned int)mt;
-            *rs.at(&sh.mass_hi[i], 0) = (unsigned int)(mt >> 32);
-        }
-        rs.sync();                                          // the leading CTA's histogram holds the row's totals
-    }
-    if (rs.rank == 0) {
-        // scan from the largest digit down: thread t owns digits n_bins-1-2t and n_bins-2-2t
-        const int d0 = n_bins - 1 - 2 * (int)threadIdx.x, d1 = d0 - 1;
-        const unsigned int c0 = d0 >= 0 ? sh.count[d0] : 0, c1 = d1 >= 0 ? sh.count[d1] : 0;
-        const unsigned long long m0 = d0 >= 0 ? mass_at(sh, d0) : 0, m1 = d1 >= 0 ? mass_at(sh, d1) : 0;
-        unsigned int cs = c0 + c1;
-        unsigned long long ms = m0 + m1;
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned int c = __shfl_up_sync(0xffffffffu, cs, o);
-            const unsigned long long m = __shfl_up_sync(0xffffffffu, ms, o);
-            if (lane >= o) {
-                cs += c;
-                ms += m;
-            }
-        }
-        if (lane == 31) {
-            sh.warp_count[warp] = cs;
-            sh.warp_mass[warp] = ms;
-        }
-        __syncthreads();
-        unsigned int cbase = carry_count;
-        unsigned long long mbase = carry_mass;
-        for (int w = 0; w < warp; w++) {
-            cbase += sh.warp_count[w];
-            mbase += sh.warp_mass[w];
-        }
-        // exclusive values before this thread's first digit
-        const unsigned int c_before = cbase + cs - (c0 + c1);
-        const unsigned long long m_before = mbase + ms - (m0 + m1);
-        auto met = [&](unsigned int c, unsigned long long m) {
-            return by_mass ? (m >= target_mass) : (c >= target_count);
-        };
-        if (c0 > 0 && !met(c_before, m_before) && met(c_before + c0, m_before + m0)) {
-            sh.found_digit[set] = (unsigned int)d0;
-            sh.found_above[set] = c_before;
-            sh.found_mass[set] = m_before;
-            sh.found_count[set] = c0;
-        } else if (c1 > 0 && !met(c_before + c0, m_before + m0) && met(c_before + c0 + c1, m_before + m0 + m1)) {
-            sh.found_digit[set] = (unsigned int)d1;
-            sh.found_above[set] = c_before + c0;
-            sh.found_mass[set] = m_before + m0;
-            sh.found_count[set] = c1;
-        }
-        __syncthreads();
-        if (sh.found_above[set] == 0xffffffffu) {
-            // target beyond everything (rounding): end at the smallest populated digit
-            if (threadIdx.x == 0) {
-                int d = 0;
-                while (d < n_bins - 1 && sh.count[d] == 0) d++;
-                unsigned int c = carry_count;
-                unsigned long long m = carry_mass;
-                for (int e = n_bins - 1; e > d; e--) {
-                    c += sh.count[e];
-                    m += mass_at(sh, e);
-                }
-                sh.found_digit[set] = (unsigned int)d;
-                sh.found_above[set] = c;
-                sh.found_mass[set] = m;
-                sh.found_count[set] = sh.count[d];
-            }
+            const unsigned int base = dg.bits | ((unsigned int)d << dg.shift);     // the digit's smallest element
+            s.m[q] = mass_by_count(base)
+                ? ((unsigned long long)((base & 0x7fffffu) | 0x800000u) * s.c[q] + lows) << ((base >> 23) - 90u) : masses;
         }
     }
-    rs.sync();                                              // the result is there (in the leading CTA)
-    Found f;
-    f.digit = *rs.at(&sh.found_digit[set], 0);
-    f.above = *rs.at(&sh.found_above[set], 0);
-    f.count = *rs.at(&sh.found_count[set], 0);
-    f.mass = *rs.at(&sh.found_mass[set], 0);
-    __syncthreads();                                        // all of this CTA's threads have read `turn` and the result
-    if (threadIdx.x == 0) sh.turn++;                        // (the other set is used next; this one stays readable for the
-    return f;                                               //  CTAs that have not read it yet until the pass after next)
+    return s;
 }
 
-// The smallest prefix of the sorted order whose count reaches target_count
-// (by_mass false) or whose mass reaches target_mass (by_mass true).
+// Finds the digit where the running (count, mass), taken from the largest digit down, first satisfies the
+// target. by_mass: cum_mass >= target_mass; else cum_count >= target_count. The carried count and mass are those of the
+// elements in larger digits of earlier passes. Every thread of every CTA of the row gets the result. A CTA tells the others
+// its slice's totals; the one whose slice holds the digit tells them the result: two barriers over the cluster.
 template <int NC>
-__device__ Prefix find_prefix(const float* __restrict__ p, const RowShare<NC>& rs, bool by_mass, unsigned int target_count,
-                              unsigned long long target_mass, Shared& sh) {
-    unsigned int bits = 0, mask = 0, above = 0, n_eq = 0;
-    unsigned long long mass = 0;
+__device__ __noinline__ Found find_digit(const RowShare<NC>& rs, const Slice<NC>& s, bool by_mass, unsigned int target_count,
+                                         unsigned long long target_mass, unsigned int carry_count, unsigned long long carry_mass,
+                                         Shared<NC>& sh) {
+    constexpr int PER = Slice<NC>::PER;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int cs = 0;
+    unsigned long long ms = 0;
+#pragma unroll
+    for (int q = 0; q < PER; q++) {
+        cs += s.c[q];
+        ms += s.m[q];
+    }
+    const unsigned int c_own = cs;
+    const unsigned long long m_own = ms;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int ct = __shfl_up_sync(0xffffffffu, cs, o);
+        const unsigned long long mt = __shfl_up_sync(0xffffffffu, ms, o);
+        if (lane >= o) {
+            cs += ct;
+            ms += mt;
+        }
+    }
+    if (lane == 31) {
+        sh.warp_count[warp] = cs;
+        sh.warp_mass[warp] = ms;
+    }
+    __syncthreads();
+    unsigned int c_before = cs - c_own;                     // this slice's elements before the thread's digits
+    unsigned long long m_before = ms - m_own;
+    for (int w = 0; w < warp; w++) {
+        c_before += sh.warp_count[w];
+        m_before += sh.warp_mass[w];
+    }
+    if (threadIdx.x == THREADS - 1) {
+        for (int r = 0; r < NC; r++) {
+            *rs.at(&sh.part_u[rs.rank], r) = c_before + c_own;
+            *rs.at(&sh.part_m[rs.rank], r) = m_before + m_own;
+        }
+    }
+    rs.sync();                                              // every slice's totals are known; the histograms have been read
+    auto met = [&](unsigned int cc, unsigned long long mm) {
+        return by_mass ? (mm >= target_mass) : (cc >= target_count);
+    };
+    unsigned int ct = carry_count, c_slice = 0;
+    unsigned long long mt = carry_mass, m_slice = 0;
+    int owner = -1, last = -1;                              // the slice that meets the target; the lowest with an element
+    for (int r = 0; r < NC; r++) {
+        if (r == rs.rank) {
+            c_slice = ct;
+            m_slice = mt;
+        }
+        const unsigned int cn = ct + sh.part_u[r];
+        const unsigned long long mn = mt + sh.part_m[r];
+        if (owner < 0 && sh.part_u[r] > 0 && !met(ct, mt) && met(cn, mn)) owner = r;
+        if (sh.part_u[r] > 0) last = r;
+        ct = cn;
+        mt = mn;
+    }
+    c_before += c_slice;
+    m_before += m_slice;
+    const bool beyond = owner < 0;                          // target beyond everything (rounding): end at the smallest populated digit
+    if (rs.rank == (beyond ? last : owner)) {
+#pragma unroll
+        for (int q = 0; q < PER; q++) {
+            const unsigned int cn = c_before + s.c[q];
+            const unsigned long long mn = m_before + s.m[q];
+            if (s.c[q] > 0 && (beyond ? cn == ct : !met(c_before, m_before) && met(cn, mn))) {
+                const Found f{(unsigned int)(s.hi - q), c_before, s.c[q], m_before};
+                for (int r = 0; r < NC; r++) *rs.at(&sh.found, r) = f;
+            }
+            c_before = cn;
+            m_before = mn;
+        }
+    }
+    rs.sync();                                              // the result is there
+    return sh.found;                                        // (written again only behind the next search's first barrier)
+}
+
+constexpr Digit FIRST_DIGIT{0u, 0u, 21, 2048};
+
+// The smallest prefix of the sorted order whose count reaches target_count
+// (by_mass false) or whose mass reaches target_mass (by_mass true). `first`: the row's slice by FIRST_DIGIT.
+template <int NC>
+__device__ __noinline__ Prefix find_prefix(const RowShare<NC>& rs, const Slice<NC>& first, bool by_mass, unsigned int target_count,
+                                           unsigned long long target_mass, Shared<NC>& sh) {
     if (by_mass && target_mass == 0) target_mass = 1;      // a draw of exactly 0 takes the first element
     if (!by_mass && target_count == 0) target_count = 1;
-    const int shifts[3] = {21, 10, 0}, nb[3] = {2048, 2048, 1024};
-    for (int r = 0; r < 3; r++) {
-        const Found f = radix_pass<NC>(p, rs, bits, mask, shifts[r], nb[r], by_mass, target_count, target_mass, above, mass, sh);
-        bits |= f.digit << shifts[r];
-        mask |= (unsigned int)(nb[r] - 1) << shifts[r];
-        above = f.above;
-        mass = f.mass;
-        n_eq = f.count;
-    }
+    Found f = find_digit<NC>(rs, first, by_mass, target_count, target_mass, 0u, 0ull, sh);
+    Digit dg{f.digit << 21, 2047u << 21, 10, 2048};
+    f = find_digit<NC>(rs, add_up<NC>(rs, dg, 1.0f, sh), by_mass, target_count, target_mass, f.above, f.mass, sh);
+    dg = Digit{dg.bits | f.digit << 10, dg.mask | 2047u << 10, 0, 1024};
+    f = find_digit<NC>(rs, add_up<NC>(rs, dg, 1.0f, sh), by_mass, target_count, target_mass, f.above, f.mass, sh);
+    const unsigned int bits = dg.bits | f.digit, n_eq = f.count;
     // `bits` is the probability at which the prefix ends; n_eq elements have exactly it
     const unsigned long long pm = mass_of(__uint_as_float(bits));
     unsigned int ties;
     if (by_mass) {
-        if (pm == 0 || target_mass <= mass) ties = 1;
+        if (pm == 0 || target_mass <= f.mass) ties = 1;
         else {
-            const unsigned long long need = target_mass - mass;
+            const unsigned long long need = target_mass - f.mass;
             const unsigned long long t = (need + pm - 1) / pm;
             ties = (unsigned int)(t < 1 ? 1 : (t > n_eq ? n_eq : t));
         }
     } else {
-        ties = target_count > above ? target_count - above : 1;
+        ties = target_count > f.above ? target_count - f.above : 1;
         if (ties > n_eq) ties = n_eq;
     }
     if (ties < 1) ties = 1;
-    return Prefix{bits, above, ties, mass + (unsigned long long)ties * pm};
+    return Prefix{bits, f.above, ties, f.mass + (unsigned long long)ties * pm};
 }
 
 // Id of the j-th (1-based) element, by ascending id, whose probability bits equal `value` (-1: there is none).
 // The CTAs of a row hold consecutive ranges of ids, so the j-th lies in the first CTA whose running count reaches j.
 template <int NC>
-__device__ int nth_equal(const float* __restrict__ p, const RowShare<NC>& rs, unsigned int value, unsigned int j, Shared& sh) {
-    const int n_mine = rs.end - rs.begin;
-    const int per = (n_mine + THREADS - 1) / THREADS;
-    const int lo = rs.begin + threadIdx.x * per, hi = min(rs.end, lo + per);
+__device__ int nth_equal(const RowShare<NC>& rs, unsigned int value, unsigned int j, Shared<NC>& sh) {
+    const int per = (rs.n + THREADS - 1) / THREADS;
+    const int lo = min(rs.n, (int)threadIdx.x * per), hi = min(rs.n, lo + per);
     unsigned int c = 0;
-    for (int i = lo; i < hi; i++) c += __float_as_uint(p[i]) == value;
+    for (int i = lo; i < hi; i++) c += __float_as_uint(rs.p[i]) == value;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned int cs = c;
 #pragma unroll
@@ -329,34 +379,25 @@ __device__ int nth_equal(const float* __restrict__ p, const RowShare<NC>& rs, un
         if (lane >= o) cs += t;
     }
     if (lane == 31) sh.scan_u[warp] = cs;
-    if (threadIdx.x == 0) sh.red_i[0] = -1;
+    if (threadIdx.x == 0) sh.id = -1;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned int tot = 0;
-        for (int w = 0; w < THREADS / 32; w++) tot += sh.scan_u[w];
-        sh.part_u = tot;                                    // equal elements in this CTA's range
-    }
-    rs.sync();
     unsigned int before = cs - c;                           // equal elements before this thread's range
-    for (int r = 0; r < rs.rank; r++) before += *rs.at(&sh.part_u, r);
     for (int w = 0; w < warp; w++) before += sh.scan_u[w];
+    if (threadIdx.x == THREADS - 1)
+        for (int r = 0; r < NC; r++) *rs.at(&sh.part_v[rs.rank], r) = before + c;       // equal elements in this CTA's range
+    rs.sync();
+    for (int r = 0; r < rs.rank; r++) before += sh.part_v[r];
     if (c > 0 && before < j && j <= before + c) {
         unsigned int seen = before;
         for (int i = lo; i < hi; i++) {
-            if (__float_as_uint(p[i]) == value && ++seen == j) {
-                sh.red_i[0] = i;
+            if (__float_as_uint(rs.p[i]) == value && ++seen == j) {
+                for (int r = 0; r < NC; r++) *rs.at(&sh.id, r) = rs.begin + i;
                 break;
             }
         }
     }
     rs.sync();
-    int r = -1;
-    for (int k = 0; k < NC; k++) {                          // at most one CTA has found it
-        const int v = *rs.at(&sh.red_i[0], k);
-        if (v >= 0) r = v;
-    }
-    rs.sync();                                              // red_i and part_u may be written again
-    return r;
+    return sh.id;                                           // (searched once a draw: id and part_v are not written again)
 }
 
 __device__ __forceinline__ double splitmix_uniform(unsigned long long* state) {
@@ -372,11 +413,20 @@ struct SampleParams {
     int top_k;
 };
 
+__device__ __forceinline__ void take_first_max(float& bv, int& bi, float v, int i) {
+    if (v > bv || (v == bv && i < bi)) {
+        bv = v;
+        bi = i;
+    }
+}
+
+constexpr int ARGMAX_THREADS = 1024;
+
 // First maximum of a row (strict >, lowest index on ties: sampler.c:124-129).
-__device__ int block_argmax(const float* __restrict__ row, int V, Shared& sh, float* max_out) {
+__device__ int block_argmax(const float* __restrict__ row, int V, ArgmaxShared& sh, float* max_out) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < V; i += THREADS) {
+    for (int i = threadIdx.x; i < V; i += ARGMAX_THREADS) {
         const float v = row[i];
         if (v > bv || (v == bv && i < bi)) {
             bv = v;
@@ -415,422 +465,459 @@ __device__ int block_argmax(const float* __restrict__ row, int V, Shared& sh, fl
     return bi == 0x7fffffff ? 0 : bi;
 }
 
-// The first maximum of a row in two steps, for vocabularies that one CTA reads too slowly: ARGMAX_PARTS CTAs
-// each take a contiguous piece of the row, then the sampling CTA reduces their results. Ties go to the lowest
-// index in both steps, so the result is the one-CTA result.
-constexpr int ARGMAX_PARTS = 32;
-constexpr int PART_THREADS = 256;
+// The ring of a sequence's recent tokens (all null: none is kept). Rows are `stride` apart; the window in use is
+// params[7] <= stride.
+struct Ring {
+    int* tokens;
+    int* n;
+    int* head;
+    int stride;
+};
 
-__device__ __forceinline__ void take_first_max(float& bv, int& bi, float v, int i) {
-    if (v > bv || (v == bv && i < bi)) {
-        bv = v;
-        bi = i;
-    }
+// ring[slot][head] = token; head advances; the count saturates at the window.
+__device__ __forceinline__ void accept_token(const Ring& ring, int slot, int window, int token) {
+    const int head = ring.head[slot] % window;
+    ring.tokens[(size_t)slot * ring.stride + head] = token;
+    ring.head[slot] = (head + 1) % window;
+    if (ring.n[slot] < window) ring.n[slot]++;
 }
 
-__global__ void __launch_bounds__(PART_THREADS)
-argmax_partial_kernel(const float* __restrict__ logits, int V, int ld, const int* __restrict__ slots,
-                      float* __restrict__ part_val, int* __restrict__ part_idx) {
-    __shared__ float red_f[PART_THREADS / 32];
-    __shared__ int red_i[PART_THREADS / 32];
-    griddep_launch();
-    griddep_wait();
-    const int c = blockIdx.x, b = blockIdx.y;
-    if (slots != nullptr && slots[b] < 0) return;          // padding row: the sampling CTA does not look
-    const float* row = logits + (size_t)b * ld;
-    const int chunk = ((V + ARGMAX_PARTS - 1) / ARGMAX_PARTS + 3) & ~3;
-    const int i0 = c * chunk, i1 = min(V, i0 + chunk);
-    float bv = -INFINITY;
-    int bi = 0x7fffffff;
-    if ((ld & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {
-        const int n4 = (i1 - i0) / 4;
-        const float4* r4 = reinterpret_cast<const float4*>(row + i0);
-        for (int j = threadIdx.x; j < n4; j += PART_THREADS) {
-            const float4 v = r4[j];
-            const int i = i0 + 4 * j;
-            take_first_max(bv, bi, v.x, i);
-            take_first_max(bv, bi, v.y, i + 1);
-            take_first_max(bv, bi, v.z, i + 2);
-            take_first_max(bv, bi, v.w, i + 3);
-        }
-        for (int i = i0 + 4 * n4 + threadIdx.x; i < i1; i += PART_THREADS) take_first_max(bv, bi, row[i], i);
-    } else {
-        for (int i = i0 + threadIdx.x; i < i1; i += PART_THREADS) take_first_max(bv, bi, row[i], i);
-    }
+// One of the reference's turns over an entry of the ring: a token that sits there c times takes it c times (sampler.c:80-106).
+__device__ __forceinline__ float penalise(float l, float repeat, float freq, float presence, int count) {
+    if (repeat != 1.0f) l = l > 0.f ? l / repeat : l * repeat;
+    l -= freq * (float)count;
+    l -= presence;
+    return l;
+}
+
+// The walk over at most MAX_CAND candidates by one CTA (sampler.c:146-186): sh.key[0, n_key) are probability bits above,
+// ~id below, each key once. A key's place in the order (probability descending, id ascending) is the number of larger keys;
+// one warp then walks the places, 32 at a time: min-p, top-p, the kept mass and the drawn place are prefixes in the same
+// integer arithmetic as the general search's. Returns the drawn id (-1: no candidate) to lane 0 of warp 0.
+template <int NC>
+__device__ int draw_from_keys(Shared<NC>& sh, unsigned int n_key, const SampleParams& sp, float p_best, double u) {
+    constexpr int TPK = THREADS / MAX_CAND;                 // threads a key
+    const unsigned int t = threadIdx.x / TPK, part = threadIdx.x % TPK;
+    unsigned int place = 0;
+    const unsigned long long own = t < n_key ? sh.key[t] : 0ull;
+    if (t < n_key)
+        for (unsigned int j = part; j < n_key; j += TPK) place += sh.key[j] > own;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float v2 = __shfl_xor_sync(0xffffffffu, bv, o);
-        const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
-        take_first_max(bv, bi, v2, i2);
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-        red_f[warp] = bv;
-        red_i[warp] = bi;
-    }
+    for (int o = TPK / 2; o > 0; o >>= 1) place += __shfl_xor_sync(0xffffffffu, place, o);
+    if (t < n_key && part == 0) sh.sorted[place] = own;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < PART_THREADS / 32; w++) take_first_max(bv, bi, red_f[w], red_i[w]);
-        part_val[(size_t)b * ARGMAX_PARTS + c] = bv;
-        part_idx[(size_t)b * ARGMAX_PARTS + c] = bi;
-    }
-}
-
-// The row's first maximum from the pieces' results (every thread of the CTA gets it).
-__device__ int argmax_from_parts(const float* __restrict__ part_val, const int* __restrict__ part_idx, int b, Shared& sh, float* max_out) {
-    if (threadIdx.x < 32) {
-        float bv = part_val[(size_t)b * ARGMAX_PARTS + threadIdx.x];
-        int bi = part_idx[(size_t)b * ARGMAX_PARTS + threadIdx.x];
+    if (threadIdx.x >= 32) return -1;
+    const unsigned int lane = threadIdx.x;
+    const unsigned int n_c = min(n_key, (unsigned int)sp.top_k);
+    constexpr int TURNS = MAX_CAND / 32;
+    unsigned long long cum[TURNS], carry = 0;               // running masses; place i is lane i % 32 of turn i / 32
+    unsigned int above_floor = 0;
+    const float floor_p = sp.min_p * p_best;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float v2 = __shfl_xor_sync(0xffffffffu, bv, o);
-            const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
-            take_first_max(bv, bi, v2, i2);
-        }
-        if (threadIdx.x == 0) {
-            sh.red_f[0] = bv;
-            sh.red_i[0] = bi;
+    for (int k = 0; k < TURNS; k++) {
+        cum[k] = 0;
+        if (k * 32u < n_c) {                                // uniform
+            const unsigned int i = k * 32 + lane;
+            const float p = i < n_c ? __uint_as_float((unsigned int)(sh.sorted[i] >> 32)) : 0.f;
+            unsigned long long m = i < n_c ? mass_of(p) : 0ull;
+            above_floor += __popc(__ballot_sync(0xffffffffu, i < n_c && p >= floor_p));
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long x = __shfl_up_sync(0xffffffffu, m, o);
+                if ((int)lane >= o) m += x;
+            }
+            cum[k] = carry + m;
+            carry = __shfl_sync(0xffffffffu, cum[k], 31);
         }
     }
-    __syncthreads();
-    const float bv = sh.red_f[0];
-    const int bi = sh.red_i[0];
-    __syncthreads();
-    *max_out = bv;
-    return bi == 0x7fffffff ? 0 : bi;
-}
-
-// A top-k of at most MAX_CAND entries is drawn by sample_top_k_kernel, everything else by sample_kernel; both are
-// launched for every step (the parameters are read on the device) and each leaves at once when the other is due.
-constexpr int MAX_CAND = 256;
-__device__ __forceinline__ bool small_top_k(const SampleParams& sp, int V) {
-    return sp.temp > 0.f && sp.top_k > 0 && sp.top_k <= MAX_CAND && sp.top_k < V;
+    unsigned int n = n_c;
+    if (sp.min_p > 0.f) n = min(n, max(above_floor, 1u));
+    // the first place below n whose running mass reaches the target (n: none)
+    auto first = [&](unsigned long long target) {
+        unsigned int at = n;
+#pragma unroll
+        for (int k = TURNS - 1; k >= 0; k--) {
+            if (k * 32u < n) {
+                const unsigned int b = __ballot_sync(0xffffffffu, k * 32 + lane < n && cum[k] >= target);
+                if (b) at = k * 32 + __ffs(b) - 1;
+            }
+        }
+        return at;
+    };
+    if (sp.top_p < 1.0f) {
+        unsigned long long target = __double2ull_ru((double)sp.top_p * 1152921504606846976.0);
+        if (target == 0) target = 1;
+        const unsigned int at = first(target);
+        if (at < n) n = at + 1;
+    }
+    if (n < 1) n = 1;
+    unsigned long long total = 0;
+#pragma unroll
+    for (int k = 0; k < TURNS; k++) {
+        const unsigned long long x = __shfl_sync(0xffffffffu, cum[k], (n - 1) & 31);
+        if (k == (int)((n - 1) >> 5)) total = x;
+    }
+    unsigned long long target = __double2ull_ru(u * (double)total);
+    if (target > total) target = total;
+    if (target == 0) target = 1;
+    unsigned int pick = first(target);
+    if (pick >= n) pick = n - 1;                            // (only through rounding: the last kept one)
+    return n_c > 0 ? (int)(0xffffffffu - (unsigned int)sh.sorted[pick]) : -1;
 }
 
 // One CTA a row, or for a large vocabulary the ROW_CTAS CTAs of a cluster (NC), each with a consecutive part of
-// the row. The row of logits is overwritten with probabilities when the temperature is positive (the
-// reference's sampler also works in place).
+// the row: penalties, the maximum, exponentials and their sum, the draw, the accepted token into the ring.
+//
+// A small top-k (sampler.c:132-186, the same decisions in another order): the maxima of groups of threads are at hand from the
+// row's maximum, and the k-th largest of them bounds the row's k-th largest from below, so the pass that forms the
+// exponentials also lists everything that can be among the k largest probabilities (equal ones included: a bound with a
+// margin above rounding). The leading CTA sorts that list and walks it. Two barriers over the cluster. The bound is used while
+// k is at most half the groups (then about 0.7 entries a group are expected above it); beyond that, and for rows with many
+// equal logits, the leading bits of the k-th largest are searched by count, and if even those leave more than MAX_CAND entries
+// (many equal logits) the whole k-th probability and the id up to which its equals belong.
+// Everything else goes through find_prefix.
+// Measured (151,936 logits a row; us a draw on the device for 1, 8 and 64 rows; before: a launch for the maximum and one for
+// each kind of draw, passes over the row in L2): top-k 20 48, 50, 200 -> 17, 17, 48; top-p 0.95 alone 156, 158, 757 -> 76, 77, 212;
+// temperature alone 70, 70, 326 -> 58, 59, 160. 512 threads a CTA, so that two share an SM: with 1,024 (whose registers fill
+// it) 64 rows took 63 us with top-k 20 and 496 with top-p, one row 15 instead of 17. A cluster a row at 32,000 logits: 12 us
+// against 18 at one row, but 45 against 19 at 64 and 268 against 86 with top-p: one CTA a row below 32,768.
 template <int NC>
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict__ params,
-              unsigned long long* __restrict__ rng, const int* __restrict__ slots, int* __restrict__ out,
-              const float* __restrict__ part_val, const int* __restrict__ part_idx) {
-    __shared__ Shared sh;
+sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict__ params, unsigned long long* __restrict__ rng,
+              const int* __restrict__ slots, int* __restrict__ out, Ring ring, int row_in_shared) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    Shared<NC>& sh = *reinterpret_cast<Shared<NC>*>(smem);
+    constexpr int GROUPS = Shared<NC>::GROUPS, LANES = Shared<NC>::LANES;      // groups of LANES lanes
+    // another CTA's shared memory may be written once that CTA runs: arrive here, wait before the first such write
+    if (NC > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     griddep_launch();
     griddep_wait();
     const SampleParams sp{params[0], params[1], params[2], (int)params[3]};
-    if (small_top_k(sp, V)) return;          // (every CTA of the launch: sample_top_k_kernel draws this step)
+    const float repeat = params[4], freq = params[5], presence = params[6];
+    const int window = ring.tokens != nullptr ? min((int)params[7], ring.stride) : 0;
     const int b = NC == 1 ? blockIdx.x : blockIdx.x / NC;
     float* row = logits + (size_t)b * ld;
     const int slot = slots ? slots[b] : b;
-    const RowShare<NC> rs(V);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    RowShare<NC> rs(V);
     if (slot < 0) {                          // padding row (all CTAs of the row leave)
+        if (NC > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (threadIdx.x == 0 && rs.rank == 0) out[b] = 0;
         return;
     }
-    if (threadIdx.x == 0) sh.turn = 0;
-    float mx;
-    const int best = part_val != nullptr ? argmax_from_parts(part_val, part_idx, b, sh, &mx) : block_argmax(row, V, sh, &mx);
-    if (sp.temp <= 0.f) {
-        if (threadIdx.x == 0 && rs.rank == 0) out[b] = best;
-        return;
-    }
-    // p_i = expf((l_i - max) / temp) * (float)(1 / sum), the sum in double (sampler.c:132-143)
-    double part = 0.0;
-    for (int base0 = rs.begin; base0 < rs.end; base0 += THREADS * LOADS) {
-        float vals[LOADS];
-#pragma unroll
-        for (int u = 0; u < LOADS; u++) {
-            const int i = base0 + u * THREADS + (int)threadIdx.x;
-            vals[u] = i < rs.end ? row[i] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < LOADS; u++) {
-            const int i = base0 + u * THREADS + (int)threadIdx.x;
-            if (i < rs.end) {
-                const float e = expf((vals[u] - mx) / sp.temp);
-                row[i] = e;
-                part += (double)e;                          // in index order within a thread
-            }
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) sh.red_d[warp] = part;
-    __syncthreads();
+    unsigned long long state = rng[slot];                   // (written by the leading CTA, behind the last barrier of all CTAs)
     if (threadIdx.x == 0) {
-        double mine = 0.0;
-        for (int w = 0; w < THREADS / 32; w++) mine += sh.red_d[w];
-        sh.part_d = mine;
+        sh.n_mine = 0;
+        sh.n_key = 0;
     }
-    rs.sync();
-    double sum = 0.0;
-    for (int r = 0; r < NC; r++) sum += *rs.at(&sh.part_d, r);       // in the CTAs' order: the same value in each of them
-    const float inv = (float)(1.0 / sum);
-    unsigned int n_floor = 0;
-    unsigned long long mass_part = 0;                       // the mass of this thread's probabilities (integers: any order)
-    for (int base0 = rs.begin; base0 < rs.end; base0 += THREADS * LOADS) {
-        float vals[LOADS];
-#pragma unroll
-        for (int u = 0; u < LOADS; u++) {
-            const int i = base0 + u * THREADS + (int)threadIdx.x;
-            vals[u] = i < rs.end ? row[i] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < LOADS; u++) {
-            const int i = base0 + u * THREADS + (int)threadIdx.x;
-            if (i < rs.end) {
-                const float pr = vals[u] * inv;
-                row[i] = pr;
-                mass_part += mass_of(pr);
-            }
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mass_part += __shfl_xor_sync(0xffffffffu, mass_part, o);
-    if (lane == 0) sh.warp_mass[warp] = mass_part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long mine = 0;
-        for (int w = 0; w < THREADS / 32; w++) mine += sh.warp_mass[w];
-        sh.part_m = mine;
-    }
-    rs.sync();                                              // the whole row holds probabilities (and part_d has been read)
-    unsigned long long row_mass = 0;
-    for (int r = 0; r < NC; r++) row_mass += *rs.at(&sh.part_m, r);
-    const float p_best = __ldcg(row + best);                // possibly written by another CTA of the row
-
-    // the kept prefix: top-k, then min-p, then top-p (sampler.c:146-175)
-    unsigned int n = (unsigned int)V;
-    if (sp.top_k > 0 && (unsigned int)sp.top_k < n) n = (unsigned int)sp.top_k;
-    if (sp.min_p > 0.f) {
-        const float floor_p = sp.min_p * p_best;
-        unsigned int c = 0;
-        for (int i = rs.begin + (int)threadIdx.x; i < rs.end; i += THREADS) c += row[i] >= floor_p;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-        if (lane == 0) sh.scan_u[warp] = c;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            unsigned int mine = 0;
-            for (int w = 0; w < THREADS / 32; w++) mine += sh.scan_u[w];
-            sh.part_u = mine;
-        }
-        rs.sync();
-        for (int r = 0; r < NC; r++) n_floor += *rs.at(&sh.part_u, r);
-        rs.sync();                                          // part_u may be written again
-        if (n_floor < 1) n_floor = 1;
-        if (n_floor < n) n = n_floor;
-    }
-    if (sp.top_p < 1.0f) {
-        const unsigned long long target = __double2ull_ru((double)sp.top_p * 1152921504606846976.0);
-        const Prefix pp = find_prefix<NC>(row, rs, true, 0, target, sh);
-        const unsigned int np = pp.above + pp.ties;
-        if (np < n) n = np;
-    }
-    if (n < 1) n = 1;
-    // mass of the kept prefix, then the draw r = U * total and the walk (sampler.c:178-186)
-    // (with nothing cut off that is the row's mass, which the pass above has added up: three passes fewer)
-    const Prefix kept = n == (unsigned int)V ? Prefix{0u, 0u, 0u, row_mass} : find_prefix<NC>(row, rs, false, n, 0, sh);
-    unsigned long long state = rng[slot];                   // (rewritten by the leading CTA only after the last barrier)
-    const double u = splitmix_uniform(&state);
-    const double r = u * (double)kept.mass;
-    unsigned long long target = __double2ull_ru(r);
-    if (target > kept.mass) target = kept.mass;
-    Prefix hit = find_prefix<NC>(row, rs, true, 0, target, sh);
-    unsigned int rank = hit.above + hit.ties;              // 1-based place in the sorted order
-    unsigned int value = hit.value, j = hit.ties;
-    if (rank > n) {                                        // only through rounding: the last kept one
-        value = kept.value;
-        j = kept.ties;
-    }
-    const int id = nth_equal<NC>(row, rs, value, j, sh);
-    if (threadIdx.x == 0 && rs.rank == 0) {
-        out[b] = id >= 0 ? id : best;
-        rng[slot] = state;
-    }
-}
-
-// The draw with a small top-k (sampler.c:132-186, the same decisions in another order). The k largest
-// probabilities are found once (a search by count, then the id up to which entries equal to the k-th belong),
-// gathered into the leading CTA and sorted by (probability descending, id ascending), which is the order that
-// the general kernel walks. min-p, top-p, the kept mass and the drawn place are then prefixes of at most k
-// entries, walked by one thread in the same integer arithmetic: three passes over the row (exponentials and their
-// sum, the leading bits of the k-th largest, the gather) instead of thirteen; seven for a row with many equal logits.
-struct Candidates {
-    unsigned long long key[MAX_CAND];      // probability bits above, ~id below: larger keys come first
-    unsigned int n;
-};
-
-template <int NC>
-__global__ void __launch_bounds__(THREADS)
-sample_top_k_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict__ params,
-                    unsigned long long* __restrict__ rng, const int* __restrict__ slots, int* __restrict__ out,
-                    const float* __restrict__ part_val, const int* __restrict__ part_idx) {
-    __shared__ Shared sh;
-    __shared__ Candidates cand;
-    griddep_launch();
-    griddep_wait();
-    const SampleParams sp{params[0], params[1], params[2], (int)params[3]};
-    if (!small_top_k(sp, V)) return;         // (every CTA of the launch)
-    const int b = NC == 1 ? blockIdx.x : blockIdx.x / NC;
-    float* row = logits + (size_t)b * ld;
-    const int slot = slots ? slots[b] : b;
-    const RowShare<NC> rs(V);
-    if (slot < 0) {                          // padding row (all CTAs of the row leave)
-        if (threadIdx.x == 0 && rs.rank == 0) out[b] = 0;
-        return;
-    }
-    if (threadIdx.x == 0) sh.turn = 0;
-    float mx;
-    const int best = part_val != nullptr ? argmax_from_parts(part_val, part_idx, b, sh, &mx) : block_argmax(row, V, sh, &mx);
-    // p_i = expf((l_i - max) / temp) * (float)(1 / sum), the sum in double, as in sample_kernel
-    double part = 0.0;
-    for (int base0 = rs.begin; base0 < rs.end; base0 += THREADS * LOADS) {
-        float vals[LOADS];
-#pragma unroll
-        for (int u = 0; u < LOADS; u++) {
-            const int i = base0 + u * THREADS + (int)threadIdx.x;
-            vals[u] = i < rs.end ? row[i] : 0.f;
-        }
-#pragma unroll
-        for (int u = 0; u < LOADS; u++) {
-            const int i = base0 + u * THREADS + (int)threadIdx.x;
-            if (i < rs.end) {
-                const float e = expf((vals[u] - mx) / sp.temp);
-                row[i] = e;
-                part += (double)e;
-            }
-        }
-    }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
-    if (lane == 0) sh.red_d[warp] = part;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double mine = 0.0;
-        for (int w = 0; w < THREADS / 32; w++) mine += sh.red_d[w];
-        sh.part_d = mine;
-    }
-    rs.sync();
-    double sum = 0.0;
-    for (int r = 0; r < NC; r++) sum += *rs.at(&sh.part_d, r);
-    const float inv = (float)(1.0 / sum);
-    if (threadIdx.x == 0) cand.n = 0;
-    for (int i = threadIdx.x; i < MAX_CAND; i += THREADS) cand.key[i] = 0ull;
-    rs.sync();                                              // the row holds the exponentials; the leading CTA's list is empty
-    const float p_best = __ldcg(row + best) * inv;
-
-    // One pass over the probabilities (the stored exponentials times inv, as the reference forms them) finds the
-    // leading eleven bits of the k-th largest. Everything with those bits or larger ones holds the k largest; when
-    // that is a short list it is gathered and sorted, and its first k entries are the k largest in the order
-    // (probability descending, id ascending). Only a row that crowds more than MAX_CAND entries there (many equal
-    // logits) takes the long way: the row normalised in place, the k-th probability to the last bit and the id up
-    // to which its equals belong.
-    const Found lead = radix_pass<NC>(row, rs, 0u, 0u, 21, 2048, false, (unsigned int)sp.top_k, 0, 0, 0, sh, inv);
-    const bool short_list = lead.above + lead.count <= (unsigned int)MAX_CAND;      // the same in every CTA of the row
-    Prefix topk{0u, 0u, 0u, 0ull};
-    int id_bound = -1;
-    float gather_scale = inv;
-    if (!short_list) {
-        for (int base0 = rs.begin; base0 < rs.end; base0 += THREADS * LOADS) {
+    // ---- the row, and each thread's first maximum
+    rs.p = row_in_shared ? reinterpret_cast<float*>(smem + sizeof(Shared<NC>)) : row + rs.begin;
+    const float* from = row + rs.begin;
+    float bv = -INFINITY;
+    int bi = 0x7fffffff;
+    auto scan = [&](const float* src, bool keep) {
+        for (int base0 = 0; base0 < rs.n; base0 += THREADS * LOADS) {
             float vals[LOADS];
 #pragma unroll
             for (int u = 0; u < LOADS; u++) {
                 const int i = base0 + u * THREADS + (int)threadIdx.x;
-                vals[u] = i < rs.end ? row[i] : 0.f;
+                vals[u] = i < rs.n ? src[i] : -INFINITY;
             }
 #pragma unroll
             for (int u = 0; u < LOADS; u++) {
                 const int i = base0 + u * THREADS + (int)threadIdx.x;
-                if (i < rs.end) row[i] = vals[u] * inv;
+                if (i < rs.n) {
+                    take_first_max(bv, bi, vals[u], rs.begin + i);
+                    if (keep) rs.p[i] = vals[u];
+                }
             }
         }
-        rs.sync();                                          // the row holds probabilities
-        topk = find_prefix<NC>(row, rs, false, (unsigned int)sp.top_k, 0, sh);
-        id_bound = nth_equal<NC>(row, rs, topk.value, topk.ties, sh);
-        gather_scale = 1.0f;
+    };
+    if (row_in_shared && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {   // (begin is a multiple of 4)
+        constexpr int LOADS4 = 5;
+        const int n4 = rs.n / 4;
+        const float4* from4 = reinterpret_cast<const float4*>(from);
+        for (int base0 = 0; base0 < n4; base0 += THREADS * LOADS4) {
+            float4 v[LOADS4];
+#pragma unroll
+            for (int u = 0; u < LOADS4; u++) {
+                const int j = base0 + u * THREADS + (int)threadIdx.x;
+                if (j < n4) v[u] = __ldcs(from4 + j);
+            }
+#pragma unroll
+            for (int u = 0; u < LOADS4; u++) {
+                const int j = base0 + u * THREADS + (int)threadIdx.x;
+                if (j < n4) {
+                    const int i = rs.begin + 4 * j;
+                    take_first_max(bv, bi, v[u].x, i);
+                    take_first_max(bv, bi, v[u].y, i + 1);
+                    take_first_max(bv, bi, v[u].z, i + 2);
+                    take_first_max(bv, bi, v[u].w, i + 3);
+                    reinterpret_cast<float4*>(rs.p)[j] = v[u];
+                }
+            }
+        }
+        for (int i = 4 * n4 + (int)threadIdx.x; i < rs.n; i += THREADS) {
+            rs.p[i] = from[i];
+            take_first_max(bv, bi, rs.p[i], rs.begin + i);
+        }
+    } else {
+        scan(from, row_in_shared != 0);
     }
-    unsigned int* cnt = rs.at(&cand.n, 0);
-    unsigned long long* keys = rs.at(&cand.key[0], 0);
-    for (int base0 = rs.begin; base0 < rs.end; base0 += THREADS * LOADS) {
+    if (window > 0 && !(repeat == 1.0f && freq == 0.0f && presence == 0.0f)) {       // sampler.c:81-84
+        const int n = min(ring.n[slot], min(window, 256));
+        const int* r = ring.tokens + (size_t)slot * ring.stride;
+        if ((int)threadIdx.x < n) sh.ring[threadIdx.x] = r[threadIdx.x];
+        __syncthreads();                                    // the ring is there, and so is the row
+        if ((int)threadIdx.x < n) {
+            const int tok = sh.ring[threadIdx.x], at = tok - rs.begin;
+            int count = 0, before = 0;
+            for (int k = 0; k < n; k++) {
+                count += sh.ring[k] == tok;
+                before += k < (int)threadIdx.x && sh.ring[k] == tok;
+            }
+            if (before == 0 && tok >= 0 && at >= 0 && at < rs.n) {       // one thread a token, in the CTA that holds it
+                float l = rs.p[at];
+                for (int k = 0; k < count; k++) l = penalise(l, repeat, freq, presence, count);
+                rs.p[at] = l;
+                row[tok] = l;
+            }
+        }
+        __syncthreads();
+        bv = -INFINITY;
+        bi = 0x7fffffff;
+        scan(rs.p, false);
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) {
+        const float v2 = __shfl_xor_sync(0xffffffffu, bv, o);
+        const int i2 = __shfl_xor_sync(0xffffffffu, bi, o);
+        take_first_max(bv, bi, v2, i2);
+    }
+    if (NC > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    const int group = rs.rank * (THREADS / LANES) + (int)threadIdx.x / LANES;
+    if (lane % LANES < NC) {                                // a lane a CTA
+        *rs.at(&sh.group_v[group], lane % LANES) = bv;
+        *rs.at(&sh.group_i[group], lane % LANES) = bi;
+    }
+    rs.sync();                                              // the maxima of all groups are in every CTA
+    // ---- the row's first maximum (warp 0), the k-th largest of the groups' maxima (all warps)
+    const bool small_k = sp.temp > 0.f && sp.top_k > 0 && sp.top_k <= MAX_CAND && sp.top_k < V;
+    const bool bounded = small_k && sp.top_k <= GROUPS / 2;
+    if (warp == 0) {
+        float v = -INFINITY;
+        int at = 0x7fffffff;
+        for (int k = lane; k < GROUPS; k += 32) take_first_max(v, at, sh.group_v[k], sh.group_i[k]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const float v2 = __shfl_xor_sync(0xffffffffu, v, o);
+            const int i2 = __shfl_xor_sync(0xffffffffu, at, o);
+            take_first_max(v, at, v2, i2);
+        }
+        if (lane == 0) {
+            sh.mx = v;
+            sh.best = at == 0x7fffffff ? 0 : at;
+        }
+    }
+    if (bounded) {
+        constexpr int TPG = THREADS / GROUPS;               // threads a group's value
+        const int g = threadIdx.x / TPG, part = threadIdx.x % TPG;
+        const float own = sh.group_v[g];
+        int place = 0;
+#pragma unroll 4
+        for (int k = part; k < GROUPS / 4; k += TPG) {
+            const float4 v = reinterpret_cast<const float4*>(sh.group_v)[k];
+            place += (v.x > own || (v.x == own && 4 * k < g)) + (v.y > own || (v.y == own && 4 * k + 1 < g))
+                   + (v.z > own || (v.z == own && 4 * k + 2 < g)) + (v.w > own || (v.w == own && 4 * k + 3 < g));
+        }
+#pragma unroll
+        for (int o = TPG / 2; o > 0; o >>= 1) place += __shfl_xor_sync(0xffffffffu, place, o);
+        if (part == 0 && place == sp.top_k - 1) sh.bound = own;
+    }
+    __syncthreads();
+    const float mx = sh.mx;
+    const int best = sh.best;
+    const bool leading = rs.rank == 0;
+    if (sp.temp <= 0.f) {
+        if (threadIdx.x == 0 && leading) {
+            out[b] = best;
+            if (window > 0) accept_token(ring, slot, window, best);
+        }
+        return;
+    }
+    // Everything whose exponential is at least `least` is listed. Probabilities are the exponentials times a rounded factor:
+    // those equal to the k-th largest come from exponentials within 2^-22 of its own, and expf is within 2^-22 of being
+    // monotonic; the margin is 2^-20. Below 1e-20 a product could be subnormal and merge more: the search by count then.
+    const float bound_e = bounded ? expf((sh.bound - mx) / sp.temp) : 0.f;
+    const bool listing = bounded && bound_e >= 1e-20f;
+    const float least = bound_e * (1.0f - 9.5367431640625e-7f);
+    // ---- p_i = expf((l_i - max) / temp) * (float)(1 / sum), the sum in double (sampler.c:132-143)
+    double part = 0.0;
+    for (int base0 = 0; base0 < rs.n; base0 += THREADS * LOADS) {
         float vals[LOADS];
 #pragma unroll
         for (int u = 0; u < LOADS; u++) {
             const int i = base0 + u * THREADS + (int)threadIdx.x;
-            vals[u] = i < rs.end ? __ldcg(row + i) : 0.f;
+            vals[u] = i < rs.n ? rs.p[i] : 0.f;
         }
 #pragma unroll
         for (int u = 0; u < LOADS; u++) {
             const int i = base0 + u * THREADS + (int)threadIdx.x;
-            const unsigned int bits = __float_as_uint(vals[u] * gather_scale);    // probabilities are not negative: bits order as values
-            const bool take = short_list ? (bits >> 21) >= lead.digit : (bits > topk.value || (bits == topk.value && i <= id_bound));
-            if (i < rs.end && take) {
-                const unsigned int at = atomicAdd(cnt, 1u);
-                if (at < (unsigned int)MAX_CAND) keys[at] = ((unsigned long long)bits << 32) | (0xffffffffu - (unsigned int)i);
-            }
-        }
-    }
-    rs.sync();                                              // the list is complete
-    if (rs.rank != 0) return;                               // (the leading CTA reads its own memory only from here on)
-    // bitonic sort, largest key first: larger probability, then lower id
-    for (int size = 2; size <= MAX_CAND; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            const int t = threadIdx.x, partner = t ^ stride;
-            if (t < MAX_CAND && partner > t) {
-                const unsigned long long a = cand.key[t], c = cand.key[partner];
-                const bool descending = (t & size) == 0;
-                if (descending ? a < c : a > c) {
-                    cand.key[t] = c;
-                    cand.key[partner] = a;
+            if (i < rs.n) {
+                const float e = expf((vals[u] - mx) / sp.temp);
+                rs.p[i] = e;
+                part += (double)e;                          // in index order within a thread
+                if (listing && e >= least) {
+                    const unsigned int at = atomicAdd(&sh.n_mine, 1u);
+                    if (at < (unsigned int)MAX_CAND)
+                        sh.mine[at] = ((unsigned long long)__float_as_uint(e) << 32) | (0xffffffffu - (unsigned int)(rs.begin + i));
                 }
             }
-            __syncthreads();
         }
     }
-    if (threadIdx.x != 0) return;
-    const unsigned int n_c = min(min(cand.n, (unsigned int)MAX_CAND), (unsigned int)sp.top_k);   // top_k, unless the row has fewer entries
-    unsigned int n = n_c;
-    if (sp.min_p > 0.f) {
-        const float floor_p = sp.min_p * p_best;
-        unsigned int c = 0;
-        while (c < n_c && __uint_as_float((unsigned int)(cand.key[c] >> 32)) >= floor_p) c++;
-        if (c < 1) c = 1;
-        if (c < n) n = c;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xffffffffu, part, o);
+    if (lane == 0) sh.red_d[warp] = part;
+    __syncthreads();
+    const unsigned int n_mine = sh.n_mine;
+    if (warp == 0) {
+        double mine = lane < WARPS ? sh.red_d[lane] : 0.0;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+        if (lane < NC) {                                    // a lane a CTA
+            *rs.at(&sh.part_d[rs.rank], lane) = mine;
+            *rs.at(&sh.part_u[rs.rank], lane) = n_mine;
+        }
+    } else if (listing && threadIdx.x - 32 < min(n_mine, (unsigned int)MAX_CAND)) {
+        *rs.at(&sh.list[rs.rank][threadIdx.x - 32], 0) = sh.mine[threadIdx.x - 32];
     }
-    if (sp.top_p < 1.0f) {
-        unsigned long long target = __double2ull_ru((double)sp.top_p * 1152921504606846976.0);
-        if (target == 0) target = 1;
-        unsigned long long cum = 0;
-        for (unsigned int i = 0; i < n; i++) {
-            cum += mass_of(__uint_as_float((unsigned int)(cand.key[i] >> 32)));
-            if (cum >= target) {
-                n = i + 1;
-                break;
+    rs.sync();                                              // sums and counts are in every CTA, the lists in the leading one
+    double sum = 0.0;
+    unsigned int listed = 0;
+    for (int r = 0; r < NC; r++) {                          // in the CTAs' order: the same value in each of them
+        sum += sh.part_d[r];
+        listed += min(sh.part_u[r], (unsigned int)MAX_CAND + 1u);
+    }
+    const float inv = (float)(1.0 / sum);
+    const float p_best = expf((mx - mx) / sp.temp) * inv;
+    const double u = splitmix_uniform(&state);
+    int id = -1;
+    if (small_k && listing && listed <= (unsigned int)MAX_CAND && inv > 0.f) {
+        if (!leading) return;                               // (the leading CTA reads its own memory only from here on)
+        if (threadIdx.x < listed) {
+            int r = 0;
+            unsigned int at = threadIdx.x;
+            while (at >= sh.part_u[r]) at -= sh.part_u[r++];
+            const unsigned long long k = sh.list[r][at];
+            const float p = __uint_as_float((unsigned int)(k >> 32)) * inv;
+            sh.key[threadIdx.x] = ((unsigned long long)__float_as_uint(p) << 32) | (unsigned int)k;
+        }
+        __syncthreads();
+        id = draw_from_keys<NC>(sh, listed, sp, p_best, u);
+    } else if (small_k) {
+        // One pass over the probabilities (the stored exponentials times inv) finds the leading eleven bits of the k-th
+        // largest. Everything with those bits or larger ones holds the k largest; when that is a short list it is gathered.
+        const Found lead = find_digit<NC>(rs, add_up<NC>(rs, FIRST_DIGIT, inv, sh), false, (unsigned int)sp.top_k, 0ull, 0u, 0ull, sh);
+        const bool short_list = lead.above + lead.count <= (unsigned int)MAX_CAND;      // the same in every CTA of the row
+        Prefix topk{0u, 0u, 0u, 0ull};
+        int id_bound = -1;
+        float gather_scale = inv;
+        if (!short_list) {
+            for (int i = threadIdx.x; i < rs.n; i += THREADS) rs.p[i] *= inv;
+            __syncthreads();                                // this CTA's part holds probabilities
+            topk = find_prefix<NC>(rs, add_up<NC>(rs, FIRST_DIGIT, 1.0f, sh), false, (unsigned int)sp.top_k, 0ull, sh);
+            id_bound = nth_equal<NC>(rs, topk.value, topk.ties, sh);
+            gather_scale = 1.0f;
+        }
+        unsigned int* cnt = rs.at(&sh.n_key, 0);
+        unsigned long long* keys = rs.at(&sh.key[0], 0);
+        for (int i = threadIdx.x; i < rs.n; i += THREADS) {
+            const unsigned int bits = __float_as_uint(rs.p[i] * gather_scale);    // probabilities are not negative: bits order as values
+            const bool take = short_list ? (bits >> 21) >= lead.digit : (bits > topk.value || (bits == topk.value && rs.begin + i <= id_bound));
+            if (take) {
+                const unsigned int at = atomicAdd(cnt, 1u);
+                if (at < (unsigned int)MAX_CAND) keys[at] = ((unsigned long long)bits << 32) | (0xffffffffu - (unsigned int)(rs.begin + i));
             }
         }
-    }
-    if (n < 1) n = 1;
-    unsigned long long total = 0;
-    for (unsigned int i = 0; i < n; i++) total += mass_of(__uint_as_float((unsigned int)(cand.key[i] >> 32)));
-    unsigned long long state = rng[slot];
-    const double u = splitmix_uniform(&state);
-    unsigned long long target = __double2ull_ru(u * (double)total);
-    if (target > total) target = total;
-    if (target == 0) target = 1;
-    unsigned int pick = n - 1;                              // (only through rounding: the last kept one)
-    unsigned long long cum = 0;
-    for (unsigned int i = 0; i < n; i++) {
-        cum += mass_of(__uint_as_float((unsigned int)(cand.key[i] >> 32)));
-        if (cum >= target) {
-            pick = i;
-            break;
+        rs.sync();                                          // the list is complete
+        if (!leading) return;
+        id = draw_from_keys<NC>(sh, min(sh.n_key, (unsigned int)MAX_CAND), sp, p_best, u);
+    } else {
+        unsigned long long mass_part = 0;                   // the mass of this thread's probabilities (integers: any order)
+        unsigned int c = 0;
+        const float floor_p = sp.min_p * p_best;
+        for (int i = threadIdx.x; i < rs.n; i += THREADS) {
+            const float pr = rs.p[i] * inv;
+            rs.p[i] = pr;
+            mass_part += mass_of(pr);
+            c += pr >= floor_p;
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            mass_part += __shfl_xor_sync(0xffffffffu, mass_part, o);
+            c += __shfl_xor_sync(0xffffffffu, c, o);
+        }
+        if (lane == 0) {
+            sh.warp_mass[warp] = mass_part;
+            sh.scan_u[warp] = c;
+        }
+        __syncthreads();                                    // this CTA's part holds probabilities
+        if (warp == 0) {
+            unsigned long long m = lane < WARPS ? sh.warp_mass[lane] : 0ull;
+            unsigned int n = lane < WARPS ? sh.scan_u[lane] : 0u;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                m += __shfl_xor_sync(0xffffffffu, m, o);
+                n += __shfl_xor_sync(0xffffffffu, n, o);
+            }
+            if (lane < NC) {
+                *rs.at(&sh.part_m[rs.rank], lane) = m;
+                *rs.at(&sh.part_v[rs.rank], lane) = n;
+            }
+        }
+        rs.sync();
+        unsigned long long row_mass = 0;
+        unsigned int n_floor = 0;
+        for (int r = 0; r < NC; r++) {
+            row_mass += sh.part_m[r];
+            n_floor += sh.part_v[r];
+        }
+        // the kept prefix: top-k, then min-p, then top-p (sampler.c:146-175)
+        unsigned int n = (unsigned int)V;
+        if (sp.top_k > 0 && (unsigned int)sp.top_k < n) n = (unsigned int)sp.top_k;
+        if (sp.min_p > 0.f) n = min(n, max(n_floor, 1u));
+        // mass of the kept prefix, then the draw r = U * total and the walk (sampler.c:178-186); with nothing cut off it is
+        // the row's mass, and a prefix that top-p ends is the one its search has found
+        const Slice<NC> first = add_up<NC>(rs, FIRST_DIGIT, 1.0f, sh);       // (both searches begin with it)
+        Prefix kept{0u, 0u, 0u, row_mass};
+        bool found = false;
+        if (sp.top_p < 1.0f) {
+            const unsigned long long target = __double2ull_ru((double)sp.top_p * 1152921504606846976.0);
+            const Prefix pp = find_prefix<NC>(rs, first, true, 0u, target, sh);
+            const unsigned int np = pp.above + pp.ties;
+            if (np <= n) {
+                n = np;
+                kept = pp;
+                found = true;
+            }
+        }
+        if (n < 1) n = 1;
+        if (!found && n < (unsigned int)V) kept = find_prefix<NC>(rs, first, false, n, 0ull, sh);
+        const double r = u * (double)kept.mass;
+        unsigned long long target = __double2ull_ru(r);
+        if (target > kept.mass) target = kept.mass;
+        const Prefix hit = find_prefix<NC>(rs, first, true, 0u, target, sh);
+        const unsigned int rank = hit.above + hit.ties;     // 1-based place in the sorted order
+        const bool within = rank <= n;                      // (beyond only through rounding: the last kept one)
+        id = nth_equal<NC>(rs, within ? hit.value : kept.value, within ? hit.ties : kept.ties, sh);
+        if (!leading) return;
     }
-    out[b] = n_c > 0 ? (int)(0xffffffffu - (unsigned int)cand.key[pick]) : best;
-    rng[slot] = state;
+    if (threadIdx.x == 0) {
+        const int token = id >= 0 ? id : best;
+        out[b] = token;
+        rng[slot] = state;
+        if (window > 0) accept_token(ring, slot, window, token);
+    }
 }
 
 // One thread per row: the reference's loop over the ring of recent tokens,
@@ -856,15 +943,10 @@ __global__ void penalties_kernel(float* __restrict__ logits, int B, int V, int l
         if (tok < 0 || tok >= V) continue;
         int count = 0;
         for (int k = 0; k < n; k++) count += r[k] == tok;
-        float l = row[tok];
-        if (repeat != 1.0f) l = l > 0.f ? l / repeat : l * repeat;
-        l -= freq * (float)count;
-        l -= presence;
-        row[tok] = l;
+        row[tok] = penalise(row[tok], repeat, freq, presence, count);
     }
 }
 
-// ring[slot][head] = token; head advances; the count saturates at the window.
 __global__ void accept_kernel(const int* __restrict__ tokens, int B, int* __restrict__ ring, int* __restrict__ ring_n,
                               int* __restrict__ ring_head, int stride, const int* __restrict__ slots,
                               const float* __restrict__ params) {
@@ -875,15 +957,12 @@ __global__ void accept_kernel(const int* __restrict__ tokens, int B, int* __rest
     if (b >= B || window <= 0) return;
     const int slot = slots ? slots[b] : b;
     if (slot < 0) return;
-    const int head = ring_head[slot] % window;
-    ring[(size_t)slot * stride + head] = tokens[b];
-    ring_head[slot] = (head + 1) % window;
-    if (ring_n[slot] < window) ring_n[slot]++;
+    accept_token(Ring{ring, ring_n, ring_head, stride}, slot, window, tokens[b]);
 }
 
-__global__ void __launch_bounds__(THREADS)
+__global__ void __launch_bounds__(ARGMAX_THREADS)
 argmax_kernel(const float* __restrict__ logits, int V, int ld, int* __restrict__ out) {
-    __shared__ Shared sh;
+    __shared__ ArgmaxShared sh;
     griddep_launch();
     griddep_wait();
     float mx;
@@ -896,58 +975,56 @@ argmax_kernel(const float* __restrict__ logits, int V, int ld, int* __restrict__
 MYNAH_API int mynah_argmax(const float* logits, int B, int V, int ld, int* out, cudaStream_t stream) {
     if (B == 0) return 0;
     MYNAH_REQUIRE(B > 0 && V > 0 && ld >= V, "argmax: bad sizes B=%d V=%d ld=%d", B, V, ld);
-    mynah_launch(argmax_kernel, dim3(B), dim3(THREADS), 0, stream, logits, V, ld, out);
+    mynah_launch(argmax_kernel, dim3(B), dim3(ARGMAX_THREADS), 0, stream, logits, V, ld, out);
     return mynah_check_launch("argmax");
 }
 
-// logits [B, ld] are overwritten. params (device): temp, top_p, min_p, top_k,
-// repeat, freq, presence as floats; they are read on the device so that a
-// captured step serves every setting. rng: one 64-bit generator state per
-// slot; slots [B] maps rows to slots (null: row b is slot b; a negative slot
-// marks a padding row). out [B] receives the token ids.
-// part_val, part_idx: scratch of B * mynah_argmax_parts() entries each for the two-step maximum, or null.
+// One draw a row of logits [B, ld], in one launch: penalties from the ring, the draw, the token into the ring. The logits
+// may be overwritten (by penalised values, and by what is left of the search where a row does not fit shared memory). params
+// (device): temp, top_p, min_p, top_k, repeat, freq, presence, window as floats; they are read on the device so that a
+// captured step serves every setting. rng: one 64-bit generator state per slot; slots [B] maps rows to slots (null: row b is
+// slot b; a negative slot marks a padding row). out [B] receives the token ids. ring, ring_n, ring_head: the slots' rings,
+// `stride` <= 256 entries a row, or null: then no penalty is taken and nothing is accepted.
 MYNAH_API int mynah_sample(float* logits, int B, int V, int ld, const float* params,
                            unsigned long long* rng, const int* slots, int* out,
-                           float* part_val, int* part_idx, cudaStream_t stream) {
+                           int* ring, int* ring_n, int* ring_head, int stride, cudaStream_t stream) {
     if (B == 0) return 0;
     MYNAH_REQUIRE(B > 0 && V > 0 && ld >= V, "sample: bad sizes B=%d V=%d ld=%d", B, V, ld);
     MYNAH_REQUIRE(params != nullptr && rng != nullptr, "sample: parameters and generator states are required");
-    MYNAH_REQUIRE((part_val == nullptr) == (part_idx == nullptr) && B <= 65535, "sample: bad scratch or too many rows");
-    if (part_val != nullptr) {
-        mynah_launch(argmax_partial_kernel, dim3(ARGMAX_PARTS, B), dim3(PART_THREADS), 0, stream, (const float*)logits, V, ld, slots, part_val, part_idx);
-        if (mynah_check_launch("argmax_partial")) return -1;
-    }
-    if (part_val != nullptr && V >= ROW_CTAS * 4096) {
-        // a large vocabulary: a cluster of ROW_CTAS CTAs a row
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)B * ROW_CTAS);
-        cfg.blockDim = dim3(THREADS);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = ROW_CTAS;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        cudaError_t e = cudaLaunchKernelEx(&cfg, sample_top_k_kernel<ROW_CTAS>, logits, V, ld, params, rng, slots, out,
-                                           (const float*)part_val, (const int*)part_idx);
-        if (e == cudaSuccess)
-            e = cudaLaunchKernelEx(&cfg, sample_kernel<ROW_CTAS>, logits, V, ld, params, rng, slots, out,
-                                   (const float*)part_val, (const int*)part_idx);
-        if (e != cudaSuccess) return mynah_fail("sample: %s", cudaGetErrorString(e));
+    MYNAH_REQUIRE(B <= 65535, "sample: too many rows");
+    MYNAH_REQUIRE((ring == nullptr) == (ring_n == nullptr) && (ring == nullptr) == (ring_head == nullptr)
+                      && (ring == nullptr || (stride > 0 && stride <= 256)), "sample: bad ring");
+    const Ring rings{ring, ring_n, ring_head, stride};
+    // A cluster a row from this vocabulary size on (see the kernel), whatever the batch: a row's draw does not depend on its
+    // company. A row that does not fit its CTAs' shared memory stays where it is.
+    const bool cluster = V >= ROW_CTAS * 4096;
+    const size_t own = cluster ? sizeof(Shared<ROW_CTAS>) : sizeof(Shared<1>);
+    const size_t part = sizeof(float) * (size_t)(cluster ? ((V + ROW_CTAS - 1) / ROW_CTAS + 3) & ~3 : V);
+    const int in_shared = own + part <= 227 * 1024;
+    const size_t smem = own + (in_shared ? part : 0);
+    auto kernel = cluster ? sample_kernel<ROW_CTAS> : sample_kernel<1>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+    if (e != cudaSuccess) return mynah_fail("sample: %s", cudaGetErrorString(e));
+    if (!cluster) {
+        mynah_launch(kernel, dim3(B), dim3(THREADS), smem, stream, logits, V, ld, params, rng, slots, out, rings, in_shared);
         return mynah_check_launch("sample");
     }
-    mynah_launch(sample_top_k_kernel<1>, dim3(B), dim3(THREADS), 0, stream, logits, V, ld, params, rng, slots, out,
-                 (const float*)part_val, (const int*)part_idx);
-    if (mynah_check_launch("sample (top-k)")) return -1;
-    mynah_launch(sample_kernel<1>, dim3(B), dim3(THREADS), 0, stream, logits, V, ld, params, rng, slots, out,
-                 (const float*)part_val, (const int*)part_idx);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)B * ROW_CTAS);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ROW_CTAS;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    e = cudaLaunchKernelEx(&cfg, kernel, logits, V, ld, params, rng, slots, out, rings, in_shared);
+    if (e != cudaSuccess) return mynah_fail("sample: %s", cudaGetErrorString(e));
     return mynah_check_launch("sample");
 }
-
-MYNAH_API int mynah_argmax_parts() { return ARGMAX_PARTS; }
 
 MYNAH_API int mynah_apply_penalties(float* logits, int B, int V, int ld, const int* ring, const int* ring_n,
                                     int window, const int* slots, const float* params, cudaStream_t stream) {

@@ -487,37 +487,23 @@ def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Te
 
 
 def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots: Optional[torch.Tensor],
-           out: Optional[torch.Tensor] = None) -> torch.Tensor:
-    """Overwrites `logits`. params: float32 [7] on the device (temp, top_p,
-    min_p, top_k, repeat, freq, presence); rng: int64 generator state per slot."""
+           out: Optional[torch.Tensor] = None, ring: Optional[tuple] = None) -> torch.Tensor:
+    """One launch. May overwrite `logits`. params: float32 [7] on the device (temp, top_p,
+    min_p, top_k, repeat, freq, presence; with `ring` an eighth, the window in use); rng: int64 generator state per slot.
+    `ring` = (tokens [slots, stride], counts, heads), int32: the penalties are taken from it before the draw and the drawn
+    token goes into it, as `apply_penalties` and `sampler_accept` would do."""
     _chk(logits, "logits", torch.float32, 2)
     _chk(rng, "rng states", torch.int64, 1)
     _chk(params, "sampling parameters", torch.float32, 1)
     B, V = logits.shape
     if out is None:
         out = torch.empty((B,), dtype=torch.int32, device=logits.device)
-    pv = pi = None
-    if V >= SAMPLE_TWO_STEP_MIN_VOCAB:
-        pv, pi = _sample_scratch(logits.device, B)
-    call("mynah_sample", ptr(logits), B, V, V, ptr(params), ptr(rng), ptr(slots), ptr(out), ptr(pv), ptr(pi), stream_ptr())
+    tokens, counts, heads = ring if ring is not None else (None, None, None)
+    if ring is not None:
+        _chk(tokens, "ring", torch.int32, 2)
+    call("mynah_sample", ptr(logits), B, V, V, ptr(params), ptr(rng), ptr(slots), ptr(out), ptr(tokens), ptr(counts), ptr(heads),
+         tokens.shape[1] if ring is not None else 0, stream_ptr())
     return out
-
-
-# From this vocabulary size on a row's maximum is found by several CTAs first (one CTA reads a long row slowly).
-SAMPLE_TWO_STEP_MIN_VOCAB = 16384
-_SAMPLE_SCRATCH: dict = {}
-
-
-def _sample_scratch(device, B: int):
-    """Scratch of the two-step maximum, kept for the life of the process (a captured step holds its address)."""
-    key = (str(device), B)
-    if key not in _SAMPLE_SCRATCH:
-        if torch.cuda.is_current_stream_capturing():
-            raise KernelError("sample: scratch memory must exist before graph capture")
-        n = B * int(lib.load().mynah_argmax_parts())
-        _SAMPLE_SCRATCH[key] = (torch.empty((n,), dtype=torch.float32, device=device),
-                                torch.empty((n,), dtype=torch.int32, device=device))
-    return _SAMPLE_SCRATCH[key]
 
 
 def apply_penalties(logits: torch.Tensor, ring: torch.Tensor, ring_n: torch.Tensor, slots: Optional[torch.Tensor],

@@ -146,13 +146,9 @@ class SamplerState:
         self.ring_head[idx] = torch.tensor(heads, dtype=torch.int32, device=self.device)
 
     def sample(self, logits: torch.Tensor, slots: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
-        """Penalties, then the draw, then the accepted token into the ring.
-        `logits` [B, V] fp32 is overwritten; `slots` int32 [B] (negative: padding)."""
+        """Penalties, then the draw, then the accepted token into the ring, in one launch.
+        `logits` [B, V] fp32 may be overwritten; `slots` int32 [B] (negative: padding)."""
         if not torch.cuda.is_current_stream_capturing():
             self.flush_resets()
-        if self.window > 0:
-            kernels.apply_penalties(logits, self.ring, self.ring_n, slots, self.params)
-        out = kernels.sample(logits, self.params, self.rng, slots, out)
-        if self.window > 0:
-            kernels.sampler_accept(out, self.ring, self.ring_n, self.ring_head, slots, self.params)
-        return out
+        return kernels.sample(logits, self.params, self.rng, slots, out,
+                              (self.ring, self.ring_n, self.ring_head) if self.window > 0 else None)

@@ -1,0 +1,68 @@
+"""The one-launch draw against the plain sampler, at the edges of its routes: lists of candidates (a bound from the groups'
+maxima, many equal logits, more places than finite logits), rows that fit shared memory or do not, rows that no 16-byte load
+can start at, and the penalties and the ring inside the launch."""
+import numpy as np
+import pytest
+import torch
+
+from plain.sampler import PlainSampler
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _rows(rng, V, kind):
+    lg = (rng.standard_normal((4, V)) * 2.0).astype(np.float32)
+    if kind == "equal":                                    # far more than 256 logits share the largest values
+        lg = np.round(lg)
+        lg[1, :] = 0.5
+    elif kind == "masked":                                 # fewer finite logits than places
+        lg[:, 7:] = -np.inf
+        lg[2, V - 1] = 3.0
+    elif kind == "sharp":                                  # all but a few exponentials vanish
+        lg *= 40.0
+    return lg
+
+
+@pytest.mark.parametrize("V,kind", [(300, "plain"), (32767, "plain"), (32768, "plain"), (65541, "plain"), (32771, "equal"),
+                                    (40000, "equal"), (1003, "equal"), (50000, "masked"), (900, "masked"), (33000, "sharp"),
+                                    (400001, "plain"), (60000, "plain")])
+@pytest.mark.parametrize("temp,top_k,top_p,min_p", [(0.6, 20, 0.95, 0.0), (1.0, 128, 0.9, 0.0), (1.0, 129, 1.0, 0.0),
+                                                    (0.8, 0, 0.9, 0.0), (1.0, 0, 1.0, 0.1), (0.9, 257, 1.0, 0.0), (0.0, 20, 1.0, 0.0)])
+def test_routes_match_plain_sampler(V, kind, temp, top_k, top_p, min_p):
+    """The same token from the same generator state. Equal logits make equal probabilities, which ids tell apart."""
+    from mynah_slm_b200.ops import kernels
+    rng = np.random.default_rng(V + top_k)
+    plain = [PlainSampler(temp=temp, top_k=top_k, top_p=top_p, min_p=min_p, rng_state=101 + i) for i in range(4)]
+    state = torch.tensor([101 + i for i in range(4)], dtype=torch.int64, device=DEV)
+    params = torch.tensor([temp, top_p, min_p, float(top_k), 1.0, 0.0, 0.0, 0.0], dtype=torch.float32, device=DEV)
+    for _ in range(3):
+        lg = _rows(rng, V, kind)
+        with np.errstate(all="ignore"):
+            want = [p.sample(lg[b].copy()) for b, p in enumerate(plain)]
+        got = kernels.sample(torch.from_numpy(lg.copy()).to(DEV), params, state, None).cpu().tolist()
+        assert got == want
+
+
+@pytest.mark.parametrize("V", [500, 40002])
+@pytest.mark.parametrize("temp,top_k", [(0.0, 0), (0.9, 20), (0.9, 0)])
+def test_penalties_and_ring_inside_the_draw(V, temp, top_k):
+    """Draw after draw with a window of five tokens: the ring holds repeats, and what it holds decides the next draw."""
+    from mynah_slm_b200.ops import kernels
+    rng, W, stride, B = np.random.default_rng(3), 5, 8, 3
+    plain = [PlainSampler(temp=temp, top_k=top_k, top_p=0.95, repeat_penalty=1.4, freq_penalty=0.3, presence_penalty=0.2,
+                          penalty_window=W, rng_state=7 + i) for i in range(B)]
+    ring = tuple(torch.zeros(shape, dtype=torch.int32, device=DEV) for shape in ((B + 1, stride), (B + 1,), (B + 1,)))
+    state = torch.tensor([7 + i for i in range(B)] + [99], dtype=torch.int64, device=DEV)
+    params = torch.tensor([temp, 0.95, 0.0, float(top_k), 1.4, 0.3, 0.2, float(W)], dtype=torch.float32, device=DEV)
+    slots = torch.tensor([0, 1, -1, 2], dtype=torch.int32, device=DEV)
+    base = rng.standard_normal((4, V)).astype(np.float32)
+    base[:, [3, V // 2, V - 2]] += 6.0                                            # three favourites: tokens come again
+    for _ in range(14):
+        lg = base + 0.3 * rng.standard_normal((4, V)).astype(np.float32)
+        want = [p.sample(lg[row].copy()) for p, row in zip(plain, (0, 1, 3))]
+        got = kernels.sample(torch.from_numpy(lg.copy()).to(DEV), params, state, slots, ring=ring).cpu().tolist()
+        assert [got[0], got[1], got[3]] == want
+        for p, t in zip(plain, want):
+            p.accept(t)
+    assert ring[1].cpu().tolist() == [W] * B + [0] and int(state[B]) == 99
