@@ -11,7 +11,7 @@
 //                    head of one sequence; a column's dim values lie in the registers of L adjacent lanes (up to
 //                    32 values a lane), which add their parts of o by shuffles in a fixed order. Keys, queries and
 //                    values of 32 tokens at a time pass through shared memory.
-//   retention_chunk  the same recurrence for prompts, a chunk of tokens at a time (see below)
+//   retention_local, _states, _out   the same recurrence for prompts, a chunk of tokens at a time (see below)
 //
 // All arithmetic is fp32. A sequence's rows are walked in order, so a prompt run whole, in pieces or token by
 // token performs the same operations in the same order.
@@ -66,6 +66,66 @@ retention_prep_kernel(const T* __restrict__ qk, float* __restrict__ qn, float* _
         if (is_k) kn[(size_t)t * n + e] = v * a.k_scale;
         else qn[(size_t)t * n + e] = v;
     }
+}
+
+// The same where eight values lie on 16-byte boundaries and a rotated pair's two halves do too: a thread takes eight of a head
+// (and fetches the eight they are paired with), so that every access is a vector and a step of any size has all its loads in
+// flight at once. 16 heads of 128, us: 4 rows 13.8 -> 2.7, 3,837 rows 57 -> 28.
+template <typename T>
+__global__ void __launch_bounds__(128)
+retention_prep_vec_kernel(const T* __restrict__ qk, float* __restrict__ qn, float* __restrict__ kn,
+                          const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                          const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, RetPrepArgs a, int n_tok,
+                          int* __restrict__ status) {
+    griddep_launch_small();
+    griddep_wait();
+    const int n = a.H * a.dim, per = n / 8;                 // pieces of eight, q's then k's
+    const int piece = blockIdx.x * blockDim.x + threadIdx.x, t = blockIdx.y + blockIdx.z * gridDim.y;
+    if (piece >= 2 * per || t >= n_tok || tok_seq[t] < 0) return;
+    const int pos = tok_pos[t];
+    const bool rotate = a.rot > 0 && cos_t != nullptr;
+    if (rotate && (pos < 0 || pos >= a.n_pos)) {
+        if (piece == 0) atomicOr(status, MYNAH_ST_POS_RANGE);
+        return;
+    }
+    const bool is_k = piece >= per;
+    const int e = (is_k ? piece - per : piece) * 8, h = e / a.dim, d = e % a.dim;
+    const T* src = qk + (size_t)t * a.ld + (is_k ? a.k_off : a.q_off) + (size_t)h * a.dim;
+    auto load = [](const T* p, float (&x)[8]) {
+        uint4 w[sizeof(T) / 2];
+#pragma unroll
+        for (int i = 0; i < (int)sizeof(T) / 2; i++) w[i] = reinterpret_cast<const uint4*>(p)[i];
+        const T* y = reinterpret_cast<const T*>(w);
+#pragma unroll
+        for (int i = 0; i < 8; i++) x[i] = to_f32(y[i]);
+    };
+    float x[8], r[8];
+    load(src + d, x);
+#pragma unroll
+    for (int j = 0; j < 8; j++) r[j] = x[j];
+    if (rotate && d < a.rot) {
+        const int half = a.rot >> 1;
+        const float* cr = cos_t + (size_t)pos * half;
+        const float* sr = sin_t + (size_t)pos * half;
+        if (a.interleaved) {
+#pragma unroll
+            for (int j = 0; j < 8; j++) {
+                const float sign = (j & 1) ? 1.f : -1.f;
+                r[j] = x[j] * cr[(d + j) >> 1] + sign * x[j ^ 1] * sr[(d + j) >> 1];
+            }
+        } else {
+            const int i = d < half ? d : d - half;
+            const float sign = d < half ? -1.f : 1.f;
+            float y[8];
+            load(src + (d < half ? d + half : d - half), y);
+#pragma unroll
+            for (int j = 0; j < 8; j++) r[j] = x[j] * cr[i + j] + sign * y[j] * sr[i + j];
+        }
+    }
+    const float scale = is_k ? a.k_scale : 1.f;
+    float4* dst = reinterpret_cast<float4*>((is_k ? kn : qn) + (size_t)t * n + e);
+    dst[0] = make_float4(r[0] * scale, r[1] * scale, r[2] * scale, r[3] * scale);
+    dst[1] = make_float4(r[4] * scale, r[5] * scale, r[6] * scale, r[7] * scale);
 }
 
 constexpr int RET_THREADS = 128;
@@ -153,297 +213,382 @@ retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn
 // With a chunk of C tokens, S the state before it and g the head's decay:
 //
 //   o_t   = sum_{s <= t} g^(t-s) (q_t . k_s) v_s  +  g^(t+1) S^T q_t                      t, s inside the chunk
-//   S_new = g^n S + sum_s g^(n-1-s) k_s v_s^T                                            n tokens in the chunk
+//   S_new = g^n S + U,   U = sum_s g^(n-1-s) k_s v_s^T                                   n tokens in the chunk
 //
-// so the 2n dependent steps of a chunk become blocks of independent multiply-adds. Two kernels:
+// U does not depend on S, and o depends on nothing but S and the chunk, so only the elementwise recurrence over the
+// chunks' states is a chain. Three kernels, all sums fp32:
 //
-//   retention_scores  the decayed scores g^(t-s) (q_t . k_s) of every chunk of every sequence, side by side (they do
-//                     not depend on the state): a CTA a chunk and head, register-tiled fp32, written to scratch
-//                     [H][rows][C]
-//   retention_chunk   the chain: a CTA takes JW columns (32, or 16 when the step has too few CTAs for the machine) of one
-//                     head of one sequence and walks the sequence's chunks in order: scores times values, the read of
-//                     the old state, the state's update. q and k of the chunk, the scores, the values and the state's
-//                     columns lie in shared memory.
+//   retention_local   U of every chunk and head, into scratch [chunk][H][dim][columns]
+//   retention_states  the chain: a thread takes four values of a state through its sequence's chunks, puts the state before
+//                     a chunk in U's place and the last one into the slot
+//   retention_out     the decayed scores of a chunk (kept in shared memory), the read of its old state, scores times values
+//
+// What bounds them: the multiply-adds (49,000 a token and head of 128 x 128, 3.1e9 a layer for 4,000 tokens of 16 heads: 88 us at
+// the FFMA rate) and the reads of shared memory that feed them; the products run in pairs (fma.rn.f32x2, the same roundings),
+// which halves the instructions beside the loads. Scratch is bounded: a step's chunks go in passes of about 96 MB of states
+// (what the cache holds), in the order of their sequences. Measured (3,837 tokens of 4 sequences,
+// 16 heads of 128), us a layer: 85 + 46 + 137; a chain of CTAs that each walked a head's 32 columns through its chunks took 625.
 //
 // The powers of g come from a table made by repeated multiplication. Sums run in another order than token by token:
 // the two forms agree to rounding.
 constexpr int RC_THREADS = 256;
 
 struct RetChunkArgs {
-    int H, dim, vd, n_slots, ldv, v_off, rows, B;
+    int H, dim, vd, n_slots, ldv, v_off, B, cols;          // cols: columns of a state in scratch (vd padded to whole tiles)
+    int first;                                              // the pass's first chunk
 };
 
-// grid (rows / C + B, H): the step's chunks are numbered sequence by sequence (layout.cuh: find_query_tile)
-template <int C>
-__global__ void __launch_bounds__(RC_THREADS)
-retention_scores_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const float* __restrict__ decay,
-                        float* __restrict__ w_out, const int* __restrict__ cu_q, RetChunkArgs a) {
-    constexpr int TT = C / 16;
-    extern __shared__ __align__(16) float sm[];
-    __shared__ float gp[C];
-    griddep_wait();
-    int b, tile;
-    if (!find_query_tile(cu_q, a.B, C, (int)blockIdx.x, b, tile)) return;
-    const int h = blockIdx.y, d = a.dim, ldr = d + 4;
-    float* qs = sm;
-    float* ks = qs + C * ldr;
-    const int tid = threadIdx.x;
-    const int t0 = cu_q[b] + tile * C, nt = min(C, cu_q[b + 1] - t0);
-    if (tid == 0) {
-        float p = 1.f;
-        const float g = decay[h];
-        for (int n = 0; n < C; n++) {
-            gp[n] = p;
-            p *= g;
-        }
-    }
-    const size_t n = (size_t)a.H * d;
-    for (int idx = tid; idx < C * (d / 4); idx += RC_THREADS) {
-        const int tt = idx / (d / 4), i4 = (idx % (d / 4)) * 4;
-        float4 qv = make_float4(0.f, 0.f, 0.f, 0.f), kv = qv;
-        if (tt < nt) {
-            const size_t src = (size_t)(t0 + tt) * n + (size_t)h * d + i4;
-            qv = *reinterpret_cast<const float4*>(qn + src);
-            kv = *reinterpret_cast<const float4*>(kn + src);
-        }
-        *reinterpret_cast<float4*>(qs + tt * ldr + i4) = qv;
-        *reinterpret_cast<float4*>(ks + tt * ldr + i4) = kv;
-    }
-    __syncthreads();
-    // thread (ta, sb) takes tokens ta + 16 u and keys sb + 16 w
-    const int ta = tid >> 4, sb = tid & 15;
-    float acc[TT][TT];
-#pragma unroll
-    for (int u = 0; u < TT; u++)
-#pragma unroll
-        for (int w = 0; w < TT; w++) acc[u][w] = 0.f;
-#pragma unroll 2
-    for (int i = 0; i < d; i += 4) {
-        float4 qv[TT], kv[TT];
-#pragma unroll
-        for (int u = 0; u < TT; u++) qv[u] = *reinterpret_cast<const float4*>(qs + (ta + 16 * u) * ldr + i);
-#pragma unroll
-        for (int w = 0; w < TT; w++) kv[w] = *reinterpret_cast<const float4*>(ks + (sb + 16 * w) * ldr + i);
-#pragma unroll
-        for (int u = 0; u < TT; u++)
-#pragma unroll
-            for (int w = 0; w < TT; w++) {
-                acc[u][w] = fmaf(qv[u].x, kv[w].x, acc[u][w]);
-                acc[u][w] = fmaf(qv[u].y, kv[w].y, acc[u][w]);
-                acc[u][w] = fmaf(qv[u].z, kv[w].z, acc[u][w]);
-                acc[u][w] = fmaf(qv[u].w, kv[w].w, acc[u][w]);
-            }
-    }
-    float* wo = w_out + ((size_t)h * a.rows + t0) * C;
-#pragma unroll
-    for (int u = 0; u < TT; u++)
-#pragma unroll
-        for (int w = 0; w < TT; w++) {
-            const int t = ta + 16 * u, s = sb + 16 * w;
-            if (t < nt) wo[(size_t)t * C + s] = s <= t ? gp[t - s] * acc[u][w] : 0.f;
-        }
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
 }
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(f32x2& c, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void mul2(f32x2& c, f32x2 a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
 
-template <typename T, int C, int JW>
-__global__ void __launch_bounds__(RC_THREADS)
-retention_chunk_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v,
-                       const float* __restrict__ decay, const float* __restrict__ w_in, float* __restrict__ state,
-                       float* __restrict__ o, const int* __restrict__ cu_q, const int* __restrict__ slots, RetChunkArgs a) {
-    constexpr int HS = 32 / JW;            // groups of lanes that share the CTA's columns (1 or 2)
-    constexpr int TPW = C / 8 / HS;        // tokens a group of lanes takes in the products with the values and the state
-    constexpr int LDW = C + 4;             // row stride of the decayed scores (rows stay 16-byte aligned)
-    extern __shared__ __align__(16) float sm[];
-    griddep_wait();
-    const int b = blockIdx.z, h = blockIdx.y;
-    const int slot = slots[b];
-    const int q0 = cu_q[b], q1 = cu_q[b + 1];
-    if (slot < 0 || slot >= a.n_slots || q1 <= q0) return;
-    const int d = a.dim, ldr = d + 4;      // row stride of q and k in shared memory (16 bytes of padding)
-    const int rpw = d / 8 / HS;            // state rows a group of lanes owns (a multiple of 4)
-    float* qs = sm;                        // [C][ldr]
-    float* ks = qs + C * ldr;              // [C][ldr]
-    float* Ss = ks + C * ldr;              // [d][JW]
-    float* Ws = Ss + d * JW;               // [C][LDW]
-    float* vs = Ws + C * LDW;              // [C][JW]
-    float* gp = vs + C * JW;               // [C + 1]: powers of the decay
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int grp = lane / JW, col = lane % JW;
-    const int j = blockIdx.x * JW + col;
-    const bool on = j < a.vd;
-    const float g = decay[h];
-    if (tid == 0) {
+struct alignas(16) Pairs { f32x2 lo, hi; };                 // four floats as two pairs, one 16-byte load
+__device__ __forceinline__ Pairs pairs_at(const float* p) { return *reinterpret_cast<const Pairs*>(p); }
+
+// gp[n] = g^n, n <= C
+template <int C>
+__device__ __forceinline__ void decay_powers(float* gp, float g) {
+    if (threadIdx.x == 0) {
         float p = 1.f;
         for (int n = 0; n <= C; n++) {
             gp[n] = p;
             p *= g;
         }
     }
-    float* sp = state + (((size_t)slot * a.H + h) * d) * a.vd;
-    for (int idx = tid; idx < d * JW; idx += RC_THREADS) {
-        const int i = idx / JW, c = blockIdx.x * JW + idx % JW;
-        Ss[idx] = c < a.vd ? sp[(size_t)i * a.vd + c] : 0.f;
+}
+
+// A chunk's rows of one head into shared memory, rows from nt on as zeros (C rows, d values, d + 4 apart).
+template <int C>
+__device__ __forceinline__ void stage_rows(float* dst, const float* __restrict__ src, size_t row, int d, int nt) {
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < C * (d / 4); idx += RC_THREADS) {
+        const int tt = idx / (d / 4), i4 = (idx % (d / 4)) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tt < nt) x = *reinterpret_cast<const float4*>(src + (size_t)tt * row + i4);
+        *reinterpret_cast<float4*>(dst + tt * (d + 4) + i4) = x;
     }
+}
+
+// A chunk's values of one head, columns [j0, j0 + JT), times `weight(token)`; what does not exist is zero.
+template <typename T, int C, int JT, typename F>
+__device__ __forceinline__ void stage_values(float* vs, const T* __restrict__ v, int ldv, int j0, int vd, int nt, F weight) {
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < C * JT; idx += RC_THREADS) {
+        const int tt = idx / JT, c = idx % JT;
+        vs[idx] = (tt < nt && j0 + c < vd) ? weight(tt) * to_f32(v[(size_t)tt * ldv + j0 + c]) : 0.f;
+    }
+}
+
+// grid (chunks of the pass, H, cols / JT): the step's chunks are numbered sequence by sequence (layout.cuh: find_query_tile).
+// Thread (ti, tj) owns state rows ti * 8 + u and columns tj * 4 + {0..3} of either half of the tile.
+template <typename T, int C, int JT>
+__global__ void __launch_bounds__(RC_THREADS, 2)
+retention_local_kernel(const float* __restrict__ kn, const T* __restrict__ v, const float* __restrict__ decay, float* __restrict__ states,
+                       const int* __restrict__ cu_q, RetChunkArgs a) {
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float gp[C + 1];
+    griddep_wait();
+    int b, tile;
+    if (!find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile)) return;
+    const int h = blockIdx.y, d = a.dim, j0 = blockIdx.z * JT;
+    const int t0 = cu_q[b] + tile * C, nt = min(C, cu_q[b + 1] - t0);
+    float* ks = sm;                        // [C][d + 4]
+    float* vs = ks + C * (d + 4);          // [C][JT]
+    decay_powers<C>(gp, decay[h]);
     const size_t n = (size_t)a.H * d;
-    // A chunk's q, k, scores and values travel through registers: the loads of chunk c + 1 are issued before chunk c
-    // is computed, all at once, so that the chain waits on no load. (C * d <= 8192: at most 8 + 8 + 4 vectors a thread.)
-    constexpr int QK_IT = 8, W_IT = C * (C / 4) / RC_THREADS > 0 ? C * (C / 4) / RC_THREADS : 1, V_IT = C * JW / RC_THREADS;
-    float4 rq[QK_IT], rk[QK_IT], rw[W_IT];
-    float rv[V_IT];
-    const int qk_total = C * (d / 4);
-    auto load_chunk = [&](int t0) {
-        const int nt = min(C, q1 - t0);
-        const float* wi = w_in + ((size_t)h * a.rows + t0) * C;
-#pragma unroll
-        for (int it = 0; it < QK_IT; it++) {
-            const int idx = tid + it * RC_THREADS;
-            const int tt = idx / (d / 4), i4 = (idx % (d / 4)) * 4;
-            rq[it] = rk[it] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (idx < qk_total && tt < nt) {
-                const size_t src = (size_t)(t0 + tt) * n + (size_t)h * d + i4;
-                rq[it] = *reinterpret_cast<const float4*>(qn + src);
-                rk[it] = *reinterpret_cast<const float4*>(kn + src);
-            }
-        }
-#pragma unroll
-        for (int it = 0; it < W_IT; it++) {
-            const int idx = tid + it * RC_THREADS;
-            const int tt = idx / (C / 4), s4 = (idx % (C / 4)) * 4;
-            rw[it] = (idx < C * (C / 4) && tt < nt) ? *reinterpret_cast<const float4*>(wi + (size_t)tt * C + s4)
-                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int it = 0; it < V_IT; it++) {
-            const int idx = tid + it * RC_THREADS;
-            const int tt = idx / JW, c = blockIdx.x * JW + idx % JW;
-            rv[it] = (tt < nt && c < a.vd) ? to_f32(v[(size_t)(t0 + tt) * a.ldv + a.v_off + (size_t)h * a.vd + c]) : 0.f;
-        }
-    };
-    auto store_chunk = [&]() {
-#pragma unroll
-        for (int it = 0; it < QK_IT; it++) {
-            const int idx = tid + it * RC_THREADS;
-            if (idx < qk_total) {
-                const int tt = idx / (d / 4), i4 = (idx % (d / 4)) * 4;
-                *reinterpret_cast<float4*>(qs + tt * ldr + i4) = rq[it];
-                *reinterpret_cast<float4*>(ks + tt * ldr + i4) = rk[it];
-            }
-        }
-#pragma unroll
-        for (int it = 0; it < W_IT; it++) {
-            const int idx = tid + it * RC_THREADS;
-            if (idx < C * (C / 4)) *reinterpret_cast<float4*>(Ws + (idx / (C / 4)) * LDW + (idx % (C / 4)) * 4) = rw[it];
-        }
-#pragma unroll
-        for (int it = 0; it < V_IT; it++) vs[tid + it * RC_THREADS] = rv[it];
-    };
-    load_chunk(q0);
-    for (int t0 = q0; t0 < q1; t0 += C) {
-        const int nt = min(C, q1 - t0);
-        __syncthreads();                                         // the chunk before is done with q, k, v, the scores
-        store_chunk();
-        __syncthreads();
-        if (t0 + C < q1) load_chunk(t0 + C);                     // in flight while this chunk is computed
-        {   // o: lane group `grp` of warp `warp` takes tokens tb + u, its lanes the columns
-            float intra[TPW], inter[TPW];
-#pragma unroll
-            for (int u = 0; u < TPW; u++) intra[u] = inter[u] = 0.f;
-            const int tb = (warp * HS + grp) * TPW;
-            const int s_end = min((tb + TPW + 3) & ~3, C);       // keys beyond the group's last token weigh nothing
-            for (int s = 0; s < s_end; s += 4) {                 // (rows beyond nt hold zeros)
-                const float v0 = vs[s * JW + col], v1 = vs[(s + 1) * JW + col];
-                const float v2 = vs[(s + 2) * JW + col], v3 = vs[(s + 3) * JW + col];
-#pragma unroll
-                for (int u = 0; u < TPW; u++) {
-                    const float4 w4 = *reinterpret_cast<const float4*>(Ws + (tb + u) * LDW + s);
-                    intra[u] = fmaf(w4.x, v0, intra[u]);
-                    intra[u] = fmaf(w4.y, v1, intra[u]);
-                    intra[u] = fmaf(w4.z, v2, intra[u]);
-                    intra[u] = fmaf(w4.w, v3, intra[u]);
-                }
-            }
-#pragma unroll 2
-            for (int i = 0; i < d; i += 4) {
-                const float s0 = Ss[i * JW + col], s1 = Ss[(i + 1) * JW + col];
-                const float s2 = Ss[(i + 2) * JW + col], s3 = Ss[(i + 3) * JW + col];
-#pragma unroll
-                for (int u = 0; u < TPW; u++) {
-                    const float4 qv = *reinterpret_cast<const float4*>(qs + (tb + u) * ldr + i);
-                    inter[u] = fmaf(qv.x, s0, inter[u]);
-                    inter[u] = fmaf(qv.y, s1, inter[u]);
-                    inter[u] = fmaf(qv.z, s2, inter[u]);
-                    inter[u] = fmaf(qv.w, s3, inter[u]);
-                }
-            }
-            if (on) {
-#pragma unroll
-                for (int u = 0; u < TPW; u++) {
-                    const int t = tb + u;
-                    if (t < nt) o[(size_t)(t0 + t) * a.H * a.vd + (size_t)h * a.vd + j] = fmaf(gp[t + 1], inter[u], intra[u]);
-                }
-            }
-        }
-        __syncthreads();                                         // every warp has read the old state
-        {   // the state's rows (warp * HS + grp) * rpw + r, column `col`
-            const float gn = gp[nt];
-            float loc[32];                                       // rpw <= 32 rows (d <= 256)
-#pragma unroll
-            for (int r = 0; r < 32; r++) loc[r] = 0.f;
-            const int row0 = (warp * HS + grp) * rpw;
-            const float* kw = ks + row0;
-#pragma unroll 2
-            for (int s = 0; s < nt; s++) {
-                const float vw = gp[nt - 1 - s] * vs[s * JW + col];
-#pragma unroll
-                for (int r4 = 0; r4 < 8; r4++) {
-                    if (r4 * 4 < rpw) {
-                        const float4 kv = *reinterpret_cast<const float4*>(kw + s * ldr + r4 * 4);
-                        loc[r4 * 4] = fmaf(kv.x, vw, loc[r4 * 4]);
-                        loc[r4 * 4 + 1] = fmaf(kv.y, vw, loc[r4 * 4 + 1]);
-                        loc[r4 * 4 + 2] = fmaf(kv.z, vw, loc[r4 * 4 + 2]);
-                        loc[r4 * 4 + 3] = fmaf(kv.w, vw, loc[r4 * 4 + 3]);
-                    }
-                }
-            }
-#pragma unroll
-            for (int r = 0; r < 32; r++)
-                if (r < rpw) {
-                    float* sl = Ss + (row0 + r) * JW + col;
-                    *sl = fmaf(gn, *sl, loc[r]);
-                }
-        }
-    }
+    stage_rows<C>(ks, kn + (size_t)t0 * n + (size_t)h * d, n, d, nt);
     __syncthreads();
-    for (int idx = tid; idx < d * JW; idx += RC_THREADS) {
-        const int i = idx / JW, c = blockIdx.x * JW + idx % JW;
-        if (c < a.vd) sp[(size_t)i * a.vd + c] = Ss[idx];
+    stage_values<T, C, JT>(vs, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd, nt,
+                           [&](int tt) { return gp[nt - 1 - tt]; });
+    __syncthreads();
+    constexpr int TJ = JT / 8;
+    const int ti = threadIdx.x / TJ, tj = threadIdx.x % TJ;
+    if (ti * 8 >= d) return;
+    f32x2 acc[8][4];
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+#pragma unroll
+        for (int w = 0; w < 4; w++) acc[u][w] = 0ull;
+    const float* kr = ks + ti * 8;
+    const float* vr = vs + tj * 4;
+#pragma unroll 2
+    for (int s = 0; s < nt; s++) {
+        const float4 k0 = *reinterpret_cast<const float4*>(kr + s * (d + 4)), k1 = *reinterpret_cast<const float4*>(kr + s * (d + 4) + 4);
+        const Pairs v0 = pairs_at(vr + s * JT), v1 = pairs_at(vr + s * JT + JT / 2);
+        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const f32x2 k2 = pack2(kk[u], kk[u]);
+            fma2(acc[u][0], k2, v0.lo);
+            fma2(acc[u][1], k2, v0.hi);
+            fma2(acc[u][2], k2, v1.lo);
+            fma2(acc[u][3], k2, v1.hi);
+        }
+    }
+    float* out = states + (((size_t)blockIdx.x * a.H + h) * d + ti * 8) * a.cols + j0 + tj * 4;
+#pragma unroll
+    for (int u = 0; u < 8; u++) {
+        *reinterpret_cast<Pairs*>(out + (size_t)u * a.cols) = Pairs{acc[u][0], acc[u][1]};
+        *reinterpret_cast<Pairs*>(out + (size_t)u * a.cols + JT / 2) = Pairs{acc[u][2], acc[u][3]};
     }
 }
 
-template <typename T, int C, int JW>
-int launch_chain(const float* qn, const float* kn, const void* v, const float* decay, const float* w, float* state, float* o,
-                 const int* cu_q, const int* slots, const RetChunkArgs& a, cudaStream_t stream) {
-    const int d = a.dim;
-    const size_t smem = ((size_t)2 * C * (d + 4) + (size_t)d * JW + (size_t)C * (C + 4) + (size_t)C * JW + C + 1 + 3) * sizeof(float);
-    if (cudaFuncSetAttribute(retention_chunk_kernel<T, C, JW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return mynah_fail("retention_scan: %zu bytes of shared memory are not to be had", smem);
-    mynah_launch(retention_chunk_kernel<T, C, JW>, dim3(ceil_div(a.vd, JW), a.H, a.B), dim3(RC_THREADS), smem, stream,
-                 qn, kn, (const T*)v, decay, w, state, o, cu_q, slots, a);
-    return mynah_check_launch("retention_scan (chunked)");
+// grid (dim * cols / 4 / 256, H, B): four values of one state a thread, through the pass's chunks of sequence b.
+__global__ void __launch_bounds__(RC_THREADS)
+retention_states_kernel(const float* __restrict__ decay, float* __restrict__ states, float* __restrict__ state,
+                        const int* __restrict__ cu_q, const int* __restrict__ slots, RetChunkArgs a, int C, int n_pass) {
+    __shared__ int parts[RC_THREADS / 32];
+    griddep_wait();
+    const int b = blockIdx.z, h = blockIdx.y;
+    const int q0 = cu_q[b], q1 = cu_q[b + 1], slot = slots[b];
+    // the sequence's first chunk number: those of the sequences before it
+    int before = 0;
+    for (int i = threadIdx.x; i < b; i += RC_THREADS) before += (cu_q[i + 1] - cu_q[i] + C - 1) / C;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if ((threadIdx.x & 31) == 0) parts[threadIdx.x >> 5] = before;
+    __syncthreads();
+    before = 0;
+#pragma unroll
+    for (int w = 0; w < RC_THREADS / 32; w++) before += parts[w];
+    const int tiles = (q1 - q0 + C - 1) / C;
+    // tile t of the sequence is number before + tiles - 1 - t; this pass holds the numbers [first, first + n_pass)
+    const int last_no = before + tiles - 1;
+    const int t_lo = max(0, last_no - (a.first + n_pass - 1)), t_hi = min(tiles, last_no - a.first + 1);
+    if (t_lo >= t_hi || slot < 0 || slot >= a.n_slots) return;
+    const int e = blockIdx.x * RC_THREADS + threadIdx.x, per_row = a.cols / 4;
+    const int i = e / per_row, c = (e % per_row) * 4;
+    if (i >= a.dim || c >= a.vd) return;
+    const float g = decay[h];
+    float gc = 1.f, gl = 1.f;                               // the decay over a whole chunk, over the sequence's last
+    for (int k = 0; k < C; k++) {
+        if (k == q1 - q0 - (tiles - 1) * C) gl = gc;
+        gc *= g;
+    }
+    if (q1 - q0 == tiles * C) gl = gc;
+    float* sp = state + (((size_t)slot * a.H + h) * a.dim + i) * a.vd + c;
+    const int have = min(4, a.vd - c);
+    float S[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) S[k] = k < have ? sp[k] : 0.f;
+    const size_t one = (size_t)a.H * a.dim * a.cols;        // floats of a chunk
+    float* at = states + ((size_t)h * a.dim + i) * a.cols + c;
+    constexpr int AHEAD = 8;
+    for (int t = t_lo; t < t_hi; t += AHEAD) {
+        float4 u[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++)
+            if (t + k < t_hi) u[k] = *reinterpret_cast<const float4*>(at + (size_t)(last_no - (t + k) - a.first) * one);
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) {
+            if (t + k < t_hi) {
+                *reinterpret_cast<float4*>(at + (size_t)(last_no - (t + k) - a.first) * one) = make_float4(S[0], S[1], S[2], S[3]);
+                const float gn = t + k == tiles - 1 ? gl : gc;
+                S[0] = fmaf(gn, S[0], u[k].x);
+                S[1] = fmaf(gn, S[1], u[k].y);
+                S[2] = fmaf(gn, S[2], u[k].z);
+                S[3] = fmaf(gn, S[3], u[k].w);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++)
+        if (k < have) sp[k] = S[k];
 }
 
-template <typename T, int C>
-int launch_chunked(const float* qn, const float* kn, const void* v, const float* decay, float* w, float* state, float* o,
-                   const int* cu_q, const int* slots, const RetChunkArgs& a, cudaStream_t stream) {
-    const size_t smem = (size_t)2 * C * (a.dim + 4) * sizeof(float);
-    if (cudaFuncSetAttribute(retention_scores_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-        return mynah_fail("retention_scan: %zu bytes of shared memory are not to be had", smem);
-    MYNAH_REQUIRE(a.rows / C + a.B <= 65535 * 32, "retention_scan: too many chunks for one launch");
-    mynah_launch(retention_scores_kernel<C>, dim3(a.rows / C + a.B, a.H), dim3(RC_THREADS), smem, stream, qn, kn, decay, w, cu_q, a);
-    if (mynah_check_launch("retention_scan (scores)") != 0) return -1;
-    // 16 columns a CTA when 32 would leave most of the machine idle (and the state's rows divide)
-    const bool narrow = a.dim % 64 == 0 && (long long)a.B * a.H * ceil_div(a.vd, 32) < mynah_sm_count();
-    return narrow ? launch_chain<T, C, 16>(qn, kn, v, decay, w, state, o, cu_q, slots, a, stream)
-                  : launch_chain<T, C, 32>(qn, kn, v, decay, w, state, o, cu_q, slots, a, stream);
+// The same grid as retention_local. Thread (ty, tx) owns tokens ty * RT + u and columns tx * 4 + {0..3} (of either half, when the
+// tile has 128). The keys' place in shared memory is used again by the old state, 32 rows at a time, and then by the values.
+template <typename T, int C, int JT>
+__global__ void __launch_bounds__(RC_THREADS, 2)
+retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v, const float* __restrict__ decay,
+                     const float* __restrict__ states, float* __restrict__ o, const int* __restrict__ cu_q,
+                     const int* __restrict__ slots, RetChunkArgs a) {
+    constexpr int RT = C / 16, G = JT / 64, LDW = C + 4, SR = 32;
+    extern __shared__ __align__(16) float sm[];
+    __shared__ float gp[C + 1];
+    griddep_wait();
+    int b, tile;
+    if (!find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile)) return;
+    const int slot = slots[b];
+    if (slot < 0 || slot >= a.n_slots) return;
+    const int h = blockIdx.y, d = a.dim, j0 = blockIdx.z * JT, ldr = d + 4;
+    const int t0 = cu_q[b] + tile * C, nt = min(C, cu_q[b + 1] - t0);
+    float* qs = sm;                        // [C][ldr]
+    float* Ws = qs + C * ldr;              // [C][LDW]
+    float* xs = Ws + C * LDW;              // [C][ldr] keys; [2][SR][JT] state rows; [C][JT] values
+    decay_powers<C>(gp, decay[h]);
+    const size_t n = (size_t)a.H * d;
+    stage_rows<C>(qs, qn + (size_t)t0 * n + (size_t)h * d, n, d, nt);
+    stage_rows<C>(xs, kn + (size_t)t0 * n + (size_t)h * d, n, d, nt);
+    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    {   // scores: tokens ty + 16 u, keys tx + 16 w; even and odd values of a head are summed apart, then added
+        f32x2 acc[RT][RT];
+#pragma unroll
+        for (int u = 0; u < RT; u++)
+#pragma unroll
+            for (int w = 0; w < RT; w++) acc[u][w] = 0ull;
+#pragma unroll 2
+        for (int i = 0; i < d; i += 4) {
+            Pairs qv[RT], kv[RT];
+#pragma unroll
+            for (int u = 0; u < RT; u++) qv[u] = pairs_at(qs + (ty + 16 * u) * ldr + i);
+#pragma unroll
+            for (int w = 0; w < RT; w++) kv[w] = pairs_at(xs + (tx + 16 * w) * ldr + i);
+#pragma unroll
+            for (int u = 0; u < RT; u++)
+#pragma unroll
+                for (int w = 0; w <= u; w++) {              // (keys behind every token of the group: not needed)
+                    fma2(acc[u][w], qv[u].lo, kv[w].lo);
+                    fma2(acc[u][w], qv[u].hi, kv[w].hi);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < RT; u++)
+#pragma unroll
+            for (int w = 0; w < RT; w++) {
+                const int t = ty + 16 * u, s = tx + 16 * w;
+                const float2 x = unpack2(acc[u][w]);
+                Ws[t * LDW + s] = s <= t ? gp[t - s] * (x.x + x.y) : 0.f;
+            }
+    }
+    __syncthreads();                                        // the scores are there, the keys are done with
+    f32x2 acc[RT][G][2];
+#pragma unroll
+    for (int u = 0; u < RT; u++)
+#pragma unroll
+        for (int w = 0; w < G; w++) acc[u][w][0] = acc[u][w][1] = 0ull;
+    // one product's four steps of k: rows [ty * RT, + RT) of `lhs` from column i, rows [i, i + 4) of `rhs`
+    auto steps = [&](const float* lhs, int ld, const float* rhs) {
+        float4 x[RT];
+#pragma unroll
+        for (int u = 0; u < RT; u++) x[u] = *reinterpret_cast<const float4*>(lhs + (ty * RT + u) * ld);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            Pairs y[G];
+#pragma unroll
+            for (int w = 0; w < G; w++) y[w] = pairs_at(rhs + k * JT + w * 64 + tx * 4);
+#pragma unroll
+            for (int u = 0; u < RT; u++) {
+                const float xk = k == 0 ? x[u].x : k == 1 ? x[u].y : k == 2 ? x[u].z : x[u].w;
+                const f32x2 x2 = pack2(xk, xk);
+#pragma unroll
+                for (int w = 0; w < G; w++) {
+                    fma2(acc[u][w][0], x2, y[w].lo);
+                    fma2(acc[u][w][1], x2, y[w].hi);
+                }
+            }
+        }
+    };
+    // ---- the old state, in pieces of SR rows; a piece is on its way while the one before is multiplied
+    const float* from = states + ((size_t)blockIdx.x * a.H + h) * d * a.cols + j0;
+    auto fetch = [&](int piece) {
+        if (piece * SR < d) {
+            float* dst = xs + (piece & 1) * SR * JT;
+#pragma unroll
+            for (int idx = threadIdx.x; idx < SR * JT / 4; idx += RC_THREADS) {
+                const int i = idx / (JT / 4), c = (idx % (JT / 4)) * 4;
+                const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst + i * JT + c);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(s), "l"(from + (size_t)(piece * SR + i) * a.cols + c) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    for (int p = 0; p * SR < d; p++) {
+        fetch(p + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float* S = xs + (p & 1) * SR * JT;
+#pragma unroll 2
+        for (int i = 0; i < SR; i += 4) steps(qs + p * SR + i, ldr, S + i * JT);
+        __syncthreads();                                    // the piece's place may be filled again
+    }
+#pragma unroll
+    for (int u = 0; u < RT; u++) {
+        const float gt = gp[ty * RT + u + 1];
+#pragma unroll
+        for (int w = 0; w < G; w++) {
+            mul2(acc[u][w][0], pack2(gt, gt));
+            mul2(acc[u][w][1], pack2(gt, gt));
+        }
+    }
+    // ---- scores times values
+    stage_values<T, C, JT>(xs, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd, nt, [](int) { return 1.f; });
+    __syncthreads();
+    const int s_end = ((ty | 1) + 1) * RT;                  // keys behind the last token of the warp's rows weigh nothing
+    for (int s = 0; s < s_end; s += 4) steps(Ws + s, LDW, xs + s * JT);
+#pragma unroll
+    for (int u = 0; u < RT; u++) {
+        const int t = ty * RT + u;
+        if (t >= nt) break;
+        float* row = o + (size_t)(t0 + t) * a.H * a.vd + (size_t)h * a.vd;
+#pragma unroll
+        for (int w = 0; w < G; w++) {
+            const int j = j0 + w * 64 + tx * 4;
+            const float2 x = unpack2(acc[u][w][0]), y = unpack2(acc[u][w][1]);
+            if (j + 3 < a.vd && (a.vd & 3) == 0) {
+                *reinterpret_cast<float4*>(row + j) = make_float4(x.x, x.y, y.x, y.y);
+            } else {
+                if (j < a.vd) row[j] = x.x;
+                if (j + 1 < a.vd) row[j + 1] = x.y;
+                if (j + 2 < a.vd) row[j + 2] = y.x;
+                if (j + 3 < a.vd) row[j + 3] = y.y;
+            }
+        }
+    }
+}
+
+// How a step's chunks go: tokens a chunk, columns a tile, padded columns of a state, chunks a pass.
+struct RetPlan {
+    int C, JT, cols, total, n_pass;
+    RetPlan(int rows, int B, int H, int dim, int vd) {
+        C = dim <= 128 ? 64 : 32;                           // (q and k of a chunk and a piece of the state: 86 KB a CTA, two an SM)
+        JT = dim <= 128 && vd > 64 ? 128 : 64;
+        cols = ceil_div(vd, JT) * JT;
+        total = rows / C + B;                               // at most
+        const long long one = (long long)H * dim * cols;
+        const long long fit = (96ll << 20) / 4 / one;
+        const int least = ceil_div(2 * mynah_sm_count(), H);
+        const int most = (int)(fit < least ? least : fit > total ? total : fit);
+        const int passes = ceil_div(total, most);
+        n_pass = ceil_div(total, passes);
+    }
+    long long floats(int H, int dim) const { return (long long)n_pass * H * dim * cols; }
+};
+
+template <typename T, int C, int JT>
+int launch_chunked(const float* qn, const float* kn, const void* v, const float* decay, float* states, float* state, float* o,
+                   const int* cu_q, const int* slots, RetChunkArgs a, const RetPlan& plan, cudaStream_t stream) {
+    const int d = a.dim;
+    const size_t local = ((size_t)C * (d + 4) + (size_t)C * JT) * sizeof(float);
+    const size_t shared_part = (size_t)C * (d + 4) > (size_t)64 * JT ? (size_t)C * (d + 4) : (size_t)64 * JT;
+    const size_t out = ((size_t)C * (d + 4) + (size_t)C * (C + 4) + shared_part) * sizeof(float);
+    if (cudaFuncSetAttribute(retention_local_kernel<T, C, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(retention_out_kernel<T, C, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess)
+        return mynah_fail("retention_scan: %zu bytes of shared memory are not to be had", out);
+    // a sequence's chunks are numbered from its last to its first, so the passes go from the last to the first too
+    for (int p = (plan.total - 1) / plan.n_pass; p >= 0; p--) {
+        a.first = p * plan.n_pass;
+        const dim3 grid(plan.n_pass, a.H, plan.cols / JT);
+        mynah_launch(retention_local_kernel<T, C, JT>, grid, dim3(RC_THREADS), local, stream, kn, (const T*)v, decay, states, cu_q, a);
+        mynah_launch(retention_states_kernel, dim3(ceil_div(d * (plan.cols / 4), RC_THREADS), a.H, a.B), dim3(RC_THREADS), 0, stream,
+                     decay, states, state, cu_q, slots, a, C, plan.n_pass);
+        mynah_launch(retention_out_kernel<T, C, JT>, grid, dim3(RC_THREADS), out, stream, qn, kn, (const T*)v, decay,
+                     (const float*)states, o, cu_q, slots, a);
+        if (mynah_check_launch("retention_scan (chunked)") != 0) return -1;
+    }
+    return 0;
 }
 
 }  // namespace
@@ -460,11 +605,16 @@ static bool retention_chunked(int dim, int max_q_len) {
     return g_ret_chunk_min > 0 && max_q_len >= g_ret_chunk_min && dim % 32 == 0 && dim <= 256;
 }
 
-// Floats of scratch that mynah_retention_scan wants for a step of `rows` rows (0: it walks token by token).
-MYNAH_API long long mynah_retention_scratch_floats(int rows, int H, int dim, int max_q_len) {
-    return retention_chunked(dim, max_q_len) ? (long long)rows * H * (dim <= 128 ? 64 : 32) : 0;
+// Floats of scratch that mynah_retention_scan wants for a step of `rows` rows (0: it walks token by token), and its launches.
+MYNAH_API long long mynah_retention_scratch_floats(int rows, int B, int H, int dim, int vd, int max_q_len, int* launches) {
+    if (!retention_chunked(dim, max_q_len) || rows <= 0) {
+        *launches = 1;
+        return 0;
+    }
+    const RetPlan plan(rows, B, H, dim, vd);
+    *launches = 3 * ceil_div(plan.total, plan.n_pass);
+    return plan.floats(H, dim);
 }
-
 
 // qk: rows that hold every head's q from column q_off and every head's k from column k_off; qn, kn: fp32 [T][H*dim].
 MYNAH_API int mynah_retention_prep(const void* qk, int ld, int q_off, int k_off, int dtype, float* qn, float* kn,
@@ -475,6 +625,20 @@ MYNAH_API int mynah_retention_prep(const void* qk, int ld, int q_off, int k_off,
     MYNAH_REQUIRE(T > 0 && H > 0 && dim > 0, "retention_prep: bad sizes");
     MYNAH_REQUIRE(rot % 2 == 0 && rot <= dim, "retention_prep: %d rotated dims do not fit a head of %d", rot, dim);
     const RetPrepArgs a{H, dim, ld, q_off, k_off, cos_t ? rot : 0, interleaved, n_pos, k_scale};
+    const int size = dtype == MYNAH_BF16 ? 2 : 4;
+    const bool vec = dim % 8 == 0 && a.rot % (interleaved ? 8 : 16) == 0 && (ld * size) % 16 == 0 && (q_off * size) % 16 == 0
+                     && (k_off * size) % 16 == 0 && (((uintptr_t)qk | (uintptr_t)qn | (uintptr_t)kn) & 15) == 0;
+    if (vec && (dtype == MYNAH_F32 || dtype == MYNAH_BF16)) {
+        const int y = T < 32768 ? T : 32768;
+        const dim3 grid(ceil_div(H * dim / 4, 128), y, ceil_div(T, y));
+        if (dtype == MYNAH_F32)
+            mynah_launch(retention_prep_vec_kernel<float>, grid, dim3(128), 0, stream, (const float*)qk, qn, kn, cos_t, sin_t, tok_seq,
+                         tok_pos, a, T, status);
+        else
+            mynah_launch(retention_prep_vec_kernel<bf16>, grid, dim3(128), 0, stream, (const bf16*)qk, qn, kn, cos_t, sin_t, tok_seq,
+                         tok_pos, a, T, status);
+        return mynah_check_launch("retention_prep");
+    }
     if (dtype == MYNAH_F32)
         mynah_launch(retention_prep_kernel<float>, dim3(T), dim3(128), 0, stream, (const float*)qk, qn, kn, cos_t, sin_t,
                      tok_seq, tok_pos, a, status);
@@ -499,12 +663,13 @@ MYNAH_API int mynah_retention_scan(const float* qn, const float* kn, const void*
     MYNAH_REQUIRE(H <= 65535 && B <= 65535, "retention_scan: too many heads or sequences for one launch");
     MYNAH_REQUIRE(v_dtype == MYNAH_F32 || v_dtype == MYNAH_BF16, "retention_scan: unsupported dtype %d", v_dtype);
     if (retention_chunked(dim, max_q_len) && scratch != nullptr && (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)scratch) & 15) == 0) {
-        const RetChunkArgs ca{H, dim, vd, n_slots, ldv, v_off, rows, B};
-        if (v_dtype == MYNAH_F32)
-            return dim <= 128 ? launch_chunked<float, 64>(qn, kn, v, decay, scratch, state, o, cu_q, slots, ca, stream)
-                              : launch_chunked<float, 32>(qn, kn, v, decay, scratch, state, o, cu_q, slots, ca, stream);
-        return dim <= 128 ? launch_chunked<bf16, 64>(qn, kn, v, decay, scratch, state, o, cu_q, slots, ca, stream)
-                          : launch_chunked<bf16, 32>(qn, kn, v, decay, scratch, state, o, cu_q, slots, ca, stream);
+        const RetPlan plan(rows, B, H, dim, vd);
+        const RetChunkArgs ca{H, dim, vd, n_slots, ldv, v_off, B, plan.cols, 0};
+        MYNAH_REQUIRE(plan.cols / plan.JT <= 65535, "retention_scan: too many columns for one launch");
+#define RET_CHUNKED(T, C, JT) launch_chunked<T, C, JT>(qn, kn, v, decay, scratch, state, o, cu_q, slots, ca, plan, stream)
+        if (v_dtype == MYNAH_F32) return plan.C == 32 ? RET_CHUNKED(float, 32, 64) : plan.JT == 64 ? RET_CHUNKED(float, 64, 64) : RET_CHUNKED(float, 64, 128);
+        return plan.C == 32 ? RET_CHUNKED(bf16, 32, 64) : plan.JT == 64 ? RET_CHUNKED(bf16, 64, 64) : RET_CHUNKED(bf16, 64, 128);
+#undef RET_CHUNKED
     }
     int L = 1;
     while (L * RET_RMAX < dim) L <<= 1;

@@ -203,7 +203,7 @@ def load() -> ctypes.CDLL:
         getattr(lib, name).restype = c_int
         getattr(lib, name).argtypes = [c_int]
     lib.mynah_retention_scratch_floats.restype = c_longlong
-    lib.mynah_retention_scratch_floats.argtypes = [c_int, c_int, c_int, c_int]
+    lib.mynah_retention_scratch_floats.argtypes = [c_int] * 6 + [P]
     lib.mynah_gated_memory_scratch_floats.restype = c_longlong
     lib.mynah_gated_memory_scratch_floats.argtypes = [c_int] * 9
     lib.mynah_moe_grouped_rows.restype = c_int

@@ -195,6 +195,39 @@ def test_retention_prep_and_scan(H, dim, vd, rot):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,dim,vd,lengths", [(2, 128, 128, [64, 65, 1, 63, 300]), (2, 128, 130, [129]), (3, 32, 66, [200, 17]),
+                                              (64, 256, 256, [700, 31, 33, 200]), (16, 128, 128, [40, 2500, 16, 3000, 1000]),
+                                              (1, 224, 65, [90])])
+def test_retention_chunks_match_the_token_by_token_kernel(dtype, H, dim, vd, lengths):
+    """Edges of chunks and of column tiles, several sequences, steps whose chunks' states take several passes; a non-zero state,
+    a sequence without a slot (left alone) and padding rows. Both sides sum in fp32 in another order: sums of up to dim + 64
+    products, whose roundings grow like the root of their number, times 2^-24, with a factor of ten to spare."""
+    from mynah_slm_b200.ops import kernels
+    g = torch.Generator(device=DEV).manual_seed(dim + vd)
+    T = sum(lengths) + 3
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)                    # noqa: E731
+    qn, kn, v = rand(T, H * dim), rand(T, H * dim) * dim ** -0.5, rand(T, H * vd).to(dtype)
+    decay = torch.linspace(0.9, 1.0, H, device=DEV) if H > 1 else torch.full((1,), 0.97, device=DEV)
+    slots = [3 + i for i in range(len(lengths))]
+    if len(lengths) > 2:
+        slots[1] = -1
+    state0 = rand(len(lengths) + 5, H, dim, vd)
+    ctx = ctx_for(lengths, slots, pad_rows=3)
+    outs = []
+    for chunk_min in (1, 0):
+        before = kernels.retention_chunk_min(chunk_min)
+        try:
+            st = state0.clone()
+            o = kernels.retention_scan(qn, kn, v, 0, decay, st, ctx, H, dim, vd)
+            at = np.cumsum([0] + lengths)
+            outs.append((torch.cat([o[at[i]:at[i + 1]] for i in range(len(lengths)) if slots[i] >= 0]), st))
+        finally:
+            kernels.retention_chunk_min(before)
+    for a, b in zip(*outs):
+        assert float((a - b).double().norm() / b.double().norm()) < 10 * (dim + 64) ** 0.5 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,D,F,E,top", [(150, 48, 56, 9, 2), (5, 40, 12, 1, 1), (3, 64, 20, 7, 7), (400, 96, 200, 70, 4),
                                         (700, 128, 320, 5, 2)])
 def test_table_routed_experts(dtype, T, D, F, E, top):
