@@ -117,43 +117,52 @@ attn_decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
         for (int j = 0; j < 8; j++) st.acc[i][j] = 0.f;
     }
 
-    const int pt_lo = pt.indptr[b], pt_cnt = pt.indptr[b + 1] - pt_lo, pt_base = pt.base[b];
+    // All keys of a split lie in one page. A warp's keys come a batch at a time, the loads of a batch all in flight before the first
+    // of them is used: with one key after the other a page was sixteen round trips to memory (2 rows behind 160 positions, 16
+    // heads of 128 in fp32: 11.7 -> 8.8 us).
+    constexpr int AHEAD = GT <= 2 ? 4 : GT <= 4 ? 2 : 1;
+    const int pt_lo = pt.indptr[b], pt_cnt = pt.indptr[b + 1] - pt_lo, lp = key_begin / PAGE_TOKENS - pt.base[b];
+    int page = (lp >= 0 && lp < pt_cnt) ? pt.ids[pt_lo + lp] : -1;
+    if (page >= pt.n_pages) page = -1;
     bool bad_page = false;
-    for (int base = key_begin + warp * kpw; base < key_end; base += WARPS * kpw) {
-        const int key = base + slot;
-        const bool valid = key < key_end && (key >= lo || key < first_end);
-        float kf[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, vf[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        bool have = false;
-        if (valid) {
-            const int lp = key / PAGE_TOKENS - pt_base;
-            int page = (lp >= 0 && lp < pt_cnt) ? pt.ids[pt_lo + lp] : -1;
-            if (page >= pt.n_pages) page = -1;
-            if (page < 0) {
-                bad_page = true;
-            } else {
-                const size_t tok = ((size_t)page * a.KV + g) * PAGE_TOKENS + key % PAGE_TOKENS;
-                if (lane_on) load8(k_cache + tok * HD + u * 8, kf);
-                const size_t vtok = ((size_t)page * KVV + gv) * PAGE_TOKENS + key % PAGE_TOKENS;
-                if (lane_on_v) load8(v_cache + vtok * VD + u * 8, vf);
+    const T* k_page = k_cache + ((size_t)max(page, 0) * a.KV + g) * PAGE_TOKENS * HD + u * 8;
+    const T* v_page = v_cache + ((size_t)max(page, 0) * KVV + gv) * PAGE_TOKENS * VD + u * 8;
+    for (int base0 = key_begin + warp * kpw; base0 < key_end; base0 += AHEAD * WARPS * kpw) {
+        float kf[AHEAD][8], vf[AHEAD][8];
+        bool have[AHEAD];
+#pragma unroll
+        for (int w = 0; w < AHEAD; w++) {
+            const int key = base0 + w * WARPS * kpw + slot;
+            const bool valid = key < key_end && (key >= lo || key < first_end);
+            have[w] = valid && page >= 0;
+            bad_page = bad_page || (valid && page < 0);
+#pragma unroll
+            for (int j = 0; j < 8; j++) kf[w][j] = vf[w][j] = 0.f;
+            if (have[w]) {
+                if (lane_on) load8(k_page + (size_t)(key % PAGE_TOKENS) * HD, kf[w]);
+                if (lane_on_v) load8(v_page + (size_t)(key % PAGE_TOKENS) * VD, vf[w]);
             }
-            have = page >= 0;
         }
 #pragma unroll
-        for (int i = 0; i < GT; i++) {
-            float d = 0.f;
+        for (int w = 0; w < AHEAD; w++) {
+            if (base0 + w * WARPS * kpw >= key_end) break;           // uniform over the warp
 #pragma unroll
-            for (int j = 0; j < 8; j++) d = fmaf(qv[i][j], kf[j], d);
-            for (int o = lpk >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
-            if (have) {
-                float sc = d * a.scale;
-                if (a.softcap > 0.f) sc = a.softcap * tanhf(sc / a.softcap);
-                const float m_new = fmaxf(st.m[i], sc);
-                const float alpha = expf(st.m[i] - m_new);
-                const float p = expf(sc - m_new);
-                st.l[i] = st.l[i] * alpha + p;
-                st.m[i] = m_new;
+            for (int i = 0; i < GT; i++) {
+                float d = 0.f;
 #pragma unroll
-                for (int j = 0; j < 8; j++) st.acc[i][j] = fmaf(p, vf[j], st.acc[i][j] * alpha);
+                for (int j = 0; j < 8; j++) d = fmaf(qv[i][j], kf[w][j], d);
+                for (int o = lpk >> 1; o > 0; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
+                if (have[w]) {
+                    float sc = d * a.scale;
+                    if (a.softcap > 0.f) sc = a.softcap * tanhf(sc / a.softcap);
+                    const float m_new = fmaxf(st.m[i], sc);
+                    const float alpha = expf(st.m[i] - m_new);
+                    const float p = expf(sc - m_new);
+                    st.l[i] = st.l[i] * alpha + p;
+                    st.m[i] = m_new;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) st.acc[i][j] = fmaf(p, vf[w][j], st.acc[i][j] * alpha);
+                }
             }
         }
     }
