@@ -22,6 +22,13 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int N>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
+// A 16-byte read of shared memory that stays where it is written: ahead of the multiply-adds it is to hide behind.
+__device__ __forceinline__ float4 read16(uint32_t at) {
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    return v;
+}
+
 // ---- rows that are not 16-byte aligned, or no multiple of four long: scalar loads, any size
 
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;   // 256 threads, 4x4 outputs each
@@ -75,20 +82,21 @@ gemm_f32_kernel(const float* __restrict__ A, const float* __restrict__ W, float*
     }
 }
 
-// ---- many rows: tiles of BM x BN outputs, a thread TM x TN of them, slabs of 32 k brought by 16-byte asynchronous
-// copies into three stages. Both operands stay as they lie in memory ([row][k], rows padded to 36 words, so that eight
-// rows' 16-byte reads meet no bank twice); a thread reads four k of its TM + TN rows at a time and walks them in order.
-// Bound by the FFMA pipes where the tiles fill the SMs. A prompt of 161 rows through the 0.6B shape (products of 1,024 to
-// 6,144 outputs): 163 us a product with the scalar kernel above for every size, 70 us with these.
+// ---- many rows: tiles of BM x BN outputs, a thread TM x TN of them, slabs of 32 or 64 k brought by 16-byte asynchronous
+// copies into three stages. Both operands stay as they lie in memory ([row][k], rows padded by 4 words, so that eight
+// rows' 16-byte reads meet no bank twice); a thread reads four k of its TM + TN rows at a time, a step ahead of their use, and
+// walks them in order. Bound by the reads of shared memory (four cycles of an SM for a warp's 16-byte read of sixteen rows, two for
+// two) and by how few warps a product of few rows makes. us for 161 rows, 4,096 x 1,024 / 1,024 x 2,048 / 6,144 x 1,024 /
+// 1,024 x 3,072 outputs x k: 73 / 64 / 74 / 90 with reads where they are used -> 55 / 46 / 72 / 66.
 
 constexpr int GRID_ROWS = 65535;                                     // tiles of rows that a launch's grid can name
-constexpr int SLAB = 32, PITCH = SLAB + 4, TILE_STAGES = 3;
+constexpr int TILE_STAGES = 3;
 
-template <int BM, int BN, int TM, int TN>
+template <int BM, int BN, int TM, int TN, int SLAB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN))
 gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                      int M, int N, int K, int lda, int ldw, int ldc) {
-    constexpr int TX = BN / TN, THREADS = TX * (BM / TM), CHUNKS = (BM + BN) * (SLAB / 4);
+    constexpr int PITCH = SLAB + 4, TX = BN / TN, THREADS = TX * (BM / TM), CHUNKS = (BM + BN) * (SLAB / 4);
     static_assert(CHUNKS % THREADS == 0, "whole rounds of copies");
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, tx = tid % TX, ty = tid / TX;
@@ -120,31 +128,37 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         copy_wait<TILE_STAGES - 2>();
         __syncthreads();                                             // slab s is there; slab s - 1 has been read by all
         fetch(s + TILE_STAGES - 1);
-        const float* as = smem + (size_t)(s % TILE_STAGES) * ((BM + BN) * PITCH);
-        const float* ws = as + BM * PITCH;
-#pragma unroll 2
+        // four k of the thread's rows a step; the next step's are on their way while these are multiplied
+        const uint32_t a_at = base + (uint32_t)((s % TILE_STAGES) * ((BM + BN) * PITCH) + ty * PITCH) * 4;
+        const uint32_t w_at = base + (uint32_t)((s % TILE_STAGES) * ((BM + BN) * PITCH) + (BM + tx) * PITCH) * 4;
+        struct Piece { float4 a[TM], w[TN]; } piece[2];
+        auto load = [&](Piece& p, int k) {
+#pragma unroll
+            for (int j = 0; j < TN; j++) p.w[j] = read16(w_at + (j * TX * PITCH + k) * 4);
+#pragma unroll
+            for (int i = 0; i < TM; i++) p.a[i] = read16(a_at + (i * (BM / TM) * PITCH + k) * 4);
+        };
+        load(piece[0], 0);
+#pragma unroll
         for (int k = 0; k < SLAB; k += 4) {
-            float4 a[TM], w[TN];
-#pragma unroll
-            for (int i = 0; i < TM; i++) a[i] = *reinterpret_cast<const float4*>(as + (ty + i * (BM / TM)) * PITCH + k);
-#pragma unroll
-            for (int j = 0; j < TN; j++) w[j] = *reinterpret_cast<const float4*>(ws + (tx + j * TX) * PITCH + k);
+            if (k + 4 < SLAB) load(piece[(k / 4 + 1) & 1], k + 4);
+            const Piece& p = piece[(k / 4) & 1];
 #pragma unroll
             for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].x, w[j].x, acc[i][j]);
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(p.a[i].x, p.w[j].x, acc[i][j]);
 #pragma unroll
             for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].y, w[j].y, acc[i][j]);
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(p.a[i].y, p.w[j].y, acc[i][j]);
 #pragma unroll
             for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].z, w[j].z, acc[i][j]);
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(p.a[i].z, p.w[j].z, acc[i][j]);
 #pragma unroll
             for (int i = 0; i < TM; i++)
 #pragma unroll
-                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i].w, w[j].w, acc[i][j]);
+                for (int j = 0; j < TN; j++) acc[i][j] = fmaf(p.a[i].w, p.w[j].w, acc[i][j]);
         }
     }
 #pragma unroll
@@ -159,10 +173,10 @@ gemm_f32_tile_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     }
 }
 
-template <int BM, int BN, int TM, int TN>
+template <int BM, int BN, int TM, int TN, int SLAB>
 int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-    auto kern = gemm_f32_tile_kernel<BM, BN, TM, TN>;
-    constexpr int smem = TILE_STAGES * (BM + BN) * PITCH * 4;
+    auto kern = gemm_f32_tile_kernel<BM, BN, TM, TN, SLAB>;
+    constexpr int smem = TILE_STAGES * (BM + BN) * (SLAB + 4) * 4;
     if (smem > 48 * 1024) {
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return mynah_fail("gemm_f32: %s", cudaGetErrorString(e));
@@ -177,12 +191,13 @@ int launch_tile(const float* A, const float* W, float* C, int M, int N, int K, i
 // multiplies. The weights' first slabs are asked for before the kernel in front has ended. Two rows of the 0.6B shape:
 // 13 to 17 us a product of a layer and 107 us for the head (622 MB, 5.8 TB/s); with the scalar kernel 163 us a product.
 
-constexpr int ROW_SLAB = 128, ROW_PITCH = ROW_SLAB + 4, ROW_THREADS = 128, ROW_MAX_M = 16;
+constexpr int ROW_THREADS = 128, ROW_MAX_M = 16;
 
-template <int BN, int MR, int STAGES>
+template <int BN, int MR, int STAGES, int ROW_SLAB>
 __global__ void __launch_bounds__(ROW_THREADS)
 gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, float* __restrict__ C,
                      int M, int N, int K, int lda, int ldw, int ldc) {
+    constexpr int ROW_PITCH = ROW_SLAB + 4;
     extern __shared__ __align__(16) float smem[];
     const int tid = threadIdx.x, n0 = blockIdx.x * BN;
     const int groups = (M + MR - 1) / MR, rows_a = groups * MR;      // input rows, rounded up; those beyond M are zeros
@@ -216,6 +231,29 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         if (s < slabs) fetch_a(s);
         copy_commit();                                               // (the first group holds all the weights' slabs too)
     }
+    constexpr int AHEAD = MR == 4 ? 8 : 16;
+    struct Piece {
+        float4 w[AHEAD / 4], a[MR][AHEAD / 4];
+        __device__ __forceinline__ void load(uint32_t wp, uint32_t ap, int k) {
+#pragma unroll
+            for (int i = 0; i < AHEAD / 4; i++) {
+                w[i] = read16(wp + (k + 4 * i) * 4);
+#pragma unroll
+                for (int r = 0; r < MR; r++) a[r][i] = read16(ap + (r * ROW_PITCH + k + 4 * i) * 4);
+            }
+        }
+        __device__ __forceinline__ void multiply(float (&acc)[MR]) const {
+#pragma unroll
+            for (int i = 0; i < AHEAD / 4; i++)
+#pragma unroll
+                for (int r = 0; r < MR; r++) {
+                    acc[r] = fmaf(a[r][i].x, w[i].x, acc[r]);
+                    acc[r] = fmaf(a[r][i].y, w[i].y, acc[r]);
+                    acc[r] = fmaf(a[r][i].z, w[i].z, acc[r]);
+                    acc[r] = fmaf(a[r][i].w, w[i].w, acc[r]);
+                }
+        }
+    };
     const int n = tid % BN, mg = tid / BN;
     const bool works = mg < groups;
     float acc[MR] = {};
@@ -230,19 +268,17 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         }
         copy_commit();
         if (works) {
-            const float* w = smem + (size_t)(s % STAGES) * stage_words + n * ROW_PITCH;
-            const float* a = smem + (size_t)(s % STAGES) * stage_words + (BN + mg * MR) * ROW_PITCH;
-#pragma unroll 8
-            for (int k = 0; k < ROW_SLAB; k += 4) {
-                const float4 wv = *reinterpret_cast<const float4*>(w + k);
-#pragma unroll
-                for (int r = 0; r < MR; r++) {
-                    const float4 av = *reinterpret_cast<const float4*>(a + r * ROW_PITCH + k);
-                    acc[r] = fmaf(av.x, wv.x, acc[r]);
-                    acc[r] = fmaf(av.y, wv.y, acc[r]);
-                    acc[r] = fmaf(av.z, wv.z, acc[r]);
-                    acc[r] = fmaf(av.w, wv.w, acc[r]);
-                }
+            const uint32_t w = base + (uint32_t)((s % STAGES) * stage_words + n * ROW_PITCH) * 4;
+            const uint32_t a = base + (uint32_t)((s % STAGES) * stage_words + (BN + mg * MR) * ROW_PITCH) * 4;
+            // the next AHEAD k are on their way from shared memory while these are multiplied
+            Piece p0, p1;
+            p0.load(w, a, 0);
+#pragma unroll 1
+            for (int k = 0; k < ROW_SLAB; k += 2 * AHEAD) {
+                p1.load(w, a, k + AHEAD);
+                p0.multiply(acc);
+                p0.load(w, a, min(k + 2 * AHEAD, ROW_SLAB - AHEAD));
+                p1.multiply(acc);
             }
         }
     }
@@ -253,9 +289,10 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
     }
 }
 
-template <int BN, int MR, int STAGES>
+template <int BN, int MR, int STAGES, int ROW_SLAB>
 int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-    auto kern = gemm_f32_rows_kernel<BN, MR, STAGES>;
+    constexpr int ROW_PITCH = ROW_SLAB + 4;
+    auto kern = gemm_f32_rows_kernel<BN, MR, STAGES, ROW_SLAB>;
     const int smem = STAGES * (BN + ceil_div(M, MR) * MR) * ROW_PITCH * 4;
     constexpr int most = STAGES * (BN + (MR == 4 ? ROW_MAX_M : MR)) * ROW_PITCH * 4;
     if (most > 48 * 1024) {
@@ -266,11 +303,11 @@ int launch_rows(const float* A, const float* W, float* C, int M, int N, int K, i
     return mynah_check_launch("gemm_f32");
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, int SLAB>
 int launch_rows_m(const float* A, const float* W, float* C, int M, int N, int K, int lda, int ldw, int ldc, cudaStream_t stream) {
-    if (M == 1) return launch_rows<BN, 1, STAGES>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    if (M == 2) return launch_rows<BN, 2, STAGES>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    return launch_rows<BN, 4, STAGES>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (M == 1) return launch_rows<BN, 1, STAGES, SLAB>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (M == 2) return launch_rows<BN, 2, STAGES, SLAB>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    return launch_rows<BN, 4, STAGES, SLAB>(A, W, C, M, N, K, lda, ldw, ldc, stream);
 }
 
 }  // namespace
@@ -295,19 +332,19 @@ MYNAH_API int mynah_gemm_f32(const float* A, const float* W, float* C, int M, in
     if (M <= ROW_MAX_M) {
         // enough CTAs that every SM streams (two an SM and more), else as many weight rows a CTA as keep its threads busy
         const int sms = mynah_sm_count();
-        if (N >= 32 * 4 * sms) return launch_rows_m<32, 3>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-        if (N >= 16 * 2 * sms) return launch_rows_m<16, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-        return launch_rows_m<8, 6>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+        if (N >= 32 * 4 * sms) return launch_rows_m<32, 3, 128>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+        if (N >= 16 * 2 * sms) return launch_rows_m<16, 4, 128>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+        // long slabs where a CTA an SM is all there is (half as many barriers; 1,024 outputs, K = 3,072: 1 row 21 -> 17 us, 2 rows 25 -> 20,
+        // 16 rows 36 -> 30); with more CTAs their shared memory would keep some waiting (8 rows of 4,096: 21 -> 25)
+        if (ceil_div(N, 8) <= sms && K >= 512) return launch_rows_m<8, 4, 256>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+        return launch_rows_m<8, 6, 128>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     }
-    // The tile with the least time by this count: waves of tiles over the SMs, a tile's time its outputs over the share
-    // of the FFMA rate that a tile of its size reaches alone on an SM.
+    // Tiles of 32 x 32 with 64 threads unless they leave SMs idle (then twice the threads a tile: 40 rows of 1,024 x 3,072 46 us against
+    // 58) or there are many (tiles of 64 x 64 read half as much from L2 and are as fast: 800 rows of 6,144 x 1,024 260 against 264;
+    // 161 rows of 4,096 x 1,024, fewer than five a SM, 69 against 55).
     const int sms = mynah_sm_count();
-    auto cost = [&](int bm, int bn, double share) {
-        const long long tiles = (long long)ceil_div(M, bm) * ceil_div(N, bn);
-        return (double)ceil_div_ll(tiles, sms) * bm * bn / share;
-    };
-    const double c128 = cost(128, 128, 0.85), c64 = cost(64, 64, 0.60), c32 = cost(32, 32, 0.35);
-    if (c128 <= c64 && c128 <= c32) return launch_tile<128, 128, 8, 8>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    if (c64 <= c32 || ceil_div(M, 32) > GRID_ROWS) return launch_tile<64, 64, 8, 4>(A, W, C, M, N, K, lda, ldw, ldc, stream);
-    return launch_tile<32, 32, 4, 2>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    const long long small = ceil_div_ll(M, 32) * ceil_div_ll(N, 32), large = ceil_div_ll(M, 64) * ceil_div_ll(N, 64);
+    if (large >= 5 * sms || ceil_div(M, 32) > GRID_ROWS) return launch_tile<64, 64, 8, 4, 32>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if (small <= sms) return launch_tile<32, 32, 4, 2, 64>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    return launch_tile<32, 32, 4, 4, 32>(A, W, C, M, N, K, lda, ldw, ldc, stream);
 }
