@@ -172,18 +172,17 @@ __device__ __forceinline__ void load_q_fragments(const PageJob& j, const bf16* _
 // The page's partial result. Where the K and V fragments come from is the caller's business: k_frag(ks, kb) gives
 // the B fragments of this warp's 16 keys for dims [16 ks, 16 ks + 16), v_frag(ks, nt, vb) those of keys
 // [16 ks, 16 ks + 16) for this warp's n-tiles nt and nt + 1; before_k() and before_v() run before the first use of
-// each (waits and barriers, if the fragments still lie in shared memory). The arithmetic, and so every bit of the
-// result, is the same whoever provides them.
-template <int HD, int VD, class SYNC, class KFRAG, class VFRAG, class BEFORE_K, class BEFORE_V>
+// each (waits and barriers, if the fragments still lie in shared memory); after_k() runs when every warp has used its K
+// fragments. put_o(head, dim, two values) and put_ml(head, maximum, sum) take the result. The arithmetic, and so every bit
+// of the result, is the same whoever provides them.
+template <int HD, int VD, class SYNC, class KFRAG, class VFRAG, class BEFORE_K, class AFTER_K, class BEFORE_V, class PUT_O, class PUT_ML>
 __device__ __forceinline__ void compute_page_core(const PageJob& job, const uint32_t (&qa)[HD / 16][4], const TcArgs& a,
-                                                  KFRAG k_frag, VFRAG v_frag, BEFORE_K before_k, BEFORE_V before_v,
-                                                  bf16* p_s, float (*red_m)[MAX_G], float (*red_l)[MAX_G],
-                                                  float* __restrict__ part_o, float* __restrict__ part_ml) {
+                                                  KFRAG k_frag, VFRAG v_frag, BEFORE_K before_k, AFTER_K after_k, BEFORE_V before_v,
+                                                  bf16* p_s, float (*red_m)[MAX_G], float (*red_l)[MAX_G], PUT_O put_o, PUT_ML put_ml) {
     constexpr int KSTEPS = HD / 16, NT = VD / 32;
     const int G = a.H / a.KV;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int k_first = job.k_first, k_last = job.k_last;
-    const size_t row0 = job.row0;
 
     before_k();
 
@@ -220,6 +219,7 @@ __device__ __forceinline__ void compute_page_core(const PageJob& job, const uint
         red_m[warp][hrow + 8] = mx[1];
     }
     SYNC::sync();
+    after_k();
     float m[2], l[2] = {0.f, 0.f};
 #pragma unroll
     for (int j = 0; j < 2; j++) {
@@ -275,21 +275,33 @@ __device__ __forceinline__ void compute_page_core(const PageJob& job, const uint
     for (int j = 0; j < 2; j++) {
         const int h = hrow + 8 * j;
         if (h < G) {
-            float* o = part_o + (row0 + (size_t)h * a.S) * VD;
 #pragma unroll
-            for (int nt = 0; nt < NT; nt++) {
-                const int d = warp * (VD / 4) + nt * 8 + (lane & 3) * 2;
-                *reinterpret_cast<float2*>(o + d) = make_float2(oc[nt][2 * j], oc[nt][2 * j + 1]);
-            }
+            for (int nt = 0; nt < NT; nt++)
+                put_o(h, warp * (VD / 4) + nt * 8 + (lane & 3) * 2, make_float2(oc[nt][2 * j], oc[nt][2 * j + 1]));
         }
     }
     if (tid < G) {
         const float ls = (red_l[0][tid] + red_l[1][tid]) + (red_l[2][tid] + red_l[3][tid]);
         const float mm = fmaxf(fmaxf(red_m[0][tid], red_m[1][tid]), fmaxf(red_m[2][tid], red_m[3][tid]));
-        part_ml[(row0 + (size_t)tid * a.S) * 2] = mm;
-        part_ml[(row0 + (size_t)tid * a.S) * 2 + 1] = ls;
+        put_ml(tid, mm, ls);
     }
 }
+
+// A page's result goes to scratch, for the merge.
+template <int VD>
+struct ToScratch {
+    float* part_o;
+    float* part_ml;
+    size_t row0;
+    int S;
+    __device__ __forceinline__ void o(int h, int d, float2 v) const {
+        *reinterpret_cast<float2*>(part_o + (row0 + (size_t)h * S) * VD + d) = v;
+    }
+    __device__ __forceinline__ void ml(int h, float m, float l) const {
+        part_ml[(row0 + (size_t)h * S) * 2] = m;
+        part_ml[(row0 + (size_t)h * S) * 2 + 1] = l;
+    }
+};
 
 // The fragments of a page's tiles in shared memory, as compute_page_core wants them.
 // K (non-transposed load): matrices 0: keys 0-7 of the warp's 16, dims k0..k0+7; 1: keys 0-7, dims +8; 2: keys 8-15,
@@ -314,13 +326,15 @@ template <int HD, int VD, int PENDING_K, int PENDING_V>
 __device__ __forceinline__ void compute_page(const PageJob& job, const uint32_t (&qa)[HD / 16][4], const TcArgs& a,
                                              uint32_t k_base, uint32_t v_base, bf16* p_s, float (*red_m)[MAX_G], float (*red_l)[MAX_G],
                                              float* __restrict__ part_o, float* __restrict__ part_ml) {
+    const ToScratch<VD> to{part_o, part_ml, job.row0, a.S};
     compute_page_core<HD, VD, SyncCta>(
         job, qa, a,
         [&](int ks, uint32_t (&kb)[4]) { load_k_frag<HD, TileSwz<HD>>(k_base, ks, kb); },
         [&](int ks, int nt, uint32_t (&vb)[4]) { load_v_frag<VD, TileSwz<VD>>(v_base, ks, nt, vb); },
         [&]() { cp_async_wait<PENDING_K>(); __syncthreads(); },       // K has landed (V may still be in flight)
+        []() {},
         [&]() { cp_async_wait<PENDING_V>(); __syncthreads(); },       // V has landed
-        p_s, red_m, red_l, part_o, part_ml);
+        p_s, red_m, red_l, [&](int h, int d, float2 v) { to.o(h, d, v); }, [&](int h, float m, float l) { to.ml(h, m, l); });
 }
 
 // One CTA a page; six CTAs an SM cover one another's waits. (Persistent CTAs that prefetch their next page were
@@ -501,6 +515,69 @@ struct FusedArgs {
     float scale, qk_eps;
 };
 
+// The group's query heads and the new key and value of a (sequence, kv head), prepared by a CTA of WARPS warps. Heads lie
+// side by side in a warp (head_prep.cuh), as in the rope/store pass, whose bits these are.
+constexpr int QPAD = 8;                               // padding of a query row in shared memory: no bank conflicts on its loads
+template <int HD>
+struct HeadPrep {
+    static constexpr int LPH = HeadLanes<HD>::LPH, HPW = HeadLanes<HD>::HPW, QLD = HD + QPAD;
+    bool rotate, has_gain;
+    float eps, rc[8], rs[8], qgv[8], kgv[8];
+    __device__ __forceinline__ void load(const float* __restrict__ cos_t, const float* __restrict__ sin_t, int pos, VecRef q_gain, VecRef k_gain, float qk_eps) {
+        const int lane = threadIdx.x & 31, li = lane % LPH;
+        rotate = cos_t != nullptr;
+        has_gain = q_gain.p != nullptr;
+        eps = qk_eps;
+        if (rotate) load_rotation<HD>(cos_t, sin_t, pos, lane, rc, rs);
+        if (has_gain) {
+            load_gain8(q_gain, li * 8, qgv);
+            load_gain8(k_gain, li * 8, kgv);
+        }
+    }
+    // norm and rotation of the group's G queries, to shared memory as bf16; rows beyond G are zero
+    __device__ __forceinline__ void queries(const bf16* __restrict__ q, int G, bf16* q_s) const {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPH, li = lane % LPH;
+        for (int hbase = warp * HPW; hbase < MAX_G; hbase += WARPS * HPW) {      // uniform over the warp
+            const int h = hbase + sub;
+            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (h < G) load8<bf16>(q + (size_t)h * HD + li * 8, v);
+            head_norm_rotate<HD>(v, has_gain, qgv, eps, rotate, rc, rs, lane);
+            if (h >= G) {
+#pragma unroll
+                for (int j = 0; j < 8; j++) v[j] = 0.f;
+            }
+            if (h < MAX_G) store8<bf16>(q_s + h * QLD + li * 8, v);
+        }
+    }
+    // the new position's key (norm, rotation) and value, 16 bytes a lane, by a whole warp: true for the lanes that hold them
+    __device__ __forceinline__ bool new_row(const bf16* __restrict__ k, const bf16* __restrict__ v, uint4& ko, uint4& vo) const {
+        const int lane = threadIdx.x & 31, sub = lane / LPH, li = lane % LPH;
+        float kv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (sub == 0) load8<bf16>(k + li * 8, kv);
+        head_norm_rotate<HD>(kv, has_gain, kgv, eps, rotate, rc, rs, lane);      // the whole warp; one lane group holds the head
+        if (sub != 0) return false;
+        vo = *reinterpret_cast<const uint4*>(v + li * 8);
+        __nv_bfloat162* kh = reinterpret_cast<__nv_bfloat162*>(&ko);
+#pragma unroll
+        for (int j = 0; j < 4; j++) kh[j] = __floats2bfloat162_rn(kv[2 * j], kv[2 * j + 1]);
+        return true;
+    }
+};
+
+template <int HD>
+__device__ __forceinline__ void query_fragments(const bf16* q_s, uint32_t (&qa)[HD / 16][4]) {
+    constexpr int QLD = HD + QPAD;
+    const int lane = threadIdx.x & 31, r0 = lane >> 2, c0 = (lane & 3) * 2;
+#pragma unroll
+    for (int ks = 0; ks < HD / 16; ks++) {
+        const int col = ks * 16 + c0;
+        qa[ks][0] = *reinterpret_cast<const uint32_t*>(q_s + r0 * QLD + col);
+        qa[ks][1] = *reinterpret_cast<const uint32_t*>(q_s + (r0 + 8) * QLD + col);
+        qa[ks][2] = *reinterpret_cast<const uint32_t*>(q_s + r0 * QLD + col + 8);
+        qa[ks][3] = *reinterpret_cast<const uint32_t*>(q_s + (r0 + 8) * QLD + col + 8);
+    }
+}
+
 template <int HD, bool MERGE>
 __global__ void __launch_bounds__(WARPS * 32)
 attn_decode_fused_kernel(const bf16* __restrict__ qkv, VecRef q_gain, VecRef k_gain,
@@ -509,8 +586,7 @@ attn_decode_fused_kernel(const bf16* __restrict__ qkv, VecRef q_gain, VecRef k_g
                          bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, FusedArgs a,
                          float* __restrict__ part_o, float* __restrict__ part_ml, unsigned* __restrict__ counters,
                          bf16* __restrict__ out, int* __restrict__ status) {
-    constexpr int CH = HD / 8, KSTEPS = HD / 16;
-    constexpr int QLD = HD + 8;                       // padded row of the query tile: no bank conflicts on its loads
+    constexpr int CH = HD / 8, KSTEPS = HD / 16, QLD = HD + QPAD;
     __shared__ __align__(128) unsigned char k_s[KEYS * HD * 2];     // reused by the merge for the pages' weights
     __shared__ __align__(128) unsigned char v_s[KEYS * HD * 2];     // reused by the merge for its series
     __shared__ __align__(16) bf16 q_s[MAX_G * QLD];   // the queries; once they are in registers, the probabilities
@@ -570,61 +646,26 @@ attn_decode_fused_kernel(const bf16* __restrict__ qkv, VecRef q_gain, VecRef k_g
         }
         cp_async_commit();
 
-        // ---- the group's queries: norm, rotation, to shared memory as bf16; rows beyond G are zero.
-        // Heads lie side by side in a warp (head_prep.cuh), as in the rope/store pass, whose bits these are.
-        constexpr int LPH = HeadLanes<HD>::LPH, HPW = HeadLanes<HD>::HPW;
-        const int sub = lane / LPH, li = lane % LPH;
-        const bool rotate = cos_t != nullptr, has_gain = q_gain.p != nullptr;
-        float rc[8], rs[8], qgv[8], kgv[8];
-        if (rotate) load_rotation<HD>(cos_t, sin_t, pos, lane, rc, rs);
-        if (has_gain) {
-            load_gain8(q_gain, li * 8, qgv);
-            load_gain8(k_gain, li * 8, kgv);
-        }
+        HeadPrep<HD> prep;
+        prep.load(cos_t, sin_t, pos, q_gain, k_gain, a.qk_eps);
         const bf16* qrow = qkv + (size_t)b * a.ldq;
-        for (int hbase = warp * HPW; hbase < MAX_G; hbase += WARPS * HPW) {      // uniform over the warp
-            const int h = hbase + sub;
-            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (h < G) load8<bf16>(qrow + (size_t)(g * G + h) * HD + li * 8, v);
-            head_norm_rotate<HD>(v, has_gain, qgv, a.qk_eps, rotate, rc, rs, lane);
-            if (h >= G) {
-#pragma unroll
-                for (int j = 0; j < 8; j++) v[j] = 0.f;
-            }
-            if (h < MAX_G) store8<bf16>(q_s + h * QLD + li * 8, v);
-        }
+        prep.queries(qrow + (size_t)(g * G) * HD, G, q_s);
         // ---- the new position's k and v, by the CTA that has its page: to the cache and into the tiles
         if (r_new >= 0 && warp == WARPS - 1) {
-            float kv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (sub == 0) load8<bf16>(qrow + (size_t)(a.H + g) * HD + li * 8, kv);
-            head_norm_rotate<HD>(kv, has_gain, kgv, a.qk_eps, rotate, rc, rs, lane);    // the whole warp; one lane group holds the head
-            if (sub == 0) {
-                const uint4 vraw = *reinterpret_cast<const uint4*>(qrow + (size_t)(a.H + a.KV + g) * HD + li * 8);
-                uint4 ko;
-                __nv_bfloat162* kh = reinterpret_cast<__nv_bfloat162*>(&ko);
-#pragma unroll
-                for (int j = 0; j < 4; j++) kh[j] = __floats2bfloat162_rn(kv[2 * j], kv[2 * j + 1]);
+            uint4 ko, vo;
+            if (prep.new_row(qrow + (size_t)(a.H + g) * HD, qrow + (size_t)(a.H + a.KV + g) * HD, ko, vo)) {
+                const int li = lane;
                 *reinterpret_cast<uint4*>(k_cache + tile + (size_t)r_new * HD + li * 8) = ko;
-                *reinterpret_cast<uint4*>(v_cache + tile + (size_t)r_new * HD + li * 8) = vraw;
+                *reinterpret_cast<uint4*>(v_cache + tile + (size_t)r_new * HD + li * 8) = vo;
                 *reinterpret_cast<uint4*>(k_s + swz<CH>(r_new, li)) = ko;       // a lane's eight elements are one 16-byte chunk
-                *reinterpret_cast<uint4*>(v_s + swz<CH>(r_new, li)) = vraw;
+                *reinterpret_cast<uint4*>(v_s + swz<CH>(r_new, li)) = vo;
             }
         }
         cp_async_wait<1>();                           // K has landed (V may still be in flight)
         __syncthreads();
 
         uint32_t qa[KSTEPS][4];
-        {
-            const int r0 = lane >> 2, c0 = (lane & 3) * 2;
-#pragma unroll
-            for (int ks = 0; ks < KSTEPS; ks++) {
-                const int col = ks * 16 + c0;
-                qa[ks][0] = *reinterpret_cast<const uint32_t*>(q_s + r0 * QLD + col);
-                qa[ks][1] = *reinterpret_cast<const uint32_t*>(q_s + (r0 + 8) * QLD + col);
-                qa[ks][2] = *reinterpret_cast<const uint32_t*>(q_s + r0 * QLD + col + 8);
-                qa[ks][3] = *reinterpret_cast<const uint32_t*>(q_s + (r0 + 8) * QLD + col + 8);
-            }
-        }
+        query_fragments<HD>(q_s, qa);
         // the page's partial result: the same code as the pages' kernel (the probabilities go where the queries were)
         PageJob job;
         job.s = s; job.g = g; job.b = b; job.page = page;
@@ -646,6 +687,172 @@ attn_decode_fused_kernel(const bf16* __restrict__ qkv, VecRef q_gain, VecRef k_g
     if (!last_flag) return;
     merge_pages<HD>(part_o, part_ml, out + (size_t)b * a.ldo + (size_t)g * G * HD, ((size_t)b * a.H + (size_t)g * G) * a.S,
                     G, a.S, n_vis, reinterpret_cast<float*>(k_s), reinterpret_cast<float*>(v_s), red_m[0]);
+}
+
+
+// The same for steps of many short sequences: one CTA a (sequence, kv head) prepares the heads, writes the new key and value,
+// walks the sequence's few pages and merges them, so nothing passes through scratch memory and one launch does what three
+// did. A page's K is fetched into its place while the page before is weighted, its V behind that; five CTAs an SM
+// cover one another's waits. A page's partial result waits in shared memory, in the words of the thread that wrote it. The
+// arithmetic is that of the pages' kernel and of merge_pages for at most as many pages as that has series (SHORT_PAGES), so a
+// sequence has the same bits by either route. Measured (16 heads of 128 on 8, 64 rows behind 32 to 128 positions, us a layer):
+// three launches of 3.3 + 9.7 + 3.5 -> 13.8, what is left being one chain of loads, products and barriers after another.
+constexpr int SHORT_PAGES = 4;
+
+template <int HD>
+__global__ void __launch_bounds__(WARPS * 32, 5)
+attn_decode_short_kernel(const bf16* __restrict__ qkv, VecRef q_gain, VecRef k_gain,
+                         const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                         const int* __restrict__ tok_pos, const int* __restrict__ kv_len, PageTable pt,
+                         bf16* __restrict__ k_cache, bf16* __restrict__ v_cache, FusedArgs a,
+                         bf16* __restrict__ out, int* __restrict__ status) {
+    constexpr int CH = HD / 8, QLD = HD + QPAD;
+    __shared__ __align__(128) unsigned char k_s[KEYS * HD * 2];
+    __shared__ __align__(128) unsigned char v_s[KEYS * HD * 2];
+    __shared__ __align__(16) bf16 q_s[MAX_G * QLD];   // the queries; once they are in registers, the probabilities
+    __shared__ float red_m[WARPS][MAX_G], red_l[WARPS][MAX_G];
+    __shared__ float2 ml_s[SHORT_PAGES][MAX_G];
+    __shared__ float w_s[SHORT_PAGES][MAX_G], inv_s[MAX_G];
+    __shared__ int page_s[SHORT_PAGES];
+    extern __shared__ __align__(16) float o_s[];      // [pages][G][HD]
+    static_assert(MAX_G * QLD >= MAX_G * KEYS, "the probabilities must fit where the queries were");
+
+    const int g = blockIdx.x, b = blockIdx.y;
+    const int G = a.H / a.KV;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    griddep_launch();
+    griddep_wait();
+    const int hi = kv_len[b];
+    const int lo = first_visible(hi, a.window);
+    const int pos = hi > 0 ? tok_pos[b] : 0;
+    int pg0 = 0, n_vis = 0;
+    if (hi > 0) {
+        pg0 = lo / PAGE_TOKENS;
+        const int pg1 = (hi - 1) / PAGE_TOKENS + 1;
+        n_vis = min(pg1 - pg0, a.S);
+        if (pg1 - pg0 > a.S && tid == 0) atomicOr(status, MYNAH_ST_SPLIT_RANGE);
+        if (cos_t != nullptr && (pos < 0 || pos >= a.n_pos)) {
+            if (tid == 0) atomicOr(status, MYNAH_ST_POS_RANGE);
+            n_vis = 0;
+        }
+    }
+    if (tid < n_vis) {
+        const int page = page_of(pt, b, (pg0 + tid) * PAGE_TOKENS);
+        if (page < 0) atomicOr(status, MYNAH_ST_PAGE_RANGE);
+        page_s[tid] = page;
+    }
+    for (int i = tid; i < SHORT_PAGES * MAX_G; i += WARPS * 32) ml_s[i / MAX_G][i % MAX_G] = make_float2(-INFINITY, 0.f);
+    __syncthreads();
+
+    const uint32_t k_base = smem_u32(k_s), v_base = smem_u32(v_s);
+    HeadPrep<HD> prep;
+    uint4 ko, vo;                                     // the new row, in the lanes of the last warp that hold it
+    bool holds = false;
+    auto new_at = [&](int p) {                        // the new position's row of page p, or -1
+        const int mp = pg0 + p;
+        return a.write_kv && pos >= mp * PAGE_TOKENS && pos < (mp + 1) * PAGE_TOKENS ? pos % PAGE_TOKENS : -1;
+    };
+    auto first_row = [&](int p) { return max(lo, (pg0 + p) * PAGE_TOKENS) % PAGE_TOKENS; };
+    auto last_row = [&](int p) { return (min(hi, (pg0 + p + 1) * PAGE_TOKENS) - 1) % PAGE_TOKENS; };
+    // one tile of page p, as a copy group of its own (empty where there is no page); the new row comes from registers
+    auto fetch = [&](int p, const bf16* cache, uint32_t base) {
+        if (p < n_vis && page_s[p] >= 0) {
+            const bf16* src = cache + ((size_t)page_s[p] * a.KV + g) * PAGE_TOKENS * HD;
+            const int r_new = new_at(p), k_first = first_row(p), k_last = last_row(p);
+            for (int i = tid; i < KEYS * CH; i += WARPS * 32) {
+                const int r = i / CH, c = i % CH;
+                if (r != r_new) cp_async_16(base + swz<CH>(r, c), src + (size_t)r * HD + c * 8, r >= k_first && r <= k_last);
+            }
+        }
+        cp_async_commit();
+    };
+    auto place = [&](int p, unsigned char* tile, const uint4& row) {
+        if (holds && p < n_vis && page_s[p] >= 0 && new_at(p) >= 0) *reinterpret_cast<uint4*>(tile + swz<CH>(new_at(p), lane)) = row;
+    };
+    fetch(0, k_cache, k_base);
+    fetch(0, v_cache, v_base);
+    uint32_t qa[HD / 16][4];
+    if (n_vis > 0) {
+        prep.load(cos_t, sin_t, pos, q_gain, k_gain, a.qk_eps);
+        const bf16* qrow = qkv + (size_t)b * a.ldq;
+        prep.queries(qrow + (size_t)(g * G) * HD, G, q_s);
+        if (a.write_kv && warp == WARPS - 1) {
+            holds = prep.new_row(qrow + (size_t)(a.H + g) * HD, qrow + (size_t)(a.H + a.KV + g) * HD, ko, vo);
+            const int p = pos / PAGE_TOKENS - pg0;
+            if (holds && p >= 0 && p < n_vis && page_s[p] >= 0) {
+                const size_t at = (((size_t)page_s[p] * a.KV + g) * PAGE_TOKENS + pos % PAGE_TOKENS) * HD + lane * 8;
+                *reinterpret_cast<uint4*>(k_cache + at) = ko;
+                *reinterpret_cast<uint4*>(v_cache + at) = vo;
+            }
+        }
+        place(0, k_s, ko);
+        place(0, v_s, vo);
+        __syncthreads();
+        query_fragments<HD>(q_s, qa);
+    }
+    const TcArgs ta{a.H, a.KV, a.ldq, a.window, a.S, a.scale, 0, 1, 0.f};
+    for (int p = 0; p < n_vis; p++) {
+        PageJob job;
+        job.s = p; job.g = g; job.b = b; job.page = page_s[p];
+        job.h_first = 1; job.h_last = 0; job.k_first = first_row(p); job.k_last = last_row(p); job.row0 = 0; job.empty = false;
+        if (job.page < 0) {                           // (uniform) reported; the tiles of the next page are still to be fetched
+            __syncthreads();
+            fetch(p + 1, k_cache, k_base);
+            place(p + 1, k_s, ko);
+        } else {
+            compute_page_core<HD, HD, SyncCta>(
+                job, qa, ta,
+                [&](int ks, uint32_t (&kb)[4]) { load_k_frag<HD, TileSwz<HD>>(k_base, ks, kb); },
+                [&](int ks, int nt, uint32_t (&vb)[4]) { load_v_frag<HD, TileSwz<HD>>(v_base, ks, nt, vb); },
+                [&]() { cp_async_wait<1>(); __syncthreads(); },       // this page's K has landed (and every warp has its queries)
+                [&]() { fetch(p + 1, k_cache, k_base); place(p + 1, k_s, ko); },
+                [&]() { cp_async_wait<1>(); __syncthreads(); },       // its V has landed (the next page's K may be in flight)
+                q_s, red_m, red_l,
+                [&](int h, int d, float2 v) { *reinterpret_cast<float2*>(o_s + ((size_t)p * G + h) * HD + d) = v; },
+                [&](int h, float m, float l) { ml_s[p][h] = make_float2(m, l); });
+            __syncthreads();                          // the probabilities and V have been read
+        }
+        fetch(p + 1, v_cache, v_base);
+        place(p + 1, v_s, vo);
+    }
+    cp_async_wait<0>();
+    __syncthreads();
+    // ---- the merge, as merge_pages does it: page s in lane s, one page a series
+    for (int i = warp; i < G; i += WARPS) {
+        const float2 ml = lane < n_vis ? ml_s[lane][i] : make_float2(-INFINITY, 0.f);
+        const float mmax = warp_max(ml.x);
+        float ls = 0.f;
+        if (lane < n_vis) {
+            const float w = ml.x == -INFINITY ? 0.f : expf(ml.x - mmax);
+            w_s[lane][i] = w;
+            ls = fmaf(ml.y, w, ls);
+        }
+        ls = warp_sum(ls);
+        if (lane == 0) inv_s[i] = ls > 0.f ? 1.0f / ls : 0.f;
+    }
+    __syncthreads();
+    bf16* orow = out + (size_t)b * a.ldo + (size_t)g * G * HD;
+    const int hrow = lane >> 2;
+#pragma unroll
+    for (int j = 0; j < 2; j++) {
+        const int h = hrow + 8 * j;
+        if (h >= G) continue;
+        const float inv = inv_s[h];
+#pragma unroll
+        for (int nt = 0; nt < HD / 32; nt++) {
+            const int d = warp * (HD / 4) + nt * 8 + (lane & 3) * 2;
+            float2 os = make_float2(0.f, 0.f);
+            for (int p = 0; p < n_vis; p++) {
+                const float w = w_s[p][h];
+                if (w != 0.f) {                       // a page without visible keys wrote nothing
+                    const float2 o = *reinterpret_cast<const float2*>(o_s + ((size_t)p * G + h) * HD + d);
+                    os.x += __fmul_rn(o.x, w);
+                    os.y += __fmul_rn(o.y, w);
+                }
+            }
+            *reinterpret_cast<__nv_bfloat162*>(orow + (size_t)h * HD + d) = __floats2bfloat162_rn(os.x * inv, os.y * inv);
+        }
+    }
 }
 
 
@@ -826,12 +1033,13 @@ attn_decode_stream_kernel(const __grid_constant__ CUtensorMap map_k, const __gri
             __syncwarp();
             if (lane == 0) mbar_arrive(smem_u32(&bars[STAGES + st]));
             released = true;
+            const ToScratch<HD> to{part_o, part_ml, job.row0, a.S};
             compute_page_core<HD, HD, SyncConsumers>(
                 job, qa, a,
                 [&](int ks, uint32_t (&kb)[4]) { kb[0] = kf[ks][0]; kb[1] = kf[ks][1]; kb[2] = kf[ks][2]; kb[3] = kf[ks][3]; },
                 [&](int ks, int nt, uint32_t (&vb)[4]) { vb[0] = vf[ks][nt / 2][0]; vb[1] = vf[ks][nt / 2][1]; vb[2] = vf[ks][nt / 2][2]; vb[3] = vf[ks][nt / 2][3]; },
-                []() {}, []() { SyncConsumers::sync(); },
-                p_s, red_m, red_l, part_o, part_ml);
+                []() {}, []() {}, []() { SyncConsumers::sync(); },
+                p_s, red_m, red_l, [&](int h, int d, float2 v) { to.o(h, d, v); }, [&](int h, float m, float l) { to.ml(h, m, l); });
         }
         if (!released && lane == 0) mbar_arrive(smem_u32(&bars[STAGES + st]));
         SyncConsumers::sync();                                     // the page's scratch (probabilities, sums) is free again
@@ -1015,6 +1223,14 @@ MYNAH_API int mynah_attn_decode_tc_capped(
     return mynah_check_launch("attn_decode_merge");
 }
 
+// Whether mynah_attn_decode_fused gives a (sequence, kv head) of a step of B sequences and at most `n_splits` pages one CTA: enough of
+// them to fill the SMs with time to spare, since a CTA walks its pages one after the other (8 kv heads, us a step of 28 layers, three launches
+// or a CTA a page -> this: 20 rows behind 180 positions 1,232 -> 1,286, 32 rows 1,360 -> 1,311, 64 rows 1,498 -> 1,406; 20 rows
+// of 16 kv heads of 64 behind 100, 16 layers, 945 -> 858).
+MYNAH_API int mynah_attn_decode_short(int B, int KV, int n_splits) {
+    return n_splits <= SHORT_PAGES && 2ll * B * KV >= 3ll * mynah_sm_count();
+}
+
 // The fused decode attention: q, k, v rows [B, (H + 2 KV) * HD] as the projection left them (with write_kv = 0
 // only the q columns are read and the cache is taken as complete); gains may be null (no per-head norm), the
 // tables may be null (no rotation; else the whole head is rotated). `counters`: B * KV words, zero before the
@@ -1041,6 +1257,15 @@ MYNAH_API int mynah_attn_decode_fused(
     float* part_o = scratch;
     float* part_ml = scratch + (size_t)B * H * n_splits * HD;
     const VecRef qg{q_gain, gain_dtype}, kg{k_gain, gain_dtype};
+    if (mynah_attn_decode_short(B, KV, n_splits)) {
+        const size_t o_bytes = (size_t)n_splits * (H / KV) * HD * sizeof(float);
+        auto kern = HD == 128 ? attn_decode_short_kernel<128> : attn_decode_short_kernel<64>;
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_PAGES * MAX_G * 128 * (int)sizeof(float));
+        if (e != cudaSuccess) return mynah_fail("attn_decode_fused: %s", cudaGetErrorString(e));
+        mynah_launch(kern, dim3(KV, B), dim3(WARPS * 32), o_bytes, stream, (const bf16*)qkv, qg, kg, cos_t, sin_t, tok_pos,
+                     kv_len, pt, (bf16*)k_cache, (bf16*)v_cache, a, (bf16*)out, status);
+        return mynah_check_launch("attn_decode_fused (short)");
+    }
     const dim3 grid(n_splits, KV, B);
     if (counters == nullptr) {
         // without counters: the pages' CTAs do not merge; the merge follows as a launch of its own (the same bits)

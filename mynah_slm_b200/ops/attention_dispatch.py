@@ -51,10 +51,10 @@ FUSED_PREP_LARGE = os.environ.get("MYNAH_FUSED_ATTN_PREP", "0") == "1"
 
 def decode_fused_ok(dtype: torch.dtype, H: int, KV: int, HD: int, rotary_dim: int, cos, B: int, n_splits: int) -> bool:
     """Whether the one-launch decode attention takes this layer in this step: the tensor-core sizes, a rotation
-    of the whole head or none, and few enough CTAs."""
+    of the whole head or none, and few enough CTAs, or many sequences of few pages (a CTA a sequence's kv head then)."""
     if not kernels.attn_decode_tc_supported(dtype, H, KV, HD):
         return False
-    if B * KV * n_splits > FUSED_DECODE_MAX_CTAS and not FUSED_PREP_LARGE:
+    if B * KV * n_splits > FUSED_DECODE_MAX_CTAS and not FUSED_PREP_LARGE and not kernels.attn_decode_short(B, KV, n_splits):
         return False
     return _tc_fits(H, KV, n_splits) and (cos is None or rotary_dim == HD)
 

@@ -478,6 +478,11 @@ def attn_decode_fused(qkv: torch.Tensor, out: torch.Tensor, B: int, H: int, KV: 
          window or 0, n_splits, ptr(scratch), ptr(counters), ptr(status), stream_ptr())
 
 
+def attn_decode_short(B: int, KV: int, n_splits: int) -> bool:
+    """Whether the one-launch decode attention gives a (sequence, kv head) one CTA (csrc/attn_decode_tc.cu)."""
+    return bool(lib.load().mynah_attn_decode_short(B, KV, n_splits))
+
+
 def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     _chk(logits, "logits", torch.float32, 2)
     B, V = logits.shape
