@@ -180,7 +180,7 @@ template <int MT>
 __global__ void __launch_bounds__(256)
 head_linear_mma_kernel(const bf16* __restrict__ in, const bf16* __restrict__ W, bf16* __restrict__ out, HeadLinearArgs a) {
     constexpr int NT = 2;
-    __shared__ __align__(16) bf16 xs[16 * MT][tilemma::MMA_LDS];
+    __shared__ __align__(16) bf16 xs[16 * MT][tilemma::block_ld(MT)];
     __shared__ int row_s[16 * MT];
     griddep_wait();
     const int t0 = blockIdx.x * 16 * MT, h = blockIdx.y;

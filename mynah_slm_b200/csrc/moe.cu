@@ -453,7 +453,7 @@ template <int MT, int NT, int ACT>
 __global__ void __launch_bounds__(MMA_WARPS * 32, 2)
 moe_gate_up_mma_kernel(const bf16* __restrict__ h, const bf16* __restrict__ w_gu, bf16* __restrict__ y,
                        const int* __restrict__ perm, const int* __restrict__ tiles, MoeArgs a) {
-    __shared__ __align__(16) bf16 xs[16 * MT][tilemma::MMA_LDS];
+    __shared__ __align__(16) bf16 xs[16 * MT][tilemma::block_ld(MT)];
     __shared__ int pair_s[16 * MT];
     griddep_wait();
     if ((int)blockIdx.x >= tiles[0]) return;
@@ -500,7 +500,7 @@ template <int MT, int NT>
 __global__ void __launch_bounds__(MMA_WARPS * 32, 2)
 moe_down_mma_kernel(const bf16* __restrict__ y, const bf16* __restrict__ w_down, float* __restrict__ o,
                     const int* __restrict__ perm, const int* __restrict__ tiles, MoeArgs a) {
-    __shared__ __align__(16) bf16 xs[16 * MT][tilemma::MMA_LDS];
+    __shared__ __align__(16) bf16 xs[16 * MT][tilemma::block_ld(MT)];
     __shared__ int pair_s[16 * MT];
     griddep_wait();
     if ((int)blockIdx.x >= tiles[0]) return;
