@@ -12,6 +12,7 @@
 //                    32 values a lane), which add their parts of o by shuffles in a fixed order. Keys, queries and
 //                    values of 32 tokens at a time pass through shared memory.
 //   retention_local, _states, _out   the same recurrence for prompts, a chunk of tokens at a time (see below)
+//   retention_step   all of a decode step's row behind its projection, the RMS and the gate with it (see below)
 //
 // All arithmetic is fp32. A sequence's rows are walked in order, so a prompt run whole, in pieces or token by
 // token performs the same operations in the same order.
@@ -207,6 +208,93 @@ retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn
             const int i = l * per + r;
             if (r < per && i < a.dim) sp[(size_t)i * a.vd + j] = S[r];
         }
+    }
+}
+
+// ---- a decode step: preparation, one token of the recurrence, the unit RMS and the gate ----
+// A CTA a (row, head), L lanes a column as in retention_scan: the state's 64 KB (128 x 128) are asked for at once and everything
+// else is worked out meanwhile, so the step is one trip to memory instead of three launches. The arithmetic and its order are those of
+// retention_prep, retention_scan and gated_rmsnorm. Rows without a sequence give zeros. Measured (16 heads of
+// 128, us against the three launches): 2 rows 8.4 / 8.7, 4 rows 8.6 / 9.5, 8 rows 9.2 / 12.8; where the CTAs no longer run side by side the
+// scan's many small ones win (16 rows 18.9 / 19.3, 32 rows 36.6 / 29.8), and one row leaves most SMs idle (8.3 / 7.9).
+struct RetStepArgs {
+    int H, dim, vd, n_slots, L, per, ld, q_off, k_off, v_off, g_off, ldo;
+    int rot, interleaved, n_pos;
+    float k_scale, eps;
+};
+
+template <typename T>
+__global__ void __launch_bounds__(512)
+retention_step_kernel(const T* __restrict__ p, const float* __restrict__ cos_t, const float* __restrict__ sin_t,
+                      const float* __restrict__ decay, float* __restrict__ state, VecRef w, T* __restrict__ out,
+                      const int* __restrict__ tok_seq, const int* __restrict__ tok_pos, const int* __restrict__ slots, RetStepArgs a,
+                      int* __restrict__ status) {
+    __shared__ float qs[128 + 32], ks[128 + 32], os[512], zs[512];    // q and k: a lane's chunk, one float apart from the next
+    griddep_launch_small();
+    griddep_wait();
+    const int h = blockIdx.x, b = blockIdx.y, tid = threadIdx.x;
+    const int slot = slots[b], pos = tok_pos[b];
+    const T* row = p + (size_t)b * a.ld;
+    T* dst = out + (size_t)b * a.ldo + (size_t)h * a.vd;
+    const bool rotate = a.rot > 0 && cos_t != nullptr;
+    const bool bad_pos = rotate && (pos < 0 || pos >= a.n_pos);
+    if (tok_seq[b] < 0 || slot < 0 || slot >= a.n_slots || bad_pos) {
+        if (tok_seq[b] >= 0 && bad_pos && tid == 0) atomicOr(status, MYNAH_ST_POS_RANGE);
+        for (int j = tid; j < a.vd; j += blockDim.x) dst[j] = from_f32<T>(0.f);
+        return;
+    }
+    const int L = a.L, per = a.per, l = tid % L, j = tid / L;
+    const bool on = j < a.vd;
+    float* sp = state + (((size_t)slot * a.H + h) * a.dim) * a.vd;
+    float S[RET_RMAX];
+#pragma unroll
+    for (int r = 0; r < RET_RMAX; r++) {
+        const int i = l * per + r;
+        S[r] = (on && r < per && i < a.dim) ? sp[(size_t)i * a.vd + j] : 0.f;
+    }
+    for (int e = tid; e < 2 * a.dim; e += blockDim.x) {
+        const bool is_k = e >= a.dim;
+        const int d = is_k ? e - a.dim : e, half = a.rot >> 1;
+        const T* src = row + (is_k ? a.k_off : a.q_off) + (size_t)h * a.dim;
+        float v = to_f32(src[d]);
+        if (rotate && d < a.rot) {
+            int i, other;
+            float sign;
+            if (a.interleaved) {
+                i = d >> 1; other = d ^ 1; sign = (d & 1) ? 1.f : -1.f;
+            } else {
+                i = d < half ? d : d - half; other = d < half ? d + half : d - half; sign = d < half ? -1.f : 1.f;
+            }
+            v = v * cos_t[(size_t)pos * half + i] + sign * to_f32(src[other]) * sin_t[(size_t)pos * half + i];
+        }
+        (is_k ? ks : qs)[d + d / per] = is_k ? v * a.k_scale : v;
+    }
+    for (int d = tid; d < a.vd; d += blockDim.x) zs[d] = to_f32(row[a.g_off + (size_t)h * a.vd + d]);
+    const float vj = on ? to_f32(row[a.v_off + (size_t)h * a.vd + j]) : 0.f, g = decay[h];
+    __syncthreads();
+    float acc = 0.f;
+#pragma unroll
+    for (int r = 0; r < RET_RMAX; r++) {
+        if (r < per && l * per + r < a.dim) {
+            S[r] = fmaf(ks[l * (per + 1) + r], vj, g * S[r]);
+            acc = fmaf(S[r], qs[l * (per + 1) + r], acc);
+        }
+    }
+    for (int m = 1; m < L; m <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    if (on && l == 0) os[j] = acc;
+#pragma unroll
+    for (int r = 0; r < RET_RMAX; r++) {
+        const int i = l * per + r;
+        if (on && r < per && i < a.dim) sp[(size_t)i * a.vd + j] = S[r];
+    }
+    __syncthreads();
+    if (tid >= 32) return;
+    float ss = 0.f;
+    for (int d = tid; d < a.vd; d += 32) ss = fmaf(os[d], os[d], ss);
+    const float r = 1.0f / sqrtf(warp_sum(ss) / (float)a.vd + a.eps);
+    for (int d = tid; d < a.vd; d += 32) {
+        const float z = zs[d], sg = 1.0f / (1.0f + expf(-z));
+        dst[d] = from_f32<T>(os[d] * r * w.at(d) * (z * sg));
     }
 }
 
@@ -533,4 +621,39 @@ MYNAH_API int mynah_retention_scan(const float* qn, const float* kn, const void*
     } else
         return mynah_fail("retention_scan: unsupported dtype %d", v_dtype);
     return mynah_check_launch("retention_scan");
+}
+
+// A decode step's rows, one a sequence: p [B, ld] holds every head's q, k, v and gate from their columns on; state as above; w [vd]
+// in w_dtype; out [B, ldo] in dtype. Keys of up to 128 values, value heads of up to 512 / (lanes a column).
+MYNAH_API int mynah_retention_step_supported(int dim, int vd) {
+    int L = 1;
+    while (L * RET_RMAX < dim) L <<= 1;
+    return dim > 0 && dim <= 128 && vd > 0 && L * vd <= 512;
+}
+// Whether it is the faster form for B rows: a CTA an SM at most, and more than a handful (figures at the kernel).
+MYNAH_API int mynah_retention_step_pays(int B, int H) {
+    return (long long)B * H >= 32 && (long long)B * H <= mynah_sm_count();
+}
+MYNAH_API int mynah_retention_step(const void* p, int ld, int q_off, int k_off, int v_off, int g_off, int dtype, const float* cos_t,
+                                   const float* sin_t, int rot, int interleaved, int n_pos, float k_scale, const float* decay,
+                                   float* state, int n_slots, const void* w, int w_dtype, float eps, void* out, int ldo, int B, int H,
+                                   int dim, int vd, const int* tok_seq, const int* tok_pos, const int* slots, int* status,
+                                   cudaStream_t stream) {
+    if (B == 0) return 0;
+    MYNAH_REQUIRE(B > 0 && H > 0 && B <= 65535 && mynah_retention_step_supported(dim, vd), "retention_step: bad sizes B=%d H=%d dim=%d vd=%d", B, H, dim, vd);
+    MYNAH_REQUIRE(rot % 2 == 0 && rot <= dim, "retention_step: %d rotated dims do not fit a head of %d", rot, dim);
+    int L = 1;
+    while (L * RET_RMAX < dim) L <<= 1;
+    const RetStepArgs a{H, dim, vd, n_slots, L, ceil_div(dim, L), ld, q_off, k_off, v_off, g_off, ldo, cos_t ? rot : 0, interleaved, n_pos, k_scale, eps};
+    const dim3 grid(H, B), block(ceil_div(L * vd, 32) * 32);
+    const VecRef wv{w, w_dtype};
+    if (dtype == MYNAH_F32)
+        mynah_launch(retention_step_kernel<float>, grid, block, 0, stream, (const float*)p, cos_t, sin_t, decay, state, wv, (float*)out, tok_seq, tok_pos,
+                     slots, a, status);
+    else if (dtype == MYNAH_BF16)
+        mynah_launch(retention_step_kernel<bf16>, grid, block, 0, stream, (const bf16*)p, cos_t, sin_t, decay, state, wv, (bf16*)out, tok_seq, tok_pos,
+                     slots, a, status);
+    else
+        return mynah_fail("retention_step: unsupported dtype %d", dtype);
+    return mynah_check_launch("retention_step");
 }

@@ -983,6 +983,36 @@ def retention_scan(qn: torch.Tensor, kn: torch.Tensor, v: torch.Tensor, v_off: i
     return o
 
 
+def retention_step_ok(p: torch.Tensor, ctx, H: int, dim: int, vd: int) -> bool:
+    """Whether `retention_step` takes a step and is the faster form: one row a sequence, heads that fit its CTA, as many CTAs as run
+    side by side."""
+    L = lib.load()
+    return (bool(ctx.is_decode) and p.shape[0] == ctx.B and bool(L.mynah_retention_step_supported(dim, vd))
+            and bool(L.mynah_retention_step_pays(ctx.B, H)))
+
+
+def retention_step(p: torch.Tensor, q_off: int, k_off: int, v_off: int, g_off: int, cos, sin, rot: int, interleaved: bool,
+                   k_scale: float, decay: torch.Tensor, state: torch.Tensor, w: torch.Tensor, eps: float, ctx, H: int, dim: int,
+                   vd: int) -> torch.Tensor:
+    """`retention_prep`, `retention_scan` and `gated_rmsnorm` (silu) for a decode step's rows, one launch; returns [B, H * vd] in
+    p's type."""
+    _rows(p, "retention_step: projection")
+    _chk(state, "retention state", torch.float32, 4)
+    _chk(decay, "decays", torch.float32, 1)
+    if tuple(state.shape[1:]) != (H, dim, vd) or decay.numel() != H or w.numel() != vd:
+        raise KernelError("retention_step: the state, the decays or the gain do not fit")
+    if max(q_off + H * dim, k_off + H * dim, v_off + H * vd, g_off + H * vd) > p.shape[1]:
+        raise KernelError("retention_step: the projection's rows are too short")
+    if cos is not None and cos.shape[1] * 2 != rot:
+        raise KernelError("retention_step: the rotation table does not match the rotated dims")
+    out = torch.empty((p.shape[0], H * vd), dtype=p.dtype, device=p.device)
+    call("mynah_retention_step", ptr(p), p.stride(0), q_off, k_off, v_off, g_off, code(p.dtype), ptr(cos), ptr(sin),
+         rot if cos is not None else 0, 1 if interleaved else 0, cos.shape[0] if cos is not None else 0, float(k_scale), ptr(decay),
+         ptr(state), state.shape[0] - 1, ptr(w), code(w.dtype), float(eps), ptr(out), H * vd, p.shape[0], H, dim, vd,
+         ptr(ctx.tok_seq), ptr(ctx.tok_pos), ptr(ctx.slots), ptr(ctx.status), stream_ptr())
+    return out
+
+
 def retention_chunk_min(n: int) -> int:
     """From how many tokens in a step's longest piece the retention recurrence runs chunk by chunk (keys that are a
     multiple of 32 values up to 256); 0: always token by token. Returns the setting before. The two forms agree to

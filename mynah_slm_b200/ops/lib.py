@@ -111,6 +111,8 @@ _SIGNATURES: dict[str, list] = {
                              P, P, P, c_int, P, c_int, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
     "mynah_delta_prep": [P, c_int, P, P, c_int, c_int, P, P, c_int, P, P, P, P, c_int, c_int, c_int, c_int, P, c_int, P],
     "mynah_delta_rule": [P, P, P, c_int, c_int, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
+    "mynah_retention_step": [P, c_int, c_int, c_int, c_int, c_int, c_int, P, P, c_int, c_int, c_int, c_float, P, P, c_int, P, c_int,
+                             c_float, P, c_int, c_int, c_int, c_int, c_int, P, P, P, P, P],
     "mynah_gated_rmsnorm": [P, P, c_int, c_int, P, c_int, P, c_int, c_int, c_int, c_float, c_int, P],
     "mynah_rmsnorm_add": [P, P, P, P, c_int, c_float, P, c_int, c_float, P, P, c_int, c_int, P],
     "mynah_rms_rows": [P, c_int, c_int, P, c_int, c_float, P, c_int, c_int, c_int, P],
@@ -204,6 +206,10 @@ def load() -> ctypes.CDLL:
                  "mynah_gated_memory_chunk_min"):
         getattr(lib, name).restype = c_int
         getattr(lib, name).argtypes = [c_int]
+    lib.mynah_retention_step_supported.restype = c_int
+    lib.mynah_retention_step_supported.argtypes = [c_int, c_int]
+    lib.mynah_retention_step_pays.restype = c_int
+    lib.mynah_retention_step_pays.argtypes = [c_int, c_int]
     lib.mynah_delta_scratch_floats.restype = c_longlong
     lib.mynah_delta_scratch_floats.argtypes = [c_int] * 8 + [P]
     lib.mynah_retention_scratch_floats.restype = c_longlong

@@ -102,6 +102,10 @@ class Retention(Mixer):
                                  vd, self.eps)
             return kernels.linear(out, self.w_o, out_dtype=self.out_dtype)
         nq = H * dim
+        if kernels.retention_step_ok(p, ctx, H, dim, vd):
+            out = kernels.retention_step(p, 0, nq, 2 * nq, 2 * nq + H * vd, self.cos, self.sin, self.rot, self.interleaved, float(dim) ** -0.5,
+                                         self.decay_t, cache.state["S"], self.ones, self.eps, ctx, H, dim, vd)
+            return kernels.linear(out, self.w_o, out_dtype=self.out_dtype)
         qn, kn = kernels.retention_prep(p, 0, nq, H, dim, self.cos, self.sin, self.rot, self.interleaved,
                                         float(dim) ** -0.5, ctx)
         o = kernels.retention_scan(qn, kn, p, 2 * nq, self.decay_t, cache.state["S"], ctx, H, dim, vd)
