@@ -16,7 +16,6 @@
 //
 // All arithmetic is fp32. A sequence's rows are walked in order, so a prompt run whole, in pieces or token by
 // token performs the same operations in the same order.
-#include "chunk_prod.cuh"
 #include "layout.cuh"
 
 namespace {
@@ -320,10 +319,29 @@ retention_step_kernel(const T* __restrict__ p, const float* __restrict__ cos_t, 
 //
 // The powers of g come from a table made by repeated multiplication. Sums run in another order than token by token:
 // the two forms agree to rounding.
+constexpr int RC_THREADS = 256;
+
 struct RetChunkArgs {
     int H, dim, vd, n_slots, ldv, v_off, B, cols;          // cols: columns of a state in scratch (vd padded to whole tiles)
     int first;                                              // the pass's first chunk
 };
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void fma2(f32x2& c, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void mul2(f32x2& c, f32x2 a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
+
+struct alignas(16) Pairs { f32x2 lo, hi; };                 // four floats as two pairs, one 16-byte load
+__device__ __forceinline__ Pairs pairs_at(const float* p) { return *reinterpret_cast<const Pairs*>(p); }
 
 // gp[n] = g^n, n <= C
 template <int C>
@@ -334,6 +352,28 @@ __device__ __forceinline__ void decay_powers(float* gp, float g) {
             gp[n] = p;
             p *= g;
         }
+    }
+}
+
+// A chunk's rows of one head into shared memory, rows from nt on as zeros (C rows, d values, d + 4 apart).
+template <int C>
+__device__ __forceinline__ void stage_rows(float* dst, const float* __restrict__ src, size_t row, int d, int nt) {
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < C * (d / 4); idx += RC_THREADS) {
+        const int tt = idx / (d / 4), i4 = (idx % (d / 4)) * 4;
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (tt < nt) x = *reinterpret_cast<const float4*>(src + (size_t)tt * row + i4);
+        *reinterpret_cast<float4*>(dst + tt * (d + 4) + i4) = x;
+    }
+}
+
+// A chunk's values of one head, columns [j0, j0 + JT), times `weight(token)`; what does not exist is zero.
+template <typename T, int C, int JT, typename F>
+__device__ __forceinline__ void stage_values(float* vs, const T* __restrict__ v, int ldv, int j0, int vd, int nt, F weight) {
+#pragma unroll 4
+    for (int idx = threadIdx.x; idx < C * JT; idx += RC_THREADS) {
+        const int tt = idx / JT, c = idx % JT;
+        vs[idx] = (tt < nt && j0 + c < vd) ? weight(tt) * to_f32(v[(size_t)tt * ldv + j0 + c]) : 0.f;
     }
 }
 
@@ -454,20 +494,14 @@ retention_states_kernel(const float* __restrict__ decay, float* __restrict__ sta
         if (k < have) sp[k] = S[k];
 }
 
-// The same grid as retention_local.
-template <int C>
-struct RetWeights {
-    const float* gp;
-    __device__ __forceinline__ void fill(float*) const {}
-    __device__ __forceinline__ float score(int t, int s, const float*) const { return gp[t - s]; }
-    __device__ __forceinline__ float before(int t) const { return gp[t + 1]; }
-};
-
+// The same grid as retention_local. Thread (ty, tx) owns tokens ty * RT + u and columns tx * 4 + {0..3} (of either half, when the
+// tile has 128). The keys' place in shared memory is used again by the old state, 32 rows at a time, and then by the values.
 template <typename T, int C, int JT>
 __global__ void __launch_bounds__(RC_THREADS, 2)
 retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v, const float* __restrict__ decay,
                      const float* __restrict__ states, float* __restrict__ o, const int* __restrict__ cu_q,
                      const int* __restrict__ slots, RetChunkArgs a) {
+    constexpr int RT = C / 16, G = JT / 64, LDW = C + 4, SR = 32;
     extern __shared__ __align__(16) float sm[];
     __shared__ float gp[C + 1];
     griddep_wait();
@@ -475,13 +509,132 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
     if (!find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile)) return;
     const int slot = slots[b];
     if (slot < 0 || slot >= a.n_slots) return;
-    const int h = blockIdx.y, d = a.dim, j0 = blockIdx.z * JT;
+    const int h = blockIdx.y, d = a.dim, j0 = blockIdx.z * JT, ldr = d + 4;
     const int t0 = cu_q[b] + tile * C, nt = min(C, cu_q[b + 1] - t0);
+    float* qs = sm;                        // [C][ldr]
+    float* Ws = qs + C * ldr;              // [C][LDW]
+    float* xs = Ws + C * LDW;              // [C][ldr] keys; [2][SR][JT] state rows; [C][JT] values
     decay_powers<C>(gp, decay[h]);
-    const size_t n = (size_t)a.H * d, at = (size_t)t0 * n + (size_t)h * d;
-    chunk_outputs<T, C, JT>(sm, qn + at, kn + at, n, d, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd,
-                            states + ((size_t)blockIdx.x * a.H + h) * d * a.cols + j0, a.cols,
-                            o + (size_t)t0 * a.H * a.vd + (size_t)h * a.vd, (size_t)a.H * a.vd, nt, RetWeights<C>{gp});
+    const size_t n = (size_t)a.H * d;
+    stage_rows<C>(qs, qn + (size_t)t0 * n + (size_t)h * d, n, d, nt);
+    stage_rows<C>(xs, kn + (size_t)t0 * n + (size_t)h * d, n, d, nt);
+    __syncthreads();
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    {   // scores: tokens ty + 16 u, keys tx + 16 w; even and odd values of a head are summed apart, then added
+        f32x2 acc[RT][RT];
+#pragma unroll
+        for (int u = 0; u < RT; u++)
+#pragma unroll
+            for (int w = 0; w < RT; w++) acc[u][w] = 0ull;
+#pragma unroll 2
+        for (int i = 0; i < d; i += 4) {
+            Pairs qv[RT], kv[RT];
+#pragma unroll
+            for (int u = 0; u < RT; u++) qv[u] = pairs_at(qs + (ty + 16 * u) * ldr + i);
+#pragma unroll
+            for (int w = 0; w < RT; w++) kv[w] = pairs_at(xs + (tx + 16 * w) * ldr + i);
+#pragma unroll
+            for (int u = 0; u < RT; u++)
+#pragma unroll
+                for (int w = 0; w <= u; w++) {              // (keys behind every token of the group: not needed)
+                    fma2(acc[u][w], qv[u].lo, kv[w].lo);
+                    fma2(acc[u][w], qv[u].hi, kv[w].hi);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < RT; u++)
+#pragma unroll
+            for (int w = 0; w < RT; w++) {
+                const int t = ty + 16 * u, s = tx + 16 * w;
+                const float2 x = unpack2(acc[u][w]);
+                Ws[t * LDW + s] = s <= t ? gp[t - s] * (x.x + x.y) : 0.f;
+            }
+    }
+    __syncthreads();                                        // the scores are there, the keys are done with
+    f32x2 acc[RT][G][2];
+#pragma unroll
+    for (int u = 0; u < RT; u++)
+#pragma unroll
+        for (int w = 0; w < G; w++) acc[u][w][0] = acc[u][w][1] = 0ull;
+    // one product's four steps of k: rows [ty * RT, + RT) of `lhs` from column i, rows [i, i + 4) of `rhs`
+    auto steps = [&](const float* lhs, int ld, const float* rhs) {
+        float4 x[RT];
+#pragma unroll
+        for (int u = 0; u < RT; u++) x[u] = *reinterpret_cast<const float4*>(lhs + (ty * RT + u) * ld);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            Pairs y[G];
+#pragma unroll
+            for (int w = 0; w < G; w++) y[w] = pairs_at(rhs + k * JT + w * 64 + tx * 4);
+#pragma unroll
+            for (int u = 0; u < RT; u++) {
+                const float xk = k == 0 ? x[u].x : k == 1 ? x[u].y : k == 2 ? x[u].z : x[u].w;
+                const f32x2 x2 = pack2(xk, xk);
+#pragma unroll
+                for (int w = 0; w < G; w++) {
+                    fma2(acc[u][w][0], x2, y[w].lo);
+                    fma2(acc[u][w][1], x2, y[w].hi);
+                }
+            }
+        }
+    };
+    // ---- the old state, in pieces of SR rows; a piece is on its way while the one before is multiplied
+    const float* from = states + ((size_t)blockIdx.x * a.H + h) * d * a.cols + j0;
+    auto fetch = [&](int piece) {
+        if (piece * SR < d) {
+            float* dst = xs + (piece & 1) * SR * JT;
+#pragma unroll
+            for (int idx = threadIdx.x; idx < SR * JT / 4; idx += RC_THREADS) {
+                const int i = idx / (JT / 4), c = (idx % (JT / 4)) * 4;
+                const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst + i * JT + c);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(s), "l"(from + (size_t)(piece * SR + i) * a.cols + c) : "memory");
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    fetch(0);
+    for (int p = 0; p * SR < d; p++) {
+        fetch(p + 1);
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();
+        const float* S = xs + (p & 1) * SR * JT;
+#pragma unroll 2
+        for (int i = 0; i < SR; i += 4) steps(qs + p * SR + i, ldr, S + i * JT);
+        __syncthreads();                                    // the piece's place may be filled again
+    }
+#pragma unroll
+    for (int u = 0; u < RT; u++) {
+        const float gt = gp[ty * RT + u + 1];
+#pragma unroll
+        for (int w = 0; w < G; w++) {
+            mul2(acc[u][w][0], pack2(gt, gt));
+            mul2(acc[u][w][1], pack2(gt, gt));
+        }
+    }
+    // ---- scores times values
+    stage_values<T, C, JT>(xs, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd, nt, [](int) { return 1.f; });
+    __syncthreads();
+    const int s_end = ((ty | 1) + 1) * RT;                  // keys behind the last token of the warp's rows weigh nothing
+    for (int s = 0; s < s_end; s += 4) steps(Ws + s, LDW, xs + s * JT);
+#pragma unroll
+    for (int u = 0; u < RT; u++) {
+        const int t = ty * RT + u;
+        if (t >= nt) break;
+        float* row = o + (size_t)(t0 + t) * a.H * a.vd + (size_t)h * a.vd;
+#pragma unroll
+        for (int w = 0; w < G; w++) {
+            const int j = j0 + w * 64 + tx * 4;
+            const float2 x = unpack2(acc[u][w][0]), y = unpack2(acc[u][w][1]);
+            if (j + 3 < a.vd && (a.vd & 3) == 0) {
+                *reinterpret_cast<float4*>(row + j) = make_float4(x.x, x.y, y.x, y.y);
+            } else {
+                if (j < a.vd) row[j] = x.x;
+                if (j + 1 < a.vd) row[j + 1] = x.y;
+                if (j + 2 < a.vd) row[j + 2] = y.x;
+                if (j + 3 < a.vd) row[j + 3] = y.y;
+            }
+        }
+    }
 }
 
 // How a step's chunks go: tokens a chunk, columns a tile, padded columns of a state, chunks a pass.
@@ -507,7 +660,8 @@ int launch_chunked(const float* qn, const float* kn, const void* v, const float*
                    const int* cu_q, const int* slots, RetChunkArgs a, const RetPlan& plan, cudaStream_t stream) {
     const int d = a.dim;
     const size_t local = ((size_t)C * (d + 4) + (size_t)C * JT) * sizeof(float);
-    const size_t out = chunk_outputs_floats<C, JT>(d) * sizeof(float);
+    const size_t shared_part = (size_t)C * (d + 4) > (size_t)64 * JT ? (size_t)C * (d + 4) : (size_t)64 * JT;
+    const size_t out = ((size_t)C * (d + 4) + (size_t)C * (C + 4) + shared_part) * sizeof(float);
     if (cudaFuncSetAttribute(retention_local_kernel<T, C, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess ||
         cudaFuncSetAttribute(retention_out_kernel<T, C, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess)
         return mynah_fail("retention_scan: %zu bytes of shared memory are not to be had", out);

@@ -794,21 +794,9 @@ def delta_rule(qn: torch.Tensor, kn: torch.Tensor, v: torch.Tensor, g: torch.Ten
         raise KernelError("delta_rule: the decay's rows do not fit")
     channel = 1 if channel_decay else 0
     o = torch.empty((T, H * vd), dtype=torch.float32, device=v.device)
-    launches = ctypes.c_int(1)
-    need = int(lib.load().mynah_delta_scratch_floats(T, ctx.B, H, dim, vd, int(ctx.max_q_len), channel, code(v.dtype),
-                                                     ctypes.addressof(launches)))
-    scratch = torch.empty((need,), dtype=torch.float32, device=v.device) if need else None
     call("mynah_delta_rule", ptr(qn), ptr(kn), ptr(v), v.stride(0), code(v.dtype), ptr(g), ptr(beta), ptr(state),
-         state.shape[0] - 1, ptr(o), ptr(ctx.cu_q), ptr(ctx.slots), ctx.B, H, G, dim, vd, channel, T, ptr(scratch), stream_ptr())
-    lib.add_launches(launches.value - 1)
+         state.shape[0] - 1, ptr(o), ptr(ctx.cu_q), ptr(ctx.slots), ctx.B, H, G, dim, vd, channel, stream_ptr())
     return o
-
-
-def delta_chunk_min(n: int) -> int:
-    """From how many tokens in a step's longest piece the bfloat16 delta rule with a decay a head runs chunk by chunk (keys that
-    are a multiple of 32 values up to 128); 0: always token by token. Returns the setting before. The two forms agree to
-    rounding."""
-    return int(lib.load().mynah_delta_chunk_min(int(n)))
 
 
 def gated_rmsnorm(o: torch.Tensor, gate: torch.Tensor, w: torch.Tensor, H: int, vd: int, eps: float,

@@ -110,7 +110,7 @@ _SIGNATURES: dict[str, list] = {
     "mynah_selective_scan": [P, c_int, P, c_int, P, c_int, c_int, P, c_int, P, P, c_int, c_int,
                              P, P, P, c_int, P, c_int, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
     "mynah_delta_prep": [P, c_int, P, P, c_int, c_int, P, P, c_int, P, P, P, P, c_int, c_int, c_int, c_int, P, c_int, P],
-    "mynah_delta_rule": [P, P, P, c_int, c_int, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, c_int, P, P],
+    "mynah_delta_rule": [P, P, P, c_int, c_int, P, P, P, c_int, P, P, P, c_int, c_int, c_int, c_int, c_int, c_int, P],
     "mynah_retention_step": [P, c_int, c_int, c_int, c_int, c_int, c_int, P, P, c_int, c_int, c_int, c_float, P, P, c_int, P, c_int,
                              c_float, P, c_int, c_int, c_int, c_int, c_int, P, P, P, P, P],
     "mynah_gated_rmsnorm": [P, P, c_int, c_int, P, c_int, P, c_int, c_int, c_int, c_float, c_int, P],
@@ -202,7 +202,7 @@ def load() -> ctypes.CDLL:
     lib.mynah_attn_decode_short.argtypes = [c_int, c_int, c_int]
     lib.mynah_gemv_decode_supported.restype = c_int
     lib.mynah_gemv_decode_supported.argtypes = [c_int, c_int, c_int]
-    for name in ("mynah_moe_plain", "mynah_retention_chunk_min", "mynah_head_linear_plain", "mynah_moe_grouped_min", "mynah_delta_chunk_min",
+    for name in ("mynah_moe_plain", "mynah_retention_chunk_min", "mynah_head_linear_plain", "mynah_moe_grouped_min",
                  "mynah_gated_memory_chunk_min"):
         getattr(lib, name).restype = c_int
         getattr(lib, name).argtypes = [c_int]
@@ -210,8 +210,6 @@ def load() -> ctypes.CDLL:
     lib.mynah_retention_step_supported.argtypes = [c_int, c_int]
     lib.mynah_retention_step_pays.restype = c_int
     lib.mynah_retention_step_pays.argtypes = [c_int, c_int]
-    lib.mynah_delta_scratch_floats.restype = c_longlong
-    lib.mynah_delta_scratch_floats.argtypes = [c_int] * 8 + [P]
     lib.mynah_retention_scratch_floats.restype = c_longlong
     lib.mynah_retention_scratch_floats.argtypes = [c_int] * 6 + [P]
     lib.mynah_gated_memory_scratch_floats.restype = c_longlong
