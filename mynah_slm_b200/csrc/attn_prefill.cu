@@ -60,7 +60,7 @@ attn_prefill_generic_kernel(const TA* __restrict__ q, TA* __restrict__ out,
                             const TC* __restrict__ k_cache, const TC* __restrict__ v_cache,
                             const int* __restrict__ cu_q, const int* __restrict__ kv_len,
                             PageTable pt, PrefillArgs a, int* __restrict__ status) {
-    extern __shared__ float smem[];
+    extern __shared__ __align__(16) float smem[];      // (read four floats at a time)
     const int HD = a.HD, VD = a.VD, KS = VEC ? HD + KPAD : HD + 1;      // padded key rows: lanes read distinct banks
     float* Ks = smem;                                  // [KT][KS]
     float* Vs = Ks + KT * KS;                          // [KT][VD]

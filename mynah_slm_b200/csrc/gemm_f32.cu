@@ -22,10 +22,11 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int N>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
-// A 16-byte read of shared memory that stays where it is written: ahead of the multiply-adds it is to hide behind.
+// A 16-byte read of shared memory that stays where it is written: ahead of the multiply-adds it is to hide behind, behind the barrier
+// that says that the slab is there (the clobber: nothing that touches memory moves across it).
 __device__ __forceinline__ float4 read16(uint32_t at) {
     float4 v;
-    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at));
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(at) : "memory");
     return v;
 }
 
