@@ -271,15 +271,34 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         if (works) {
             const uint32_t w = base + (uint32_t)((s % STAGES) * stage_words + n * ROW_PITCH) * 4;
             const uint32_t a = base + (uint32_t)((s % STAGES) * stage_words + (BN + mg * MR) * ROW_PITCH) * 4;
-            // the next AHEAD k are on their way from shared memory while these are multiplied
-            Piece p0, p1;
-            p0.load(w, a, 0);
+            if constexpr (BN == 16) {
+                // two CTAs an SM and more cover one another's reads; the registers of reading ahead only cost (16 rows, 6,144 x 1,024: 20.7 us
+                // against 19.6; 9,728 x 2,560: 79.0 / 74.8; 12 rows of 16,384 x 1,024: 46.8 / 43.7)
+                const float* wf = smem + (size_t)(s % STAGES) * stage_words + n * ROW_PITCH;
+                const float* af = smem + (size_t)(s % STAGES) * stage_words + (BN + mg * MR) * ROW_PITCH;
+#pragma unroll 8
+                for (int k = 0; k < ROW_SLAB; k += 4) {
+                    const float4 wv = *reinterpret_cast<const float4*>(wf + k);
+#pragma unroll
+                    for (int r = 0; r < MR; r++) {
+                        const float4 av = *reinterpret_cast<const float4*>(af + r * ROW_PITCH + k);
+                        acc[r] = fmaf(av.x, wv.x, acc[r]);
+                        acc[r] = fmaf(av.y, wv.y, acc[r]);
+                        acc[r] = fmaf(av.z, wv.z, acc[r]);
+                        acc[r] = fmaf(av.w, wv.w, acc[r]);
+                    }
+                }
+            } else {
+                // the next AHEAD k are on their way from shared memory while these are multiplied
+                Piece p0, p1;
+                p0.load(w, a, 0);
 #pragma unroll 1
-            for (int k = 0; k < ROW_SLAB; k += 2 * AHEAD) {
-                p1.load(w, a, k + AHEAD);
-                p0.multiply(acc);
-                p0.load(w, a, min(k + 2 * AHEAD, ROW_SLAB - AHEAD));
-                p1.multiply(acc);
+                for (int k = 0; k < ROW_SLAB; k += 2 * AHEAD) {
+                    p1.load(w, a, k + AHEAD);
+                    p0.multiply(acc);
+                    p0.load(w, a, min(k + 2 * AHEAD, ROW_SLAB - AHEAD));
+                    p1.multiply(acc);
+                }
             }
         }
     }
@@ -341,11 +360,13 @@ MYNAH_API int mynah_gemm_f32(const float* A, const float* W, float* C, int M, in
         return launch_rows_m<8, 6, 128>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     }
     // Tiles of 32 x 32 with 64 threads unless they leave SMs idle (then twice the threads a tile: 40 rows of 1,024 x 3,072 46 us against
-    // 58) or there are many (tiles of 64 x 64 read half as much from L2 and are as fast: 800 rows of 6,144 x 1,024 260 against 264;
-    // 161 rows of 4,096 x 1,024, fewer than five a SM, 69 against 55).
+    // 58) or there are many and a tile of 64 is more than half full (tiles of 64 x 64 read half as much from L2: 800 rows of 6,144 x 1,024 260
+    // against 264, 64 rows of 151,936 x 1,024 477 / 496; 32 rows 466 / 259; 161 rows of 4,096 x 1,024, fewer than five a SM, 69 / 55).
+    // The larger the product the better they stand against the tile of 128 x 128 without reads ahead that they took the place of: rows of
+    // 6,144 x 1,024, us: 500 246 -> 170, 1,024 369 -> 312, 2,048 735 -> 591, 4,000 1,342 -> 1,146.
     const int sms = mynah_sm_count();
     const long long small = ceil_div_ll(M, 32) * ceil_div_ll(N, 32), large = ceil_div_ll(M, 64) * ceil_div_ll(N, 64);
-    if (large >= 5 * sms || ceil_div(M, 32) > GRID_ROWS) return launch_tile<64, 64, 8, 4, 32>(A, W, C, M, N, K, lda, ldw, ldc, stream);
+    if ((large >= 5 * sms && M > 32) || ceil_div(M, 32) > GRID_ROWS) return launch_tile<64, 64, 8, 4, 32>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     if (small <= sms) return launch_tile<32, 32, 4, 2, 64>(A, W, C, M, N, K, lda, ldw, ldc, stream);
     return launch_tile<32, 32, 4, 4, 32>(A, W, C, M, N, K, lda, ldw, ldc, stream);
 }

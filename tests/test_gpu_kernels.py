@@ -134,11 +134,11 @@ def test_gemm_f32_is_true_fp32_and_cut_invariant(M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(1, 1, 4), (1, 1024, 3072), (2, 4096, 1024), (3, 33, 132), (4, 4735, 128), (5, 4736, 260), (13, 18943, 124),
-                                   (16, 18944, 512), (17, 31, 36), (32, 33, 68), (33, 1000, 1024), (65, 4100, 96), (129, 129, 32), (300, 3000, 640),
+                                   (16, 18944, 512), (17, 31, 36), (32, 33, 68), (32, 48000, 68), (33, 48000, 36), (33, 1000, 1024), (65, 4100, 96), (129, 129, 32), (300, 3000, 640),
                                    (512, 4607, 100), (509, 6144, 1024), (1025, 2500, 36),
                                    (8, 3071, 32), (8, 3072, 32), (16, 3072, 36), (16, 9000, 28), (4, 8192, 32), (4, 8193, 32)])
 def test_gemm_f32_kernels_walk_the_same_chain(M, N, K):
-    """Aligned rows take the tiled kernel (all three tiles are among these) and the few-rows kernel, rows at an odd pitch the
+    """Aligned rows take the tiled kernel (both tiles, and 32 rows of many outputs) and the few-rows kernel, rows at an odd pitch the
     general one: the same bits."""
     k = _k()
     g = torch.Generator().manual_seed(M + N + K)
