@@ -117,10 +117,11 @@ attn_decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
         for (int j = 0; j < 8; j++) st.acc[i][j] = 0.f;
     }
 
-    // All keys of a split lie in one page. A warp's keys come a batch at a time, the loads of a batch all in flight before the first
-    // of them is used: with one key after the other a page was sixteen round trips to memory (2 rows behind 160 positions, 16
-    // heads of 128 in fp32: 11.7 -> 8.8 us).
-    constexpr int AHEAD = GT <= 2 ? 4 : GT <= 4 ? 2 : 1;
+    // All keys of a split lie in one page, which is looked up once. In fp32 a warp's keys come in pairs, both keys' loads in flight before
+    // the first is used; more of them cost the registers that let other CTAs cover the wait (8 heads of 64, 32 rows behind 2,000
+    // positions, us one at a time / two / four: fp32 61.6 / 58.4 / 70.6; bfloat16, whose conversions take registers of their own, 67.1 / 73.1 /
+    // 110.3; with the page looked up for every key 63.7 and 75.2. One row behind 500, 16 heads of 128 in fp32: 11.7 / 11.4 / 11.2; 12.2).
+    constexpr int AHEAD = sizeof(T) == 4 ? 2 : 1;
     const int pt_lo = pt.indptr[b], pt_cnt = pt.indptr[b + 1] - pt_lo, lp = key_begin / PAGE_TOKENS - pt.base[b];
     int page = (lp >= 0 && lp < pt_cnt) ? pt.ids[pt_lo + lp] : -1;
     if (page >= pt.n_pages) page = -1;
