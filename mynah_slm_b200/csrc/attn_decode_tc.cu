@@ -1223,12 +1223,19 @@ MYNAH_API int mynah_attn_decode_tc_capped(
     return mynah_check_launch("attn_decode_merge");
 }
 
-// Whether mynah_attn_decode_fused gives a (sequence, kv head) of a step of B sequences and at most `n_splits` pages one CTA: enough of
-// them to fill the SMs with time to spare, since a CTA walks its pages one after the other (8 kv heads, us a step of 28 layers, three launches
-// or a CTA a page -> this: 20 rows behind 180 positions 1,232 -> 1,286, 32 rows 1,360 -> 1,311, 64 rows 1,498 -> 1,406; 20 rows
-// of 16 kv heads of 64 behind 100, 16 layers, 945 -> 858).
-MYNAH_API int mynah_attn_decode_short(int B, int KV, int n_splits) {
-    return n_splits <= SHORT_PAGES && 2ll * B * KV >= 3ll * mynah_sm_count();
+// Whether mynah_attn_decode_fused gives a (sequence, kv head) of a step of B sequences and at most `n_splits` pages one CTA. It walks its pages
+// one after the other, so either the step has CTAs enough to cover that (three an SM), or the pages are one, or a group of eight
+// heads and more makes its preparation the larger part, which a CTA a page repeats; and with one head a group, where there is little to
+// prepare, the CTAs must all run side by side (five an SM). us a layer, a CTA a page or three launches -> this: 28 rows of 8 kv heads of 128, 250
+// positions: groups of 1, 2, 4 11.9, 12.2, 12.9 -> 13.9, 14.2, 13.9, groups of 8 of 64 13.6 -> 11.9; 32 rows, one page, groups of 2 9.1 -> 8.8;
+// 64 rows, 250 positions, groups of 1, 2, 4, 8 20.4, 20.7, 22.8, 23.1 -> 18.4, 18.7, 19.0, 14.6; 64 rows of 16 kv heads of 64, groups of 1,
+// one page 10.2 -> 13.2; 250 rows of 8, 100 positions, groups of 1, 2, 4 35.4, 39.2, 46.7 -> 35.7, 35.8, 36.4.
+MYNAH_API int mynah_attn_decode_short(int B, int H, int KV, int n_splits) {
+    if (n_splits > SHORT_PAGES || KV <= 0) return 0;
+    const long long ctas = (long long)B * KV, sms = mynah_sm_count();
+    const int G = H / KV;
+    if (2 * ctas < 3 * sms || (G == 1 && ctas > 5 * sms)) return 0;
+    return n_splits == 1 || G >= 8 || ctas >= 3 * sms;
 }
 
 // The fused decode attention: q, k, v rows [B, (H + 2 KV) * HD] as the projection left them (with write_kv = 0
@@ -1257,7 +1264,7 @@ MYNAH_API int mynah_attn_decode_fused(
     float* part_o = scratch;
     float* part_ml = scratch + (size_t)B * H * n_splits * HD;
     const VecRef qg{q_gain, gain_dtype}, kg{k_gain, gain_dtype};
-    if (mynah_attn_decode_short(B, KV, n_splits)) {
+    if (mynah_attn_decode_short(B, H, KV, n_splits)) {
         const size_t o_bytes = (size_t)n_splits * (H / KV) * HD * sizeof(float);
         auto kern = HD == 128 ? attn_decode_short_kernel<128> : attn_decode_short_kernel<64>;
         const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SHORT_PAGES * MAX_G * 128 * (int)sizeof(float));

@@ -54,7 +54,7 @@ def decode_fused_ok(dtype: torch.dtype, H: int, KV: int, HD: int, rotary_dim: in
     of the whole head or none, and few enough CTAs, or many sequences of few pages (a CTA a sequence's kv head then)."""
     if not kernels.attn_decode_tc_supported(dtype, H, KV, HD):
         return False
-    if B * KV * n_splits > FUSED_DECODE_MAX_CTAS and not FUSED_PREP_LARGE and not kernels.attn_decode_short(B, KV, n_splits):
+    if B * KV * n_splits > FUSED_DECODE_MAX_CTAS and not FUSED_PREP_LARGE and not kernels.attn_decode_short(B, H, KV, n_splits):
         return False
     return _tc_fits(H, KV, n_splits) and (cos is None or rotary_dim == HD)
 

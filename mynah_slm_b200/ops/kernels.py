@@ -478,9 +478,9 @@ def attn_decode_fused(qkv: torch.Tensor, out: torch.Tensor, B: int, H: int, KV: 
          window or 0, n_splits, ptr(scratch), ptr(counters), ptr(status), stream_ptr())
 
 
-def attn_decode_short(B: int, KV: int, n_splits: int) -> bool:
+def attn_decode_short(B: int, H: int, KV: int, n_splits: int) -> bool:
     """Whether the one-launch decode attention gives a (sequence, kv head) one CTA (csrc/attn_decode_tc.cu)."""
-    return bool(lib.load().mynah_attn_decode_short(B, KV, n_splits))
+    return bool(lib.load().mynah_attn_decode_short(B, H, KV, n_splits))
 
 
 def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:

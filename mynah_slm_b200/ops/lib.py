@@ -199,7 +199,7 @@ def load() -> ctypes.CDLL:
     lib.mynah_gemm_tcgen05_splits_k.restype = c_int
     lib.mynah_gemm_tcgen05_splits_k.argtypes = [c_int, c_int, c_int, c_int]
     lib.mynah_attn_decode_short.restype = c_int
-    lib.mynah_attn_decode_short.argtypes = [c_int, c_int, c_int]
+    lib.mynah_attn_decode_short.argtypes = [c_int, c_int, c_int, c_int]
     lib.mynah_gemv_decode_supported.restype = c_int
     lib.mynah_gemv_decode_supported.argtypes = [c_int, c_int, c_int]
     for name in ("mynah_moe_plain", "mynah_retention_chunk_min", "mynah_head_linear_plain", "mynah_moe_grouped_min",

@@ -14,9 +14,12 @@ def test_short_sequences_have_the_bits_of_the_separate_launches(H, KV, HD, windo
     """Lengths at a page's first and last row, of one page to four, padding rows, rows behind the last position no numbers."""
     from mynah_slm_b200.ops import kernels as k
     g = torch.Generator(device=DEV).manual_seed(H + KV)
-    B = 240 // KV + 8
+    B = 480 // KV + 8
     lens = [[1, 64, 65, 128, 0, 129, 192, 193, 256, 37][b % 10] for b in range(B)]
-    assert k.attn_decode_short(B, KV, 4) and not k.attn_decode_short(B, KV, 5) and not k.attn_decode_short(8, 8, 4)
+    assert k.attn_decode_short(B, H, KV, 4) and not k.attn_decode_short(B, H, KV, 5) and not k.attn_decode_short(8, 8, 8, 4)
+    # where a CTA a page or three launches are the faster form (figures at the rule)
+    assert not k.attn_decode_short(28, 16, 8, 3) and not k.attn_decode_short(64, 16, 16, 1) and not k.attn_decode_short(250, 8, 8, 4)
+    assert k.attn_decode_short(28, 16, 8, 1) and k.attn_decode_short(28, 64, 8, 4) and k.attn_decode_short(250, 16, 8, 4)
     indptr, ids = [0], []
     for n in lens:
         ids += list(range(len(ids), len(ids) + -(-n // 64)))
