@@ -633,7 +633,7 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
             }
         }
     };
-    if (row_in_shared && (ld & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {   // (begin is a multiple of 4)
+    if ((ld & 3) == 0 && (reinterpret_cast<uintptr_t>(logits) & 15) == 0) {   // (begin is a multiple of 4)
         constexpr int LOADS4 = 5;
         const int n4 = rs.n / 4;
         const float4* from4 = reinterpret_cast<const float4*>(from);
@@ -642,7 +642,7 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
 #pragma unroll
             for (int u = 0; u < LOADS4; u++) {
                 const int j = base0 + u * THREADS + (int)threadIdx.x;
-                if (j < n4) v[u] = __ldcs(from4 + j);
+                if (j < n4) v[u] = row_in_shared ? __ldcs(from4 + j) : from4[j];
             }
 #pragma unroll
             for (int u = 0; u < LOADS4; u++) {
@@ -653,13 +653,14 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
                     take_first_max(bv, bi, v[u].y, i + 1);
                     take_first_max(bv, bi, v[u].z, i + 2);
                     take_first_max(bv, bi, v[u].w, i + 3);
-                    reinterpret_cast<float4*>(rs.p)[j] = v[u];
+                    if (row_in_shared) reinterpret_cast<float4*>(rs.p)[j] = v[u];
                 }
             }
         }
         for (int i = 4 * n4 + (int)threadIdx.x; i < rs.n; i += THREADS) {
-            rs.p[i] = from[i];
-            take_first_max(bv, bi, rs.p[i], rs.begin + i);
+            const float x = from[i];
+            if (row_in_shared) rs.p[i] = x;
+            take_first_max(bv, bi, x, rs.begin + i);
         }
     } else {
         scan(from, row_in_shared != 0);
@@ -816,9 +817,18 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
         id = draw_from_keys<NC>(sh, listed, sp, p_best, u);
     } else if (small_k) {
         // One pass over the probabilities (the stored exponentials times inv) finds the leading eleven bits of the k-th
-        // largest. Everything with those bits or larger ones holds the k largest; when that is a short list it is gathered.
-        const Found lead = find_digit<NC>(rs, add_up<NC>(rs, FIRST_DIGIT, inv, sh), false, (unsigned int)sp.top_k, 0ull, 0u, 0ull, sh);
-        const bool short_list = lead.above + lead.count <= (unsigned int)MAX_CAND;      // the same in every CTA of the row
+        // largest, a second one, where those leave a long list, eleven more. Everything with those bits or larger ones holds the k
+        // largest; when that is a short list it is gathered.
+        Found lead = find_digit<NC>(rs, add_up<NC>(rs, FIRST_DIGIT, inv, sh), false, (unsigned int)sp.top_k, 0ull, 0u, 0ull, sh);
+        unsigned int lead_bits = lead.digit;
+        int lead_shift = FIRST_DIGIT.shift;
+        if (lead.above + lead.count > (unsigned int)MAX_CAND) {                         // the same in every CTA of the row
+            const Digit next{lead.digit << 21, 2047u << 21, 10, 2048};
+            lead = find_digit<NC>(rs, add_up<NC>(rs, next, inv, sh), false, (unsigned int)sp.top_k, 0ull, lead.above, lead.mass, sh);
+            lead_bits = lead_bits << 11 | lead.digit;
+            lead_shift = next.shift;
+        }
+        const bool short_list = lead.above + lead.count <= (unsigned int)MAX_CAND;
         Prefix topk{0u, 0u, 0u, 0ull};
         int id_bound = -1;
         float gather_scale = inv;
@@ -833,7 +843,7 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
         unsigned long long* keys = rs.at(&sh.key[0], 0);
         for (int i = threadIdx.x; i < rs.n; i += THREADS) {
             const unsigned int bits = __float_as_uint(rs.p[i] * gather_scale);    // probabilities are not negative: bits order as values
-            const bool take = short_list ? (bits >> 21) >= lead.digit : (bits > topk.value || (bits == topk.value && rs.begin + i <= id_bound));
+            const bool take = short_list ? (bits >> lead_shift) >= lead_bits : (bits > topk.value || (bits == topk.value && rs.begin + i <= id_bound));
             if (take) {
                 const unsigned int at = atomicAdd(cnt, 1u);
                 if (at < (unsigned int)MAX_CAND) keys[at] = ((unsigned long long)bits << 32) | (0xffffffffu - (unsigned int)(rs.begin + i));
@@ -996,11 +1006,13 @@ MYNAH_API int mynah_sample(float* logits, int B, int V, int ld, const float* par
                       && (ring == nullptr || (stride > 0 && stride <= 256)), "sample: bad ring");
     const Ring rings{ring, ring_n, ring_head, stride};
     // A cluster a row from this vocabulary size on (see the kernel), whatever the batch: a row's draw does not depend on its
-    // company. A row that does not fit its CTAs' shared memory stays where it is.
+    // company. A row stays where it is when its CTAs' shared memory cannot hold it, or when it would leave an SM to one CTA while the step has
+    // more CTAs than SMs (262,144 logits, us a draw from shared memory / where they are: 8 rows top-k 20 23 / 25, top-p 116 / 132; 32 rows
+    // 62 / 40 and 338 / 203; 256 rows greedy 204 / 155, top-k 20 412 / 315, top-p 2,076 / 1,560).
     const bool cluster = V >= ROW_CTAS * 4096;
     const size_t own = cluster ? sizeof(Shared<ROW_CTAS>) : sizeof(Shared<1>);
     const size_t part = sizeof(float) * (size_t)(cluster ? ((V + ROW_CTAS - 1) / ROW_CTAS + 3) & ~3 : V);
-    const int in_shared = own + part <= 227 * 1024;
+    const int in_shared = own + part <= 113 * 1024 || (own + part <= 227 * 1024 && B * (cluster ? ROW_CTAS : 1) <= mynah_sm_count());
     const size_t smem = own + (in_shared ? part : 0);
     auto kernel = cluster ? sample_kernel<ROW_CTAS> : sample_kernel<1>;
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);

@@ -19,6 +19,10 @@ def _rows(rng, V, kind):
     elif kind == "masked":                                 # fewer finite logits than places
         lg[:, 7:] = -np.inf
         lg[2, V - 1] = 3.0
+    elif kind == "crowd":                                  # 400 of the largest probabilities share their leading eleven bits
+        lg = np.minimum(lg, 2.0)
+        for b in range(4):
+            lg[b, rng.permutation(V)[:400]] = 9.0 + 2e-4 * rng.permutation(400)
     elif kind == "sharp":                                  # all but a few exponentials vanish
         lg *= 40.0
     return lg
@@ -26,7 +30,7 @@ def _rows(rng, V, kind):
 
 @pytest.mark.parametrize("V,kind", [(300, "plain"), (32767, "plain"), (32768, "plain"), (65541, "plain"), (32771, "equal"),
                                     (40000, "equal"), (1003, "equal"), (50000, "masked"), (900, "masked"), (33000, "sharp"),
-                                    (400001, "plain"), (60000, "plain")])
+                                    (400001, "plain"), (60000, "plain"), (400004, "plain"), (5000, "crowd"), (40000, "crowd")])
 @pytest.mark.parametrize("temp,top_k,top_p,min_p", [(0.6, 20, 0.95, 0.0), (1.0, 128, 0.9, 0.0), (1.0, 129, 1.0, 0.0),
                                                     (0.8, 0, 0.9, 0.0), (1.0, 0, 1.0, 0.1), (0.9, 257, 1.0, 0.0), (0.0, 20, 1.0, 0.0)])
 def test_routes_match_plain_sampler(V, kind, temp, top_k, top_p, min_p):
@@ -42,6 +46,20 @@ def test_routes_match_plain_sampler(V, kind, temp, top_k, top_p, min_p):
             want = [p.sample(lg[b].copy()) for b, p in enumerate(plain)]
         got = kernels.sample(torch.from_numpy(lg.copy()).to(DEV), params, state, None).cpu().tolist()
         assert got == want
+
+
+@pytest.mark.parametrize("V,rows", [(30000, 160), (200003, 24)])
+def test_many_rows_draw_as_few_do(V, rows):
+    """Steps of more CTAs than SMs leave long rows where they are, small ones take them into shared memory: the same tokens."""
+    from mynah_slm_b200.ops import kernels
+    lg = torch.randn((rows, V), generator=torch.Generator(device=DEV).manual_seed(V), device=DEV) * 2.0
+    for temp, top_k in ((0.0, 0), (0.9, 20), (0.9, 200), (1.0, 0)):
+        params = torch.tensor([temp, 0.9, 0.0, float(top_k), 1.0, 0.0, 0.0, 0.0], dtype=torch.float32, device=DEV)
+        many, few = (torch.arange(5, 5 + rows, dtype=torch.int64, device=DEV) for _ in range(2))
+        got = kernels.sample(lg.clone(), params, many, None)
+        for at in range(0, rows, 6):
+            assert torch.equal(kernels.sample(lg[at:at + 6].clone(), params, few[at:at + 6], None), got[at:at + 6])
+        assert torch.equal(many, few)
 
 
 @pytest.mark.parametrize("V", [500, 40002])
