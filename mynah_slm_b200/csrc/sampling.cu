@@ -930,46 +930,6 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
     }
 }
 
-// One thread per row: the reference's loop over the ring of recent tokens,
-// entry by entry (a token that sits in the ring c times is penalised c times).
-// The ring rows are `stride` apart; the window in use is params[7] <= stride.
-__global__ void penalties_kernel(float* __restrict__ logits, int B, int V, int ld, const int* __restrict__ ring,
-                                 const int* __restrict__ ring_n, int stride, const int* __restrict__ slots,
-                                 const float* __restrict__ params) {
-    griddep_launch();
-    griddep_wait();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const float repeat = params[4], freq = params[5], presence = params[6];
-    const int window = min((int)params[7], stride);
-    if (window <= 0 || (repeat == 1.0f && freq == 0.0f && presence == 0.0f)) return;   // sampler.c:81-84
-    const int slot = slots ? slots[b] : b;
-    if (slot < 0) return;
-    const int n = min(ring_n[slot], window);
-    const int* r = ring + (size_t)slot * stride;
-    float* row = logits + (size_t)b * ld;
-    for (int i = 0; i < n; i++) {
-        const int tok = r[i];
-        if (tok < 0 || tok >= V) continue;
-        int count = 0;
-        for (int k = 0; k < n; k++) count += r[k] == tok;
-        row[tok] = penalise(row[tok], repeat, freq, presence, count);
-    }
-}
-
-__global__ void accept_kernel(const int* __restrict__ tokens, int B, int* __restrict__ ring, int* __restrict__ ring_n,
-                              int* __restrict__ ring_head, int stride, const int* __restrict__ slots,
-                              const float* __restrict__ params) {
-    griddep_launch();
-    griddep_wait();
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    const int window = min((int)params[7], stride);
-    if (b >= B || window <= 0) return;
-    const int slot = slots ? slots[b] : b;
-    if (slot < 0) return;
-    accept_token(Ring{ring, ring_n, ring_head, stride}, slot, window, tokens[b]);
-}
-
 __global__ void __launch_bounds__(ARGMAX_THREADS)
 argmax_kernel(const float* __restrict__ logits, int V, int ld, int* __restrict__ out) {
     __shared__ ArgmaxShared sh;
@@ -1038,13 +998,6 @@ MYNAH_API int mynah_sample(float* logits, int B, int V, int ld, const float* par
     return mynah_check_launch("sample");
 }
 
-MYNAH_API int mynah_apply_penalties(float* logits, int B, int V, int ld, const int* ring, const int* ring_n,
-                                    int window, const int* slots, const float* params, cudaStream_t stream) {
-    if (B == 0 || window == 0) return 0;
-    mynah_launch(penalties_kernel, dim3(ceil_div(B, 64)), dim3(64), 0, stream, logits, B, V, ld, ring, ring_n, window, slots, params);
-    return mynah_check_launch("apply_penalties");
-}
-
 namespace {
 // After a sampled decode step: the sampled token becomes the sequence's next
 // input, one position further on.
@@ -1066,11 +1019,4 @@ MYNAH_API int mynah_decode_advance(int* tokens, const int* sampled, int* tok_pos
     if (B == 0) return 0;
     mynah_launch(decode_advance_kernel, dim3(ceil_div(B, 64)), dim3(64), 0, stream, tokens, sampled, tok_pos, kv_len, slots, B);
     return mynah_check_launch("decode_advance");
-}
-
-MYNAH_API int mynah_sampler_accept(const int* tokens, int B, int* ring, int* ring_n, int* ring_head, int window,
-                                   const int* slots, const float* params, cudaStream_t stream) {
-    if (B == 0 || window == 0) return 0;
-    mynah_launch(accept_kernel, dim3(ceil_div(B, 64)), dim3(64), 0, stream, tokens, B, ring, ring_n, ring_head, window, slots, params);
-    return mynah_check_launch("sampler_accept");
 }

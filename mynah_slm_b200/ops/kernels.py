@@ -497,7 +497,7 @@ def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots:
     """One launch. May overwrite `logits`. params: float32 [7] on the device (temp, top_p,
     min_p, top_k, repeat, freq, presence; with `ring` an eighth, the window in use); rng: int64 generator state per slot.
     `ring` = (tokens [slots, stride], counts, heads), int32: the penalties are taken from it before the draw and the drawn
-    token goes into it, as `apply_penalties` and `sampler_accept` would do."""
+    token goes into it."""
     _chk(logits, "logits", torch.float32, 2)
     _chk(rng, "rng states", torch.int64, 1)
     _chk(params, "sampling parameters", torch.float32, 1)
@@ -510,22 +510,6 @@ def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots:
     call("mynah_sample", ptr(logits), B, V, V, ptr(params), ptr(rng), ptr(slots), ptr(out), ptr(tokens), ptr(counts), ptr(heads),
          tokens.shape[1] if ring is not None else 0, stream_ptr())
     return out
-
-
-def apply_penalties(logits: torch.Tensor, ring: torch.Tensor, ring_n: torch.Tensor, slots: Optional[torch.Tensor],
-                    params: torch.Tensor) -> None:
-    _chk(logits, "logits", torch.float32, 2)
-    _chk(ring, "ring", torch.int32, 2)
-    B, V = logits.shape
-    call("mynah_apply_penalties", ptr(logits), B, V, V, ptr(ring), ptr(ring_n), ring.shape[1], ptr(slots),
-         ptr(params), stream_ptr())
-
-
-def sampler_accept(tokens: torch.Tensor, ring: torch.Tensor, ring_n: torch.Tensor, ring_head: torch.Tensor,
-                   slots: Optional[torch.Tensor], params: torch.Tensor) -> None:
-    _chk(tokens, "tokens", torch.int32, 1)
-    call("mynah_sampler_accept", ptr(tokens), tokens.numel(), ptr(ring), ptr(ring_n), ptr(ring_head),
-         ring.shape[1], ptr(slots), ptr(params), stream_ptr())
 
 
 def decode_advance(tokens: torch.Tensor, sampled: torch.Tensor, tok_pos: torch.Tensor, kv_len: torch.Tensor,

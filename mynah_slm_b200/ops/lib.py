@@ -81,9 +81,7 @@ _SIGNATURES: dict[str, list] = {
     "mynah_set_pdl": [c_int],
     "mynah_gemm_tcgen05_reset": [P],
     "mynah_sample": [P, c_int, c_int, c_int, P, P, P, P, P, P, P, c_int, P],
-    "mynah_apply_penalties": [P, c_int, c_int, c_int, P, P, c_int, P, P, P],
     "mynah_decode_advance": [P, P, P, P, P, c_int, P],
-    "mynah_sampler_accept": [P, c_int, P, P, P, c_int, P, P, P],
     "mynah_l2_prefetch": [P, P, c_int, P],
     "mynah_attn_prefill_tcgen05_stages": [c_int],
     "mynah_wait_probe": [P, P, ctypes.c_ulonglong, P],

@@ -437,6 +437,7 @@ def test_sample_padding_rows_and_slot_mapping():
 
 
 def test_penalties_and_ring_match_plain():
+    """Greedy draws with penalties from a ring: the penalised logits, the drawn tokens and what the ring then holds."""
     k = _k()
     rng = np.random.default_rng(13)
     V, W, stride, B = 300, 5, 8, 3
@@ -444,21 +445,23 @@ def test_penalties_and_ring_match_plain():
     ring = torch.zeros((B, stride), dtype=torch.int32, device=DEV)
     ring_n = torch.zeros(B, dtype=torch.int32, device=DEV)
     ring_head = torch.zeros(B, dtype=torch.int32, device=DEV)
+    state = torch.zeros(B, dtype=torch.int64, device=DEV)
     params = torch.tensor([0.0, 1.0, 0.0, 0.0, 1.3, 0.2, 0.1, float(W)], dtype=torch.float32, device=DEV)
     slots = torch.arange(B, dtype=torch.int32, device=DEV)
     for step in range(12):
-        toks = rng.integers(0, 6, size=B).astype(np.int32)                           # few ids: repeats inside the window
-        for b in range(B):
-            plain[b].accept(int(toks[b]))
-        k.sampler_accept(torch.from_numpy(toks).to(DEV), ring, ring_n, ring_head, slots, params)
         lg = rng.standard_normal((B, V)).astype(np.float32)
+        lg[:, :6] += 5.0                                                             # few ids: repeats inside the window
         ref = lg.copy()
         for b in range(B):
             plain[b].apply_penalties(ref[b])
         d = torch.from_numpy(lg.copy()).to(DEV)
-        k.apply_penalties(d, ring, ring_n, slots, params)
+        got = k.sample(d, params, state, slots, ring=(ring, ring_n, ring_head)).cpu().tolist()
         assert np.allclose(d.cpu().numpy(), ref, rtol=1e-6, atol=1e-6), step
-    assert ring_n.cpu().tolist() == [W] * B
+        assert got == ref.argmax(axis=1).tolist(), step
+        for b in range(B):
+            plain[b].accept(got[b])
+        assert ring_n.cpu().tolist() == [min(step + 1, W)] * B
+    assert ring_head.cpu().tolist() == [12 % W] * B
 
 
 def test_refusals_are_errors_not_wrong_results():
