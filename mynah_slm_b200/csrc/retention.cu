@@ -338,7 +338,6 @@ __device__ __forceinline__ float2 unpack2(f32x2 v) {
     return r;
 }
 __device__ __forceinline__ void fma2(f32x2& c, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
-__device__ __forceinline__ void mul2(f32x2& c, f32x2 a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
 
 struct alignas(16) Pairs { f32x2 lo, hi; };                 // four floats as two pairs, one 16-byte load
 __device__ __forceinline__ Pairs pairs_at(const float* p) { return *reinterpret_cast<const Pairs*>(p); }
@@ -557,7 +556,7 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
 #pragma unroll
         for (int w = 0; w < G; w++) acc[u][w][0] = acc[u][w][1] = 0ull;
     // one product's four steps of k: rows [ty * RT, + RT) of `lhs` from column i, rows [i, i + 4) of `rhs`
-    auto steps = [&](const float* lhs, int ld, const float* rhs) {
+    auto steps = [&](const float* lhs, int ld, const float* rhs, f32x2 (&acc)[RT][G][2]) {
         float4 x[RT];
 #pragma unroll
         for (int u = 0; u < RT; u++) x[u] = *reinterpret_cast<const float4*>(lhs + (ty * RT + u) * ld);
@@ -599,32 +598,31 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
         __syncthreads();
         const float* S = xs + (p & 1) * SR * JT;
 #pragma unroll 2
-        for (int i = 0; i < SR; i += 4) steps(qs + p * SR + i, ldr, S + i * JT);
+        for (int i = 0; i < SR; i += 4) steps(qs + p * SR + i, ldr, S + i * JT, acc);
         __syncthreads();                                    // the piece's place may be filled again
     }
-#pragma unroll
-    for (int u = 0; u < RT; u++) {
-        const float gt = gp[ty * RT + u + 1];
-#pragma unroll
-        for (int w = 0; w < G; w++) {
-            mul2(acc[u][w][0], pack2(gt, gt));
-            mul2(acc[u][w][1], pack2(gt, gt));
-        }
-    }
-    // ---- scores times values
+    // ---- scores times values, summed apart from the state's part: the roundings of a sum are of its own size
     stage_values<T, C, JT>(xs, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd, nt, [](int) { return 1.f; });
     __syncthreads();
     const int s_end = ((ty | 1) + 1) * RT;                  // keys behind the last token of the warp's rows weigh nothing
-    for (int s = 0; s < s_end; s += 4) steps(Ws + s, LDW, xs + s * JT);
+    f32x2 within[RT][G][2];
+#pragma unroll
+    for (int u = 0; u < RT; u++)
+#pragma unroll
+        for (int w = 0; w < G; w++) within[u][w][0] = within[u][w][1] = 0ull;
+    for (int s = 0; s < s_end; s += 4) steps(Ws + s, LDW, xs + s * JT, within);
 #pragma unroll
     for (int u = 0; u < RT; u++) {
         const int t = ty * RT + u;
         if (t >= nt) break;
+        const f32x2 gt = pack2(gp[t + 1], gp[t + 1]);
         float* row = o + (size_t)(t0 + t) * a.H * a.vd + (size_t)h * a.vd;
 #pragma unroll
         for (int w = 0; w < G; w++) {
             const int j = j0 + w * 64 + tx * 4;
-            const float2 x = unpack2(acc[u][w][0]), y = unpack2(acc[u][w][1]);
+            fma2(within[u][w][0], gt, acc[u][w][0]);
+            fma2(within[u][w][1], gt, acc[u][w][1]);
+            const float2 x = unpack2(within[u][w][0]), y = unpack2(within[u][w][1]);
             if (j + 3 < a.vd && (a.vd & 3) == 0) {
                 *reinterpret_cast<float4*>(row + j) = make_float4(x.x, x.y, y.x, y.y);
             } else {
