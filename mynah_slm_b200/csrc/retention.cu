@@ -11,11 +11,12 @@
 //                    head of one sequence; a column's dim values lie in the registers of L adjacent lanes (up to
 //                    32 values a lane), which add their parts of o by shuffles in a fixed order. Keys, queries and
 //                    values of 32 tokens at a time pass through shared memory.
-//   retention_local, _states, _out   the same recurrence for prompts, a chunk of tokens at a time (see below)
+//   retention_local, _states, _out   the same recurrence for pieces of 16 tokens and more, a chunk of tokens at a time (see below)
 //   retention_step   all of a decode step's row behind its projection, the RMS and the gate with it (see below)
 //
-// All arithmetic is fp32. A sequence's rows are walked in order, so a prompt run whole, in pieces or token by
-// token performs the same operations in the same order.
+// All arithmetic is fp32. Which form a sequence's rows take depends on their number alone, so a step's rows have the same bits in any
+// company. Token by token the rows are walked in order, whatever pieces they come in; chunk by chunk the sums run in another
+// order (the forms agree to rounding), so a prompt run whole and the same prompt in pieces differ by roundings.
 #include "layout.cuh"
 
 namespace {
@@ -138,29 +139,30 @@ struct RetArgs {
     int L, per;                            // lanes a column (a power of two <= 32), values a lane (<= RET_RMAX)
 };
 
-template <typename T>
-__global__ void __launch_bounds__(RET_THREADS)
-retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v,
-                      const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ o,
-                      const int* __restrict__ cu_q, const int* __restrict__ slots, RetArgs a) {
-    extern __shared__ float sm[];
-    griddep_wait();
-    const int b = blockIdx.z, h = blockIdx.y;
-    const int slot = slots[b];
-    const int q0 = cu_q[b], q1 = cu_q[b + 1];
-    if (slot < 0 || slot >= a.n_slots || q1 <= q0) return;
+// Rows [q0, q1) of one sequence and head, columns [j0, j0 + THREADS / L), by a CTA of THREADS threads that stages TB tokens at a time in
+// `sm` (walk_floats). A column's arithmetic does not depend on THREADS or TB.
+__host__ __device__ constexpr size_t walk_floats(int threads, int tb, int L, int per) {
+    return (size_t)2 * tb * (per + 1) * L + (size_t)tb * (threads / L);
+}
+template <typename T, int THREADS, int TB>
+__device__ __forceinline__ void walk_tokens(float* sm, const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v,
+                                            float g, float* __restrict__ state, float* __restrict__ o, int q0, int q1, int slot, int h, int j0,
+                                            const RetArgs& a) {
+    qn += (size_t)h * a.dim;
+    kn += (size_t)h * a.dim;
+    v += a.v_off + (size_t)h * a.vd;
+    o += (size_t)h * a.vd;
     const int L = a.L, per = a.per;
-    const int JT = RET_THREADS / L;
+    const int JT = THREADS / L;
     const int l = threadIdx.x % L, jl = threadIdx.x / L;
-    const int j = blockIdx.x * JT + jl;
+    const int j = j0 + jl;
     const bool on = j < a.vd;
     const int CS = per + 1;                                      // floats of a lane's chunk (padded against bank conflicts)
     const int rowf = CS * L;
     float* ks = sm;                                              // [TB][rowf]
-    float* qs = ks + RET_TB * rowf;                              // [TB][rowf]
-    float* vs = qs + RET_TB * rowf;                              // [TB][JT]
-    for (int i = threadIdx.x; i < 2 * RET_TB * rowf; i += RET_THREADS) ks[i] = 0.f;    // slots beyond dim stay zero
-    const float g = decay[h];
+    float* qs = ks + TB * rowf;                                  // [TB][rowf]
+    float* vs = qs + TB * rowf;                                  // [TB][JT]
+    for (int i = threadIdx.x; i < 2 * TB * rowf; i += THREADS) ks[i] = 0.f;    // slots beyond dim stay zero
     float S[RET_RMAX];
     float* sp = state + (((size_t)slot * a.H + h) * a.dim) * a.vd;
 #pragma unroll
@@ -169,20 +171,19 @@ retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn
         S[r] = (on && r < per && i < a.dim) ? sp[(size_t)i * a.vd + j] : 0.f;
     }
     const int n = a.H * a.dim;
-    for (int t0 = q0; t0 < q1; t0 += RET_TB) {
-        const int nt = min(RET_TB, q1 - t0);
+    for (int t0 = q0; t0 < q1; t0 += TB) {
+        const int nt = min(TB, q1 - t0);
         __syncthreads();
-        for (int idx = threadIdx.x; idx < nt * a.dim; idx += RET_THREADS) {
+        for (int idx = threadIdx.x; idx < nt * a.dim; idx += THREADS) {
             const int tt = idx / a.dim, i = idx % a.dim;
-            const size_t src = (size_t)(t0 + tt) * n + (size_t)h * a.dim + i;
+            const size_t src = (size_t)(t0 + tt) * n + i;
             const int dst = tt * rowf + (i / per) * CS + i % per;
             ks[dst] = kn[src];
             qs[dst] = qn[src];
         }
-        for (int idx = threadIdx.x; idx < nt * JT; idx += RET_THREADS) {
+        for (int idx = threadIdx.x; idx < nt * JT; idx += THREADS) {
             const int tt = idx / JT, c = idx % JT;
-            const int col = blockIdx.x * JT + c;
-            vs[idx] = col < a.vd ? to_f32(v[(size_t)(t0 + tt) * a.ldv + a.v_off + (size_t)h * a.vd + col]) : 0.f;
+            vs[idx] = j0 + c < a.vd ? to_f32(v[(size_t)(t0 + tt) * a.ldv + j0 + c]) : 0.f;
         }
         __syncthreads();
         for (int tt = 0; tt < nt; tt++) {
@@ -198,7 +199,7 @@ retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn
                 }
             }
             for (int m = 1; m < L; m <<= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
-            if (on && l == 0) o[(size_t)(t0 + tt) * a.H * a.vd + (size_t)h * a.vd + j] = acc;
+            if (on && l == 0) o[(size_t)(t0 + tt) * a.H * a.vd + j] = acc;
         }
     }
     if (on) {
@@ -208,6 +209,20 @@ retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn
             if (r < per && i < a.dim) sp[(size_t)i * a.vd + j] = S[r];
         }
     }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(RET_THREADS)
+retention_scan_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v,
+                      const float* __restrict__ decay, float* __restrict__ state, float* __restrict__ o,
+                      const int* __restrict__ cu_q, const int* __restrict__ slots, RetArgs a) {
+    extern __shared__ float scan_sm[];
+    griddep_wait();
+    const int b = blockIdx.z, h = blockIdx.y;
+    const int slot = slots[b];
+    const int q0 = cu_q[b], q1 = cu_q[b + 1];
+    if (slot < 0 || slot >= a.n_slots || q1 <= q0) return;
+    walk_tokens<T, RET_THREADS, RET_TB>(scan_sm, qn, kn, v, decay[h], state, o, q0, q1, slot, h, blockIdx.x * (RET_THREADS / a.L), a);
 }
 
 // ---- a decode step: preparation, one token of the recurrence, the unit RMS and the gate ----
@@ -317,13 +332,23 @@ retention_step_kernel(const T* __restrict__ p, const float* __restrict__ cos_t, 
 // (what the cache holds), in the order of their sequences. Measured (3,837 tokens of 4 sequences,
 // 16 heads of 128), us a layer: 85 + 46 + 137; a chain of CTAs that each walked a head's 32 columns through its chunks took 625.
 //
+// Sequences of fewer than 16 rows in such a step are walked token by token, by the CTAs of retention_out that have their rows: a
+// decode row beside a prompt costs a row's work, and has the bits it has among its like.
+//
+// Where no sequence has more than one chunk nothing is a chain: retention_out reads the old state from its slot and leaves the
+// new one there, one launch instead of three. us with the preparation and the gated norm, 16 heads of 128: one sequence of 20, 48,
+// 64 rows 36.2, 40.3, 42.4 -> 23.4, 28.5, 31.1; 16 of 32 83 -> 41; 64 of 40 424 -> 175; a prompt of 70 beside 60 decode rows 322 -> 103.
+//
 // The powers of g come from a table made by repeated multiplication. Sums run in another order than token by token:
 // the two forms agree to rounding.
 constexpr int RC_THREADS = 256;
+constexpr int WALK_TB = 16;                                 // tokens staged at a time where the chunks' CTAs walk a short sequence
 
 struct RetChunkArgs {
     int H, dim, vd, n_slots, ldv, v_off, B, cols;          // cols: columns of a state in scratch (vd padded to whole tiles)
     int first;                                              // the pass's first chunk
+    int least;                                              // rows from which a sequence goes chunk by chunk
+    RetArgs walk;                                           // shorter ones are walked token by token
 };
 
 typedef unsigned long long f32x2;
@@ -338,6 +363,7 @@ __device__ __forceinline__ float2 unpack2(f32x2 v) {
     return r;
 }
 __device__ __forceinline__ void fma2(f32x2& c, f32x2 a, f32x2 b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ void mul2(f32x2& c, f32x2 a) { asm("mul.rn.f32x2 %0, %0, %1;" : "+l"(c) : "l"(a)); }
 
 struct alignas(16) Pairs { f32x2 lo, hi; };                 // four floats as two pairs, one 16-byte load
 __device__ __forceinline__ Pairs pairs_at(const float* p) { return *reinterpret_cast<const Pairs*>(p); }
@@ -376,6 +402,37 @@ __device__ __forceinline__ void stage_values(float* vs, const T* __restrict__ v,
     }
 }
 
+// A thread's part of U from a chunk's keys (rows ldk apart) and values in shared memory: eight state rows, four columns of either half
+// of the tile. WEIGH: the values are yet to be multiplied by the powers of the decay.
+template <int JT, bool WEIGH>
+__device__ __forceinline__ void chunk_update(const float* kr, int ldk, const float* vr, int nt, const float* gp, f32x2 (&acc)[8][4]) {
+#pragma unroll
+    for (int u = 0; u < 8; u++)
+#pragma unroll
+        for (int w = 0; w < 4; w++) acc[u][w] = 0ull;
+#pragma unroll 2
+    for (int s = 0; s < nt; s++) {
+        const float4 k0 = *reinterpret_cast<const float4*>(kr + s * ldk), k1 = *reinterpret_cast<const float4*>(kr + s * ldk + 4);
+        Pairs v0 = pairs_at(vr + s * JT), v1 = pairs_at(vr + s * JT + JT / 2);
+        if (WEIGH) {
+            const f32x2 w = pack2(gp[nt - 1 - s], gp[nt - 1 - s]);
+            mul2(v0.lo, w);
+            mul2(v0.hi, w);
+            mul2(v1.lo, w);
+            mul2(v1.hi, w);
+        }
+        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const f32x2 k2 = pack2(kk[u], kk[u]);
+            fma2(acc[u][0], k2, v0.lo);
+            fma2(acc[u][1], k2, v0.hi);
+            fma2(acc[u][2], k2, v1.lo);
+            fma2(acc[u][3], k2, v1.hi);
+        }
+    }
+}
+
 // grid (chunks of the pass, H, cols / JT): the step's chunks are numbered sequence by sequence (layout.cuh: find_query_tile).
 // Thread (ti, tj) owns state rows ti * 8 + u and columns tj * 4 + {0..3} of either half of the tile.
 template <typename T, int C, int JT>
@@ -386,7 +443,7 @@ retention_local_kernel(const float* __restrict__ kn, const T* __restrict__ v, co
     __shared__ float gp[C + 1];
     griddep_wait();
     int b, tile;
-    if (!find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile)) return;
+    if (!find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile) || cu_q[b + 1] - cu_q[b] < a.least) return;
     const int h = blockIdx.y, d = a.dim, j0 = blockIdx.z * JT;
     const int t0 = cu_q[b] + tile * C, nt = min(C, cu_q[b + 1] - t0);
     float* ks = sm;                        // [C][d + 4]
@@ -398,30 +455,10 @@ retention_local_kernel(const float* __restrict__ kn, const T* __restrict__ v, co
     stage_values<T, C, JT>(vs, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd, nt,
                            [&](int tt) { return gp[nt - 1 - tt]; });
     __syncthreads();
-    constexpr int TJ = JT / 8;
-    const int ti = threadIdx.x / TJ, tj = threadIdx.x % TJ;
+    const int ti = threadIdx.x / (JT / 8), tj = threadIdx.x % (JT / 8);
     if (ti * 8 >= d) return;
     f32x2 acc[8][4];
-#pragma unroll
-    for (int u = 0; u < 8; u++)
-#pragma unroll
-        for (int w = 0; w < 4; w++) acc[u][w] = 0ull;
-    const float* kr = ks + ti * 8;
-    const float* vr = vs + tj * 4;
-#pragma unroll 2
-    for (int s = 0; s < nt; s++) {
-        const float4 k0 = *reinterpret_cast<const float4*>(kr + s * (d + 4)), k1 = *reinterpret_cast<const float4*>(kr + s * (d + 4) + 4);
-        const Pairs v0 = pairs_at(vr + s * JT), v1 = pairs_at(vr + s * JT + JT / 2);
-        const float kk[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-#pragma unroll
-        for (int u = 0; u < 8; u++) {
-            const f32x2 k2 = pack2(kk[u], kk[u]);
-            fma2(acc[u][0], k2, v0.lo);
-            fma2(acc[u][1], k2, v0.hi);
-            fma2(acc[u][2], k2, v1.lo);
-            fma2(acc[u][3], k2, v1.hi);
-        }
-    }
+    chunk_update<JT, false>(ks + ti * 8, d + 4, vs + tj * 4, nt, gp, acc);
     float* out = states + (((size_t)blockIdx.x * a.H + h) * d + ti * 8) * a.cols + j0 + tj * 4;
 #pragma unroll
     for (int u = 0; u < 8; u++) {
@@ -452,7 +489,7 @@ retention_states_kernel(const float* __restrict__ decay, float* __restrict__ sta
     // tile t of the sequence is number before + tiles - 1 - t; this pass holds the numbers [first, first + n_pass)
     const int last_no = before + tiles - 1;
     const int t_lo = max(0, last_no - (a.first + n_pass - 1)), t_hi = min(tiles, last_no - a.first + 1);
-    if (t_lo >= t_hi || slot < 0 || slot >= a.n_slots) return;
+    if (t_lo >= t_hi || slot < 0 || slot >= a.n_slots || q1 - q0 < a.least) return;
     const int e = blockIdx.x * RC_THREADS + threadIdx.x, per_row = a.cols / 4;
     const int i = e / per_row, c = (e % per_row) * 4;
     if (i >= a.dim || c >= a.vd) return;
@@ -495,19 +532,31 @@ retention_states_kernel(const float* __restrict__ decay, float* __restrict__ sta
 
 // The same grid as retention_local. Thread (ty, tx) owns tokens ty * RT + u and columns tx * 4 + {0..3} (of either half, when the
 // tile has 128). The keys' place in shared memory is used again by the old state, 32 rows at a time, and then by the values.
-template <typename T, int C, int JT>
+// ONE: grid (B, H, cols / JT), a sequence's only chunk: the old state comes from its slot (vd a multiple of 4), whose columns of this
+// tile nobody else touches, and the new one goes there, in the operations of retention_local and retention_states.
+template <typename T, int C, int JT, bool ONE>
 __global__ void __launch_bounds__(RC_THREADS, 2)
 retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn, const T* __restrict__ v, const float* __restrict__ decay,
-                     const float* __restrict__ states, float* __restrict__ o, const int* __restrict__ cu_q,
+                     const float* __restrict__ states, float* state, float* __restrict__ o, const int* __restrict__ cu_q,
                      const int* __restrict__ slots, RetChunkArgs a) {
     constexpr int RT = C / 16, G = JT / 64, LDW = C + 4, SR = 32;
     extern __shared__ __align__(16) float sm[];
     __shared__ float gp[C + 1];
     griddep_wait();
-    int b, tile;
-    if (!find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile)) return;
+    int b = blockIdx.x, tile = 0;
+    if (!ONE && !find_query_tile(cu_q, a.B, C, a.first + (int)blockIdx.x, b, tile)) return;
     const int slot = slots[b];
-    if (slot < 0 || slot >= a.n_slots) return;
+    if (slot < 0 || slot >= a.n_slots || cu_q[b + 1] <= cu_q[b]) return;
+    if (cu_q[b + 1] - cu_q[b] < a.least) {                  // (uniform)
+        if (tile == 0) {
+            const int wide = RC_THREADS / a.walk.L, j_end = min(a.vd, ((int)blockIdx.z + 1) * JT);
+            for (int j = blockIdx.z * JT; j < j_end; j += wide) {
+                walk_tokens<T, RC_THREADS, WALK_TB>(sm, qn, kn, v, decay[blockIdx.y], state, o, cu_q[b], cu_q[b + 1], slot, blockIdx.y, j, a.walk);
+                __syncthreads();                            // shared memory is free again
+            }
+        }
+        return;
+    }
     const int h = blockIdx.y, d = a.dim, j0 = blockIdx.z * JT, ldr = d + 4;
     const int t0 = cu_q[b] + tile * C, nt = min(C, cu_q[b + 1] - t0);
     float* qs = sm;                        // [C][ldr]
@@ -533,12 +582,14 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
 #pragma unroll
             for (int w = 0; w < RT; w++) kv[w] = pairs_at(xs + (tx + 16 * w) * ldr + i);
 #pragma unroll
-            for (int u = 0; u < RT; u++)
+            for (int u = 0; u < RT; u++) {
+                if (16 * u >= nt) break;                    // uniform: no token of the group exists
 #pragma unroll
                 for (int w = 0; w <= u; w++) {              // (keys behind every token of the group: not needed)
                     fma2(acc[u][w], qv[u].lo, kv[w].lo);
                     fma2(acc[u][w], qv[u].hi, kv[w].hi);
                 }
+            }
         }
 #pragma unroll
         for (int u = 0; u < RT; u++)
@@ -578,7 +629,10 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
         }
     };
     // ---- the old state, in pieces of SR rows; a piece is on its way while the one before is multiplied
-    const float* from = states + ((size_t)blockIdx.x * a.H + h) * d * a.cols + j0;
+    const int ldS = ONE ? a.vd : a.cols;
+    float* own = ONE ? state + (((size_t)slot * a.H + h) * d) * a.vd + j0 : nullptr;
+    const float* from = ONE ? own : states + ((size_t)blockIdx.x * a.H + h) * d * a.cols + j0;
+    const bool busy = (ty & ~1) * RT < nt;                  // a token of the warp's rows exists
     auto fetch = [&](int piece) {
         if (piece * SR < d) {
             float* dst = xs + (piece & 1) * SR * JT;
@@ -586,7 +640,8 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
             for (int idx = threadIdx.x; idx < SR * JT / 4; idx += RC_THREADS) {
                 const int i = idx / (JT / 4), c = (idx % (JT / 4)) * 4;
                 const uint32_t s = (uint32_t)__cvta_generic_to_shared(dst + i * JT + c);
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(s), "l"(from + (size_t)(piece * SR + i) * a.cols + c) : "memory");
+                const bool in = !ONE || j0 + c < a.vd;      // (beyond the state's columns: zeros, nothing read)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" :: "r"(s), "l"(from + (in ? (size_t)(piece * SR + i) * ldS + c : 0)), "r"(in ? 16 : 0) : "memory");
             }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
@@ -598,18 +653,20 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
         __syncthreads();
         const float* S = xs + (p & 1) * SR * JT;
 #pragma unroll 2
-        for (int i = 0; i < SR; i += 4) steps(qs + p * SR + i, ldr, S + i * JT, acc);
+        for (int i = 0; i < SR; i += 4)
+            if (busy) steps(qs + p * SR + i, ldr, S + i * JT, acc);
         __syncthreads();                                    // the piece's place may be filled again
     }
     // ---- scores times values, summed apart from the state's part: the roundings of a sum are of its own size
+    if (ONE) stage_rows<C>(qs, kn + (size_t)t0 * n + (size_t)h * d, n, d, nt);      // (the keys once more, where the queries were)
     stage_values<T, C, JT>(xs, v + (size_t)t0 * a.ldv + a.v_off + (size_t)h * a.vd, a.ldv, j0, a.vd, nt, [](int) { return 1.f; });
     __syncthreads();
-    const int s_end = ((ty | 1) + 1) * RT;                  // keys behind the last token of the warp's rows weigh nothing
     f32x2 within[RT][G][2];
 #pragma unroll
     for (int u = 0; u < RT; u++)
 #pragma unroll
         for (int w = 0; w < G; w++) within[u][w][0] = within[u][w][1] = 0ull;
+    const int s_end = busy ? ((ty | 1) + 1) * RT : 0;       // keys behind the last token of the warp's rows weigh nothing
     for (int s = 0; s < s_end; s += 4) steps(Ws + s, LDW, xs + s * JT, within);
 #pragma unroll
     for (int u = 0; u < RT; u++) {
@@ -633,16 +690,39 @@ retention_out_kernel(const float* __restrict__ qn, const float* __restrict__ kn,
             }
         }
     }
+    if constexpr (ONE) {                                    // the state
+        const int ti = threadIdx.x / (JT / 8), tj = threadIdx.x % (JT / 8);
+        if (ti * 8 >= d) return;
+        f32x2 U[8][4];
+        chunk_update<JT, true>(qs + ti * 8, ldr, xs + tj * 4, nt, gp, U);
+        const float gn = gp[nt];
+#pragma unroll
+        for (int half = 0; half < 2; half++) {
+            const int c = tj * 4 + half * (JT / 2);
+            if (j0 + c >= a.vd) continue;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                float4* at = reinterpret_cast<float4*>(own + (size_t)(ti * 8 + u) * a.vd + c);
+                const float4 S = *at;
+                const float2 x = unpack2(U[u][2 * half]), y = unpack2(U[u][2 * half + 1]);
+                *at = make_float4(fmaf(gn, S.x, x.x), fmaf(gn, S.y, x.y), fmaf(gn, S.z, y.x), fmaf(gn, S.w, y.y));
+            }
+        }
+    }
 }
 
 // How a step's chunks go: tokens a chunk, columns a tile, padded columns of a state, chunks a pass.
 struct RetPlan {
     int C, JT, cols, total, n_pass;
-    RetPlan(int rows, int B, int H, int dim, int vd) {
+    bool one;                                               // no sequence has more than one chunk, and a launch does it all
+    RetPlan(int rows, int B, int H, int dim, int vd, int max_q_len) {
         C = dim <= 128 ? 64 : 32;                           // (q and k of a chunk and a piece of the state: 86 KB a CTA, two an SM)
-        JT = dim <= 128 && vd > 64 ? 128 : 64;
+        one = max_q_len <= C && vd % 4 == 0;
+        total = one ? B : rows / C + B;                     // at most
+        // narrow tiles while even those leave no SM two CTAs (16 heads of 128: one sequence of 200 rows 43.9 -> 38.2 us, of 300 rows, with 160
+        // narrow CTAs, 45.4 -> 48.5)
+        JT = dim <= 128 && vd > 64 && (long long)total * H * ceil_div(vd, 64) > mynah_sm_count() ? 128 : 64;
         cols = ceil_div(vd, JT) * JT;
-        total = rows / C + B;                               // at most
         const long long one = (long long)H * dim * cols;
         const long long fit = (96ll << 20) / 4 / one;
         const int least = ceil_div(2 * mynah_sm_count(), H);
@@ -650,7 +730,8 @@ struct RetPlan {
         const int passes = ceil_div(total, most);
         n_pass = ceil_div(total, passes);
     }
-    long long floats(int H, int dim) const { return (long long)n_pass * H * dim * cols; }
+    long long floats(int H, int dim) const { return one ? 0 : (long long)n_pass * H * dim * cols; }
+    int launches() const { return one ? 1 : 3 * ceil_div(total, n_pass); }
 };
 
 template <typename T, int C, int JT>
@@ -660,9 +741,16 @@ int launch_chunked(const float* qn, const float* kn, const void* v, const float*
     const size_t local = ((size_t)C * (d + 4) + (size_t)C * JT) * sizeof(float);
     const size_t shared_part = (size_t)C * (d + 4) > (size_t)64 * JT ? (size_t)C * (d + 4) : (size_t)64 * JT;
     const size_t out = ((size_t)C * (d + 4) + (size_t)C * (C + 4) + shared_part) * sizeof(float);
+    if (walk_floats(RC_THREADS, WALK_TB, a.walk.L, a.walk.per) * sizeof(float) > out) return mynah_fail("retention_scan: a short sequence's walk does not fit");
     if (cudaFuncSetAttribute(retention_local_kernel<T, C, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess ||
-        cudaFuncSetAttribute(retention_out_kernel<T, C, JT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess)
+        cudaFuncSetAttribute(retention_out_kernel<T, C, JT, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(retention_out_kernel<T, C, JT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024) != cudaSuccess)
         return mynah_fail("retention_scan: %zu bytes of shared memory are not to be had", out);
+    if (plan.one) {
+        mynah_launch(retention_out_kernel<T, C, JT, true>, dim3(a.B, a.H, plan.cols / JT), dim3(RC_THREADS), out, stream, qn, kn, (const T*)v, decay,
+                     (const float*)nullptr, state, o, cu_q, slots, a);
+        return mynah_check_launch("retention_scan (one chunk)");
+    }
     // a sequence's chunks are numbered from its last to its first, so the passes go from the last to the first too
     for (int p = (plan.total - 1) / plan.n_pass; p >= 0; p--) {
         a.first = p * plan.n_pass;
@@ -670,8 +758,8 @@ int launch_chunked(const float* qn, const float* kn, const void* v, const float*
         mynah_launch(retention_local_kernel<T, C, JT>, grid, dim3(RC_THREADS), local, stream, kn, (const T*)v, decay, states, cu_q, a);
         mynah_launch(retention_states_kernel, dim3(ceil_div(d * (plan.cols / 4), RC_THREADS), a.H, a.B), dim3(RC_THREADS), 0, stream,
                      decay, states, state, cu_q, slots, a, C, plan.n_pass);
-        mynah_launch(retention_out_kernel<T, C, JT>, grid, dim3(RC_THREADS), out, stream, qn, kn, (const T*)v, decay,
-                     (const float*)states, o, cu_q, slots, a);
+        mynah_launch(retention_out_kernel<T, C, JT, false>, grid, dim3(RC_THREADS), out, stream, qn, kn, (const T*)v, decay,
+                     (const float*)states, state, o, cu_q, slots, a);
         if (mynah_check_launch("retention_scan (chunked)") != 0) return -1;
     }
     return 0;
@@ -679,7 +767,7 @@ int launch_chunked(const float* qn, const float* kn, const void* v, const float*
 
 }  // namespace
 
-// 0: every step walks token by token; otherwise prompts whose longest piece has at least this many tokens go chunk by chunk.
+// 0: every sequence is walked token by token; otherwise those that bring at least this many tokens go chunk by chunk.
 static int g_ret_chunk_min = 16;
 MYNAH_API int mynah_retention_chunk_min(int n) {
     const int before = g_ret_chunk_min;
@@ -697,8 +785,8 @@ MYNAH_API long long mynah_retention_scratch_floats(int rows, int B, int H, int d
         *launches = 1;
         return 0;
     }
-    const RetPlan plan(rows, B, H, dim, vd);
-    *launches = 3 * ceil_div(plan.total, plan.n_pass);
+    const RetPlan plan(rows, B, H, dim, vd, max_q_len);
+    *launches = plan.launches();
     return plan.floats(H, dim);
 }
 
@@ -737,8 +825,8 @@ MYNAH_API int mynah_retention_prep(const void* qk, int ld, int q_off, int k_off,
 }
 
 // v: rows whose columns [v_off + h * vd, ...) are head h's values; decay: fp32 [H]; state: fp32 [n_slots + 1][H][dim][vd];
-// o: fp32 [T][H * vd]. max_q_len: the most tokens a sequence brings (chooses between the two forms of the recurrence);
-// rows: the step's rows; scratch: mynah_retention_scratch_floats(...) floats, or null (token by token).
+// o: fp32 [T][H * vd]. max_q_len: no sequence brings more tokens; rows: the step's rows; scratch: mynah_retention_scratch_floats(...)
+// floats (null where those are 0, or to have every sequence walked token by token).
 MYNAH_API int mynah_retention_scan(const float* qn, const float* kn, const void* v, int ldv, int v_off, int v_dtype,
                                    const float* decay, float* state, int n_slots, float* o, const int* cu_q,
                                    const int* slots, int B, int H, int dim, int vd, int max_q_len, int rows, float* scratch,
@@ -748,21 +836,22 @@ MYNAH_API int mynah_retention_scan(const float* qn, const float* kn, const void*
     MYNAH_REQUIRE(dim <= 512, "retention_scan: keys of %d values exceed the 512 that the kernel stages", dim);
     MYNAH_REQUIRE(H <= 65535 && B <= 65535, "retention_scan: too many heads or sequences for one launch");
     MYNAH_REQUIRE(v_dtype == MYNAH_F32 || v_dtype == MYNAH_BF16, "retention_scan: unsupported dtype %d", v_dtype);
-    if (retention_chunked(dim, max_q_len) && scratch != nullptr && (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)scratch) & 15) == 0) {
-        const RetPlan plan(rows, B, H, dim, vd);
-        const RetChunkArgs ca{H, dim, vd, n_slots, ldv, v_off, B, plan.cols, 0};
+    int L = 1;
+    while (L * RET_RMAX < dim) L <<= 1;
+    const int per = ceil_div(dim, L);
+    const int JT = RET_THREADS / L;
+    const RetArgs a{B, H, dim, vd, n_slots, ldv, v_off, L, per};
+    const RetPlan plan(rows, B, H, dim, vd, max_q_len);
+    if (retention_chunked(dim, max_q_len) && (plan.one ? ((uintptr_t)state & 15) == 0 : scratch != nullptr) &&
+        (((uintptr_t)qn | (uintptr_t)kn | (uintptr_t)scratch) & 15) == 0) {
+        const RetChunkArgs ca{H, dim, vd, n_slots, ldv, v_off, B, plan.cols, 0, g_ret_chunk_min, a};
         MYNAH_REQUIRE(plan.cols / plan.JT <= 65535, "retention_scan: too many columns for one launch");
 #define RET_CHUNKED(T, C, JT) launch_chunked<T, C, JT>(qn, kn, v, decay, scratch, state, o, cu_q, slots, ca, plan, stream)
         if (v_dtype == MYNAH_F32) return plan.C == 32 ? RET_CHUNKED(float, 32, 64) : plan.JT == 64 ? RET_CHUNKED(float, 64, 64) : RET_CHUNKED(float, 64, 128);
         return plan.C == 32 ? RET_CHUNKED(bf16, 32, 64) : plan.JT == 64 ? RET_CHUNKED(bf16, 64, 64) : RET_CHUNKED(bf16, 64, 128);
 #undef RET_CHUNKED
     }
-    int L = 1;
-    while (L * RET_RMAX < dim) L <<= 1;
-    const int per = ceil_div(dim, L);
-    const int JT = RET_THREADS / L;
-    const RetArgs a{B, H, dim, vd, n_slots, ldv, v_off, L, per};
-    const size_t smem = ((size_t)2 * RET_TB * (per + 1) * L + (size_t)RET_TB * JT) * sizeof(float);
+    const size_t smem = walk_floats(RET_THREADS, RET_TB, L, per) * sizeof(float);
     const dim3 grid(ceil_div(vd, JT), H, B);
     if (v_dtype == MYNAH_F32) {
         if (smem > 48 * 1024) cudaFuncSetAttribute(retention_scan_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

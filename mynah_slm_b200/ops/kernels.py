@@ -1005,9 +1005,8 @@ def retention_step(p: torch.Tensor, q_off: int, k_off: int, v_off: int, g_off: i
 
 
 def retention_chunk_min(n: int) -> int:
-    """From how many tokens in a step's longest piece the retention recurrence runs chunk by chunk (keys that are a
-    multiple of 32 values up to 256); 0: always token by token. Returns the setting before. The two forms agree to
-    rounding."""
+    """From how many tokens in a step a sequence's retention runs chunk by chunk (keys that are a multiple of 32 values up to
+    256); 0: always token by token. Returns the setting before. The two forms agree to rounding."""
     return int(lib.load().mynah_retention_chunk_min(int(n)))
 
 

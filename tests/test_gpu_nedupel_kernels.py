@@ -256,6 +256,39 @@ def test_retention_chunks_keep_their_distance_from_64_bits():
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,dim,vd", [(2, 128, 128), (20, 128, 192), (3, 32, 66), (2, 256, 36), (1, 96, 20), (2, 40, 24)])
+def test_a_piece_of_the_retention_has_the_same_bits_in_any_step(dtype, H, dim, vd):
+    """Pieces about the length from which they go chunk by chunk, of one chunk, of several: in one step, in a step of short ones, and
+    each alone, given their own length or a captured step's capacity. Outputs and states."""
+    from mynah_slm_b200.engine.engine import _prompt_rows_bucket
+    from mynah_slm_b200.ops import kernels
+    g = torch.Generator(device=DEV).manual_seed(dim + vd)
+    lengths = [15, 64, 1, 16, 300, 33, 17]
+    rand = lambda *s: torch.randn(s, generator=g, device=DEV)                    # noqa: E731
+    T = sum(lengths)
+    qn, kn, v = rand(T, H * dim), rand(T, H * dim) * dim ** -0.5, rand(T, H * vd).to(dtype)
+    decay = torch.linspace(0.9, 1.0, H, device=DEV)
+    state0 = rand(10, H, dim, vd)
+    at = np.cumsum([0] + lengths)
+
+    def run(which, capacity):
+        rows = torch.cat([torch.arange(at[i], at[i + 1], device=DEV) for i in which])
+        ctx = ctx_for([lengths[i] for i in which], [8 - i for i in which])
+        ctx.max_q_len = capacity or ctx.max_q_len
+        st = state0.clone()
+        o = kernels.retention_scan(qn[rows].contiguous(), kn[rows].contiguous(), v[rows].contiguous(), 0, decay, st, ctx, H, dim, vd)
+        return dict(zip(which, torch.split(o, [lengths[i] for i in which]))), st
+
+    whole, st_whole = run(range(len(lengths)), None)
+    short = [i for i, n in enumerate(lengths) if n <= 64]
+    steps = [run(short, None), run(short, _prompt_rows_bucket(sum(lengths[i] for i in short)))]
+    steps += [run([i], c) for i, n in enumerate(lengths) for c in (None, _prompt_rows_bucket(n))]
+    for out, st in steps:
+        for i, o in out.items():
+            assert torch.equal(o, whole[i]) and torch.equal(st[8 - i], st_whole[8 - i]), lengths[i]
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,D,F,E,top", [(150, 48, 56, 9, 2), (5, 40, 12, 1, 1), (3, 64, 20, 7, 7), (400, 96, 200, 70, 4),
                                         (700, 128, 320, 5, 2)])
 def test_table_routed_experts(dtype, T, D, F, E, top):
