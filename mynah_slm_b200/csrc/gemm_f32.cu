@@ -271,9 +271,9 @@ gemm_f32_rows_kernel(const float* __restrict__ A, const float* __restrict__ W, f
         if (works) {
             const uint32_t w = base + (uint32_t)((s % STAGES) * stage_words + n * ROW_PITCH) * 4;
             const uint32_t a = base + (uint32_t)((s % STAGES) * stage_words + (BN + mg * MR) * ROW_PITCH) * 4;
-            if constexpr (BN == 16) {
+            if constexpr (BN == 16 && MR == 4) {
                 // two CTAs an SM and more cover one another's reads; the registers of reading ahead only cost (16 rows, 6,144 x 1,024: 20.7 us
-                // against 19.6; 9,728 x 2,560: 79.0 / 74.8; 12 rows of 16,384 x 1,024: 46.8 / 43.7)
+                // against 19.6; 9,728 x 2,560: 79.0 / 74.8; 12 rows of 16,384 x 1,024: 46.8 / 43.7; two rows of 6,144 x 1,024 the other way: 10.9 / 11.2)
                 const float* wf = smem + (size_t)(s % STAGES) * stage_words + n * ROW_PITCH;
                 const float* af = smem + (size_t)(s % STAGES) * stage_words + (BN + mg * MR) * ROW_PITCH;
 #pragma unroll 8

@@ -871,7 +871,10 @@ MYNAH_API int mynah_retention_step_supported(int dim, int vd) {
     while (L * RET_RMAX < dim) L <<= 1;
     return dim > 0 && dim <= 128 && vd > 0 && L * vd <= 512;
 }
-// Whether it is the faster form for B rows: a CTA an SM at most, and more than a handful (figures at the kernel).
+// Whether it is the faster form for B rows: a CTA an SM at most, and more than a handful (figures at the kernel). Smaller states move the
+// upper end out and leave the lower one without a loss, us against the three launches: 8 heads of 64 1 row 6.5 / 9.1, 64 rows
+// 8.1 / 13.2; 32 heads of 32 1 row 7.0 / 8.6, 64 rows 8.6 / 20.9; 64 heads of 128 2 rows 9.6 / 13.2, 4 rows 17.3 / 17.3; within
+// the rule it never loses.
 MYNAH_API int mynah_retention_step_pays(int B, int H) {
     return (long long)B * H >= 32 && (long long)B * H <= mynah_sm_count();
 }

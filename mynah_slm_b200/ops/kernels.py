@@ -492,19 +492,25 @@ def argmax(logits: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Te
     return out
 
 
-def _check_ring(ring: tuple, params: torch.Tensor, rows: int, by_slot: bool) -> None:
-    """The kernel reads the window from params[7] and, for every slot, reads and writes a row of tokens, a count and a head."""
-    if len(ring) != 3:
-        raise KernelError("sample: a ring is (tokens, counts, heads)")
-    for t, name, dim in zip(ring, ("ring", "ring counts", "ring heads"), (2, 1, 1)):
-        if t.dtype != torch.int32 or t.dim() != dim or not t.is_contiguous():
-            raise KernelError(f"sample: {name} must be contiguous int32 of {dim} dimensions")
-    if not ring[0].shape[0] == ring[1].numel() == ring[2].numel():
-        raise KernelError(f"sample: {ring[0].shape[0]} rows in the ring, {ring[1].numel()} counts, {ring[2].numel()} heads")
-    if not by_slot and ring[0].shape[0] < rows:
-        raise KernelError(f"sample: {ring[0].shape[0]} rows in the ring for {rows} rows of logits")
-    if params.numel() < 8:
-        raise KernelError("sample: with a ring the parameters are eight, the last of them the window")
+class Ring(tuple):
+    """The rings of recent tokens that a draw reads and feeds: (tokens [slots, stride], counts [slots], heads [slots]), int32. The kernel
+    reads and writes a row, a count and a head for every slot, so a ring is checked when it is made."""
+    __slots__ = ()
+
+    def __new__(cls, tokens: torch.Tensor, counts: torch.Tensor, heads: torch.Tensor) -> "Ring":
+        for t, name, dim in ((tokens, "ring", 2), (counts, "ring counts", 1), (heads, "ring heads", 1)):
+            if t.dtype != torch.int32 or t.dim() != dim or not t.is_contiguous():
+                raise KernelError(f"sample: {name} must be contiguous int32 of {dim} dimensions")
+        if not tokens.shape[0] == counts.numel() == heads.numel() or not tokens.device == counts.device == heads.device:
+            raise KernelError(f"sample: {tokens.shape[0]} rows in the ring, {counts.numel()} counts, {heads.numel()} heads, "
+                              "on one device each, do not go together")
+        return super().__new__(cls, (tokens, counts, heads))
+
+    def check(self, params: torch.Tensor, rows: int, by_slot: bool) -> None:
+        if not by_slot and self[0].shape[0] < rows:
+            raise KernelError(f"sample: {self[0].shape[0]} rows in the ring for {rows} rows of logits")
+        if params.numel() < 8:
+            raise KernelError("sample: with a ring the parameters are eight, the last of them the window")
 
 
 def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots: Optional[torch.Tensor],
@@ -519,13 +525,14 @@ def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots:
     B, V = logits.shape
     if out is None:
         out = torch.empty((B,), dtype=torch.int32, device=logits.device)
-    tokens, counts, heads = ring if ring is not None else (None, None, None)
-    if params.numel() < 7:
-        raise KernelError(f"sample: {params.numel()} parameters, seven are read")
     if ring is not None:
-        _check_ring(ring, params, B, slots is not None)
-        for t in ring:
-            _chk(t, "ring")
+        if type(ring) is not Ring:
+            ring = Ring(*ring)
+        ring.check(params, B, slots is not None)
+        _chk(ring[0], "ring")
+    elif params.numel() < 7:
+        raise KernelError(f"sample: {params.numel()} parameters, seven are read")
+    tokens, counts, heads = ring if ring is not None else (None, None, None)
     call("mynah_sample", ptr(logits), B, V, V, ptr(params), ptr(rng), ptr(slots), ptr(out), ptr(tokens), ptr(counts), ptr(heads),
          tokens.shape[1] if ring is not None else 0, stream_ptr())
     return out

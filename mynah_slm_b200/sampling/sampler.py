@@ -88,6 +88,7 @@ class SamplerState:
         self.ring = torch.zeros((max_seqs, max(window, 1)), dtype=torch.int32, device=device)
         self.ring_n = torch.zeros((max_seqs,), dtype=torch.int32, device=device)
         self.ring_head = torch.zeros((max_seqs,), dtype=torch.int32, device=device)
+        self._rings = kernels.Ring(self.ring, self.ring_n, self.ring_head)
         self.params = torch.zeros((8,), dtype=torch.float32, device=device)
         self.active_window = window
         self._params_host: Optional[SamplingParams] = None
@@ -151,4 +152,4 @@ class SamplerState:
         if not torch.cuda.is_current_stream_capturing():
             self.flush_resets()
         return kernels.sample(logits, self.params, self.rng, slots, out,
-                              (self.ring, self.ring_n, self.ring_head) if self.window > 0 else None)
+                              self._rings if self.window > 0 else None)

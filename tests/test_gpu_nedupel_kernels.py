@@ -95,7 +95,8 @@ def test_latent_prep_and_cache_rows(H, dim, rd, r, interleaved):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,H,n_in,n_out,aligned", [(70, 3, 16, 40, True), (1, 1, 6, 13, False), (130, 5, 100, 70, False),
-                                                    (9, 2, 64, 150, True), (200, 3, 96, 96, True)])
+                                                    (9, 2, 64, 150, True), (200, 3, 96, 96, True), (5, 2, 1032, 72, True),
+                                                    (16, 2, 2080, 40, True)])
 def test_head_linear(dtype, T, H, n_in, n_out, aligned):
     from mynah_slm_b200.ops import kernels
     rng = np.random.default_rng(T + n_in)
@@ -290,7 +291,9 @@ def test_a_piece_of_the_retention_has_the_same_bits_in_any_step(dtype, H, dim, v
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,D,F,E,top", [(150, 48, 56, 9, 2), (5, 40, 12, 1, 1), (3, 64, 20, 7, 7), (400, 96, 200, 70, 4),
-                                        (700, 128, 320, 5, 2)])
+                                        (700, 128, 320, 5, 2),
+                                        # rows in several blocks of 1,024 values, with whole and short last blocks
+                                        (140, 1032, 1536, 3, 2), (270, 2088, 264, 2, 1), (270, 256, 2048, 3, 1)])
 def test_table_routed_experts(dtype, T, D, F, E, top):
     from mynah_slm_b200.ops import kernels
     rng = np.random.default_rng(T + E)

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from mynah_slm_b200.ops.kernels import _check_ring
+from mynah_slm_b200.ops.kernels import Ring
 from mynah_slm_b200.ops.lib import KernelError
 
 
@@ -11,12 +11,18 @@ def _ring(rows=4, stride=8, counts=4, heads=4, dtype=torch.int32):
 
 
 def test_a_ring_that_fits_is_taken():
-    _check_ring(_ring(), torch.zeros(8), 4, False)
-    _check_ring(_ring(), torch.zeros(8), 9, True)                    # rows go by slot: more rows than slots is the caller's business
+    Ring(*_ring()).check(torch.zeros(8), 4, False)
+    Ring(*_ring()).check(torch.zeros(8), 9, True)                    # rows go by slot: more rows than slots is the caller's business
 
 
-@pytest.mark.parametrize("ring,params,rows", [(_ring(counts=3), 8, 4), (_ring(heads=3), 8, 4), (_ring(heads=1, counts=1), 8, 1),
-                                              (_ring(dtype=torch.int64), 8, 4), (_ring(), 7, 4), (_ring(), 8, 5), (_ring()[:2], 8, 4)])
-def test_a_ring_that_does_not_fit_is_refused(ring, params, rows):
+@pytest.mark.parametrize("parts", [_ring(counts=3), _ring(heads=3), _ring(heads=1, counts=1), _ring(dtype=torch.int64),
+                                   (torch.zeros((8, 4), dtype=torch.int32).t(),) + _ring()[1:]])
+def test_parts_that_do_not_fit_are_refused(parts):
     with pytest.raises(KernelError):
-        _check_ring(ring, torch.zeros(params), rows, False)
+        Ring(*parts)
+
+
+@pytest.mark.parametrize("params,rows", [(7, 4), (8, 5)])
+def test_a_draw_that_does_not_fit_is_refused(params, rows):
+    with pytest.raises(KernelError):
+        Ring(*_ring()).check(torch.zeros(params), rows, False)
