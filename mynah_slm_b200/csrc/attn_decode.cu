@@ -66,7 +66,7 @@ struct HeadState {
     float m[GT], l[GT], acc[GT][8];
 };
 
-template <typename T, int GT>
+template <typename T, int GT, int AHEAD>
 __global__ void __launch_bounds__(WARPS * 32)
 attn_decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache, const T* __restrict__ v_cache,
                          const int* __restrict__ kv_len, PageTable pt, DecodeArgs a,
@@ -117,11 +117,7 @@ attn_decode_split_kernel(const T* __restrict__ q, const T* __restrict__ k_cache,
         for (int j = 0; j < 8; j++) st.acc[i][j] = 0.f;
     }
 
-    // All keys of a split lie in one page, which is looked up once. In fp32 a warp's keys come in pairs, both keys' loads in flight before
-    // the first is used; more of them cost the registers that let other CTAs cover the wait (8 heads of 64, 32 rows behind 2,000
-    // positions, us one at a time / two / four: fp32 61.6 / 58.4 / 70.6; bfloat16, whose conversions take registers of their own, 67.1 / 73.1 /
-    // 110.3; with the page looked up for every key 63.7 and 75.2. One row behind 500, 16 heads of 128 in fp32: 11.7 / 11.4 / 11.2; 12.2).
-    constexpr int AHEAD = sizeof(T) == 4 ? 2 : 1;
+    // All keys of a split lie in one page, which is looked up once. A warp takes AHEAD keys at a time, their loads in flight together.
     const int pt_lo = pt.indptr[b], pt_cnt = pt.indptr[b + 1] - pt_lo, lp = key_begin / PAGE_TOKENS - pt.base[b];
     int page = (lp >= 0 && lp < pt_cnt) ? pt.ids[pt_lo + lp] : -1;
     if (page >= pt.n_pages) page = -1;
@@ -266,12 +262,21 @@ int launch_decode(const void* q, void* out, int B, const DecodeArgs& a, const vo
     const T* qp = (const T*)q;
     const T* kp = (const T*)k_cache;
     const T* vp = (const T*)v_cache;
-    if (gt == 1)
-        attn_decode_split_kernel<T, 1><<<grid, WARPS * 32, 0, stream>>>(qp, kp, vp, kv_len, pt, a, part_o, part_ml, status);
-    else if (gt == 2)
-        attn_decode_split_kernel<T, 2><<<grid, WARPS * 32, 0, stream>>>(qp, kp, vp, kv_len, pt, a, part_o, part_ml, status);
-    else
-        attn_decode_split_kernel<T, 4><<<grid, WARPS * 32, 0, stream>>>(qp, kp, vp, kv_len, pt, a, part_o, part_ml, status);
+    // In fp32 two keys a warp's turn, four while a few CTAs an SM leave each wait uncovered: more keys take the registers that let other
+    // CTAs cover it, and bfloat16's conversions take registers of their own (us with one key / two / four; with the page looked up
+    // for every key: 8 heads of 64, 32 rows behind 2,000 positions fp32 61.6 / 58.4 / 70.6; 63.7, bfloat16 67.1 / 73.1 / 110.3; 75.2;
+    // 4 heads of 256 in fp32, 256 CTAs 14.8 / 13.8 / 13.0; 16.1, 512 CTAs 19.1 / 18.1 / 18.1; 20.4).
+    const bool few = (long long)grid.x * grid.y * grid.z <= 3ll * mynah_sm_count();
+    auto go = [&](auto kern) { kern<<<grid, WARPS * 32, 0, stream>>>(qp, kp, vp, kv_len, pt, a, part_o, part_ml, status); };
+    if constexpr (sizeof(T) == 4) {
+        if (gt == 1) few ? go(attn_decode_split_kernel<T, 1, 4>) : go(attn_decode_split_kernel<T, 1, 2>);
+        else if (gt == 2) few ? go(attn_decode_split_kernel<T, 2, 4>) : go(attn_decode_split_kernel<T, 2, 2>);
+        else go(attn_decode_split_kernel<T, 4, 2>);
+    } else {
+        if (gt == 1) go(attn_decode_split_kernel<T, 1, 1>);
+        else if (gt == 2) go(attn_decode_split_kernel<T, 2, 1>);
+        else go(attn_decode_split_kernel<T, 4, 1>);
+    }
     if (mynah_check_launch("attn_decode_split")) return -1;
     const int threads = a.VD >= 128 ? 128 : (a.VD >= 64 ? 64 : 32);
     attn_decode_combine_kernel<T><<<dim3(a.H, B), threads, 0, stream>>>(part_o, part_ml, (T*)out, kv_len, a.window, a.chunk, a.keep_first, a.H, a.VD, a.S, a.ldo,

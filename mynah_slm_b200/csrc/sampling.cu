@@ -581,10 +581,10 @@ __device__ int draw_from_keys(Shared<NC>& sh, unsigned int n_key, const SamplePa
 // temperature alone 70, 70, 326 -> 58, 59, 160. 512 threads a CTA, so that two share an SM: with 1,024 (whose registers fill
 // it) 64 rows took 63 us with top-k 20 and 496 with top-p, one row 15 instead of 17. A cluster a row at 32,000 logits: 12 us
 // against 18 at one row, but 45 against 19 at 64 and 268 against 86 with top-p: one CTA a row below 32,768.
-template <int NC>
+template <int NC, bool IN_SHARED>
 __global__ void __launch_bounds__(THREADS)
 sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict__ params, unsigned long long* __restrict__ rng,
-              const int* __restrict__ slots, int* __restrict__ out, Ring ring, int row_in_shared) {
+              const int* __restrict__ slots, int* __restrict__ out, Ring ring) {
     extern __shared__ __align__(16) unsigned char smem[];
     Shared<NC>& sh = *reinterpret_cast<Shared<NC>*>(smem);
     constexpr int GROUPS = Shared<NC>::GROUPS, LANES = Shared<NC>::LANES;      // groups of LANES lanes
@@ -611,7 +611,7 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
         sh.n_key = 0;
     }
     // ---- the row, and each thread's first maximum
-    rs.p = row_in_shared ? reinterpret_cast<float*>(smem + sizeof(Shared<NC>)) : row + rs.begin;
+    rs.p = IN_SHARED ? reinterpret_cast<float*>(smem + sizeof(Shared<NC>)) : row + rs.begin;
     const float* from = row + rs.begin;
     float bv = -INFINITY;
     int bi = 0x7fffffff;
@@ -642,7 +642,7 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
 #pragma unroll
             for (int u = 0; u < LOADS4; u++) {
                 const int j = base0 + u * THREADS + (int)threadIdx.x;
-                if (j < n4) v[u] = row_in_shared ? __ldcs(from4 + j) : from4[j];
+                if (j < n4) v[u] = IN_SHARED ? __ldcs(from4 + j) : from4[j];
             }
 #pragma unroll
             for (int u = 0; u < LOADS4; u++) {
@@ -653,17 +653,17 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
                     take_first_max(bv, bi, v[u].y, i + 1);
                     take_first_max(bv, bi, v[u].z, i + 2);
                     take_first_max(bv, bi, v[u].w, i + 3);
-                    if (row_in_shared) reinterpret_cast<float4*>(rs.p)[j] = v[u];
+                    if (IN_SHARED) reinterpret_cast<float4*>(rs.p)[j] = v[u];
                 }
             }
         }
         for (int i = 4 * n4 + (int)threadIdx.x; i < rs.n; i += THREADS) {
             const float x = from[i];
-            if (row_in_shared) rs.p[i] = x;
+            if (IN_SHARED) rs.p[i] = x;
             take_first_max(bv, bi, x, rs.begin + i);
         }
     } else {
-        scan(from, row_in_shared != 0);
+        scan(from, IN_SHARED);
     }
     if (window > 0 && !(repeat == 1.0f && freq == 0.0f && presence == 0.0f)) {       // sampler.c:81-84
         const int n = min(ring.n[slot], min(window, 256));
@@ -972,13 +972,13 @@ MYNAH_API int mynah_sample(float* logits, int B, int V, int ld, const float* par
     const bool cluster = V >= ROW_CTAS * 4096;
     const size_t own = cluster ? sizeof(Shared<ROW_CTAS>) : sizeof(Shared<1>);
     const size_t part = sizeof(float) * (size_t)(cluster ? ((V + ROW_CTAS - 1) / ROW_CTAS + 3) & ~3 : V);
-    const int in_shared = own + part <= 113 * 1024 || (own + part <= 227 * 1024 && B * (cluster ? ROW_CTAS : 1) <= mynah_sm_count());
+    const bool in_shared = own + part <= 113 * 1024 || (own + part <= 227 * 1024 && B * (cluster ? ROW_CTAS : 1) <= mynah_sm_count());
     const size_t smem = own + (in_shared ? part : 0);
-    auto kernel = cluster ? sample_kernel<ROW_CTAS> : sample_kernel<1>;
+    auto kernel = cluster ? (in_shared ? sample_kernel<ROW_CTAS, true> : sample_kernel<ROW_CTAS, false>) : (in_shared ? sample_kernel<1, true> : sample_kernel<1, false>);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
     if (e != cudaSuccess) return mynah_fail("sample: %s", cudaGetErrorString(e));
     if (!cluster) {
-        mynah_launch(kernel, dim3(B), dim3(THREADS), smem, stream, logits, V, ld, params, rng, slots, out, rings, in_shared);
+        mynah_launch(kernel, dim3(B), dim3(THREADS), smem, stream, logits, V, ld, params, rng, slots, out, rings);
         return mynah_check_launch("sample");
     }
     cudaLaunchConfig_t cfg = {};
@@ -993,7 +993,7 @@ MYNAH_API int mynah_sample(float* logits, int B, int V, int ld, const float* par
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, logits, V, ld, params, rng, slots, out, rings, in_shared);
+    e = cudaLaunchKernelEx(&cfg, kernel, logits, V, ld, params, rng, slots, out, rings);
     if (e != cudaSuccess) return mynah_fail("sample: %s", cudaGetErrorString(e));
     return mynah_check_launch("sample");
 }

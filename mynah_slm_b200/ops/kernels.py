@@ -507,10 +507,13 @@ class Ring(tuple):
         return super().__new__(cls, (tokens, counts, heads))
 
     def check(self, params: torch.Tensor, rows: int, by_slot: bool) -> None:
+        """Raises unless a draw of so many rows with these parameters can use the ring."""
         if not by_slot and self[0].shape[0] < rows:
             raise KernelError(f"sample: {self[0].shape[0]} rows in the ring for {rows} rows of logits")
         if params.numel() < 8:
             raise KernelError("sample: with a ring the parameters are eight, the last of them the window")
+        if not self[0].is_cuda and params.is_cuda:
+            raise KernelError("ring is not on a CUDA device")
 
 
 def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots: Optional[torch.Tensor],
@@ -525,16 +528,19 @@ def sample(logits: torch.Tensor, params: torch.Tensor, rng: torch.Tensor, slots:
     B, V = logits.shape
     if out is None:
         out = torch.empty((B,), dtype=torch.int32, device=logits.device)
+    tokens = counts = heads = None
+    stride = 0
     if ring is not None:
         if type(ring) is not Ring:
             ring = Ring(*ring)
-        ring.check(params, B, slots is not None)
-        _chk(ring[0], "ring")
+        tokens, counts, heads = ring
+        stride = tokens.shape[1]
+        if params.numel() < 8 or not tokens.is_cuda or (slots is None and tokens.shape[0] < B):
+            ring.check(params, B, slots is not None)
     elif params.numel() < 7:
         raise KernelError(f"sample: {params.numel()} parameters, seven are read")
-    tokens, counts, heads = ring if ring is not None else (None, None, None)
     call("mynah_sample", ptr(logits), B, V, V, ptr(params), ptr(rng), ptr(slots), ptr(out), ptr(tokens), ptr(counts), ptr(heads),
-         tokens.shape[1] if ring is not None else 0, stream_ptr())
+         stride, stream_ptr())
     return out
 
 
