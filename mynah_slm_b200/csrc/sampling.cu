@@ -62,7 +62,9 @@ struct Histogram {
     unsigned int lo[BINS], hi[BINS];
 };
 constexpr int LOW_BITS = 11;
-__device__ __forceinline__ bool mass_by_count(unsigned int bits) { return (bits >> 23) - 90u <= 127u - 90u; }
+// (a CTA with more than 2^21 elements could overflow the low word: it sums the masses themselves, `span` 0)
+constexpr unsigned int SPAN = 128 - 90;
+__device__ __forceinline__ bool mass_by_count(unsigned int bits, unsigned int span) { return (bits >> 23) - 90u < span; }
 
 template <int NC>
 struct Shared {
@@ -108,15 +110,18 @@ __device__ __forceinline__ void add_mass(Histogram& h, unsigned int d, unsigned 
 // A row is shared by NC CTAs (NC = 1, or the ROW_CTAS CTAs of a cluster): CTA r works on the elements
 // [r * chunk, (r + 1) * chunk) and the CTAs meet through distributed shared memory. Every CTA of a row runs
 // the same code with the same decisions, so the cluster barriers below are reached by all of them.
-template <int NC>
+template <int NC, bool IN_SHARED>
 struct RowShare {
     int rank, begin, n;                                     // this CTA's elements: `n` from `begin` on
     float* p;                                               // where it keeps them: shared memory, or the row itself if too long
+    bool wide;                                              // more elements a CTA than mass_by_count can add up (never in shared memory)
+    __device__ __forceinline__ unsigned int span() const { return IN_SHARED || !wide ? SPAN : 0u; }
     __device__ static int chunk(int V) { return NC == 1 ? V : ((V + NC - 1) / NC + 3) & ~3; }
     __device__ explicit RowShare(int V) {
         rank = NC == 1 ? 0 : (int)cg::this_cluster().block_rank();
         begin = min(V, rank * chunk(V));
         n = min(V, begin + chunk(V)) - begin;
+        wide = !IN_SHARED && chunk(V) > 1 << 21;            // the same in every CTA of the row
     }
     __device__ __forceinline__ void sync() const {
         if (NC == 1) __syncthreads();
@@ -147,8 +152,8 @@ struct Slice {
 // Counts and masses of a pass. Probabilities crowd into a few digits where the logits do: a warp whose 32 elements fall into
 // at most four digits adds each digit up over the warp and lets one lane do the atomics. Counts and masses are integers, so
 // the order of the additions does not matter.
-template <int NC>
-__device__ __noinline__ void fill_histogram(const RowShare<NC>& rs, const Digit dg, float scale, Shared<NC>& sh) {
+template <int NC, bool IN_SHARED>
+__device__ __noinline__ void fill_histogram(const RowShare<NC, IN_SHARED>& rs, const Digit dg, float scale, Shared<NC>& sh) {
     for (int i = threadIdx.x; i < BINS; i += THREADS) {
         sh.h.count[i] = 0;
         sh.h.lo[i] = 0;
@@ -184,7 +189,7 @@ __device__ __noinline__ void fill_histogram(const RowShare<NC>& rs, const Digit 
                     const bool same = ((left >> lane) & 1u) && d == ds;
                     const unsigned int grp = __ballot_sync(0xffffffffu, same);
                     const unsigned int bs = __shfl_sync(0xffffffffu, bits, src);
-                    if (__popc(grp) >= 8 && (mass_by_count(bs))) {
+                    if (__popc(grp) >= 8 && mass_by_count(bs, rs.span())) {
                         const unsigned int low = same ? bits & low_mask : 0u;
                         const unsigned int lo = __reduce_add_sync(0xffffffffu, low & ((1u << LOW_BITS) - 1u));
                         const unsigned int hi = __reduce_add_sync(0xffffffffu, low >> LOW_BITS);
@@ -199,7 +204,7 @@ __device__ __noinline__ void fill_histogram(const RowShare<NC>& rs, const Digit 
             }
             if ((left >> lane) & 1u) {
                 atomicAdd(&sh.h.count[d], 1u);
-                if (mass_by_count(bits)) {
+                if (mass_by_count(bits, rs.span())) {
                     const unsigned int low = bits & low_mask, lo = low & ((1u << LOW_BITS) - 1u), hi = low >> LOW_BITS;
                     if (lo) atomicAdd(&sh.h.lo[d], lo);
                     if (hi) atomicAdd(&sh.h.hi[d], hi);
@@ -212,9 +217,9 @@ __device__ __noinline__ void fill_histogram(const RowShare<NC>& rs, const Digit 
 }
 
 // This CTA's slice of a pass over the row. The histograms may be filled again behind find_digit's first barrier.
-template <int NC>
-__device__ __forceinline__ Slice<NC> add_up(const RowShare<NC>& rs, const Digit dg, float scale, Shared<NC>& sh) {
-    fill_histogram<NC>(rs, dg, scale, sh);
+template <int NC, bool IN_SHARED>
+__device__ __forceinline__ Slice<NC> add_up(const RowShare<NC, IN_SHARED>& rs, const Digit dg, float scale, Shared<NC>& sh) {
+    fill_histogram<NC, IN_SHARED>(rs, dg, scale, sh);
     rs.sync();                                              // every CTA's histogram is complete
     Slice<NC> s;
     s.hi = dg.n_bins - 1 - (rs.rank * Slice<NC>::WIDE + (int)threadIdx.x * Slice<NC>::PER);
@@ -239,7 +244,7 @@ __device__ __forceinline__ Slice<NC> add_up(const RowShare<NC>& rs, const Digit 
                 masses += ((unsigned long long)hi[r] << 32) | lo[r];
             }
             const unsigned int base = dg.bits | ((unsigned int)d << dg.shift);     // the digit's smallest element
-            s.m[q] = mass_by_count(base)
+            s.m[q] = mass_by_count(base, rs.span())
                 ? ((unsigned long long)((base & 0x7fffffu) | 0x800000u) * s.c[q] + lows) << ((base >> 23) - 90u) : masses;
         }
     }
@@ -250,8 +255,8 @@ __device__ __forceinline__ Slice<NC> add_up(const RowShare<NC>& rs, const Digit 
 // target. by_mass: cum_mass >= target_mass; else cum_count >= target_count. The carried count and mass are those of the
 // elements in larger digits of earlier passes. Every thread of every CTA of the row gets the result. A CTA tells the others
 // its slice's totals; the one whose slice holds the digit tells them the result: two barriers over the cluster.
-template <int NC>
-__device__ __noinline__ Found find_digit(const RowShare<NC>& rs, const Slice<NC>& s, bool by_mass, unsigned int target_count,
+template <int NC, bool IN_SHARED>
+__device__ __noinline__ Found find_digit(const RowShare<NC, IN_SHARED>& rs, const Slice<NC>& s, bool by_mass, unsigned int target_count,
                                          unsigned long long target_mass, unsigned int carry_count, unsigned long long carry_mass,
                                          Shared<NC>& sh) {
     constexpr int PER = Slice<NC>::PER;
@@ -334,16 +339,16 @@ constexpr Digit FIRST_DIGIT{0u, 0u, 21, 2048};
 
 // The smallest prefix of the sorted order whose count reaches target_count
 // (by_mass false) or whose mass reaches target_mass (by_mass true). `first`: the row's slice by FIRST_DIGIT.
-template <int NC>
-__device__ __noinline__ Prefix find_prefix(const RowShare<NC>& rs, const Slice<NC>& first, bool by_mass, unsigned int target_count,
+template <int NC, bool IN_SHARED>
+__device__ __noinline__ Prefix find_prefix(const RowShare<NC, IN_SHARED>& rs, const Slice<NC>& first, bool by_mass, unsigned int target_count,
                                            unsigned long long target_mass, Shared<NC>& sh) {
     if (by_mass && target_mass == 0) target_mass = 1;      // a draw of exactly 0 takes the first element
     if (!by_mass && target_count == 0) target_count = 1;
-    Found f = find_digit<NC>(rs, first, by_mass, target_count, target_mass, 0u, 0ull, sh);
+    Found f = find_digit<NC, IN_SHARED>(rs, first, by_mass, target_count, target_mass, 0u, 0ull, sh);
     Digit dg{f.digit << 21, 2047u << 21, 10, 2048};
-    f = find_digit<NC>(rs, add_up<NC>(rs, dg, 1.0f, sh), by_mass, target_count, target_mass, f.above, f.mass, sh);
+    f = find_digit<NC, IN_SHARED>(rs, add_up<NC, IN_SHARED>(rs, dg, 1.0f, sh), by_mass, target_count, target_mass, f.above, f.mass, sh);
     dg = Digit{dg.bits | f.digit << 10, dg.mask | 2047u << 10, 0, 1024};
-    f = find_digit<NC>(rs, add_up<NC>(rs, dg, 1.0f, sh), by_mass, target_count, target_mass, f.above, f.mass, sh);
+    f = find_digit<NC, IN_SHARED>(rs, add_up<NC, IN_SHARED>(rs, dg, 1.0f, sh), by_mass, target_count, target_mass, f.above, f.mass, sh);
     const unsigned int bits = dg.bits | f.digit, n_eq = f.count;
     // `bits` is the probability at which the prefix ends; n_eq elements have exactly it
     const unsigned long long pm = mass_of(__uint_as_float(bits));
@@ -365,8 +370,8 @@ __device__ __noinline__ Prefix find_prefix(const RowShare<NC>& rs, const Slice<N
 
 // Id of the j-th (1-based) element, by ascending id, whose probability bits equal `value` (-1: there is none).
 // The CTAs of a row hold consecutive ranges of ids, so the j-th lies in the first CTA whose running count reaches j.
-template <int NC>
-__device__ int nth_equal(const RowShare<NC>& rs, unsigned int value, unsigned int j, Shared<NC>& sh) {
+template <int NC, bool IN_SHARED>
+__device__ int nth_equal(const RowShare<NC, IN_SHARED>& rs, unsigned int value, unsigned int j, Shared<NC>& sh) {
     const int per = (rs.n + THREADS - 1) / THREADS;
     const int lo = min(rs.n, (int)threadIdx.x * per), hi = min(rs.n, lo + per);
     unsigned int c = 0;
@@ -599,7 +604,7 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
     float* row = logits + (size_t)b * ld;
     const int slot = slots ? slots[b] : b;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    RowShare<NC> rs(V);
+    RowShare<NC, IN_SHARED> rs(V);
     if (slot < 0) {                          // padding row (all CTAs of the row leave)
         if (NC > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         if (threadIdx.x == 0 && rs.rank == 0) out[b] = 0;
@@ -819,12 +824,12 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
         // One pass over the probabilities (the stored exponentials times inv) finds the leading eleven bits of the k-th
         // largest, a second one, where those leave a long list, eleven more. Everything with those bits or larger ones holds the k
         // largest; when that is a short list it is gathered.
-        Found lead = find_digit<NC>(rs, add_up<NC>(rs, FIRST_DIGIT, inv, sh), false, (unsigned int)sp.top_k, 0ull, 0u, 0ull, sh);
+        Found lead = find_digit<NC, IN_SHARED>(rs, add_up<NC, IN_SHARED>(rs, FIRST_DIGIT, inv, sh), false, (unsigned int)sp.top_k, 0ull, 0u, 0ull, sh);
         unsigned int lead_bits = lead.digit;
         int lead_shift = FIRST_DIGIT.shift;
         if (lead.above + lead.count > (unsigned int)MAX_CAND) {                         // the same in every CTA of the row
             const Digit next{lead.digit << 21, 2047u << 21, 10, 2048};
-            lead = find_digit<NC>(rs, add_up<NC>(rs, next, inv, sh), false, (unsigned int)sp.top_k, 0ull, lead.above, lead.mass, sh);
+            lead = find_digit<NC, IN_SHARED>(rs, add_up<NC, IN_SHARED>(rs, next, inv, sh), false, (unsigned int)sp.top_k, 0ull, lead.above, lead.mass, sh);
             lead_bits = lead_bits << 11 | lead.digit;
             lead_shift = next.shift;
         }
@@ -835,8 +840,8 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
         if (!short_list) {
             for (int i = threadIdx.x; i < rs.n; i += THREADS) rs.p[i] *= inv;
             __syncthreads();                                // this CTA's part holds probabilities
-            topk = find_prefix<NC>(rs, add_up<NC>(rs, FIRST_DIGIT, 1.0f, sh), false, (unsigned int)sp.top_k, 0ull, sh);
-            id_bound = nth_equal<NC>(rs, topk.value, topk.ties, sh);
+            topk = find_prefix<NC, IN_SHARED>(rs, add_up<NC, IN_SHARED>(rs, FIRST_DIGIT, 1.0f, sh), false, (unsigned int)sp.top_k, 0ull, sh);
+            id_bound = nth_equal<NC, IN_SHARED>(rs, topk.value, topk.ties, sh);
             gather_scale = 1.0f;
         }
         unsigned int* cnt = rs.at(&sh.n_key, 0);
@@ -898,12 +903,12 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
         if (sp.min_p > 0.f) n = min(n, max(n_floor, 1u));
         // mass of the kept prefix, then the draw r = U * total and the walk (sampler.c:178-186); with nothing cut off it is
         // the row's mass, and a prefix that top-p ends is the one its search has found
-        const Slice<NC> first = add_up<NC>(rs, FIRST_DIGIT, 1.0f, sh);       // (both searches begin with it)
+        const Slice<NC> first = add_up<NC, IN_SHARED>(rs, FIRST_DIGIT, 1.0f, sh);       // (both searches begin with it)
         Prefix kept{0u, 0u, 0u, row_mass};
         bool found = false;
         if (sp.top_p < 1.0f) {
             const unsigned long long target = __double2ull_ru((double)sp.top_p * 1152921504606846976.0);
-            const Prefix pp = find_prefix<NC>(rs, first, true, 0u, target, sh);
+            const Prefix pp = find_prefix<NC, IN_SHARED>(rs, first, true, 0u, target, sh);
             const unsigned int np = pp.above + pp.ties;
             if (np <= n) {
                 n = np;
@@ -912,14 +917,14 @@ sample_kernel(float* __restrict__ logits, int V, int ld, const float* __restrict
             }
         }
         if (n < 1) n = 1;
-        if (!found && n < (unsigned int)V) kept = find_prefix<NC>(rs, first, false, n, 0ull, sh);
+        if (!found && n < (unsigned int)V) kept = find_prefix<NC, IN_SHARED>(rs, first, false, n, 0ull, sh);
         const double r = u * (double)kept.mass;
         unsigned long long target = __double2ull_ru(r);
         if (target > kept.mass) target = kept.mass;
-        const Prefix hit = find_prefix<NC>(rs, first, true, 0u, target, sh);
+        const Prefix hit = find_prefix<NC, IN_SHARED>(rs, first, true, 0u, target, sh);
         const unsigned int rank = hit.above + hit.ties;     // 1-based place in the sorted order
         const bool within = rank <= n;                      // (beyond only through rounding: the last kept one)
-        id = nth_equal<NC>(rs, within ? hit.value : kept.value, within ? hit.ties : kept.ties, sh);
+        id = nth_equal<NC, IN_SHARED>(rs, within ? hit.value : kept.value, within ? hit.ties : kept.ties, sh);
         if (!leading) return;
     }
     if (threadIdx.x == 0) {

@@ -62,6 +62,29 @@ def test_many_rows_draw_as_few_do(V, rows):
         assert torch.equal(many, few)
 
 
+def test_a_row_of_very_many_logits():
+    """Tens of millions of equal probabilities a digit: their summed masses exceed what counts and low bits can hold in 32 bits. Half of
+    the row is e times as likely as the other half; the walk goes through the first half by id, then through the second. A place
+    may be off by as much as the two sums' roundings make of 40 million (2^-22 of the place: 10)."""
+    from mynah_slm_b200.ops import kernels
+    half = 20_000_003
+    lg = torch.zeros((1, 2 * half), device=DEV)
+    lg[0, half:] = -1.0
+    params = torch.tensor([1.0, 1.0, 0.0, 0.0, 1.0, 0.0, 0.0, 0.0], dtype=torch.float32, device=DEV)
+    share = 1.0 / (1.0 + np.exp(-1.0))
+    sides = set()
+    for seed in range(1, 9):
+        z = (seed + 0x9E3779B97F4A7C15) & (2 ** 64 - 1)
+        z = ((z ^ (z >> 30)) * 0xBF58476D1CE4E5B9) & (2 ** 64 - 1)
+        z = ((z ^ (z >> 27)) * 0x94D049BB133111EB) & (2 ** 64 - 1)
+        u = ((z ^ (z >> 31)) >> 11) / 2.0 ** 53
+        want = u / share * half if u < share else half + (u - share) / (1.0 - share) * half
+        got = int(kernels.sample(lg.clone(), params, torch.tensor([seed], dtype=torch.int64, device=DEV), None).item())
+        assert abs(got - want) < 32, (seed, got, want)
+        sides.add(u < share)
+    assert len(sides) == 2
+
+
 @pytest.mark.parametrize("V", [500, 40002])
 @pytest.mark.parametrize("temp,top_k", [(0.0, 0), (0.9, 20), (0.9, 0)])
 def test_penalties_and_ring_inside_the_draw(V, temp, top_k):
